@@ -601,7 +601,8 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     uint64_t capX = fullP, capY = fullP, capZ = fullQ;
     if (c->prm.sized_tables) {
         CU(cudaMemsetAsync(regs, 0, 3 * kSketchRegs * 4, st));
-        k_sketch<<<grid_for(jp.nP > jp.nQ ? jp.nP : jp.nQ, sm, 2), 256, 0, st>>>(jp.P, jp.nP, jp.Q, jp.nQ, regs);
+        k_sketch<<<grid_for(jp.nP > jp.nQ ? jp.nP : jp.nQ, sm, 4, kSketchThreads), kSketchThreads, 0, st>>>(
+            jp.P, jp.nP, jp.Q, jp.nQ, regs);
         CHECK_LAUNCH();
         std::vector<uint32_t> hr(3 * kSketchRegs);
         CU(cudaMemcpyAsync(hr.data(), regs, 3 * kSketchRegs * 4, cudaMemcpyDeviceToHost, st));
@@ -751,8 +752,9 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     const uint32_t cap_b = 1u << (c->prm.block_lg - 1);
     // tiny rows get their own warp launch in the single pass only
     const bool tiny = jp.single_pass && !jp.aggregate && !jp.count_only;
-    k_row_work<<<grid_for((uint64_t)n * 32, sm), 256, 0, st>>>(rc, n, cap_w, cap_b, jp.aggregate, tiny, jp.sum, ucap, cls,
-                                                                &sc->outj, sc->outj_cls);
+    const uint32_t lanes = row_work_lanes((double)jp.nP / n);
+    k_row_work<<<grid_for((uint64_t)n << lanes, sm), 256, 0, st>>>(rc, n, lanes, cap_w, cap_b, jp.aggregate, tiny, jp.sum,
+                                                                    ucap, cls, &sc->outj, sc->outj_cls);
     CHECK_LAUNCH();
     uint32_t* list_w = lists;
     uint32_t* list_b = lists + n;

@@ -740,49 +740,76 @@ static __global__ void __launch_bounds__(1024) k_rows_bitmap(RowCtx c, const uin
 }
 
 // Per-row candidate count w = sum over y in R_x of |S_y|, u = min(w, m) and
-// the row class (0: empty, or outside sel's A-tiles).  One warp per row.  With check_range set
+// the row class (0: empty, or outside sel's A-tiles).  With check_range set
 // (join-aggregate, 32-bit per-group counters) a row of 2^32 or more
 // candidates raises kErrCountRange.
-static __global__ void k_row_work(RowCtx c, uint32_t n, uint32_t cap_w, uint32_t cap_b, bool check_range, bool tiny, SumAcc sel,
-                           uint32_t* __restrict__ ucap, uint8_t* __restrict__ cls, unsigned long long* outj,
-                           unsigned long long* outj_cls) {
-    const uint32_t lane = lane_id();
+//
+// A row's entries are a chain of dependent loads (row bounds, y id, S bounds),
+// so the rows in flight bound the time: 2^lg lanes take a row, about as many
+// as a row has entries on average (row_work_lanes), and a row of more than
+// 4 x 2^lg entries is finished by its whole warp.  A warp for every row took
+// 281 us for 1M rows of 10 entries.  The sums are added up per CTA in shared
+// memory, then one atomic a CTA and counter.
+static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, uint32_t lg, uint32_t cap_w,
+                                                         uint32_t cap_b, bool check_range, bool tiny, SumAcc sel,
+                                                         uint32_t* __restrict__ ucap, uint8_t* __restrict__ cls,
+                                                         unsigned long long* outj, unsigned long long* outj_cls) {
+    __shared__ unsigned long long s_acc[6];
+    if (threadIdx.x < 6) s_acc[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t lane = lane_id(), G = 1u << lg, gl = lane & (G - 1), per = 32 >> lg;
     const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    unsigned long long acc = 0, acc_cls[6] = {0, 0, 0, 0, 0, 0};
-    for (uint64_t x = gw; x < n; x += nwarps) {
-        if (sel.tiles && !sel.selected(c.id2x[x])) {  // summaries over a slice of A-tiles
-            if (lane == 0) {
-                ucap[x] = 0;
-                cls[x] = 0;
-            }
-            continue;
+    for (uint64_t x0 = gw * per; x0 < n; x0 += nwarps * per) {
+        const uint64_t x = x0 + (lane >> lg);
+        uint32_t e0 = 0, e1 = 0;
+        const bool live = x < n && !(sel.tiles && !sel.selected(c.id2x[x]));  // summaries over a slice of A-tiles
+        if (live) {
+            e0 = c.JR_R[x];
+            e1 = c.JR_R[x + 1];
         }
-        uint32_t e0 = c.JR_R[x], e1 = c.JR_R[x + 1];
         unsigned long long w = 0;
-        for (uint32_t e = e0 + lane; e < e1; e += 32) {
-            uint64_t r = (uint64_t)c.IC_R[e] * c.T;
-            w += c.JR_S[r + c.T] - c.JR_S[r];
+        const uint32_t head = min(e1, e0 + 4 * G);
+        uint32_t y[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) y[k] = e0 + gl + k * G < head ? __ldg(&c.IC_R[e0 + gl + k * G]) : kEmpty32;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++)
+            if (y[k] != kEmpty32) {
+                const uint64_t r = (uint64_t)y[k] * c.T;
+                w += __ldg(&c.JR_S[r + c.T]) - __ldg(&c.JR_S[r]);
+            }
+        // the rest of the warp's long rows, all lanes on one row at a time
+        for (uint32_t longs = __ballot_sync(0xffffffffu, gl == 0 && head < e1); longs; longs &= longs - 1) {
+            const int src = __ffs(longs) - 1;
+            const uint32_t b = __shfl_sync(0xffffffffu, head, src), e = __shfl_sync(0xffffffffu, e1, src);
+            unsigned long long v = 0;
+#pragma unroll 4
+            for (uint32_t k = b + lane; k < e; k += 32) {
+                const uint64_t r = (uint64_t)__ldg(&c.IC_R[k]) * c.T;
+                v += __ldg(&c.JR_S[r + c.T]) - __ldg(&c.JR_S[r]);
+            }
+            v = warp_sum(v);
+            if ((int)lane == src) w += v;
         }
-        w = warp_sum(w);
-        if (lane == 0) {
-            uint32_t u = (uint32_t)(w < c.m ? w : c.m);
-            ucap[x] = u;
+        for (uint32_t o = G >> 1; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+        if (gl == 0 && x < n) {
+            const uint32_t u = (uint32_t)(w < c.m ? w : c.m);
             const uint32_t k = row_class(w, u, cap_w, cap_b, tiny);
+            ucap[x] = u;
             cls[x] = (uint8_t)k;
             if (check_range && w >= 0xFFFFFFFFull) raise_error(c.err, kErrCountRange);
-            acc += w;
-#pragma unroll
-            for (uint32_t j = 1; j < 6; j++) acc_cls[j] += (j == k) ? w : 0ull;
+            if (w) {
+                atomicAdd(&s_acc[0], w);
+                atomicAdd(&s_acc[k], w);
+            }
         }
     }
-    if (lane == 0 && acc) {
-        atomicAdd(outj, acc);
-#pragma unroll
-        for (uint32_t j = 1; j < 6; j++)
-            if (acc_cls[j]) atomicAdd(&outj_cls[j], acc_cls[j]);
-    }
+    __syncthreads();
+    if (threadIdx.x < 6 && s_acc[threadIdx.x]) atomicAdd(threadIdx.x ? &outj_cls[threadIdx.x] : outj, s_acc[threadIdx.x]);
 }
+// Lanes a row (log2) for rows of `per_row` entries on average.
+inline uint32_t row_work_lanes(double per_row) { return per_row > 64 ? 5 : (per_row > 24 ? 4 : (per_row > 8 ? 3 : 2)); }
 
 struct ClassSrc {
     const uint8_t* cls;

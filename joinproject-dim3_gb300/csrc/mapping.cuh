@@ -52,6 +52,9 @@ __device__ __forceinline__ uint32_t table_find(DevTable t, uint32_t key) {
     return kNotFound;
 }
 
+// Tuples a thread of the sketch pass holds in flight.
+constexpr uint32_t kMapIlp = 4;
+
 // Table sizing.  A table built for a relation's tuple count (load factor
 // 1/2 if every key were distinct) is far larger than its distinct keys when
 // keys repeat -- 2^26 slots, 512 MB, for the 2M vertices of a 20M-edge graph
@@ -104,23 +107,44 @@ inline uint64_t sketch_capacity(double est, uint64_t full, uint32_t slack_pct) {
 }
 
 // Registers of P's first and y columns and Q's first column, kSketchRegs
-// each, merged into regs (zeroed by the caller).
-static __global__ void __launch_bounds__(256) k_sketch(const uint2* __restrict__ P, uint64_t nP,
-                                                       const uint2* __restrict__ Q, uint64_t nQ, uint32_t* regs) {
+// each, merged into regs (zeroed by the caller).  Bound by the latency of the
+// tuple loads, so kMapIlp of them are in flight a thread, at
+// kSketchThreads x 4 threads an SM; a CTA's registers are merged with an
+// atomic only where they raise the total (few do once the first CTAs have
+// merged).  2 x 10M tuples: 151 us at 256 x 2 threads an SM and one load in
+// flight.
+constexpr int kSketchThreads = 512;
+static __global__ void __launch_bounds__(kSketchThreads) k_sketch(const uint2* __restrict__ P, uint64_t nP,
+                                                                  const uint2* __restrict__ Q, uint64_t nQ,
+                                                                  uint32_t* regs) {
     __shared__ uint32_t r[3 * kSketchRegs];
     for (uint32_t k = threadIdx.x; k < 3 * kSketchRegs; k += blockDim.x) r[k] = 0;
     __syncthreads();
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nP; i += stride) {
-        const uint2 p = P[i];
-        sketch_add_if_larger(r, p.x);
-        sketch_add_if_larger(r + kSketchRegs, p.y);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint64_t i = first; i < nP; i += kMapIlp * stride) {
+        uint2 p[kMapIlp];
+#pragma unroll
+        for (uint32_t k = 0; k < kMapIlp; k++)
+            if (i + k * stride < nP) p[k] = __ldg(&P[i + k * stride]);
+#pragma unroll
+        for (uint32_t k = 0; k < kMapIlp; k++)
+            if (i + k * stride < nP) {
+                sketch_add_if_larger(r, p[k].x);
+                sketch_add_if_larger(r + kSketchRegs, p[k].y);
+            }
     }
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nQ; i += stride)
-        sketch_add_if_larger(r + 2 * kSketchRegs, Q[i].x);
+    for (uint64_t i = first; i < nQ; i += kMapIlp * stride) {
+        uint32_t q[kMapIlp];
+#pragma unroll
+        for (uint32_t k = 0; k < kMapIlp; k++)
+            if (i + k * stride < nQ) q[k] = __ldg(&Q[i + k * stride].x);
+#pragma unroll
+        for (uint32_t k = 0; k < kMapIlp; k++)
+            if (i + k * stride < nQ) sketch_add_if_larger(r + 2 * kSketchRegs, q[k]);
+    }
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < 3 * kSketchRegs; k += blockDim.x)
-        if (r[k]) atomicMax(&regs[k], r[k]);
+        if (r[k] > __ldcg(&regs[k])) atomicMax(&regs[k], r[k]);
 }
 
 // Build pass over the larger relation P: insert its first column into tx and
@@ -135,27 +159,58 @@ static __global__ void k_insert_p(const uint2* __restrict__ P, uint64_t n, DevTa
 
 // Semi-join of Q against ty (mapping_y's probe, dim3.hpp:816-827): keep the
 // tuples whose y occurs in P as (c, y id), insert their first column into tz.
-static __global__ void k_probe_q(const uint2* __restrict__ Q, uint64_t n, DevTable ty, DevTable tz, uint2* __restrict__ Qk,
-                          unsigned long long* nkept, uint32_t* err) {
-    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t i = i0 + threadIdx.x;
-        bool keep = false;
-        uint2 q = make_uint2(0, 0);
-        uint32_t yid = kNotFound;
-        if (i < n) {
-            q = Q[i];
-            yid = table_find(ty, q.y);
-            keep = (yid != kNotFound);
-            if (keep) table_insert(tz, q.x, err);
+// The kept tuples of a CTA's kProbeItems x 256 tuples take one range of Qk:
+// one atomic on the shared counter per 1024 tuples.  (One per warp and 32
+// tuples serialised on its address: 431 us for 10M tuples, 893 us for 20M.)
+constexpr uint32_t kProbeItems = 4;
+static __global__ void __launch_bounds__(256) k_probe_q(const uint2* __restrict__ Q, uint64_t n, DevTable ty,
+                                                        DevTable tz, uint2* __restrict__ Qk, unsigned long long* nkept,
+                                                        uint32_t* err) {
+    __shared__ uint32_t s_cnt[8];
+    __shared__ unsigned long long s_base;
+    const uint32_t wib = threadIdx.x >> 5, lt = lanemask_lt();
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < n; i0 += kProbeItems * stride) {
+        uint2 q[kProbeItems];
+        uint32_t yid[kProbeItems], b[kProbeItems], cnt = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kProbeItems; k++) {
+            const uint64_t i = i0 + k * stride + threadIdx.x;
+            if (i < n) q[k] = __ldg(&Q[i]);
         }
-        uint32_t b = __ballot_sync(0xffffffffu, keep);
-        if (b) {
-            unsigned long long base = 0;
-            int leader = __ffs(b) - 1;
-            if ((int)lane_id() == leader) base = atomicAdd(nkept, (unsigned long long)__popc(b));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (keep) Qk[base + __popc(b & lanemask_lt())] = make_uint2(q.x, yid);
+#pragma unroll
+        for (uint32_t k = 0; k < kProbeItems; k++) {
+            yid[k] = kNotFound;
+            if (i0 + k * stride + threadIdx.x < n) {
+                yid[k] = table_find(ty, q[k].y);
+                if (yid[k] != kNotFound) table_insert(tz, q[k].x, err);
+            }
         }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t k = 0; k < kProbeItems; k++) {
+            b[k] = __ballot_sync(0xffffffffu, yid[k] != kNotFound);
+            cnt += __popc(b[k]);
+        }
+        if (lane_id() == 0) s_cnt[wib] = cnt;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t t = 0;
+            for (uint32_t w = 0; w < 8; w++) {
+                const uint32_t c = s_cnt[w];
+                s_cnt[w] = t;
+                t += c;
+            }
+            s_base = t ? atomicAdd(nkept, (unsigned long long)t) : 0ull;
+        }
+        __syncthreads();
+        unsigned long long pos = s_base + s_cnt[wib];
+#pragma unroll
+        for (uint32_t k = 0; k < kProbeItems; k++) {
+            if (yid[k] != kNotFound) Qk[pos + __popc(b[k] & lt)] = make_uint2(q[k].x, yid[k]);
+            pos += __popc(b[k]);
+        }
+        __syncthreads();  // s_cnt and s_base are rewritten by the next round
     }
 }
 
