@@ -140,8 +140,8 @@ struct dim3g_relset {
     char* mem = nullptr;
     size_t mem_bytes = 0;
     RelPools P{};
-    uint64_t* bsum = nullptr;
-    uint64_t bsum_n = 0;
+    unsigned long long* scan_state = nullptr;  // of the build's four scans
+    uint64_t scan_words[4] = {};
     QueryScratch qs;  // scratch of dim3g_relset_join (grow-only)
     unsigned long long* h_need = nullptr;  // pinned: yt keys needed, err
     uint64_t launches_build = 0;
@@ -190,11 +190,10 @@ int relset_plan(dim3g_relset* s, const dim3g_relation* rels, uint32_t n, uint64_
                  o_ICy = L.add<uint32_t>(s->ntot), o_VSy = L.add<uint32_t>(s->ntot), o_err = L.add<uint32_t>(4),
                  o_need = L.add<unsigned long long>(2), o_yoff = L.add<uint64_t>(n + 1),
                  o_roles = L.add<uint8_t>(n), o_fneed = L.add<unsigned long long>(1);
-    uint64_t sn = scan_storage(s->tabtot);
-    const uint64_t s2 = scan_storage(s->ntot + 1), s3 = scan_storage(s->yt_cap);
-    if (s2 > sn) sn = s2;
-    if (s3 > sn) sn = s3;
-    const size_t o_bsum = L.add<uint64_t>(sn);
+    s->scan_words[0] = s->scan_words[1] = scan_storage(s->tabtot);
+    s->scan_words[2] = scan_storage(s->ntot + 1);
+    s->scan_words[3] = scan_storage(s->yt_cap);
+    const size_t o_scan = L.add<unsigned long long>(s->scan_words[0] + s->scan_words[1] + s->scan_words[2] + s->scan_words[3]);
     if (s->mem && s->mem_bytes < L.total) {
         cudaFree(s->mem);
         s->mem = nullptr;
@@ -239,8 +238,7 @@ int relset_plan(dim3g_relset* s, const dim3g_relation* rels, uint32_t n, uint64_
     P.yoff = (uint64_t*)(m + o_yoff);
     P.roles = (const uint8_t*)(m + o_roles);
     P.f_need = (unsigned long long*)(m + o_fneed);
-    s->bsum = (uint64_t*)(m + o_bsum);
-    s->bsum_n = sn;
+    s->scan_state = (unsigned long long*)(m + o_scan);
     BCU(cudaMemcpy((void*)P.in, s->h_in.data(), n * sizeof(RelIn), cudaMemcpyHostToDevice));
     BCU(cudaMemcpy((void*)P.tup_off, s->h_tup_off.data(), (n + 1) * 8, cudaMemcpyHostToDevice));
     BCU(cudaMemcpy((void*)P.tab_off, s->h_tab_off.data(), (n + 1) * 8, cudaMemcpyHostToDevice));
@@ -342,30 +340,30 @@ int relset_enqueue_build(dim3g_relset* s, cudaStream_t st, uint64_t& launches) {
     BCU(cudaMemsetAsync(P.degF, 0, (s->ntot + 1) * 4, st));
     BCU(cudaMemsetAsync(P.cnt_yt, 0, s->yt_cap * 4, st));
     BCU(cudaMemsetAsync(P.err, 0, 16, st));
+    BCU(cudaMemsetAsync(s->scan_state, 0, (s->scan_words[0] + s->scan_words[1] + s->scan_words[2] + s->scan_words[3]) * 8,
+                        st));
     if (s->ntot) {
         k_ix_insert<<<elem_grid(s->ntot, sm), 256, 0, st>>>(P);
         BLAUNCH();
     }
     k_ix_layout<<<1, 1024, 0, st>>>(P, s->tile_lg);
     BLAUNCH();
-    device_scan(OccupiedSrc{P.TF}, AssignIdDst{P.TF, P.id2f}, s->tabtot, s->bsum, nullptr, st);
-    launches += scan_launches(s->tabtot);
-    device_scan(OccupiedSrc{P.TY}, AssignIdDst{P.TY, P.id2y}, s->tabtot, s->bsum, nullptr, st);
-    launches += scan_launches(s->tabtot);
-    BCU(cudaGetLastError());
+    using IdJob = ScanJob<OccupiedSrc, AssignIdDst>;
+    using PtrJob = ScanJob<BoundSrc<U32Src>, BoundDst<RowPtrDst>>;
+    unsigned long long* w[4] = {s->scan_state, w[0] + s->scan_words[0], w[1] + s->scan_words[1], w[2] + s->scan_words[2]};
+    device_scan2(IdJob{OccupiedSrc{P.TF}, AssignIdDst{P.TF, P.id2f}, s->tabtot, w[0], nullptr},
+                 IdJob{OccupiedSrc{P.TY}, AssignIdDst{P.TY, P.id2y}, s->tabtot, w[1], nullptr}, P.err, st);
+    BLAUNCH();
     if (s->ntot) {
         k_ix_map<<<elem_grid(s->ntot, sm), 256, 0, st>>>(P);
         BLAUNCH();
     }
     // row pointers up to the id / key counts the layout found (the launch
     // covers the tuple-count bounds; past the counts nothing is read or written)
-    device_scan(BoundSrc<U32Src>{U32Src{P.degF}, P.f_need}, BoundDst<RowPtrDst>{RowPtrDst{P.JRf, P.curF}, P.f_need},
-                s->ntot + 1, s->bsum, nullptr, st);
-    launches += scan_launches(s->ntot + 1);
-    device_scan(BoundSrc<U32Src>{U32Src{P.cnt_yt}, P.yt_need}, BoundDst<RowPtrDst>{RowPtrDst{P.JRy, P.curY}, P.yt_need},
-                s->yt_cap, s->bsum, nullptr, st);
-    launches += scan_launches(s->yt_cap);
-    BCU(cudaGetLastError());
+    device_scan2(PtrJob{{U32Src{P.degF}, P.f_need}, {RowPtrDst{P.JRf, P.curF}, P.f_need}, s->ntot + 1, w[2], nullptr},
+                 PtrJob{{U32Src{P.cnt_yt}, P.yt_need}, {RowPtrDst{P.JRy, P.curY}, P.yt_need}, s->yt_cap, w[3], nullptr},
+                 P.err, st);
+    BLAUNCH();
     if (s->ntot) {
         k_ix_scatter<<<elem_grid(s->ntot, sm), 256, 0, st>>>(P);
         BLAUNCH();
@@ -387,7 +385,6 @@ struct QueryPlan {
     uint32_t* lists = nullptr;             // 3 x nrows
     unsigned long long* ncls = nullptr;    // rows per class 0..8
     uint32_t* next_row = nullptr;          // 8 dynamic counters (4..6: split block launches)
-    uint64_t* bsum = nullptr;
     uint32_t* part = nullptr;              // class-list partition: per-tile bucket offsets
     unsigned long long* pbase = nullptr;   // its bucket starts (8)
 };
@@ -395,7 +392,7 @@ struct QueryPlan {
 // Device layout of a query pass's scratch (every size monotone in the
 // arguments, so scratch laid out for maxima fits every smaller pass).
 struct QLayout {
-    size_t qin, qt, qr, ymap, ICq, JRq, ucap, cls, wrow, rc, rs, res, lists, ncls, next, bsum, part, pbase, total;
+    size_t qin, qt, qr, ymap, ICq, JRq, ucap, cls, wrow, rc, rs, res, lists, ncls, next, part, pbase, total;
 };
 QLayout query_layout(uint32_t nq, uint64_t ntot, uint64_t nrows) {
     Layout L;
@@ -415,7 +412,6 @@ QLayout query_layout(uint32_t nq, uint64_t ntot, uint64_t nrows) {
     o.lists = L.add<uint32_t>(4 * nrows);
     o.ncls = L.add<unsigned long long>(24);  // [16..18]: block-class rows by hash-set size
     o.next = L.add<uint32_t>(8);
-    o.bsum = L.add<uint64_t>(scan_storage(nrows));
     o.part = L.add<uint32_t>(8 * ((nrows + kPartTile - 1) / kPartTile));
     o.pbase = L.add<unsigned long long>(8);
     o.total = L.total;
@@ -517,7 +513,6 @@ int query_plan(dim3g_relset* s, QueryScratch& qs, const dim3g_query* q, uint32_t
     qp.lists = (uint32_t*)(m + o.lists);
     qp.ncls = (unsigned long long*)(m + o.ncls);
     qp.next_row = (uint32_t*)(m + o.next);
-    qp.bsum = (uint64_t*)(m + o.bsum);
     qp.part = (uint32_t*)(m + o.part);
     qp.pbase = (unsigned long long*)(m + o.pbase);
     return DIM3G_OK;

@@ -17,6 +17,7 @@ enum DeviceError : uint32_t {
     kErrCountRange = 8u,    // a per-group count could exceed 32 bits
     kErrDenseTimeout = 16u, // a wait of the dense product ran out of time
     kErrStreamTimeout = 32u,  // a wait of the streamed bitmap rows ran out of time
+    kErrScanTimeout = 64u,  // a tile of a prefix sum waited too long for the tiles before it
 };
 
 __device__ __forceinline__ void raise_error(uint32_t* err, uint32_t bit) { atomicOr(err, bit); }

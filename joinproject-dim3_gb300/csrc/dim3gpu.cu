@@ -116,6 +116,7 @@ struct Scalars {
     unsigned long long dense_base;   // single-pass start of the dense block's pairs (~0: past the capacity)
     unsigned int err;
     unsigned long long nrows_b[3];  // block-class rows by hash-set size (single pass, block_split)
+    unsigned long long nbucket[kRowBuckets], list_cur[kRowBuckets];  // rows per bucket, list cursors (k_row_lists)
     unsigned int next_row[8];      // dynamic row counters of the CTA classes (4..6: block_split launches)
     unsigned int pad;
 };
@@ -140,8 +141,6 @@ struct dim3g_ctx {
     void* d_sum = nullptr;  // per-A-tile summary accumulators
     size_t d_sum_bytes = 0;
     Scalars* h_sc = nullptr;  // pinned
-    cudaStream_t aux = nullptr;  // side stream: R's CSR build alongside S's (fork/join by events)
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaEvent_t ev[6] = {};
     cudaEvent_t evc[8] = {};  // per row-class kernel timing
     cudaEvent_t evd[4] = {};  // dense block: selection, operands, product, light pass
@@ -180,13 +179,15 @@ int fail(dim3g_ctx* c, int code, const char* fmt, ...) {
         c->launches++;         \
     } while (0)
 
-// device_scan plus launch accounting (three kernels when n > 0).
+// One scan with its own zeroing, with launch accounting.  state:
+// scan_storage(n) words.
 template <class Src, class Dst>
-int run_scan(dim3g_ctx* c, Src src, Dst dst, uint64_t n, uint64_t* bsum, unsigned long long* total,
-             cudaStream_t on = nullptr) {
-    device_scan(src, dst, n, bsum, total, on ? on : c->stream);
+int run_scan(dim3g_ctx* c, Src src, Dst dst, uint64_t n, unsigned long long* state, unsigned long long* total,
+             uint32_t* err) {
+    CU(cudaMemsetAsync(state, 0, scan_storage(n) * 8, c->stream));
+    device_scan(ScanJob<Src, Dst>{src, dst, n, state, total}, err, c->stream);
     CU(cudaGetLastError());
-    c->launches += scan_launches(n);
+    c->launches += n != 0;
     return DIM3G_OK;
 }
 #define SCAN(...)                                \
@@ -194,7 +195,6 @@ int run_scan(dim3g_ctx* c, Src src, Dst dst, uint64_t n, uint64_t* bsum, unsigne
         int r_ = run_scan(c, __VA_ARGS__);       \
         if (r_) return r_;                       \
     } while (0)
-
 
 unsigned grid_for(uint64_t n, int sm, int per_sm = 8, int block = 256) {
     uint64_t b = (n + block - 1) / block;
@@ -284,6 +284,7 @@ constexpr uint64_t kDenseMinCand = (uint64_t)1 << 26;  // smaller heavy work sta
 
 struct DensePlan {
     bool on = false;
+    bool counted = false; // the rows per class are in the host's scalars
     uint32_t nd = 0;      // rows of the block: list_m[0 .. nd) (the bitmap classes' rows, huge ones first)
     uint32_t Wd = 0;      // bitmap words per row (allocated)
     uint32_t Wm = 0;      // bitmap words per row holding z < m
@@ -349,6 +350,7 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
     CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
     if (c->h_sc->err) return fail(c, DIM3G_ERR_DEVICE, "device bound violated in row binning (flags %u)", c->h_sc->err);
+    dp->counted = true;
     const uint64_t n_heavy = c->h_sc->nrows[3] + c->h_sc->nrows[4];
     const uint64_t cd_all = c->h_sc->outj_cls[3] + c->h_sc->outj_cls[4];
     skip = 2;  // no heavy rows, or too little heavy work
@@ -471,7 +473,7 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
         uint32_t* tcnt = ws_get<uint32_t>(c, ntile + 1);
         uint32_t* toff = ws_get<uint32_t>(c, ntile + 1);
         uint32_t* tcur = ws_get<uint32_t>(c, ntile + 1);
-        uint64_t* bsum = ws_get<uint64_t>(c, scan_storage(ntile + 1));
+        unsigned long long* bsum = ws_get<unsigned long long>(c, scan_storage(ntile + 1));
         if (!A32 || !B32 || !tcnt || !toff || !tcur || !bsum)
             return fail(c, DIM3G_ERR_NOMEM, "workspace allocation failed (dense counts)");
         unsigned int* flag = bin_n + kDenseBins + 1;
@@ -492,7 +494,7 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
         CHECK_LAUNCH();
         k_dense_maxcnt<<<grid_for(ntile, sm), 256, 0, st>>>(tcnt, ntile, flag + 1);
         CHECK_LAUNCH();
-        SCAN(U32Src{tcnt}, RowPtrDst{toff, tcur}, ntile + 1, bsum, ltotal);
+        SCAN(U32Src{tcnt}, RowPtrDst{toff, tcur}, ntile + 1, bsum, ltotal, &sc->err);
         unsigned int hflag[2] = {0, 0};
         unsigned long long hl = 0;
         CU(cudaMemcpyAsync(hflag, flag, 8, cudaMemcpyDeviceToHost, st));
@@ -538,11 +540,11 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
         const uint64_t nc = nd * cpr;
         uint32_t* cc = ws_get<uint32_t>(c, nc + 1);
         coff = ws_get<unsigned long long>(c, nc + 1);
-        uint64_t* bsum = ws_get<uint64_t>(c, scan_storage(nc + 1));
+        unsigned long long* bsum = ws_get<unsigned long long>(c, scan_storage(nc + 1));
         if (!cc || !coff || !bsum) return fail(c, DIM3G_ERR_NOMEM, "workspace allocation failed (dense chunks)");
         k_dense_chunks<<<grid_for(nc * 8, sm), 256, 0, st>>>((uint32_t)nd, D, (uint32_t)Wd, cpr, cc);
         CHECK_LAUNCH();
-        SCAN(U32Src{cc}, OffDst{coff}, nc + 1, bsum, nullptr);
+        SCAN(U32Src{cc}, OffDst{coff}, nc + 1, bsum, nullptr, &sc->err);
     }
     CU(cudaEventRecord(c->evd[3], st));
     {
@@ -556,6 +558,8 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
     c->stats.heavy_y = (uint32_t)best_k;
     c->stats.dense_kp = Kp;
     c->stats.dense_light = (uint64_t)best_light;
+    c->h_sc->nrows[3] = n_heavy - nd;
+    c->h_sc->nrows[4] = 0;
     dp->on = true;
     dp->nd = (uint32_t)nd;
     dp->Wd = (uint32_t)Wd;
@@ -587,20 +591,27 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     const int sm = c->sm_count;
     CU(cudaEventRecord(c->ev[0], st));
 
-    Scalars* sc = ws_get<Scalars>(c, 1);
     const uint64_t fullP = next_pow2(jp.nP * 2 < 1024 ? 1024 : jp.nP * 2);
     const uint64_t fullQ = next_pow2(jp.nQ * 2 < 1024 ? 1024 : jp.nQ * 2);
+    // what starts at zero, in one block: scalars, sketch registers, the
+    // states of the three id scans (room for tuple-sized tables)
+    const uint64_t sP = scan_storage(fullP), sQ = scan_storage(fullQ);
+    const size_t sc_bytes = round_up(sizeof(Scalars), 256), regs_bytes = 3 * kSketchRegs * 4;
+    const size_t zero_bytes = sc_bytes + regs_bytes + (2 * sP + sQ) * 8;
+    char* zero = ws_get<char>(c, zero_bytes);
     uint2* Qk = ws_get<uint2>(c, jp.nQ);
     uint2* Pm = ws_get<uint2>(c, jp.nP);
     uint32_t* id2x = ws_get<uint32_t>(c, jp.nP);
     uint32_t* id2z = ws_get<uint32_t>(c, round_up(jp.nQ, 1024) + 1024);  // whole 1024-id chunks (dense emission)
-    uint32_t* regs = ws_get<uint32_t>(c, 3 * kSketchRegs);
-    if (!sc || !Qk || !Pm || !id2x || !id2z || !regs) return fail(c, DIM3G_ERR_NOMEM, "workspace allocation failed (mapping)");
+    if (!zero || !Qk || !Pm || !id2x || !id2z) return fail(c, DIM3G_ERR_NOMEM, "workspace allocation failed (mapping)");
+    Scalars* sc = (Scalars*)zero;
+    uint32_t* regs = (uint32_t*)(zero + sc_bytes);
+    unsigned long long* states = (unsigned long long*)(zero + sc_bytes + regs_bytes);
+    CU(cudaMemsetAsync(zero, 0, zero_bytes, st));
 
     // table capacities from the distinct-key sketch (see mapping.cuh)
     uint64_t capX = fullP, capY = fullP, capZ = fullQ;
     if (c->prm.sized_tables) {
-        CU(cudaMemsetAsync(regs, 0, 3 * kSketchRegs * 4, st));
         k_sketch<<<grid_for(jp.nP > jp.nQ ? jp.nP : jp.nQ, sm, 4, kSketchThreads), kSketchThreads, 0, st>>>(
             jp.P, jp.nP, jp.Q, jp.nQ, regs);
         CHECK_LAUNCH();
@@ -624,24 +635,25 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     for (int attempt = 0;; attempt++) {
         const bool sized = capX < fullP || capY < fullP || capZ < fullQ;
         const uint64_t lim = sized ? kSizedProbeLimit : 0;
-        tx = DevTable{ws_get<unsigned long long>(c, capX), capX - 1, lim};
-        ty = DevTable{ws_get<unsigned long long>(c, capY), capY - 1, lim};
-        tz = DevTable{ws_get<unsigned long long>(c, capZ), capZ - 1, lim};
-        const uint64_t capM = capX > capY ? (capX > capZ ? capX : capZ) : (capY > capZ ? capY : capZ);
-        uint64_t* bsum = ws_get<uint64_t>(c, scan_storage(capM));
-        if (!tx.slots || !ty.slots || !tz.slots || !bsum) return fail(c, DIM3G_ERR_NOMEM, "workspace allocation failed (mapping)");
-        CU(cudaMemsetAsync(sc, 0, sizeof(Scalars), st));
-        CU(cudaMemsetAsync(tx.slots, 0xff, capX * 8, st));
-        CU(cudaMemsetAsync(ty.slots, 0xff, capY * 8, st));
-        CU(cudaMemsetAsync(tz.slots, 0xff, capZ * 8, st));
+        unsigned long long* slots = ws_get<unsigned long long>(c, capX + capY + capZ);
+        if (!slots) return fail(c, DIM3G_ERR_NOMEM, "workspace allocation failed (mapping)");
+        tx = DevTable{slots, capX - 1, lim};
+        ty = DevTable{slots + capX, capY - 1, lim};
+        tz = DevTable{slots + capX + capY, capZ - 1, lim};
+        CU(cudaMemsetAsync(slots, 0xff, (capX + capY + capZ) * 8, st));
+        if (attempt) CU(cudaMemsetAsync(zero, 0, zero_bytes, st));
 
+        using IdJob = ScanJob<OccupiedSrc, AssignIdDst>;
         k_insert_p<<<grid_for(jp.nP, sm), 256, 0, st>>>(jp.P, jp.nP, tx, ty, &sc->err);
         CHECK_LAUNCH();
-        SCAN(OccupiedSrc{ty.slots}, AssignIdDst{ty.slots, nullptr}, capY, bsum, &sc->ny);
-        SCAN(OccupiedSrc{tx.slots}, AssignIdDst{tx.slots, id2x}, capX, bsum, &sc->nx);
+        device_scan2(IdJob{OccupiedSrc{ty.slots}, AssignIdDst{ty.slots, nullptr}, capY, states, &sc->ny},
+                     IdJob{OccupiedSrc{tx.slots}, AssignIdDst{tx.slots, id2x}, capX, states + sP, &sc->nx}, &sc->err, st);
+        CHECK_LAUNCH();
         k_probe_q<<<grid_for(jp.nQ, sm), 256, 0, st>>>(jp.Q, jp.nQ, ty, tz, Qk, &sc->nkept, &sc->err);
         CHECK_LAUNCH();
-        SCAN(OccupiedSrc{tz.slots}, AssignIdDst{tz.slots, id2z}, capZ, bsum, &sc->nz);
+        device_scan(IdJob{OccupiedSrc{tz.slots}, AssignIdDst{tz.slots, id2z}, capZ, states + 2 * sP, &sc->nz}, &sc->err,
+                    st);
+        CHECK_LAUNCH();
         CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
         if (sized && attempt == 0 && c->h_sc->err == kErrProbeLimit) {
@@ -682,13 +694,15 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     S.z_tiles = T;
     const uint64_t nyt = (uint64_t)k * T;
 
-    uint32_t* degx = ws_get<uint32_t>(c, (uint64_t)n + 1);
-    uint32_t* curx = ws_get<uint32_t>(c, (uint64_t)n + 1);
-    uint32_t* JR_R = ws_get<uint32_t>(c, (uint64_t)n + 1);
+    // zeroed: both histograms, the rows' distinct counts, the scans' states
+    const uint64_t n1 = (uint64_t)n + 1, k1 = nyt + 1, sR = scan_storage(n1), sS = scan_storage(k1);
+    const uint64_t zero2 = round_up(2 * n1 + k1, 2) * 4 + (sR + sS) * 8;
+    uint32_t* degx = (uint32_t*)ws_get<char>(c, zero2);
+    uint32_t* curx = ws_get<uint32_t>(c, n1);
+    uint32_t* JR_R = ws_get<uint32_t>(c, n1);
     uint32_t* IC_R = ws_get<uint32_t>(c, jp.nP);
-    uint32_t* cnt_yt = ws_get<uint32_t>(c, nyt + 1);
-    uint32_t* cur_yt = ws_get<uint32_t>(c, nyt + 1);
-    uint32_t* JR_S = ws_get<uint32_t>(c, nyt + 1);
+    uint32_t* cur_yt = ws_get<uint32_t>(c, k1);
+    uint32_t* JR_S = ws_get<uint32_t>(c, k1);
     uint32_t* IC_S = ws_get<uint32_t>(c, nq);
     uint32_t* VS = nullptr;  // the value paths read the pairs in ISV
     // +2: the streamed bitmap rows copy 16-byte-aligned supersets of S
@@ -696,39 +710,30 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     uint2* ISV = ws_get<uint2>(c, nq + 2);
     uint32_t* Zq = ws_get<uint32_t>(c, nq);
     uint32_t* ucap = ws_get<uint32_t>(c, n);
-    uint8_t* cls = ws_get<uint8_t>(c, n);
+    uint8_t* bucket = ws_get<uint8_t>(c, n);
     uint32_t* lists = ws_get<uint32_t>(c, (uint64_t)4 * n);
-    uint32_t* cnt = ws_get<uint32_t>(c, (uint64_t)n + 1);  // cnt[n] = 0 closes the offsets scan
-    unsigned long long* off = ws_get<unsigned long long>(c, (uint64_t)n + 1);
-    uint64_t* bsum2 = ws_get<uint64_t>(c, scan_storage((nyt > n ? nyt : n) + 1));
-    uint64_t* bsum_r = ws_get<uint64_t>(c, scan_storage((uint64_t)n + 1));
-    if (!degx || !curx || !JR_R || !IC_R || !cnt_yt || !cur_yt || !JR_S || !IC_S || !ISV || !Zq || !ucap || !cls || !lists ||
-        !cnt || !off || !bsum2 || !bsum_r)
+    unsigned long long* off = ws_get<unsigned long long>(c, n1);
+    unsigned long long* bsum2 = ws_get<unsigned long long>(c, sR);
+    if (!degx || !curx || !JR_R || !IC_R || !cur_yt || !JR_S || !IC_S || !ISV || !Zq || !ucap || !bucket || !lists ||
+        !off || !bsum2)
         return fail(c, DIM3G_ERR_NOMEM, "workspace allocation failed (CSR)");
+    uint32_t* cnt = degx + n1;  // cnt[n] = 0 closes the offsets scan
+    uint32_t* cnt_yt = cnt + n1;
+    unsigned long long* st_r = (unsigned long long*)(degx + round_up(2 * n1 + k1, 2));
 
-    // The two CSRs are independent: R's (by x) on the side stream while S's
-    // (by (y, z tile)) runs here; both are latency-bound scatters, so they
-    // overlap.  Joined before the row classification.
-    const cudaStream_t ax = c->aux;
-    CU(cudaEventRecord(c->ev_fork, st));
-    CU(cudaStreamWaitEvent(ax, c->ev_fork, 0));
-    CU(cudaMemsetAsync(degx, 0, ((uint64_t)n + 1) * 4, ax));
-    k_map_p<<<grid_for(jp.nP, sm), 256, 0, ax>>>(jp.P, jp.nP, tx, ty, Pm, degx);
+    // The two CSRs -- R's by x, S's by (y, z tile) -- are independent and
+    // latency-bound, so each step builds both in one launch.
+    CU(cudaMemsetAsync(degx, 0, zero2, st));
+    const unsigned g_csr = grid_for(jp.nP > nq ? jp.nP : nq, sm);
+    k_map<<<dim3(g_csr, 2), 256, 0, st>>>(MapArgs{jp.P, jp.nP, tx, ty, Pm, degx, Qk, nq, tz, T, tile_shift, Zq, cnt_yt});
     CHECK_LAUNCH();
-    {
-        int r = run_scan(c, U32Src{degx}, RowPtrDst{JR_R, curx}, (uint64_t)n + 1, bsum_r, nullptr, ax);
-        if (r) return r;
-    }
-    k_scatter_r<<<grid_for(jp.nP, sm), 256, 0, ax>>>(Pm, jp.nP, curx, IC_R);
+    using PtrJob = ScanJob<U32Src, RowPtrDst>;
+    device_scan2(PtrJob{U32Src{degx}, RowPtrDst{JR_R, curx}, n1, st_r, nullptr},
+                 PtrJob{U32Src{cnt_yt}, RowPtrDst{JR_S, cur_yt}, k1, st_r + sR, nullptr}, &sc->err, st);
     CHECK_LAUNCH();
-    CU(cudaEventRecord(c->ev_join, ax));
-    CU(cudaMemsetAsync(cnt_yt, 0, (nyt + 1) * 4, st));
-    k_map_q<<<grid_for(nq, sm), 256, 0, st>>>(Qk, nq, tz, T, tile_shift, Zq, cnt_yt);
+    k_scatter<<<dim3(g_csr, 2), 256, 0, st>>>(
+        ScatterArgs{Pm, jp.nP, curx, IC_R, Qk, Zq, nq, T, tile_shift, cur_yt, IC_S, ISV});
     CHECK_LAUNCH();
-    SCAN(U32Src{cnt_yt}, RowPtrDst{JR_S, cur_yt}, nyt + 1, bsum2, nullptr);
-    k_scatter_s<<<grid_for(nq, sm), 256, 0, st>>>(Qk, Zq, nq, T, tile_shift, cur_yt, IC_S, VS, ISV);
-    CHECK_LAUNCH();
-    CU(cudaStreamWaitEvent(st, c->ev_join, 0));
 
     RowCtx rc{};
     rc.JR_R = JR_R;
@@ -748,37 +753,24 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     rc.id2z = id2z;
     rc.out = nullptr;
     rc.err = &sc->err;
-    const uint32_t cap_w = 1u << (c->prm.warp_lg - 1);
-    const uint32_t cap_b = 1u << (c->prm.block_lg - 1);
-    // tiny rows get their own warp launch in the single pass only
-    const bool tiny = jp.single_pass && !jp.aggregate && !jp.count_only;
+    // tiny rows get their own warp launch, and the block class is split by
+    // hash-set size (2^lg slots for 2u keys), in the single pass only
+    const bool single = jp.single_pass && !jp.aggregate && !jp.count_only;
+    const bool block_split = single && !jp.sum.tiles && c->prm.block_split &&
+                             !(c->prm.prefetch_rows && c->prm.cta_rr == 3);
+    const RowBuckets rb{1u << (c->prm.warp_lg - 1), 1u << (c->prm.block_lg - 1), single, block_split,
+                        1u << (c->prm.block_lg - 3), 1u << (c->prm.block_lg - 2)};
     const uint32_t lanes = row_work_lanes((double)jp.nP / n);
-    k_row_work<<<grid_for((uint64_t)n << lanes, sm), 256, 0, st>>>(rc, n, lanes, cap_w, cap_b, jp.aggregate, tiny, jp.sum,
-                                                                    ucap, cls, &sc->outj, sc->outj_cls);
+    k_row_work<<<grid_for((uint64_t)n << lanes, sm), 256, 0, st>>>(rc, n, lanes, rb, jp.aggregate, jp.sum, ucap, bucket,
+                                                                    &sc->outj, sc->outj_cls, sc->nbucket);
     CHECK_LAUNCH();
     uint32_t* list_w = lists;
     uint32_t* list_b = lists + n;
     uint32_t* list_m = lists + 2 * (uint64_t)n;
     uint32_t* list_t = lists + 3 * (uint64_t)n;
-    SCAN(ClassSrc{cls, 1}, ListDst{list_w, nullptr}, n, bsum2, &sc->nrows[1]);
-    SCAN(ClassSrc{cls, 2}, ListDst{list_b, nullptr}, n, bsum2, &sc->nrows[2]);
-    const bool block_split = jp.single_pass && !jp.aggregate && !jp.count_only && !jp.sum.tiles &&
-                             c->prm.block_split && !(c->prm.prefetch_rows && c->prm.cta_rr == 3);
-    if (block_split) {
-        // the same rows again, ordered by hash-set size: u <= 2^(b-3), then
-        // u <= 2^(b-2), then the rest (b = block_lg; 2^lg slots for 2u keys)
-        const uint32_t b = c->prm.block_lg;
-        SCAN(BlockSizeSrc{cls, ucap, 0u, 1u << (b - 3)}, ListDst{list_b, nullptr}, n, bsum2, &sc->nrows_b[0]);
-        SCAN(BlockSizeSrc{cls, ucap, 1u << (b - 3), 1u << (b - 2)}, ListDst{list_b, &sc->nrows_b[0]}, n, bsum2,
-             &sc->nrows_b[1]);
-        SCAN(BlockSizeSrc{cls, ucap, 1u << (b - 2), 0xFFFFFFFFu}, ListDst{list_b, &sc->nrows_b[0], &sc->nrows_b[1]}, n,
-             bsum2, &sc->nrows_b[2]);
-    }
-    // bitmap rows: class 4 (huge) first, then class 3
-    SCAN(ClassSrc{cls, 4}, ListDst{list_m, nullptr}, n, bsum2, &sc->nrows[4]);
-    SCAN(ClassSrc{cls, 3}, ListDst{list_m, &sc->nrows[4]}, n, bsum2, &sc->nrows[3]);
-    if (tiny) SCAN(ClassSrc{cls, 5}, ListDst{list_t, nullptr}, n, bsum2, &sc->nrows[5]);
-    CU(cudaMemsetAsync(cnt, 0, ((uint64_t)n + 1) * 4, st));
+    k_row_lists<<<(unsigned)((n + kListTile - 1) / kListTile), 256, 0, st>>>(bucket, n, sc->nbucket, sc->list_cur, lists,
+                                                                             sc->nrows, sc->nrows_b);
+    CHECK_LAUNCH();
     CU(cudaEventRecord(c->ev[2], st));
     DensePlan dp;
     {
@@ -861,32 +853,46 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
                 list_m, dp.nd, dp.D, dp.Wd, dp.Wm, dp.cpr, dp.coff, id2x, id2z, out, nullptr, &sc->dense_base);
             CHECK_LAUNCH();
         }
+        // Launches whose class holds no row are left out: from the class
+        // counts where the host has them, else from u <= m (a launch over an
+        // empty list is about 3 us of a small join).
+        const Scalars& h = *c->h_sc;
+        const bool has_m = dp.counted ? h.nrows[3] + h.nrows[4] != 0 : m > rb.cap_b;
+        const bool has_b[3] = {!dp.counted || h.nrows_b[0], dp.counted ? h.nrows_b[1] != 0 : m > rb.cap_s,
+                               dp.counted ? h.nrows_b[2] != 0 : m > rb.cap_m};
+        const bool has_any_b = !dp.counted || h.nrows[2], has_w = !dp.counted || h.nrows[1],
+                   has_t = !dp.counted || h.nrows[5];
         // the cross-segment gather's threshold per row class, measured on
         // the 2-hop (bitmap rows 45.5 -> 44.7 ms at 160, block rows 26.3 ->
         // 25.7 at 560, warp rows 2.62 -> 2.58 at 160; every setting exact)
         rc.flat_avg = kFlatAvgBitmap;
-        if (c->prm.stream_rows && stream_smem_bytes(bm_words) <= kMaxSmemOptin) {
+        if (!has_m) {
+        } else if (c->prm.stream_rows && stream_smem_bytes(bm_words) <= kMaxSmemOptin) {
             const size_t ss_s = stream_smem_bytes(bm_words);
             k_stream_bitmap<<<resident_grid(k_stream_bitmap, kStreamThreads, ss_s, sm), kStreamThreads, ss_s, st>>>(
                 rc, rs, L.m, L.n3, L.n4, bm_words);
+            CHECK_LAUNCH();
         } else {
             k_single_bitmap<<<resident_grid(k_single_bitmap, blk_m, ss_m, sm), blk_m, ss_m, st>>>(rc, rs, L.m, L.n3,
                                                                                              L.n4, bm_words);
+            CHECK_LAUNCH();
         }
-        CHECK_LAUNCH();
         CU(cudaEventRecord(c->evc[5], st));
         CU(cudaMemcpyAsync(&sc->cursor_at[0], &sc->cursor, 8, cudaMemcpyDeviceToDevice, st));
         rc.flat_avg = kFlatAvgBlock;
-        if (c->prm.prefetch_rows && c->prm.cta_rr == 3) {
+        if (!has_any_b) {
+        } else if (c->prm.prefetch_rows && c->prm.cta_rr == 3) {
             const size_t ss_p = (((size_t)1 << c->prm.block_lg) + (size_t)kPfWorkers * kStage) * 4;
             k_single_block_pf<<<resident_grid(k_single_block_pf, kPfThreads, ss_p, sm), kPfThreads, ss_p, st>>>(
                 rc, rs, L.b, L.nb, c->prm.block_lg);
+            CHECK_LAUNCH();
         } else if (block_split) {
             // three launches over list_b's three parts, smallest sets first
             const uint32_t b = c->prm.block_lg;
             const unsigned long long* skip[3][2] = {{nullptr, nullptr}, {&sc->nrows_b[0], nullptr},
                                                     {&sc->nrows_b[0], &sc->nrows_b[1]}};
             for (uint32_t k = 0; k < 3; k++) {
+                if (!has_b[k]) continue;
                 const int thr = k < 2 ? (int)kBlockSplitThreads : blk_b;
                 const uint32_t lg = b - 2 + k;
                 const size_t ss = ((size_t)1 << lg << 2) + (size_t)(thr / 32) * kStage * 4;
@@ -897,18 +903,21 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         } else {
             k_single_block<<<resident_grid(k_single_block, blk_b, ss_b, sm), blk_b, ss_b, st>>>(
                 rc, rs, L.b, L.nb, c->prm.block_lg, nullptr, nullptr, 2);
+            CHECK_LAUNCH();
         }
-        CHECK_LAUNCH();
         CU(cudaEventRecord(c->evc[6], st));
         CU(cudaMemcpyAsync(&sc->cursor_at[1], &sc->cursor, 8, cudaMemcpyDeviceToDevice, st));
         rc.flat_avg = kFlatAvgWarp;
-        k_single_warp<<<resident_grid(k_single_warp, 32 * wps, ss_w, sm), 32 * wps, ss_w, st>>>(rc, rs, L.w, L.nw,
-                                                                                           c->prm.warp_lg, kStage);
-        CHECK_LAUNCH();
-        k_single_warp<<<resident_grid(k_single_warp, 32 * wpt, ss_t, sm), 32 * wpt, ss_t, st>>>(rc, rs, list_t,
-                                                                                           &sc->nrows[5], kTinyLg,
-                                                                                           kTinyStage);
-        CHECK_LAUNCH();
+        if (has_w) {
+            k_single_warp<<<resident_grid(k_single_warp, 32 * wps, ss_w, sm), 32 * wps, ss_w, st>>>(
+                rc, rs, L.w, L.nw, c->prm.warp_lg, kStage);
+            CHECK_LAUNCH();
+        }
+        if (has_t) {
+            k_single_warp<<<resident_grid(k_single_warp, 32 * wpt, ss_t, sm), 32 * wpt, ss_t, st>>>(
+                rc, rs, list_t, &sc->nrows[5], kTinyLg, kTinyStage);
+            CHECK_LAUNCH();
+        }
         CU(cudaEventRecord(c->evc[7], st));
         CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
         CU(cudaEventRecord(c->ev[3], st));
@@ -958,7 +967,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     k_rows_warp<false><<<g_w, 32 * wpc, smem_w, st>>>(rc, L.w, L.nw, c->prm.warp_lg);
     CHECK_LAUNCH();
     CU(cudaEventRecord(c->evc[3], st));
-    SCAN(U32Src{cnt}, OffDst{off}, (uint64_t)n + 1, bsum2, &sc->total);
+    SCAN(U32Src{cnt}, OffDst{off}, (uint64_t)n + 1, bsum2, &sc->total, &sc->err);
     CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
     CU(cudaEventRecord(c->ev[3], st));
     CU(cudaStreamSynchronize(st));
@@ -1234,9 +1243,6 @@ int dim3g_create(int device, dim3g_ctx** out) {
     dim3g_ctx* c = new dim3g_ctx();
     c->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&c->aux, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaMallocHost((void**)&c->h_sc, sizeof(Scalars)) != cudaSuccess) {
         cudaGetLastError();
@@ -1299,9 +1305,6 @@ void dim3g_destroy(dim3g_ctx* c) {
         if (e) cudaEventDestroy(e);
     for (auto& e : c->evd)
         if (e) cudaEventDestroy(e);
-    if (c->ev_fork) cudaEventDestroy(c->ev_fork);
-    if (c->ev_join) cudaEventDestroy(c->ev_join);
-    if (c->aux) cudaStreamDestroy(c->aux);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
 }
@@ -1675,7 +1678,7 @@ int dim3g_mapper_insert(dim3g_mapper* m, const uint32_t* keys, uint64_t n, int32
     uint32_t* dk;
     int32_t* di;
     if ((r = mapper_stage(m, keys, n, &dk, &di))) return r;
-    uint64_t* bsum = ws_get<uint64_t>(c, scan_storage(n));
+    unsigned long long* bsum = ws_get<unsigned long long>(c, scan_storage(n));
     unsigned long long* total = ws_get<unsigned long long>(c, 1);
     uint32_t* err = ws_get<uint32_t>(c, 1);
     if (!bsum || !total || !err) return fail(c, DIM3G_ERR_NOMEM, "mapper scratch allocation failed");
@@ -1684,7 +1687,7 @@ int dim3g_mapper_insert(dim3g_mapper* m, const uint32_t* keys, uint64_t n, int32
     CU(cudaMemsetAsync(err, 0, 4, st));
     k_mapper_claim<<<grid_for(n, c->sm_count), 256, 0, st>>>(t, dk, n, err);
     CHECK_LAUNCH();
-    SCAN(FirstOccSrc{t, dk}, AssignNewIdDst{t, dk, (long long)m->cnt}, n, bsum, total);
+    SCAN(FirstOccSrc{t, dk}, AssignNewIdDst{t, dk, (long long)m->cnt}, n, bsum, total, err);
     k_mapper_gather<<<grid_for(n, c->sm_count), 256, 0, st>>>(t, dk, n, di);
     CHECK_LAUNCH();
     unsigned long long h_total = 0;

@@ -739,6 +739,22 @@ static __global__ void __launch_bounds__(1024) k_rows_bitmap(RowCtx c, const uin
     }
 }
 
+// The rows' lists.  A row's bucket: 0 warp class; 1..3 block class, by
+// distinct bound u <= cap_s, u <= cap_m, larger where the launches are split
+// by hash-set size (else all 1); 4 huge and 5 other bitmap rows; 6 tiny rows;
+// kRowBuckets none.
+constexpr uint32_t kRowBuckets = 7;
+struct RowBuckets {
+    uint32_t cap_w, cap_b;  // row_class bounds
+    bool tiny, split;
+    uint32_t cap_s, cap_m;
+    __device__ __forceinline__ uint32_t of(uint32_t cls, uint32_t u) const {
+        if (cls == 1) return 0;
+        if (cls == 2) return !split || u <= cap_s ? 1u : (u <= cap_m ? 2u : 3u);
+        return cls == 0 ? kRowBuckets : (cls == 4 ? 4u : (cls == 3 ? 5u : 6u));
+    }
+};
+
 // Per-row candidate count w = sum over y in R_x of |S_y|, u = min(w, m) and
 // the row class (0: empty, or outside sel's A-tiles).  With check_range set
 // (join-aggregate, 32-bit per-group counters) a row of 2^32 or more
@@ -748,14 +764,16 @@ static __global__ void __launch_bounds__(1024) k_rows_bitmap(RowCtx c, const uin
 // so the rows in flight bound the time: 2^lg lanes take a row, about as many
 // as a row has entries on average (row_work_lanes), and a row of more than
 // 4 x 2^lg entries is finished by its whole warp.  A warp for every row took
-// 281 us for 1M rows of 10 entries.  The sums are added up per CTA in shared
-// memory, then one atomic a CTA and counter.
-static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, uint32_t lg, uint32_t cap_w,
-                                                         uint32_t cap_b, bool check_range, bool tiny, SumAcc sel,
-                                                         uint32_t* __restrict__ ucap, uint8_t* __restrict__ cls,
-                                                         unsigned long long* outj, unsigned long long* outj_cls) {
+// 281 us for 1M rows of 10 entries.  The sums and the rows per bucket are
+// added up per CTA in shared memory, then one atomic a CTA and counter.
+static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, uint32_t lg, RowBuckets rb,
+                                                         bool check_range, SumAcc sel, uint32_t* __restrict__ ucap,
+                                                         uint8_t* __restrict__ bucket, unsigned long long* outj,
+                                                         unsigned long long* outj_cls, unsigned long long* nbucket) {
     __shared__ unsigned long long s_acc[6];
+    __shared__ uint32_t s_n[kRowBuckets + 1];
     if (threadIdx.x < 6) s_acc[threadIdx.x] = 0;
+    if (threadIdx.x <= kRowBuckets) s_n[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t lane = lane_id(), G = 1u << lg, gl = lane & (G - 1), per = 32 >> lg;
     const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -795,9 +813,10 @@ static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, u
         for (uint32_t o = G >> 1; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
         if (gl == 0 && x < n) {
             const uint32_t u = (uint32_t)(w < c.m ? w : c.m);
-            const uint32_t k = row_class(w, u, cap_w, cap_b, tiny);
+            const uint32_t k = row_class(w, u, rb.cap_w, rb.cap_b, rb.tiny), q = rb.of(k, u);
             ucap[x] = u;
-            cls[x] = (uint8_t)k;
+            bucket[x] = (uint8_t)q;
+            atomicAdd(&s_n[q], 1u);
             if (check_range && w >= 0xFFFFFFFFull) raise_error(c.err, kErrCountRange);
             if (w) {
                 atomicAdd(&s_acc[0], w);
@@ -807,34 +826,68 @@ static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, u
     }
     __syncthreads();
     if (threadIdx.x < 6 && s_acc[threadIdx.x]) atomicAdd(threadIdx.x ? &outj_cls[threadIdx.x] : outj, s_acc[threadIdx.x]);
+    if (threadIdx.x < kRowBuckets && s_n[threadIdx.x])
+        atomicAdd(&nbucket[threadIdx.x], (unsigned long long)s_n[threadIdx.x]);
 }
 // Lanes a row (log2) for rows of `per_row` entries on average.
 inline uint32_t row_work_lanes(double per_row) { return per_row > 64 ? 5 : (per_row > 24 ? 4 : (per_row > 8 ? 3 : 2)); }
 
-struct ClassSrc {
-    const uint8_t* cls;
-    uint8_t want;
-    __device__ uint64_t operator()(uint64_t i) const { return cls[i] == want ? 1u : 0u; }
-};
-// Block-class (class 2) rows whose distinct bound u is in (lo, hi].
-struct BlockSizeSrc {
-    const uint8_t* cls;
-    const uint32_t* ucap;
-    uint32_t lo, hi;
-    __device__ uint64_t operator()(uint64_t i) const {
-        return cls[i] == 2 && ucap[i] > lo && ucap[i] <= hi ? 1u : 0u;
+// Every row into its bucket's list: list_w, list_b (buckets 1, 2, 3 in
+// turn), list_m (4 then 5: the huge rows first) and list_t.  k_row_work has
+// counted the buckets (nbucket), so where each starts is known; a CTA ranks
+// its kListTile rows in shared memory and takes one range of each bucket from
+// its cursor.  One launch (a prefix sum per bucket was three each).  Rows of
+// a tile stay in order and together; the order of tiles is unspecified.  The
+// class counts go to n[1..5] and nb[0..2].
+constexpr uint32_t kListItems = 8, kListTile = 256 * kListItems;
+static __global__ void __launch_bounds__(256) k_row_lists(const uint8_t* __restrict__ bucket, uint32_t n,
+                                                          const unsigned long long* __restrict__ nbucket,
+                                                          unsigned long long* cursor, uint32_t* __restrict__ lists,
+                                                          unsigned long long* nrows, unsigned long long* nrows_b) {
+    __shared__ uint32_t s_n[kRowBuckets + 1];
+    __shared__ uint32_t* s_at[kRowBuckets];
+    if (threadIdx.x <= kRowBuckets) s_n[threadIdx.x] = 0;
+    __syncthreads();
+    const uint64_t t0 = (uint64_t)blockIdx.x * kListTile;
+    const uint32_t lane = lane_id();
+    uint32_t b[kListItems], rank[kListItems];
+#pragma unroll
+    for (uint32_t k = 0; k < kListItems; k++) {
+        const uint64_t x = t0 + k * 256 + threadIdx.x;
+        b[k] = x < n ? bucket[x] : kRowBuckets;
     }
-};
-// list[*base + *base2 + rank] = row (bases: counts of rows placed before
-// this class; either may be null).
-struct ListDst {
-    uint32_t* list;
-    const unsigned long long* base;
-    const unsigned long long* base2 = nullptr;
-    __device__ void operator()(uint64_t i, uint64_t e, uint64_t v) const {
-        if (v) list[(base ? *base : 0) + (base2 ? *base2 : 0) + e] = (uint32_t)i;
+#pragma unroll
+    for (uint32_t k = 0; k < kListItems; k++) {
+        const unsigned grp = __match_any_sync(0xffffffffu, b[k]);
+        const int leader = __ffs(grp) - 1;
+        uint32_t r = 0;
+        if ((int)lane == leader) r = atomicAdd(&s_n[b[k]], (uint32_t)__popc(grp));
+        rank[k] = __shfl_sync(0xffffffffu, r, leader) + __popc(grp & lanemask_lt());
     }
-};
+    __syncthreads();
+    if (threadIdx.x < kRowBuckets) {
+        const uint32_t q = threadIdx.x;
+        uint32_t* list = lists + (q == 0 ? 0ull : (q <= 3 ? 1ull : (q <= 5 ? 2ull : 3ull))) * n;
+        unsigned long long at = s_n[q] ? atomicAdd(&cursor[q], (unsigned long long)s_n[q]) : 0ull;
+        if (q == 2 || q == 3) at += nbucket[1];
+        if (q == 3) at += nbucket[2];
+        if (q == 5) at += nbucket[4];
+        s_at[q] = list + at;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        nrows[1] = nbucket[0];
+        nrows[2] = nbucket[1] + nbucket[2] + nbucket[3];
+        nrows[3] = nbucket[5];
+        nrows[4] = nbucket[4];
+        nrows[5] = nbucket[6];
+        for (int k = 0; k < 3; k++) nrows_b[k] = nbucket[1 + k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < kListItems; k++)
+        if (b[k] < kRowBuckets) s_at[b[k]][rank[k]] = (uint32_t)(t0 + k * 256 + threadIdx.x);
+}
+
 struct OffDst {
     unsigned long long* off;
     __device__ void operator()(uint64_t i, uint64_t e, uint64_t) const { off[i] = e; }

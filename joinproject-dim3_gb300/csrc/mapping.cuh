@@ -231,27 +231,40 @@ struct AssignIdDst {
     }
 };
 
-// P -> (x id, y id); per-x degree histogram.
-static __global__ void k_map_p(const uint2* __restrict__ P, uint64_t n, DevTable tx, DevTable ty, uint2* __restrict__ Pm,
-                        uint32_t* __restrict__ degx) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint2 p = P[i];
-        uint32_t xi = table_find(tx, p.x);
-        uint32_t yi = table_find(ty, p.y);
-        Pm[i] = make_uint2(xi, yi);
-        atomicAdd(&degx[xi], 1u);
-    }
-}
-
-// Q' = (z value, y id) -> z id; histogram over the (y, z tile) CSR key
-// y*T + z/TB.
-static __global__ void k_map_q(const uint2* __restrict__ Qk, uint64_t n, DevTable tz, uint32_t T, uint32_t tile_shift,
-                        uint32_t* __restrict__ zid, uint32_t* __restrict__ cnt_yt) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint2 q = Qk[i];
-        uint32_t zi = table_find(tz, q.x);
-        zid[i] = zi;
-        atomicAdd(&cnt_yt[(uint64_t)q.y * T + (zi >> tile_shift)], 1u);
+// P -> (x id, y id) with the per-x degree histogram (blockIdx.y 0), and Q' =
+// (z value, y id) -> z id with the histogram over the (y, z tile) CSR key
+// y*T + z/TB (blockIdx.y 1): independent passes in one launch, so the one's
+// tail overlaps the other.
+struct MapArgs {
+    const uint2* P;
+    uint64_t nP;
+    DevTable tx, ty;
+    uint2* Pm;
+    uint32_t* degx;
+    const uint2* Qk;
+    uint64_t nQ;
+    DevTable tz;
+    uint32_t T, tile_shift;
+    uint32_t* zid;
+    uint32_t* cnt_yt;
+};
+static __global__ void __launch_bounds__(256) k_map(MapArgs a) {
+    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    if (blockIdx.y == 0) {
+        for (uint64_t i = first; i < a.nP; i += stride) {
+            const uint2 p = __ldg(&a.P[i]);
+            const uint32_t xi = table_find(a.tx, p.x);
+            const uint32_t yi = table_find(a.ty, p.y);
+            a.Pm[i] = make_uint2(xi, yi);
+            atomicAdd(&a.degx[xi], 1u);
+        }
+    } else {
+        for (uint64_t i = first; i < a.nQ; i += stride) {
+            const uint2 q = __ldg(&a.Qk[i]);
+            const uint32_t zi = table_find(a.tz, q.x);
+            a.zid[i] = zi;
+            atomicAdd(&a.cnt_yt[(uint64_t)q.y * a.T + (zi >> a.tile_shift)], 1u);
+        }
     }
 }
 
@@ -269,30 +282,38 @@ struct RowPtrDst {
     }
 };
 
-static __global__ void k_scatter_r(const uint2* __restrict__ Pm, uint64_t n, uint32_t* __restrict__ cursor,
-                            uint32_t* __restrict__ ic) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint2 p = Pm[i];
-        uint32_t pos = atomicAdd(&cursor[p.x], 1u);
-        ic[pos] = p.y;
-    }
-}
-
-// S CSR by (y id, z tile): z ids into ic and, beside them, z values into vs
-// (the write pass emits values without a gather through id2z).
-// vs, isv (either may be null): the z values beside the ids, and the z id
-// and z value of each entry side by side for the expansion paths that emit
-// values (one 8-byte load or copy per candidate).
-static __global__ void k_scatter_s(const uint2* __restrict__ Qk, const uint32_t* __restrict__ zid, uint64_t n, uint32_t T,
-                            uint32_t tile_shift, uint32_t* __restrict__ cursor, uint32_t* __restrict__ ic,
-                            uint32_t* __restrict__ vs, uint2* __restrict__ isv) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint2 q = Qk[i];
-        uint32_t zi = zid[i];
-        uint32_t pos = atomicAdd(&cursor[(uint64_t)q.y * T + (zi >> tile_shift)], 1u);
-        ic[pos] = zi;
-        if (vs) vs[pos] = q.x;
-        if (isv) isv[pos] = make_uint2(zi, q.x);
+// The CSR entries (launched as k_map): R's y ids by x (blockIdx.y 0), and S by
+// (y id, z tile) (blockIdx.y 1): z ids into ic and, beside them (isv, may be
+// null), the z id and z value of each entry side by side for the expansion
+// paths that emit values (one 8-byte load or copy per candidate).
+struct ScatterArgs {
+    const uint2* Pm;
+    uint64_t nP;
+    uint32_t* curx;
+    uint32_t* ic_r;
+    const uint2* Qk;
+    const uint32_t* zid;
+    uint64_t nQ;
+    uint32_t T, tile_shift;
+    uint32_t* cur_yt;
+    uint32_t* ic_s;
+    uint2* isv;
+};
+static __global__ void __launch_bounds__(256) k_scatter(ScatterArgs a) {
+    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    if (blockIdx.y == 0) {
+        for (uint64_t i = first; i < a.nP; i += stride) {
+            const uint2 p = __ldg(&a.Pm[i]);
+            a.ic_r[atomicAdd(&a.curx[p.x], 1u)] = p.y;
+        }
+    } else {
+        for (uint64_t i = first; i < a.nQ; i += stride) {
+            const uint2 q = __ldg(&a.Qk[i]);
+            const uint32_t zi = __ldg(&a.zid[i]);
+            const uint32_t pos = atomicAdd(&a.cur_yt[(uint64_t)q.y * a.T + (zi >> a.tile_shift)], 1u);
+            a.ic_s[pos] = zi;
+            if (a.isv) a.isv[pos] = make_uint2(zi, q.x);
+        }
     }
 }
 

@@ -1,6 +1,13 @@
-// scan.cuh -- device-wide exclusive prefix sums (reduce / scan-of-sums /
-// apply), driven by functors so one pass both computes and consumes the
-// prefix (CSR row pointers, table compaction, output offsets).
+// scan.cuh -- device-wide exclusive prefix sums in one launch, driven by
+// functors so one pass both computes and consumes the prefix (CSR row
+// pointers, table compaction, output offsets).
+//
+// Decoupled look-back: tiles are numbered by a ticket, so a tile waits only
+// on tiles whose CTAs already run.  A tile publishes its sum, adds up its
+// predecessors' published words 32 at a time back to the nearest inclusive
+// prefix, and publishes its own.  Items are read once and a scan is one
+// launch.  (Sum of tiles, scan of the sums, apply -- three launches and two
+// reads -- were 45 of the 53 kernels of a small join, at about 3 us each.)
 #pragma once
 #include "common.cuh"
 
@@ -10,104 +17,96 @@ constexpr int kScanBlock = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanBlock * kScanItems;
 
-// Src:  __device__ uint64_t operator()(uint64_t i) const      -- value of item i
-// Dst:  __device__ void operator()(uint64_t i, uint64_t excl, uint64_t v) const
-template <class Src>
-__global__ void __launch_bounds__(kScanBlock) k_scan_reduce(Src src, uint64_t n, uint64_t* block_sums) {
-    __shared__ uint64_t sm[kScanBlock / 32 + 1];
-    uint64_t base = (uint64_t)blockIdx.x * kScanTile;
-    uint64_t acc = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        uint64_t i = base + (uint64_t)k * kScanBlock + threadIdx.x;
-        if (i < n) acc += src(i);
-    }
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint64_t t = 0;
-        for (int w = 0; w < kScanBlock / 32; w++) t += sm[w];
-        block_sums[blockIdx.x] = t;
-    }
-}
+// A tile's word: sum << 2 | state (sums stay below 2^62).
+constexpr unsigned long long kScanSum = 1, kScanPrefix = 2;
+// Polls of one look-back window before a tile gives up (about a second).
+constexpr uint32_t kScanPolls = 1u << 21;
 
-// Single-block exclusive scan of nb block sums in place; writes the grand
-// total to *total.
-static __global__ void __launch_bounds__(1024) k_scan_sums(uint64_t* sums, uint64_t nb, unsigned long long* total) {
-    __shared__ uint64_t sm[1024 / 32 + 1];
-    uint64_t carry = 0;
-    for (uint64_t c = 0; c < nb; c += 1024) {
-        uint64_t i = c + threadIdx.x;
-        uint64_t v = i < nb ? sums[i] : 0;
-        uint64_t t;
-        uint64_t e = block_excl_scan<1024>(v, sm, &t);
-        if (i < nb) sums[i] = carry + e;
-        carry += t;
-    }
-    if (threadIdx.x == 0 && total) *total = carry;
-}
-
+// One scan.  Src: uint64_t operator()(i), the value of item i, i < n.
+// Dst: void operator()(i, prefix, value).  state: scan_storage(n) zeroed
+// words.  *total (may be null) receives the sum.
 template <class Src, class Dst>
-__global__ void __launch_bounds__(kScanBlock) k_scan_apply(Src src, uint64_t n, const uint64_t* block_sums, Dst dst) {
+struct ScanJob {
+    Src src;
+    Dst dst;
+    uint64_t n;
+    unsigned long long* state;
+    unsigned long long* total;
+};
+
+inline uint64_t scan_blocks(uint64_t n) { return (n + kScanTile - 1) / kScanTile; }
+inline uint64_t scan_storage(uint64_t n) { return scan_blocks(n) + 1; }
+
+// Exclusive prefix of tile `tile` (its sum: `sum`), by one warp.
+__device__ __forceinline__ uint64_t scan_look_back(unsigned long long* state, uint64_t tile, uint64_t sum,
+                                                   uint32_t* err) {
+    volatile unsigned long long* w = state + 1;
+    const uint32_t lane = lane_id();
+    if (tile == 0) {
+        if (lane == 0) w[0] = sum << 2 | kScanPrefix;
+        return 0;
+    }
+    if (lane == 0) w[tile] = sum << 2 | kScanSum;
+    uint64_t before = 0;
+    for (uint64_t end = tile;; end -= 32) {  // lane l reads tile end - 1 - l
+        unsigned long long v = kScanPrefix;
+        uint32_t polls = 0;
+        for (;;) {
+            if (lane < end) v = w[end - 1 - lane];
+            if (__all_sync(0xffffffffu, (v & 3) != 0)) break;
+            if (++polls == kScanPolls) {
+                if (lane == 0) raise_error(err, kErrScanTimeout);
+                break;
+            }
+        }
+        const uint32_t done = __ballot_sync(0xffffffffu, (v & 3) == kScanPrefix);
+        const uint32_t last = done ? __ffs(done) - 1 : 31;
+        before += warp_sum<uint64_t>(lane <= last ? v >> 2 : 0ull);
+        if (done || polls == kScanPolls || end <= 32) break;
+    }
+    if (lane == 0) w[tile] = (before + sum) << 2 | kScanPrefix;
+    return before;
+}
+
+// Up to two scans of one kind (blockIdx.y) in one launch.
+template <class Src, class Dst>
+__global__ void __launch_bounds__(kScanBlock) k_scan(ScanJob<Src, Dst> a, ScanJob<Src, Dst> b, uint32_t* err) {
     __shared__ uint64_t sm[kScanBlock / 32 + 1];
-    uint64_t base = (uint64_t)blockIdx.x * kScanTile;
+    __shared__ uint64_t s_tile, s_before;
+    const ScanJob<Src, Dst> j = blockIdx.y ? b : a;
+    const uint64_t nb = (j.n + kScanTile - 1) / kScanTile;
+    if (blockIdx.x >= nb) return;
+    if (threadIdx.x == 0) s_tile = atomicAdd(j.state, 1ull);
+    __syncthreads();
+    const uint64_t tile = s_tile;
     // Each thread owns kScanItems consecutive items so the scan order is the
     // item order.
-    uint64_t v[kScanItems];
-    uint64_t local = 0;
-    uint64_t first = base + (uint64_t)threadIdx.x * kScanItems;
+    const uint64_t first = tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
+    uint64_t v[kScanItems], local = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        uint64_t i = first + k;
-        v[k] = i < n ? src(i) : 0;
+        const uint64_t i = first + k;
+        v[k] = i < j.n ? j.src(i) : 0;
         local += v[k];
     }
-    uint64_t t;
-    uint64_t e = block_excl_scan<kScanBlock>(local, sm, &t) + block_sums[blockIdx.x];
+    uint64_t sum;
+    uint64_t e = block_excl_scan<kScanBlock>(local, sm, &sum);
+    if (threadIdx.x < 32) {
+        const uint64_t before = scan_look_back(j.state, tile, sum, err);
+        if (threadIdx.x == 0) {
+            s_before = before;
+            if (tile == nb - 1 && j.total) *j.total = before + sum;
+        }
+    }
+    __syncthreads();
+    e += s_before;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        uint64_t i = first + k;
-        if (i < n) dst(i, e, v[k]);
+        const uint64_t i = first + k;
+        if (i < j.n) j.dst(i, e, v[k]);
         e += v[k];
     }
 }
-
-// Host driver.  block_sums must hold scan_storage(n) entries; total
-// (device) receives the sum of all items.  Up to kScanSumsDirect block sums
-// are scanned by one CTA; more are scanned by the same three kernels one
-// level up (their own block sums stored after them).
-inline uint64_t scan_blocks(uint64_t n) { return (n + kScanTile - 1) / kScanTile; }
-constexpr uint64_t kScanSumsDirect = 32768;
-inline uint64_t scan_storage(uint64_t n) {
-    uint64_t nb = scan_blocks(n), s = nb + 1;
-    while (nb > kScanSumsDirect) {
-        nb = scan_blocks(nb);
-        s += nb + 1;
-    }
-    return s;
-}
-// Number of kernel launches device_scan makes for n items.
-inline uint64_t scan_launches(uint64_t n) {
-    uint64_t nb = scan_blocks(n), k = 0;
-    if (nb == 0) return 0;
-    k = 3;
-    while (nb > kScanSumsDirect) {
-        nb = scan_blocks(nb);
-        k += 2;
-    }
-    return k;
-}
-
-struct SumsSrc {
-    const uint64_t* a;
-    __device__ uint64_t operator()(uint64_t i) const { return a[i]; }
-};
-// In place: k_scan_apply reads all items of a thread before writing them.
-struct SumsDst {
-    uint64_t* a;
-    __device__ void operator()(uint64_t i, uint64_t e, uint64_t) const { a[i] = e; }
-};
 
 // A scan whose length is only known on the device: items at or past *lim
 // count as 0 and are neither read nor written (the launch still covers the
@@ -127,24 +126,16 @@ struct BoundDst {
     }
 };
 
+// Host launches; the states are zeroed by the caller.  An empty scan launches
+// nothing and leaves *total as it is (zeroed with the rest).
 template <class Src, class Dst>
-inline void device_scan(Src src, Dst dst, uint64_t n, uint64_t* block_sums, unsigned long long* total, cudaStream_t st);
-
-inline void scan_block_sums(uint64_t* sums, uint64_t nb, unsigned long long* total, cudaStream_t st) {
-    if (nb <= kScanSumsDirect) k_scan_sums<<<1, 1024, 0, st>>>(sums, nb, total);
-    else device_scan(SumsSrc{sums}, SumsDst{sums}, nb, sums + nb + 1, total, st);
+inline void device_scan(const ScanJob<Src, Dst>& j, uint32_t* err, cudaStream_t st) {
+    if (j.n) k_scan<<<(unsigned)scan_blocks(j.n), kScanBlock, 0, st>>>(j, j, err);
 }
-
 template <class Src, class Dst>
-inline void device_scan(Src src, Dst dst, uint64_t n, uint64_t* block_sums, unsigned long long* total, cudaStream_t st) {
-    uint64_t nb = scan_blocks(n);
-    if (nb == 0) {
-        if (total) cudaMemsetAsync(total, 0, sizeof(uint64_t), st);
-        return;
-    }
-    k_scan_reduce<<<(unsigned)nb, kScanBlock, 0, st>>>(src, n, block_sums);
-    scan_block_sums(block_sums, nb, total, st);
-    k_scan_apply<<<(unsigned)nb, kScanBlock, 0, st>>>(src, n, block_sums, dst);
+inline void device_scan2(const ScanJob<Src, Dst>& a, const ScanJob<Src, Dst>& b, uint32_t* err, cudaStream_t st) {
+    const uint64_t n = a.n > b.n ? a.n : b.n;
+    if (n) k_scan<<<dim3((unsigned)scan_blocks(n), 2), kScanBlock, 0, st>>>(a, b, err);
 }
 
 }  // namespace dim3g
