@@ -349,7 +349,7 @@ int relset_enqueue_build(dim3g_relset* s, cudaStream_t st, uint64_t& launches) {
     k_ix_layout<<<1, 1024, 0, st>>>(P, s->tile_lg);
     BLAUNCH();
     using IdJob = ScanJob<OccupiedSrc, AssignIdDst>;
-    using PtrJob = ScanJob<BoundSrc<U32Src>, BoundDst<RowPtrDst>>;
+    using PtrJob = ScanJob<U32Src, RowPtrDst>;
     unsigned long long* w[4] = {s->scan_state, w[0] + s->scan_words[0], w[1] + s->scan_words[1], w[2] + s->scan_words[2]};
     device_scan2(IdJob{OccupiedSrc{P.TF}, AssignIdDst{P.TF, P.id2f}, s->tabtot, w[0], nullptr},
                  IdJob{OccupiedSrc{P.TY}, AssignIdDst{P.TY, P.id2y}, s->tabtot, w[1], nullptr}, P.err, st);
@@ -360,9 +360,8 @@ int relset_enqueue_build(dim3g_relset* s, cudaStream_t st, uint64_t& launches) {
     }
     // row pointers up to the id / key counts the layout found (the launch
     // covers the tuple-count bounds; past the counts nothing is read or written)
-    device_scan2(PtrJob{{U32Src{P.degF}, P.f_need}, {RowPtrDst{P.JRf, P.curF}, P.f_need}, s->ntot + 1, w[2], nullptr},
-                 PtrJob{{U32Src{P.cnt_yt}, P.yt_need}, {RowPtrDst{P.JRy, P.curY}, P.yt_need}, s->yt_cap, w[3], nullptr},
-                 P.err, st);
+    device_scan2(PtrJob{U32Src{P.degF}, RowPtrDst{P.JRf, P.curF}, s->ntot + 1, w[2], nullptr, P.f_need},
+                 PtrJob{U32Src{P.cnt_yt}, RowPtrDst{P.JRy, P.curY}, s->yt_cap, w[3], nullptr, P.yt_need}, P.err, st);
     BLAUNCH();
     if (s->ntot) {
         k_ix_scatter<<<elem_grid(s->ntot, sm), 256, 0, st>>>(P);

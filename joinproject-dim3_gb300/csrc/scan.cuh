@@ -14,7 +14,7 @@
 namespace dim3g {
 
 constexpr int kScanBlock = 256;
-constexpr int kScanItems = 8;
+constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanBlock * kScanItems;
 
 // A tile's word: sum << 2 | state (sums stay below 2^62).
@@ -22,9 +22,12 @@ constexpr unsigned long long kScanSum = 1, kScanPrefix = 2;
 // Polls of one look-back window before a tile gives up (about a second).
 constexpr uint32_t kScanPolls = 1u << 21;
 
-// One scan.  Src: uint64_t operator()(i), the value of item i, i < n.
+// One scan.  Src: uint32_t operator()(i), the value of item i, i < n (a
+// tile's values add up to less than 2^32).
 // Dst: void operator()(i, prefix, value).  state: scan_storage(n) zeroed
-// words.  *total (may be null) receives the sum.
+// words.  *total (may be null) receives the sum.  lim (may be null): the
+// length where only the device knows it (the launch covers the host's bound
+// n; tiles at or past *lim end at once).
 template <class Src, class Dst>
 struct ScanJob {
     Src src;
@@ -32,6 +35,7 @@ struct ScanJob {
     uint64_t n;
     unsigned long long* state;
     unsigned long long* total;
+    const unsigned long long* lim = nullptr;
 };
 
 inline uint64_t scan_blocks(uint64_t n) { return (n + kScanTile - 1) / kScanTile; }
@@ -71,60 +75,55 @@ __device__ __forceinline__ uint64_t scan_look_back(unsigned long long* state, ui
 // Up to two scans of one kind (blockIdx.y) in one launch.
 template <class Src, class Dst>
 __global__ void __launch_bounds__(kScanBlock) k_scan(ScanJob<Src, Dst> a, ScanJob<Src, Dst> b, uint32_t* err) {
-    __shared__ uint64_t sm[kScanBlock / 32 + 1];
+    constexpr int kWarps = kScanBlock / 32;
+    __shared__ uint32_t s_warp[kWarps];
     __shared__ uint64_t s_tile, s_before;
     const ScanJob<Src, Dst> j = blockIdx.y ? b : a;
-    const uint64_t nb = (j.n + kScanTile - 1) / kScanTile;
+    const uint64_t n = j.lim && *j.lim < j.n ? *j.lim : j.n;
+    const uint64_t nb = (n + kScanTile - 1) / kScanTile;
     if (blockIdx.x >= nb) return;
     if (threadIdx.x == 0) s_tile = atomicAdd(j.state, 1ull);
     __syncthreads();
     const uint64_t tile = s_tile;
-    // Each thread owns kScanItems consecutive items so the scan order is the
-    // item order.
-    const uint64_t first = tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-    uint64_t v[kScanItems], local = 0;
+    const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
+    // A warp owns 32 x kScanItems consecutive items, lane l of step k the
+    // item 32 k + l, so loads and stores are coalesced; the prefixes of a
+    // step come from a warp scan.  (kScanItems consecutive items a thread
+    // made every store of a warp touch 32 sectors.)
+    const uint64_t first = tile * kScanTile + wib * (32 * kScanItems) + lane;
+    uint32_t v[kScanItems], e[kScanItems], run = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        const uint64_t i = first + k;
-        v[k] = i < j.n ? j.src(i) : 0;
-        local += v[k];
+        const uint64_t i = first + 32 * k;
+        v[k] = i < n ? (uint32_t)j.src(i) : 0u;
     }
-    uint64_t sum;
-    uint64_t e = block_excl_scan<kScanBlock>(local, sm, &sum);
-    if (threadIdx.x < 32) {
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        const uint32_t inc = warp_incl_scan(v[k]);
+        e[k] = run + inc - v[k];
+        run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) s_warp[wib] = run;
+    __syncthreads();
+    if (wib == 0) {
+        const uint32_t t = lane < kWarps ? s_warp[lane] : 0u;
+        const uint32_t inc = warp_incl_scan(t);
+        const uint64_t sum = __shfl_sync(0xffffffffu, inc, kWarps - 1);
+        if (lane < kWarps) s_warp[lane] = inc - t;
         const uint64_t before = scan_look_back(j.state, tile, sum, err);
-        if (threadIdx.x == 0) {
+        if (lane == 0) {
             s_before = before;
             if (tile == nb - 1 && j.total) *j.total = before + sum;
         }
     }
     __syncthreads();
-    e += s_before;
+    const uint64_t at = s_before + s_warp[wib];
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        const uint64_t i = first + k;
-        if (i < j.n) j.dst(i, e, v[k]);
-        e += v[k];
+        const uint64_t i = first + 32 * k;
+        if (i < n) j.dst(i, at + e[k], v[k]);
     }
 }
-
-// A scan whose length is only known on the device: items at or past *lim
-// count as 0 and are neither read nor written (the launch still covers the
-// host's upper bound n, and blocks past the limit do no memory traffic).
-template <class Src>
-struct BoundSrc {
-    Src s;
-    const unsigned long long* lim;
-    __device__ uint64_t operator()(uint64_t i) const { return i < *lim ? s(i) : 0u; }
-};
-template <class Dst>
-struct BoundDst {
-    Dst d;
-    const unsigned long long* lim;
-    __device__ void operator()(uint64_t i, uint64_t e, uint64_t v) const {
-        if (i < *lim) d(i, e, v);
-    }
-};
 
 // Host launches; the states are zeroed by the caller.  An empty scan launches
 // nothing and leaves *total as it is (zeroed with the rest).
