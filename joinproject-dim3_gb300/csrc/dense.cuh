@@ -34,6 +34,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "expand.cuh"
 
 namespace dim3g {
 
@@ -125,7 +126,7 @@ static __global__ void k_dense_fill_a(const uint32_t* __restrict__ JR_R, const u
 
 // B[z][h] = 1 for every S entry (z, hy[h]); blockIdx.y = column h, the
 // x blocks split its S row.
-static __global__ void k_dense_fill_b(const uint32_t* __restrict__ JR_S, const uint32_t* __restrict__ IC_S, uint32_t T,
+static __global__ void k_dense_fill_b(const uint32_t* __restrict__ JR_S, ZIds IC_S, uint32_t T,
                                       const uint32_t* __restrict__ hy, uint8_t* __restrict__ B, uint32_t Kp) {
     const uint32_t h = blockIdx.y, y = hy[h];
     const uint32_t e1 = JR_S[(unsigned long long)(y + 1) * T];
@@ -151,7 +152,7 @@ static __global__ void k_dense_cnt_a(const uint32_t* __restrict__ JR_R, const ui
         }
     }
 }
-static __global__ void k_dense_cnt_b(const uint32_t* __restrict__ JR_S, const uint32_t* __restrict__ IC_S, uint32_t T,
+static __global__ void k_dense_cnt_b(const uint32_t* __restrict__ JR_S, ZIds IC_S, uint32_t T,
                                      const uint32_t* __restrict__ hy, uint32_t* __restrict__ B32, uint32_t Kp) {
     const uint32_t h = blockIdx.y, y = hy[h];
     const uint32_t e1 = JR_S[(unsigned long long)(y + 1) * T];
@@ -646,7 +647,7 @@ struct LightScatter {  // summaries: candidates into their tile's bucket
 
 template <class V>
 static __global__ void k_dense_light(const uint32_t* __restrict__ JR_R, const uint32_t* __restrict__ IC_R,
-                                     const uint32_t* __restrict__ JR_S, const uint32_t* __restrict__ IC_S, uint32_t T,
+                                     const uint32_t* __restrict__ JR_S, ZIds IC_S, uint32_t T,
                                      const uint32_t* __restrict__ rows, uint32_t nd, const int32_t* __restrict__ hid,
                                      V visit) {
     const uint32_t lane = threadIdx.x & 31;

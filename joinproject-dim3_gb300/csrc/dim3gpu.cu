@@ -345,6 +345,7 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
     if (mode == 0 || (jp.aggregate && !jp.sum.tiles)) return DIM3G_OK;
     const int kind = !jp.sum.tiles ? kDenseBits : (jp.aggregate ? kDenseSumCount : kDenseSumProject);
     const bool bits = kind == kDenseBits;
+    const ZIds zids = rc.IC_S ? ZIds{rc.IC_S, 1} : ZIds{(const uint32_t*)rc.ISV, 2};
     cudaStream_t st = c->stream;
     const int sm = c->sm_count;
     CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
@@ -463,7 +464,7 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
         CU(cudaMemsetAsync(B, 0, Np * Kp, st));
         k_dense_fill_a<<<grid_for(nd * 32, sm), 256, 0, st>>>(rc.JR_R, rc.IC_R, list_m, (uint32_t)nd, hid, A, Kp);
         CHECK_LAUNCH();
-        k_dense_fill_b<<<dim3(16, (unsigned)best_k), 256, 0, st>>>(rc.JR_S, rc.IC_S, rc.T, hy, B, Kp);
+        k_dense_fill_b<<<dim3(16, (unsigned)best_k), 256, 0, st>>>(rc.JR_S, zids, rc.T, hy, B, Kp);
         CHECK_LAUNCH();
     } else {
         // multiplicities, then e4m3 codes (a multiplicity above 16 keeps the
@@ -483,13 +484,13 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
         CU(cudaMemsetAsync(tcnt, 0, (ntile + 1) * 4, st));
         k_dense_cnt_a<<<grid_for(nd * 32, sm), 256, 0, st>>>(rc.JR_R, rc.IC_R, list_m, (uint32_t)nd, hid, A32, Kp);
         CHECK_LAUNCH();
-        k_dense_cnt_b<<<dim3(16, (unsigned)best_k), 256, 0, st>>>(rc.JR_S, rc.IC_S, rc.T, hy, B32, Kp);
+        k_dense_cnt_b<<<dim3(16, (unsigned)best_k), 256, 0, st>>>(rc.JR_S, zids, rc.T, hy, B32, Kp);
         CHECK_LAUNCH();
         k_dense_to_fp8<<<grid_for(Mp * Kp, sm), 256, 0, st>>>(A32, A, Mp * Kp, flag);
         CHECK_LAUNCH();
         k_dense_to_fp8<<<grid_for(Np * Kp, sm), 256, 0, st>>>(B32, B, Np * Kp, flag);
         CHECK_LAUNCH();
-        k_dense_light<<<grid_for(nd * 32, sm), 256, 0, st>>>(rc.JR_R, rc.IC_R, rc.JR_S, rc.IC_S, rc.T, list_m,
+        k_dense_light<<<grid_for(nd * 32, sm), 256, 0, st>>>(rc.JR_R, rc.IC_R, rc.JR_S, zids, rc.T, list_m,
                                                              (uint32_t)nd, hid, LightCount{tcnt, nt});
         CHECK_LAUNCH();
         k_dense_maxcnt<<<grid_for(ntile, sm), 256, 0, st>>>(tcnt, ntile, flag + 1);
@@ -506,7 +507,7 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
         if (hflag[0] || hflag[1] > kDenseBucketMax || hl >= 0xFFFFFFFFull) return DIM3G_OK;
         uint16_t* lb = ws_get<uint16_t>(c, hl + 1);
         if (!lb) return fail(c, DIM3G_ERR_NOMEM, "workspace allocation failed (dense light buckets)");
-        k_dense_light<<<grid_for(nd * 32, sm), 256, 0, st>>>(rc.JR_R, rc.IC_R, rc.JR_S, rc.IC_S, rc.T, list_m,
+        k_dense_light<<<grid_for(nd * 32, sm), 256, 0, st>>>(rc.JR_R, rc.IC_R, rc.JR_S, zids, rc.T, list_m,
                                                              (uint32_t)nd, hid, LightScatter{tcur, lb, nt});
         CHECK_LAUNCH();
         ds = DenseSum{list_m, (uint32_t)nd, rc.id2x, rc.id2z, toff, lb, jp.sum};
@@ -532,7 +533,7 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
     uint32_t cpr = 0;
     unsigned long long* coff = nullptr;
     if (bits) {
-        k_dense_light<<<grid_for(nd * 32, sm), 256, 0, st>>>(rc.JR_R, rc.IC_R, rc.JR_S, rc.IC_S, rc.T, list_m,
+        k_dense_light<<<grid_for(nd * 32, sm), 256, 0, st>>>(rc.JR_R, rc.IC_R, rc.JR_S, zids, rc.T, list_m,
                                                              (uint32_t)nd, hid, LightOr{D, (uint32_t)Wd});
         CHECK_LAUNCH();
         // chunk popcounts and their offsets
@@ -703,18 +704,22 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     uint32_t* IC_R = ws_get<uint32_t>(c, jp.nP);
     uint32_t* cur_yt = ws_get<uint32_t>(c, k1);
     uint32_t* JR_S = ws_get<uint32_t>(c, k1);
-    uint32_t* IC_S = ws_get<uint32_t>(c, nq);
+    // S's entries: the single pass reads (z id, z value) pairs, COUNT and the
+    // count pass ids, ordered output and the join-project summaries both
+    const bool single = jp.single_pass && !jp.aggregate && !jp.count_only;
+    const bool want_ids = !single, want_pairs = !jp.aggregate && !jp.count_only;
+    uint32_t* IC_S = want_ids ? ws_get<uint32_t>(c, nq) : nullptr;
     uint32_t* VS = nullptr;  // the value paths read the pairs in ISV
     // +2: the streamed bitmap rows copy 16-byte-aligned supersets of S
     // segments, up to one pair past the last one
-    uint2* ISV = ws_get<uint2>(c, nq + 2);
+    uint2* ISV = want_pairs ? ws_get<uint2>(c, nq + 2) : nullptr;
     uint32_t* Zq = ws_get<uint32_t>(c, nq);
     uint32_t* ucap = ws_get<uint32_t>(c, n);
     uint8_t* bucket = ws_get<uint8_t>(c, n);
     uint32_t* lists = ws_get<uint32_t>(c, (uint64_t)4 * n);
     unsigned long long* off = ws_get<unsigned long long>(c, n1);
     unsigned long long* bsum2 = ws_get<unsigned long long>(c, sR);
-    if (!degx || !curx || !JR_R || !IC_R || !cur_yt || !JR_S || !IC_S || !ISV || !Zq || !ucap || !bucket || !lists ||
+    if (!degx || !curx || !JR_R || !IC_R || !cur_yt || !JR_S || (want_ids && !IC_S) || (want_pairs && !ISV) || !Zq || !ucap || !bucket || !lists ||
         !off || !bsum2)
         return fail(c, DIM3G_ERR_NOMEM, "workspace allocation failed (CSR)");
     uint32_t* cnt = degx + n1;  // cnt[n] = 0 closes the offsets scan
@@ -755,7 +760,6 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     rc.err = &sc->err;
     // tiny rows get their own warp launch, and the block class is split by
     // hash-set size (2^lg slots for 2u keys), in the single pass only
-    const bool single = jp.single_pass && !jp.aggregate && !jp.count_only;
     const bool block_split = single && !jp.sum.tiles && c->prm.block_split &&
                              !(c->prm.prefetch_rows && c->prm.cta_rr == 3);
     const RowBuckets rb{1u << (c->prm.warp_lg - 1), 1u << (c->prm.block_lg - 1), single, block_split,

@@ -77,6 +77,14 @@ struct RowCtx {
     uint32_t* next_row;    // dynamic row counters of the CTA classes
 };
 
+// The z ids of S's entries, from the id array or from the (z id, z value)
+// pairs (step 2).
+struct ZIds {
+    const uint32_t* a;
+    uint32_t step;
+    __device__ __forceinline__ uint32_t operator[](uint64_t j) const { return __ldg(&a[j * step]); }
+};
+
 __device__ __forceinline__ uint32_t ceil_log2(uint32_t v) { return v <= 1 ? 0 : 32 - __clz(v - 1); }
 
 // Insert z into an open-addressing set of 2^lg 32-bit slots in shared memory.
