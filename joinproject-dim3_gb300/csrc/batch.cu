@@ -612,10 +612,9 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
             k_b_single_warp<<<resident(k_b_single_warp, 32 * wps, ss_w, sm), 32 * wps, ss_w, st>>>(
                 Q, BatchRows{lw, &n[1], nullptr, nullptr}, tu.warp_lg, kStage);
             BLAUNCH();
-            const uint32_t wpt = warps_for(warp_row_words(kTinyLg, kTinyStage) * 4);
-            const size_t ss_t = (size_t)wpt * warp_row_words(kTinyLg, kTinyStage) * 4;
-            k_b_single_warp<<<resident(k_b_single_warp, 32 * wpt, ss_t, sm), 32 * wpt, ss_t, st>>>(
-                Q, BatchRows{lt, &n[5], nullptr, nullptr}, kTinyLg, kTinyStage);
+            const size_t ss_t = 8 * kPackWords * 4;
+            k_b_single_pack<<<resident(k_b_single_pack, 256, ss_t, sm), 256, ss_t, st>>>(
+                Q, BatchRows{lt, &n[5], nullptr, nullptr});
             BLAUNCH();
         } else {
             const unsigned g_t = (unsigned)(2 * sm);
@@ -631,10 +630,11 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
             k_b_agg_warp<<<resident(k_b_agg_warp, 32 * wpa, ss_w, sm), 32 * wpa, ss_w, st>>>(
                 Q, BatchRows{lw, &n[1], nullptr, nullptr}, tu.warp_lg, kStage);
             BLAUNCH();
-            const uint32_t wpt = warps_for(agg_warp_words(kTinyLg, kTinyStage) * 4);
-            const size_t ss_t = (size_t)wpt * agg_warp_words(kTinyLg, kTinyStage) * 4;
+            constexpr uint32_t tiny_lg = 9, tiny_stage = 256;
+            const uint32_t wpt = warps_for(agg_warp_words(tiny_lg, tiny_stage) * 4);
+            const size_t ss_t = (size_t)wpt * agg_warp_words(tiny_lg, tiny_stage) * 4;
             k_b_agg_warp<<<resident(k_b_agg_warp, 32 * wpt, ss_t, sm), 32 * wpt, ss_t, st>>>(
-                Q, BatchRows{lt, &n[5], nullptr, nullptr}, kTinyLg, kTinyStage);
+                Q, BatchRows{lt, &n[5], nullptr, nullptr}, tiny_lg, tiny_stage);
             BLAUNCH();
         }
     }
@@ -651,6 +651,7 @@ int set_batch_attributes(dim3g_ctx* ctx) {
     BCU(cudaFuncSetAttribute(k_b_single_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, bm));
     BCU(cudaFuncSetAttribute(k_b_single_block, cudaFuncAttributeMaxDynamicSharedMemorySize, blk));
     BCU(cudaFuncSetAttribute(k_b_single_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    BCU(cudaFuncSetAttribute(k_b_single_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * kPackWords * 4)));
     BCU(cudaFuncSetAttribute(k_b_agg_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 << 14 << 2));
     BCU(cudaFuncSetAttribute(k_b_agg_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     return DIM3G_OK;

@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include "expand.cuh"
 #include "mapping.cuh"
+#include "packed.cuh"
 #include "single.cuh"
 
 namespace dim3g {
@@ -703,6 +704,47 @@ static __global__ void __launch_bounds__(256) k_b_single_warp(QueryPools Q, Batc
             cur_q = qi;
         }
         single_warp_row(s_c[wib], x, tab, sink, warp_lg);
+    }
+    sink.flush();
+}
+
+// Tiny rows: packs of rows of one query (packed.cuh), at most 8 warps a CTA
+// with a context slot each.  A pack ends where the list goes on to another
+// query.
+static __global__ void __launch_bounds__(256, 4) k_b_single_pack(QueryPools Q, BatchRows L) {
+    extern __shared__ uint32_t smem[];
+    __shared__ RowCtx s_c[8];
+    const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
+    uint32_t* tab = smem + (size_t)wib * kPackWords;
+    PackSink sink{reinterpret_cast<uint2*>(tab + (1u << kPackLg)), nullptr, Reserve{nullptr, 0}};
+    uint32_t cur_q = 0xFFFFFFFFu;
+    const uint32_t nrows = (uint32_t)*L.n_a, warps = gridDim.x * nw;
+    uint32_t take = (nrows + warps - 1) / warps;
+    take = take > 32 ? 32 : take;
+    for (uint64_t r0 = (uint64_t)(blockIdx.x * nw + wib) * take; r0 < nrows; r0 += (uint64_t)warps * take) {
+        const uint32_t n = (uint32_t)min((uint64_t)take, nrows - r0);
+        const uint32_t g = lane < n ? L.list[r0 + lane] : 0xFFFFFFFFu;
+        for (uint32_t lo = 0; lo < n;) {
+            const uint32_t g0 = __shfl_sync(0xffffffffu, g, lo);
+            const uint32_t qi = cur_q != 0xFFFFFFFFu && g0 >= (uint32_t)Q.qrow_off[cur_q] &&
+                                        g0 < (uint32_t)Q.qrow_off[cur_q + 1]
+                                    ? cur_q
+                                    : seg_find(Q.qrow_off, Q.nq, g0);
+            const uint32_t q_lo = (uint32_t)Q.qrow_off[qi], q_hi = (uint32_t)Q.qrow_off[qi + 1];
+            const uint32_t other = __ballot_sync(0xffffffffu, lane >= lo && lane < n && (g < q_lo || g >= q_hi));
+            const uint32_t hi = other ? __ffs(other) - 1 : n;
+            if (qi != cur_q) {
+                sink.flush();
+                __syncwarp();
+                if (lane == 0) s_c[wib] = Q.rc[qi];
+                __syncwarp();
+                sink.rs = Q.rs[qi];
+                sink.out = s_c[wib].out;
+                cur_q = qi;
+            }
+            pack_rows(s_c[wib], lane >= lo && lane < hi ? g - q_lo : 0u, lo, hi, tab, sink);
+            lo = hi;
+        }
     }
     sink.flush();
 }

@@ -32,6 +32,7 @@
 #include "scan.cuh"
 #include "single.cuh"
 #include "stream.cuh"
+#include "packed.cuh"
 #include "prefetch.cuh"
 
 using namespace dim3g;
@@ -848,8 +849,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         const size_t ss_b = smem_b + (size_t)(blk_b / 32) * kStage * 4;
         const uint32_t wps = warps_per_cta(warp_row_words(c->prm.warp_lg, kStage) * 4);
         const size_t ss_w = (size_t)wps * warp_row_words(c->prm.warp_lg, kStage) * 4;
-        const uint32_t wpt = warps_per_cta(warp_row_words(kTinyLg, kTinyStage) * 4);
-        const size_t ss_t = (size_t)wpt * warp_row_words(kTinyLg, kTinyStage) * 4;
+        const size_t ss_t = 8 * kPackWords * 4;
         if (dp.on) {
             k_dense_reserve<<<1, 1, 0, st>>>(dp.coff + (uint64_t)dp.nd * dp.cpr, &sc->cursor, cap, &sc->dense_base);
             CHECK_LAUNCH();
@@ -918,8 +918,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
             CHECK_LAUNCH();
         }
         if (has_t) {
-            k_single_warp<<<resident_grid(k_single_warp, 32 * wpt, ss_t, sm), 32 * wpt, ss_t, st>>>(
-                rc, rs, list_t, &sc->nrows[5], kTinyLg, kTinyStage);
+            k_single_pack<<<resident_grid(k_single_pack, 256, ss_t, sm), 256, ss_t, st>>>(rc, rs, list_t, &sc->nrows[5]);
             CHECK_LAUNCH();
         }
         CU(cudaEventRecord(c->evc[7], st));
@@ -1267,6 +1266,8 @@ int dim3g_create(int device, dim3g_ctx** out) {
               cudaFuncSetAttribute(k_rows_bitmap<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_m) == cudaSuccess &&
               cudaFuncSetAttribute(k_rows_bitmap<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_m) == cudaSuccess &&
               cudaFuncSetAttribute(k_single_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_wmax) == cudaSuccess &&
+              cudaFuncSetAttribute(k_single_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * kPackWords * 4)) ==
+                  cudaSuccess &&
               cudaFuncSetAttribute(k_single_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    ((1 << 14) + 32 * (int)kStage) * 4) == cudaSuccess &&
               cudaFuncSetAttribute(k_single_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize,

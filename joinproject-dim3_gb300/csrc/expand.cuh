@@ -22,10 +22,9 @@ namespace dim3g {
 constexpr uint32_t kEmpty32 = 0xFFFFFFFFu;
 constexpr uint32_t kHugeRow = 1u << 16;
 constexpr uint32_t kWarpWorkMax = 1u << 14;  // candidates a single warp takes alone
-// Tiny rows (few distinct z, few candidates) run in the warp kernel with a
-// 2^kTinyLg-slot table and a kTinyStage-pair stage: about 3 KB of shared
-// memory per warp, so the latency-bound row walk runs at full occupancy.
-constexpr uint32_t kTinyU = 128, kTinyW = 4096, kTinyLg = 8, kTinyStage = 256;
+// Tiny rows (few distinct z, few candidates) are expanded many to a warp
+// (packed.cuh).
+constexpr uint32_t kTinyU = 256, kTinyW = 4096;
 
 // A hash-class row dedups with a bitmap over the whole z domain instead of
 // a hash set when that bitmap fits the kernel's table memory (2^slots_lg
