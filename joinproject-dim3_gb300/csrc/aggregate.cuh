@@ -1,25 +1,34 @@
-// aggregate.cuh -- COUNT(*) GROUP BY (x, z): the write pass of the
-// join-aggregate (SpmmAggregate with a COUNT plug-in, dim3.hpp:1271-1310).
+// aggregate.cuh -- COUNT(*) GROUP BY (x, z) (SpmmAggregate with a COUNT
+// plug-in, dim3.hpp:1271-1310).
 //
-// The count pass is the join-project count pass (distinct z per row).  The
-// write pass expands each row again with a per-z counter -- a shared-memory
-// hash map (z -> count) for classes 1 and 2, a shared-memory counter array
-// over one z tile for classes 3/4 -- and then emits every (x, z, count) of
-// the row at off[x] + a row-local slot.  Counts are exact: each expansion
-// candidate is one joining (R tuple, S tuple) pair.
+// Each row is expanded with a counter per distinct z and then emits every
+// (x, z, count).  Counts are exact: each expansion candidate is one joining
+// (R tuple, S tuple) pair.  Row forms:
+//   tiny rows    packs of rows to a warp (packed.cuh), a shared map row, z ->
+//                count, groups staged across packs
+//   map rows     one CTA a row, a shared map z -> count (or a counter per z
+//                where the domain is small), CTA width and map by row size
+//   ranked rows  one CTA a row and z tile: a bitmap of the z that occur, their
+//                ranks by popcount, then a counter per rank -- two passes over
+//                the candidates, memory by the distinct z and not the domain
+// The groups go to a reserved range of a global cursor (rows in any order), or,
+// for ordered output and callers that size the output first, to the row's
+// exact offset from a count pass.
 #pragma once
 #include "common.cuh"
 #include "expand.cuh"
+#include "packed.cuh"
+#include "single.cuh"
 
 namespace dim3g {
 
 struct AggOut {
     unsigned long long* cnt;  // one count per output pair
     SumAcc sum;               // sum.tiles set: summaries instead of output
+    Reserve rs;               // cursor and capacity (cursor null: rows at c.off)
 };
 
-// Summary emission: per-lane sums over the occupied map slots [s0, s1)
-// (stride 32) or over the nonzero direct counters.
+// Per-lane sums of a summary.
 struct GroupSums {
     unsigned long long g = 0, cs = 0, h = 0;
     __device__ __forceinline__ void add(uint32_t xv, uint32_t zv, uint32_t cnt) {
@@ -28,20 +37,6 @@ struct GroupSums {
         h += group_hash(xv, zv, cnt);
     }
 };
-__device__ __forceinline__ void sum_map_slots(const RowCtx& c, const uint32_t* keys, const uint32_t* vals,
-                                              uint32_t s0, uint32_t s1, uint32_t xv, GroupSums& gs) {
-    for (uint32_t s = s0 + lane_id(); s < s1; s += 32) {
-        const uint32_t key = keys[s];
-        if (key != kEmpty32) gs.add(xv, __ldg(&c.id2z[key]), vals[s]);
-    }
-}
-__device__ __forceinline__ void sum_counters(const RowCtx& c, const uint32_t* ctr, uint32_t s0, uint32_t s1,
-                                             uint32_t lo, uint32_t xv, GroupSums& gs) {
-    for (uint32_t s = s0 + lane_id(); s < s1; s += 32) {
-        const uint32_t v = ctr[s];
-        if (v) gs.add(xv, __ldg(&c.id2z[lo + s]), v);
-    }
-}
 
 // Shared-memory map slot of z (inserting it if absent).
 __device__ __forceinline__ uint32_t smem_map_slot(uint32_t* keys, uint32_t lg, uint32_t z, uint32_t* err) {
@@ -61,7 +56,7 @@ __device__ __forceinline__ uint32_t smem_map_slot(uint32_t* keys, uint32_t lg, u
     return 0xFFFFFFFFu;
 }
 
-// Counting "sets" for warp_expand: they count every candidate and report no
+// Counting "sets" for the expansion: they take every candidate and report no
 // first insertions (emission happens after the expansion).
 struct CountMap {
     uint32_t* keys;
@@ -84,242 +79,432 @@ struct CountTile {
         return false;
     }
 };
+struct MarkTile {  // ranked rows, first pass
+    uint32_t* bm;
+    uint32_t lo;
+    __device__ __forceinline__ bool insert(uint32_t z, bool act) {
+        const uint32_t zl = z - lo;
+        if (act) atomicOr(&bm[zl >> 5], 1u << (zl & 31));
+        return false;
+    }
+};
+// Ranked rows, second pass: rank of z = set bits below it.  A warp's words
+// start at wbase[w >> wsh]; pre[w] counts the bits of the warp's earlier
+// words.
+struct RankedTile {
+    const uint32_t* bm;
+    const uint16_t* pre;
+    const uint32_t* wbase;
+    uint32_t wsh;
+    __device__ __forceinline__ uint32_t rank(uint32_t zl) const {
+        const uint32_t w = zl >> 5;
+        return wbase[w >> wsh] + pre[w] + __popc(bm[w] & ((1u << (zl & 31)) - 1u));
+    }
+};
+struct CountRanked {
+    RankedTile t;
+    uint32_t lo, r0, n;  // counters of ranks [r0, r0 + n)
+    uint32_t* ctr;
+    uint32_t* zl;  // the ranks' z: written by the candidate that finds a zero count
+    __device__ __forceinline__ bool insert(uint32_t z, bool act) {
+        if (act) {
+            const uint32_t r = t.rank(z - lo) - r0;
+            if (r < n && atomicAdd(&ctr[r], 1u) == 0) zl[r] = z;
+        }
+        return false;
+    }
+};
 struct NullSink {
     static constexpr bool kValues = false;
     template <uint32_t N>
     __device__ __forceinline__ void take(const uint32_t (&)[N], const uint32_t (&)[N]) {}
+    template <uint32_t N>
+    __device__ __forceinline__ void take(const uint32_t (&)[N], const uint32_t (&)[N], const uint32_t (&)[N]) {}
 };
 
-// Warp-collective emission of occupied map slots [s0, s1) with stride 32.
-// shared_pos: CTA-wide row-local slot counter; nullptr for a warp-owned row
-// (then *local_pos is the running slot).
-__device__ __forceinline__ void emit_map_slots_warp(const RowCtx& c, AggOut ao, const uint32_t* keys,
-                                                    const uint32_t* vals, uint32_t s0, uint32_t s1, uint32_t xv,
-                                                    unsigned long long base, uint32_t lim, uint32_t* shared_pos,
-                                                    uint32_t* local_pos) {
-    const uint32_t lane = lane_id();
-    for (uint32_t sb = s0; sb < s1; sb += 32) {
-        uint32_t s = sb + lane;
-        uint32_t key = (s < s1) ? keys[s] : kEmpty32;
-        bool occ = key != kEmpty32;
-        uint32_t b = __ballot_sync(0xffffffffu, occ);
-        if (!b) continue;
-        uint32_t pb;
-        if (shared_pos) {
-            pb = 0;
-            if (lane == 0) pb = atomicAdd(shared_pos, (uint32_t)__popc(b));
-            pb = __shfl_sync(0xffffffffu, pb, 0);
-        } else {
-            pb = *local_pos;
-            *local_pos += __popc(b);
-        }
-        if (occ) {
-            uint32_t pos = pb + __popc(b & lanemask_lt());
-            if (pos < lim) {
-                c.out[base + pos] = make_uint2(xv, __ldg(&c.id2z[key]));
-                ao.cnt[base + pos] = vals[s];
-            } else {
-                raise_error(c.err, kErrOutputBound);
-            }
-        }
-    }
-}
-
 // A map-class row counts with one counter per z of the whole domain instead
-// of a z -> count hash map when the m counters fit the kernel's map memory
-// (2^words_lg words) and scanning them costs little against the row's
-// candidates (m <= 8 u).
+// of a z -> count hash map when the m counters fit the map memory (2^words_lg
+// words) and scanning them costs little against the row's candidates
+// (m <= 8 u).
 __device__ __forceinline__ bool use_row_counters(uint32_t m, uint32_t u, uint32_t words_lg) {
     return (uint64_t)m <= (1ull << words_lg) && (uint64_t)m <= 8ull * u;
 }
 
-// Warp-collective emission of the nonzero direct counters ctr[s0, s1): the
-// counter index is the z id.  shared_pos / local_pos as above.
-__device__ __forceinline__ void emit_counters_warp(const RowCtx& c, AggOut ao, const uint32_t* ctr, uint32_t s0,
-                                                   uint32_t s1, uint32_t xv, unsigned long long base, uint32_t lim,
-                                                   uint32_t* shared_pos, uint32_t* local_pos) {
-    const uint32_t lane = lane_id();
-    for (uint32_t sb = s0; sb < s1; sb += 32) {
-        const uint32_t s = sb + lane;
-        const uint32_t v = (s < s1) ? ctr[s] : 0u;
-        const uint32_t b = __ballot_sync(0xffffffffu, v != 0);
-        if (!b) continue;
-        uint32_t pb;
-        if (shared_pos) {
-            pb = 0;
-            if (lane == 0) pb = atomicAdd(shared_pos, (uint32_t)__popc(b));
-            pb = __shfl_sync(0xffffffffu, pb, 0);
+// Where n groups of row x go (warp-uniform; ~0: nowhere).  Cursor: a
+// reservation ending past the capacity writes nothing.  Offsets: the row's
+// next n places (*s_pos counts them), checked against its count.
+__device__ __forceinline__ unsigned long long group_place(const RowCtx& c, const AggOut& ao, uint32_t x, uint32_t n,
+                                                          uint32_t* s_pos) {
+    unsigned long long base = 0;
+    if (lane_id() == 0) {
+        if (ao.rs.cursor) {
+            base = atomicAdd(ao.rs.cursor, (unsigned long long)n);
+            if (base + n > ao.rs.cap) base = ~0ull;
         } else {
-            pb = *local_pos;
-            *local_pos += __popc(b);
-        }
-        if (v) {
-            const uint32_t pos = pb + __popc(b & lanemask_lt());
-            if (pos < lim) {
-                c.out[base + pos] = make_uint2(xv, __ldg(&c.id2z[s]));
-                ao.cnt[base + pos] = v;
-            } else {
+            const uint32_t p = atomicAdd(s_pos, n);
+            base = c.off[x] + p;
+            if (p + n > c.cnt[x]) {
                 raise_error(c.err, kErrOutputBound);
+                base = ~0ull;
             }
+        }
+    }
+    return __shfl_sync(0xffffffffu, base, 0);
+}
+
+// ------------------------------------------------------------- map rows
+// The whole CTA: row x through a map of 2^lg keys and counts at smem.  Called
+// after a barrier that follows the previous row; *s_pos is 0 by the first
+// barrier in here.
+__device__ __forceinline__ void agg_map_row(const RowCtx& c, const AggOut& ao, uint32_t x, uint32_t* smem, uint32_t lg,
+                                            CtaChunks* cc, uint32_t* s_pos) {
+    const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
+    const uint32_t u = c.ucap[x], e0 = c.JR_R[x], e1 = c.JR_R[x + 1], ne = e1 - e0;
+    const bool direct = use_row_counters(c.m, u, lg + 1);
+    uint32_t rl = ceil_log2(2 * u);
+    rl = rl < 5 ? 5 : (rl > lg ? lg : rl);
+    uint32_t* keys = smem;
+    uint32_t* vals = direct ? smem : smem + (1u << rl);
+    const uint32_t span = direct ? c.m : 1u << rl;
+    uint4* t4 = reinterpret_cast<uint4*>(smem);
+    if (direct) {
+        for (uint32_t s = threadIdx.x; s < (span + 3) / 4; s += blockDim.x) t4[s] = make_uint4(0, 0, 0, 0);
+    } else {
+        for (uint32_t s = threadIdx.x; s < span / 4; s += blockDim.x) {
+            t4[s] = make_uint4(kEmpty32, kEmpty32, kEmpty32, kEmpty32);
+            t4[s + span / 4] = make_uint4(0, 0, 0, 0);
+        }
+    }
+    if (threadIdx.x == 0) *s_pos = 0;
+    const uint64_t pol = l2_keep_policy();
+    const bool staged = ne <= kRowBlk;
+    if (staged) balanced_stage(c, e0, ne, 0, c.T, cc, pol, wib, nw);
+    __syncthreads();
+    NullSink sink;
+    CountTile ct{smem, 0};
+    CountMap cm{keys, vals, rl, c.err};
+    if (staged) {
+        if (direct) balanced_expand(c, ne, ct, sink, cc->st.seg.s0, cc->st.seg.incl, cc->ctot, pol, wib, nw);
+        else balanced_expand(c, ne, cm, sink, cc->st.seg.s0, cc->st.seg.incl, cc->ctot, pol, wib, nw);
+    } else {
+        if (direct) cta_expand_balanced(c, e0, e1, 0, c.T, ct, sink, cc);
+        else cta_expand_balanced(c, e0, e1, 0, c.T, cm, sink, cc);
+    }
+    __syncthreads();
+    // the warps' equal parts of the map, whole groups of 32 slots
+    const uint32_t per = (((span + nw - 1) / nw) + 31) & ~31u;
+    const uint32_t s0 = min(span, wib * per), s1 = min(span, s0 + per);
+    const uint32_t xv = c.id2x[x];
+    if (ao.sum.tiles) {
+        GroupSums gs;
+        for (uint32_t s = s0 + lane; s < s1; s += 32) {
+            const uint32_t v = vals[s];
+            if (v) gs.add(xv, __ldg(&c.id2z[direct ? s : keys[s]]), v);
+        }
+        ao.sum.commit(xv, gs.g, gs.cs, gs.h);
+        return;
+    }
+    uint32_t n = 0;
+    for (uint32_t s = s0 + lane; s < s1; s += 32) n += vals[s] != 0;
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (n == 0) return;
+    unsigned long long base = group_place(c, ao, x, n, s_pos);
+    if (base == ~0ull) return;
+    for (uint32_t sb = s0; sb < s1; sb += 128) {  // four id gathers in flight
+        uint32_t v[4], z[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            const uint32_t s = sb + k * 32 + lane;
+            v[k] = s < s1 ? vals[s] : 0u;
+            z[k] = v[k] ? __ldg(&c.id2z[direct ? s : keys[s]]) : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            const uint32_t b = __ballot_sync(0xffffffffu, v[k] != 0);
+            if (v[k]) {
+                const unsigned long long pos = base + __popc(b & lanemask_lt());
+                st_stream(&c.out[pos], make_uint2(xv, z[k]));
+                __stcs(&ao.cnt[pos], (unsigned long long)v[k]);
+            }
+            base += __popc(b);
         }
     }
 }
 
-// Class 1 write pass: one warp per row; per warp 2^lg keys + 2^lg counts.
-static __global__ void __launch_bounds__(256) k_agg_warp(RowCtx c, AggOut ao, const uint32_t* __restrict__ rows,
-                                                  const unsigned long long* __restrict__ nrows_p, uint32_t warp_lg) {
-    extern __shared__ uint32_t smem[];
+// ---------------------------------------------------------- ranked rows
+// Shared memory of a ranked row: the tile's bitmap words (padded to the
+// warps' word ranges), a 16-bit prefix a word, then as many (counter, z)
+// pairs as fit.
+struct RankLayout {
+    uint32_t wsh;    // words a warp ranks (log2, at least 7)
+    uint32_t words;  // bitmap words, a multiple of the warps' ranges
+    uint32_t cap;    // ranks counted at a time
+};
+__host__ __device__ inline RankLayout rank_layout(uint32_t tile_width, uint32_t warps, size_t smem) {
+    RankLayout l;
+    const uint32_t w = (tile_width + 31) / 32, per = (w + warps - 1) / warps;
+    l.wsh = 7;
+    while ((1u << l.wsh) < per) l.wsh++;
+    l.words = ((w + (1u << l.wsh) - 1) >> l.wsh) << l.wsh;
+    l.cap = (uint32_t)((smem - (size_t)l.words * 6) / 8);
+    return l;
+}
+
+// A row (or row and tile) of the ranked class: item number, row, its entries
+// and first value.
+struct RankHead {
+    uint32_t item, x, e0, e1, xv;
+};
+__device__ __forceinline__ RankHead rank_head(const RowCtx& c, uint32_t item, uint32_t x) {
+    return RankHead{item, x, c.JR_R[x], c.JR_R[x + 1], c.id2x[x]};
+}
+
+// The whole CTA: row h.x over tile t.  Groups go to the cursor, or (offsets)
+// to the row's next places.  Called after a barrier that follows the previous
+// row; *s_pos as the caller keeps it for the row.  ahead() runs on thread 0
+// during the first pass (the other warps take its share of the pieces).
+template <class Ahead>
+__device__ __forceinline__ void agg_ranked_tile(const RowCtx& c, const AggOut& ao, const RankHead& h, uint32_t t,
+                                                uint32_t* smem, const RankLayout& l, CtaChunks* cc, uint32_t* s_pos,
+                                                uint32_t* s_wbase, unsigned long long* s_base, Ahead ahead) {
     const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
-    uint32_t* keys = smem + ((size_t)wib << (warp_lg + 1));
-    uint32_t* vals = keys + (1u << warp_lg);
-    const uint32_t nrows = (uint32_t)*nrows_p;
-    for (uint32_t ri = blockIdx.x * nw + wib; ri < nrows; ri += gridDim.x * nw) {
-        const uint32_t x = rows[ri];
-        const uint32_t u = c.ucap[x];
-        const bool sum = ao.sum.tiles != nullptr;
-        NullSink sink;
-        uint32_t pos = 0;
-        if (use_row_counters(c.m, u, warp_lg + 1)) {
-            for (uint32_t s = lane; s < c.m; s += 32) keys[s] = 0;  // keys + vals: one counter array
-            __syncwarp();
-            CountTile set{keys, 0};
-            warp_expand(c, c.JR_R[x], c.JR_R[x + 1], 0, 0, 0, c.T, set, sink);
-            __syncwarp();
-            if (sum) {
-                GroupSums gs;
-                sum_counters(c, keys, 0, c.m, 0, c.id2x[x], gs);
-                ao.sum.commit(c.id2x[x], gs.g, gs.cs, gs.h);
-            } else {
-                emit_counters_warp(c, ao, keys, 0, c.m, c.id2x[x], c.off[x], c.cnt[x], nullptr, &pos);
+    const uint32_t x = h.x, e0 = h.e0, e1 = h.e1, ne = e1 - e0, lo = t * c.tile_width, xv = h.xv;
+    uint32_t* bm = smem;
+    uint16_t* pre = reinterpret_cast<uint16_t*>(smem + l.words);
+    uint32_t* ctr = smem + l.words + l.words / 2;
+    uint32_t* zl = ctr + l.cap;
+    const uint64_t pol = l2_keep_policy();
+    const bool staged = ne <= kRowBlk;
+    NullSink sink;
+    uint4* b4 = reinterpret_cast<uint4*>(bm);
+    for (uint32_t w = threadIdx.x; w < l.words / 4; w += blockDim.x) b4[w] = make_uint4(0, 0, 0, 0);
+    if (staged) balanced_stage(c, e0, ne, t, t + 1, cc, pol, wib, nw);
+    if (threadIdx.x == 0) cc->n = 0;
+    __syncthreads();
+    if (threadIdx.x == 0) ahead();
+    __syncwarp();
+    MarkTile mark{bm, lo};
+    if (staged) balanced_expand(c, ne, mark, sink, cc->st.seg.s0, cc->st.seg.incl, cc->ctot, pol, wib, nw, &cc->n, kDynPiece);
+    else cta_expand_balanced(c, e0, e1, t, t + 1, mark, sink, cc);
+    __syncthreads();
+    // ranks: every warp's words, then the warps' bases
+    const uint32_t w0 = wib << l.wsh, w1 = min(l.words, w0 + (1u << l.wsh));
+    uint32_t run = 0;
+    for (uint32_t w = w0 + 4 * lane; w < w1; w += 128) {  // four words a lane
+        const uint4 b = b4[w >> 2];
+        const uint32_t n0 = __popc(b.x), n1 = n0 + __popc(b.y), n2 = n1 + __popc(b.z), n3 = n2 + __popc(b.w);
+        const uint32_t inc = warp_incl_scan(n3), p = run + inc - n3;
+        *reinterpret_cast<uint2*>(pre + w) = make_uint2(p | (p + n0) << 16, (p + n1) | (p + n2) << 16);
+        run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) s_wbase[wib] = run;
+    if (threadIdx.x == 0) cc->n = 0;
+    __syncthreads();
+    if (wib == 0) {
+        const uint32_t v = lane < nw ? s_wbase[lane] : 0u, inc = warp_incl_scan(v);
+        const uint32_t d = __shfl_sync(0xffffffffu, inc, 31);
+        __syncwarp();
+        s_wbase[lane] = inc - v;
+        if (lane == 0) s_wbase[32] = d;
+    }
+    __syncthreads();
+    const uint32_t d = s_wbase[32];
+    // the reservation's round trip passes while the other warps set up the
+    // window; read after the next barriers
+    if (wib == 0 && d && !ao.sum.tiles) {
+        const unsigned long long base = group_place(c, ao, x, d, s_pos);
+        if (lane == 0) *s_base = base;
+    }
+    GroupSums gs;
+    const RankedTile rt{bm, pre, s_wbase, l.wsh};
+    for (uint32_t r0 = 0; r0 < d; r0 += l.cap) {
+        const uint32_t n = min(l.cap, d - r0);
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) ctr[i] = 0;
+        __syncthreads();
+        CountRanked cr{rt, lo, r0, n, ctr, zl};
+        if (staged) balanced_expand(c, ne, cr, sink, cc->st.seg.s0, cc->st.seg.incl, cc->ctot, pol, wib, nw, &cc->n, kDynPiece);
+        else cta_expand_balanced(c, e0, e1, t, t + 1, cr, sink, cc);
+        __syncthreads();
+        if (ao.sum.tiles) {
+            for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) gs.add(xv, __ldg(&c.id2z[zl[i]]), ctr[i]);
+        } else if (*s_base != ~0ull) {
+            const unsigned long long base = *s_base + r0;
+            for (uint32_t ib = threadIdx.x; ib < n; ib += 4 * blockDim.x) {  // four id gathers in flight
+                uint32_t z[4], v[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++) {
+                    const uint32_t i = ib + k * blockDim.x;
+                    z[k] = i < n ? __ldg(&c.id2z[zl[i]]) : 0u;
+                    v[k] = i < n ? ctr[i] : 0u;
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++) {
+                    const uint32_t i = ib + k * blockDim.x;
+                    if (i < n) {
+                        st_stream(&c.out[base + i], make_uint2(xv, z[k]));
+                        __stcs(&ao.cnt[base + i], (unsigned long long)v[k]);
+                    }
+                }
             }
-            __syncwarp();
-            continue;
         }
-        uint32_t lg = ceil_log2(2 * u);
-        lg = lg < 5 ? 5 : (lg > warp_lg ? warp_lg : lg);
+        if (threadIdx.x == 0) cc->n = 0;
+        __syncthreads();  // the next window's counters; the next row's bitmap
+    }
+    if (ao.sum.tiles) ao.sum.commit(xv, gs.g, gs.cs, gs.h);
+}
+
+// ------------------------------------------------------------ tiny rows
+// (x, z, count) groups staged across the rows of one warp and one query,
+// reserved once per `cap` groups (see PairStageSink).
+struct GroupStage {
+    uint2* pairs;      // cap (x value, z value)
+    uint32_t* counts;  // cap counts
+    uint2* out;
+    unsigned long long* out_cnt;
+    Reserve rs;
+    uint32_t cap;      // at least 32
+    uint32_t n = 0;
+    __device__ __forceinline__ void flush() {
+        if (n == 0) return;
+        unsigned long long base = 0;
+        if (lane_id() == 0) base = atomicAdd(rs.cursor, (unsigned long long)n);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        __syncwarp();
+        if (base + n <= rs.cap)
+            for (uint32_t i = lane_id(); i < n; i += 32) {
+                st_stream(&out[base + i], pairs[i]);
+                __stcs(&out_cnt[base + i], (unsigned long long)counts[i]);
+            }
+        __syncwarp();
+        n = 0;
+    }
+    // warp-collective: the lanes with `have` add one group each
+    __device__ __forceinline__ void add(bool have, uint32_t xv, uint32_t zv, uint32_t cnt) {
+        const uint32_t b = __ballot_sync(0xffffffffu, have);
+        if (!b) return;
+        if (n + __popc(b) > cap) flush();
+        if (have) {
+            const uint32_t pos = n + __popc(b & lanemask_lt());
+            pairs[pos] = make_uint2(xv, zv);
+            counts[pos] = cnt;
+        }
+        n += __popc(b);
+        __syncwarp();
+    }
+};
+
+// Slots (log2) of a warp's map, staged groups, shared words a warp.
+constexpr uint32_t kAggPackLg = 9, kAggPackStage = 128;
+constexpr size_t kAggPackWords = ((size_t)2 << kAggPackLg) + 3 * kAggPackStage;
+static_assert(kTinyU <= (1u << (kAggPackLg - 1)), "a small row fits a pack");
+
+// Rows of lanes [lo, hi) (x: the lane's row) as packs into the warp's map.
+__device__ __forceinline__ void agg_pack_rows(const RowCtx& c, uint32_t x, uint32_t lo, uint32_t hi, uint32_t* keys,
+                                              GroupStage& gs) {
+    const uint32_t lane = lane_id();
+    uint32_t u = 0, e0 = 0, ne = 0, xv = 0;
+    if (lane >= lo && lane < hi) {
+        u = c.ucap[x];
+        e0 = c.JR_R[x];
+        ne = c.JR_R[x + 1] - e0;
+        xv = c.id2x[x];
+    }
+    for (uint32_t first = lo; first < hi;) {
+        uint32_t sum;
+        const uint32_t end = pack_end(u, first, hi, c.m, 1u << (kAggPackLg - 1), &sum);
+        const bool in = lane >= first && lane < end;
+        uint32_t lg = ceil_log2(2 * sum);
+        lg = lg < 5 ? 5 : lg;
+        uint32_t* vals = keys + (1u << lg);
         for (uint32_t s = lane; s < (1u << lg); s += 32) {
             keys[s] = kEmpty32;
             vals[s] = 0;
         }
         __syncwarp();
         CountMap set{keys, vals, lg, c.err};
-        warp_expand(c, c.JR_R[x], c.JR_R[x + 1], 0, 0, 0, c.T, set, sink);
+        NullSink sink;
+        pack_expand<false>(c, e0, in ? ne : 0u, in ? (lane - first) * c.m : 0u, xv, set, sink);
         __syncwarp();
-        if (sum) {
-            GroupSums gs;
-            sum_map_slots(c, keys, vals, 0, 1u << lg, c.id2x[x], gs);
-            ao.sum.commit(c.id2x[x], gs.g, gs.cs, gs.h);
-        } else {
-            emit_map_slots_warp(c, ao, keys, vals, 0, 1u << lg, c.id2x[x], c.off[x], c.cnt[x], nullptr, &pos);
+        for (uint32_t sb = 0; sb < (1u << lg); sb += 32) {
+            const uint32_t key = keys[sb + lane];
+            const bool have = key != kEmpty32;
+            const uint32_t r = have ? key / c.m : 0u;
+            const uint32_t gx = __shfl_sync(0xffffffffu, xv, first + r);
+            gs.add(have, gx, have ? __ldg(&c.id2z[key - r * c.m]) : 0u, have ? vals[sb + lane] : 0u);
         }
         __syncwarp();
+        first = end;
     }
 }
 
-// Class 2 write pass: one CTA per row.
-static __global__ void __launch_bounds__(256) k_agg_block(RowCtx c, AggOut ao, const uint32_t* __restrict__ rows,
-                                                   const unsigned long long* __restrict__ nrows_p, uint32_t block_lg) {
+// ------------------------------------------------------------- one join
+static __global__ void __launch_bounds__(256, 4) k_agg_pack(RowCtx c, AggOut ao, const uint32_t* __restrict__ rows,
+                                                         const unsigned long long* __restrict__ nrows_p) {
+    extern __shared__ uint32_t smem[];
+    const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
+    uint32_t* keys = smem + (size_t)wib * kAggPackWords;
+    uint32_t* stage = keys + (2u << kAggPackLg);
+    GroupStage gs{reinterpret_cast<uint2*>(stage), stage + 2 * kAggPackStage, c.out, ao.cnt, ao.rs, kAggPackStage};
+    const uint32_t nrows = (uint32_t)*nrows_p, warps = gridDim.x * nw;
+    uint32_t take = (nrows + warps - 1) / warps;
+    take = take > 32 ? 32 : take;
+    for (uint64_t r0 = (uint64_t)(blockIdx.x * nw + wib) * take; r0 < nrows; r0 += (uint64_t)warps * take) {
+        const uint32_t n = (uint32_t)min((uint64_t)take, nrows - r0);
+        agg_pack_rows(c, lane < n ? rows[r0 + lane] : 0u, 0, n, keys, gs);
+    }
+    gs.flush();
+}
+
+// Map rows rows[skip0 + skip1 + i], i < *nrows_p (skips: device counts, either
+// may be null), maps of up to 2^lg keys; row counter c.next_row[ctr].
+static __global__ void __launch_bounds__(1024, 1) k_agg_map(RowCtx c, AggOut ao, const uint32_t* __restrict__ rows,
+                                                         const unsigned long long* __restrict__ nrows_p, uint32_t lg,
+                                                         const unsigned long long* skip0,
+                                                         const unsigned long long* skip1, uint32_t ctr) {
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t s_pos, s_row;
-    const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5;
-    const uint32_t nw_lg = 31 - __clz(nw);
-    uint32_t* keys = smem;
-    uint32_t* vals = smem + (1u << block_lg);
+    __shared__ CtaChunks s_cc;
     const uint32_t nrows = (uint32_t)*nrows_p;
-    for (uint32_t ri = cta_next_row(&c.next_row[2], &s_row); ri < nrows; ri = cta_next_row(&c.next_row[2], &s_row)) {
-        const uint32_t x = rows[ri];
-        const uint32_t u = c.ucap[x];
-        const bool direct = use_row_counters(c.m, u, block_lg + 1);
-        uint32_t lg = ceil_log2(2 * u);
-        lg = lg < 5 ? 5 : (lg > block_lg ? block_lg : lg);
-        if (direct) {
-            for (uint32_t s = threadIdx.x; s < c.m; s += blockDim.x) keys[s] = 0;
-        } else {
-            for (uint32_t s = threadIdx.x; s < (1u << lg); s += blockDim.x) {
-                keys[s] = kEmpty32;
-                vals[s] = 0;
-            }
-        }
-        if (threadIdx.x == 0) s_pos = 0;
-        __syncthreads();
-        NullSink sink;
-        if (direct) {
-            CountTile set{keys, 0};
-            warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, 0, c.T, set, sink);
-        } else {
-            CountMap set{keys, vals, lg, c.err};
-            warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, 0, c.T, set, sink);
-        }
-        __syncthreads();
-        const uint32_t span = direct ? c.m : (1u << lg);
-        const uint32_t per = (((span + nw - 1) / nw) + 31) & ~31u;
-        const uint32_t s0 = min(span, wib * per), s1 = min(span, s0 + per);
-        if (ao.sum.tiles) {
-            GroupSums gs;
-            if (direct) sum_counters(c, keys, s0, s1, 0, c.id2x[x], gs);
-            else sum_map_slots(c, keys, vals, s0, s1, c.id2x[x], gs);
-            ao.sum.commit(c.id2x[x], gs.g, gs.cs, gs.h);
-        } else if (direct) {
-            emit_counters_warp(c, ao, keys, s0, s1, c.id2x[x], c.off[x], c.cnt[x], &s_pos, nullptr);
-        } else {
-            emit_map_slots_warp(c, ao, keys, vals, s0, s1, c.id2x[x], c.off[x], c.cnt[x], &s_pos, nullptr);
-        }
-    }
+    rows += (skip0 ? *skip0 : 0ull) + (skip1 ? *skip1 : 0ull);
+    for (uint32_t ri = cta_next_row(&c.next_row[ctr], &s_row); ri < nrows; ri = cta_next_row(&c.next_row[ctr], &s_row))
+        agg_map_row(c, ao, rows[ri], smem, lg, &s_cc, &s_pos);
 }
 
-// Classes 3/4 write pass: one CTA per row; a counter per z of one tile.
-static __global__ void __launch_bounds__(1024) k_agg_tile(RowCtx c, AggOut ao, const uint32_t* __restrict__ rows,
-                                                   const unsigned long long* __restrict__ n3,
-                                                   const unsigned long long* __restrict__ n4) {
-    extern __shared__ uint32_t ctr[];
-    __shared__ uint32_t s_pos, s_row;
-    const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
-    const uint32_t nw_lg = 31 - __clz(nw);
-    const uint32_t nrows = (uint32_t)(*n3 + *n4);
-    for (uint32_t ri = cta_next_row(&c.next_row[3], &s_row); ri < nrows; ri = cta_next_row(&c.next_row[3], &s_row)) {
-        const uint32_t x = rows[ri];
-        const bool sum = ao.sum.tiles != nullptr;
-        const unsigned long long base = sum ? 0 : c.off[x];
-        const uint32_t lim = sum ? 0 : c.cnt[x], xv = c.id2x[x];
-        GroupSums gs;
+// Ranked rows (classes 4, then 3).  Cursor and summaries: one CTA a row and
+// tile, so a huge row's tiles run side by side; offsets: one CTA a row.  The
+// next item is claimed and its header loaded during the current one.
+static __global__ void __launch_bounds__(1024, 1) k_agg_ranked(RowCtx c, AggOut ao, const uint32_t* __restrict__ rows,
+                                                            const unsigned long long* __restrict__ n3,
+                                                            const unsigned long long* __restrict__ n4, RankLayout l) {
+    extern __shared__ uint32_t smem[];
+    __shared__ uint32_t s_pos, s_wbase[33];
+    __shared__ unsigned long long s_base;
+    __shared__ RankHead s_head[2];
+    __shared__ CtaChunks s_cc;
+    const uint32_t per = ao.rs.cursor || ao.sum.tiles ? c.T : 1u;
+    const uint32_t items = (uint32_t)(*n3 + *n4) * per;
+    auto claim = [&](RankHead* dst) {
+        const uint32_t i = atomicAdd(&c.next_row[3], 1u);
+        *dst = i < items ? rank_head(c, i, rows[i / per]) : RankHead{i, 0, 0, 0, 0};
+    };
+    if (threadIdx.x == 0) claim(&s_head[0]);
+    __syncthreads();
+    for (uint32_t k = 0;; k ^= 1) {
+        const RankHead h = s_head[k];
+        if (h.item >= items) break;
         if (threadIdx.x == 0) s_pos = 0;
-        for (uint32_t t = 0; t < c.T; t++) {
-            const uint32_t lo = t * c.tile_width;
-            const uint32_t width = min(c.tile_width, c.m - lo);
-            for (uint32_t w = threadIdx.x; w < width; w += blockDim.x) ctr[w] = 0;
-            __syncthreads();
-            CountTile set{ctr, lo};
-            NullSink sink;
-            warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, t, t + 1, set, sink);
-            __syncthreads();
-            if (sum) {
-                for (uint32_t wb = wib * 32; wb < width; wb += nw * 32)
-                    sum_counters(c, ctr, wb, min(width, wb + 32), lo, xv, gs);
+        if (per == c.T) {
+            agg_ranked_tile(c, ao, h, h.item % per, smem, l, &s_cc, &s_pos, s_wbase, &s_base,
+                            [&] { claim(&s_head[k ^ 1]); });
+        } else {
+            for (uint32_t t = 0; t < c.T; t++) {
+                agg_ranked_tile(c, ao, h, t, smem, l, &s_cc, &s_pos, s_wbase, &s_base, [&] {
+                    if (t == 0) claim(&s_head[k ^ 1]);
+                });
                 __syncthreads();
-                continue;
             }
-            // emit the nonzero counters of this tile
-            for (uint32_t wb = wib * 32; wb < width; wb += nw * 32) {
-                uint32_t w = wb + lane;
-                uint32_t v = w < width ? ctr[w] : 0;
-                uint32_t b = __ballot_sync(0xffffffffu, v != 0);
-                if (!b) continue;
-                uint32_t pb = 0;
-                if (lane == 0) pb = atomicAdd(&s_pos, (uint32_t)__popc(b));
-                pb = __shfl_sync(0xffffffffu, pb, 0);
-                if (v) {
-                    uint32_t pos = pb + __popc(b & lanemask_lt());
-                    if (pos < lim) {
-                        c.out[base + pos] = make_uint2(xv, __ldg(&c.id2z[lo + w]));
-                        ao.cnt[base + pos] = v;
-                    } else {
-                        raise_error(c.err, kErrOutputBound);
-                    }
-                }
-            }
-            __syncthreads();
         }
-        if (sum) ao.sum.commit(xv, gs.g, gs.cs, gs.h);
+        __syncthreads();
     }
 }
 

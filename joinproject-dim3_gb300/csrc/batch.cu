@@ -113,8 +113,6 @@ uint32_t warps_for(size_t per_warp) {
 struct QueryScratch {
     char* qmem = nullptr;
     size_t qmem_bytes = 0;
-    uint32_t* agg = nullptr;  // COUNT tile counters + touched lists
-    size_t agg_bytes = 0;
     QueryRes* h_res = nullptr;  // pinned
     uint32_t h_res_n = 0;
     QueryScratch() = default;
@@ -122,7 +120,6 @@ struct QueryScratch {
     QueryScratch& operator=(const QueryScratch&) = delete;
     ~QueryScratch() {
         if (qmem) cudaFree(qmem);
-        if (agg) cudaFree(agg);
         if (h_res) cudaFreeHost(h_res);
     }
 };
@@ -566,8 +563,8 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
         if (op == 1 && !qp.has_count) continue;
         const uint8_t k0 = op ? 8 : 0;
         unsigned long long* n = qp.ncls + 8 * op;  // n[1..5]: rows of classes k0+1..k0+5
-        unsigned long long* nb = qp.ncls + 16;  // block-class rows by hash-set size (project, split)
-        const bool split = op == 0 && tu.block_split;
+        unsigned long long* nb = qp.ncls + 16 + 4 * op;  // block-class rows by hash-set size (split)
+        const bool split = tu.block_split;
         {
             // the class lists (and the CTA class by hash-set size) in one partition
             const uint32_t b = tu.block_lg;
@@ -617,24 +614,31 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
                 Q, BatchRows{lt, &n[5], nullptr, nullptr});
             BLAUNCH();
         } else {
-            const unsigned g_t = (unsigned)(2 * sm);
-            k_b_agg_tile<<<g_t, 512, 0, st>>>(Q, BatchRows{lm, &n[4], &n[3], &qp.next_row[2]}, qs.agg,
-                                              1u << s->tile_lg);
+            const size_t ss_m = 200 << 10;
+            k_b_agg_ranked<<<resident(k_b_agg_ranked, 1024, ss_m, sm), 1024, ss_m, st>>>(
+                Q, BatchRows{lm, &n[4], &n[3], &qp.next_row[2]}, ss_m);
             BLAUNCH();
-            const size_t ss_b = (size_t)2 << tu.block_lg << 2;
-            k_b_agg_block<<<resident(k_b_agg_block, 256, ss_b, sm), 256, ss_b, st>>>(
-                Q, BatchRows{lb, &n[2], nullptr, &qp.next_row[3]}, tu.block_lg);
-            BLAUNCH();
-            const uint32_t wpa = warps_for(agg_warp_words(tu.warp_lg, kStage) * 4);
-            const size_t ss_w = (size_t)wpa * agg_warp_words(tu.warp_lg, kStage) * 4;
-            k_b_agg_warp<<<resident(k_b_agg_warp, 32 * wpa, ss_w, sm), 32 * wpa, ss_w, st>>>(
-                Q, BatchRows{lw, &n[1], nullptr, nullptr}, tu.warp_lg, kStage);
-            BLAUNCH();
-            constexpr uint32_t tiny_lg = 9, tiny_stage = 256;
-            const uint32_t wpt = warps_for(agg_warp_words(tiny_lg, tiny_stage) * 4);
-            const size_t ss_t = (size_t)wpt * agg_warp_words(tiny_lg, tiny_stage) * 4;
-            k_b_agg_warp<<<resident(k_b_agg_warp, 32 * wpt, ss_t, sm), 32 * wpt, ss_t, st>>>(
-                Q, BatchRows{lt, &n[5], nullptr, nullptr}, tiny_lg, tiny_stage);
+            auto map_rows = [&](const BatchRows& rows, uint32_t lg) -> int {
+                const int thr = lg >= 14 ? 1024 : (lg == 13 ? 512 : (lg == 12 ? 256 : 128));
+                const size_t ss = (size_t)8 << lg;
+                k_b_agg_map<<<resident(k_b_agg_map, thr, ss, sm), thr, ss, st>>>(Q, rows, lg);
+                BLAUNCH();
+                return DIM3G_OK;
+            };
+            int r = DIM3G_OK;
+            const uint32_t b = tu.block_lg;
+            if (split) {
+                r = map_rows(BatchRows{lb, &nb[2], nullptr, &qp.next_row[6], &nb[0], &nb[1]}, b);
+                if (!r) r = map_rows(BatchRows{lb, &nb[1], nullptr, &qp.next_row[5], &nb[0], nullptr}, b - 1);
+                if (!r) r = map_rows(BatchRows{lb, &nb[0], nullptr, &qp.next_row[4]}, b - 2);
+            } else {
+                r = map_rows(BatchRows{lb, &n[2], nullptr, &qp.next_row[3]}, b);
+            }
+            if (!r) r = map_rows(BatchRows{lw, &n[1], nullptr, &qp.next_row[0]}, tu.warp_lg);
+            if (r) return r;
+            const size_t ss_t = 8 * kAggPackWords * 4;
+            k_b_agg_pack<<<resident(k_b_agg_pack, 256, ss_t, sm), 256, ss_t, st>>>(
+                Q, BatchRows{lt, &n[5], nullptr, nullptr});
             BLAUNCH();
         }
     }
@@ -652,25 +656,9 @@ int set_batch_attributes(dim3g_ctx* ctx) {
     BCU(cudaFuncSetAttribute(k_b_single_block, cudaFuncAttributeMaxDynamicSharedMemorySize, blk));
     BCU(cudaFuncSetAttribute(k_b_single_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     BCU(cudaFuncSetAttribute(k_b_single_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * kPackWords * 4)));
-    BCU(cudaFuncSetAttribute(k_b_agg_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 << 14 << 2));
-    BCU(cudaFuncSetAttribute(k_b_agg_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    return DIM3G_OK;
-}
-
-int ensure_agg_scratch(dim3g_relset* s, QueryScratch& qs) {
-    dim3g_ctx* ctx = s->ctx;
-    const size_t need = (size_t)2 * I::sm_count(ctx) * 2 * ((size_t)1 << s->tile_lg) * 4;
-    if (qs.agg_bytes >= need) return DIM3G_OK;
-    if (qs.agg) cudaFree(qs.agg);
-    qs.agg = nullptr;
-    qs.agg_bytes = 0;
-    if (cudaMalloc(&qs.agg, need) != cudaSuccess) {
-        cudaGetLastError();
-        return I::fail(ctx, DIM3G_ERR_NOMEM, "COUNT scratch: device allocation of %zu bytes failed", need);
-    }
-    // counters start at zero; every row resets the counters it touched
-    BCU(cudaMemset(qs.agg, 0, need));
-    qs.agg_bytes = need;
+    BCU(cudaFuncSetAttribute(k_b_agg_map, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 << 14));
+    BCU(cudaFuncSetAttribute(k_b_agg_ranked, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10));
+    BCU(cudaFuncSetAttribute(k_b_agg_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * kAggPackWords * 4)));
     return DIM3G_OK;
 }
 
@@ -803,7 +791,7 @@ void dim3g_relset_destroy(dim3g_relset* s) {
 }
 
 uint64_t dim3g_relset_bytes(const dim3g_relset* s) {
-    return s ? (uint64_t)(s->mem_bytes + s->qs.qmem_bytes + s->qs.agg_bytes) : 0;
+    return s ? (uint64_t)(s->mem_bytes + s->qs.qmem_bytes) : 0;
 }
 
 int dim3g_relset_join(dim3g_relset* s, dim3g_query* q, uint32_t n) {
@@ -814,7 +802,6 @@ int dim3g_relset_join(dim3g_relset* s, dim3g_query* q, uint32_t n) {
     cudaStream_t st = I::stream(ctx);
     QueryPlan qp;
     int r = query_plan(s, s->qs, q, n, qp);
-    if (!r && qp.has_count) r = ensure_agg_scratch(s, s->qs);
     if (!r) r = query_upload(s, qp);
     if (r) return r;
     uint64_t launches = 0;
@@ -859,7 +846,6 @@ int dim3g_batch_create(dim3g_ctx* ctx, const dim3g_relation* rels, const dim3g_q
     if (!r) r = relset_sketch(&b->set, b->rels.data(), 2 * n);
     if (!r) r = relset_plan(&b->set, b->rels.data(), 2 * n, 0);
     if (!r) r = query_plan(&b->set, b->set.qs, b->queries.data(), n, b->qp);
-    if (!r && b->qp.has_count) r = ensure_agg_scratch(&b->set, b->set.qs);
     if (!r) r = batch_capture(b);
     if (r) {
         delete b;
@@ -994,7 +980,7 @@ int dim3g_batch_info(const dim3g_batch* b, float* ms_last, uint64_t* launches_pe
     if (!b) return DIM3G_ERR_INVALID;
     if (ms_last) *ms_last = b->ms_last;
     if (launches_per_run) *launches_per_run = b->launches_per_run;
-    if (device_bytes) *device_bytes = (uint64_t)(b->set.mem_bytes + b->set.qs.qmem_bytes + b->set.qs.agg_bytes);
+    if (device_bytes) *device_bytes = (uint64_t)(b->set.mem_bytes + b->set.qs.qmem_bytes);
     return DIM3G_OK;
 }
 
@@ -1230,9 +1216,7 @@ int dim3g_server_create(dim3g_relset* set, uint32_t lanes, uint32_t max_batch, u
             return I::fail(ctx, DIM3G_ERR_NOMEM, "server lane pinned staging");
         }
         L->qs.h_res_n = max_batch;
-        r = ensure_agg_scratch(set, L->qs);
-        if (r) return r;
-        fixed += L->qs.qmem_bytes + L->qs.agg_bytes;
+        fixed += L->qs.qmem_bytes;
         S->lanes.push_back(std::move(L));
     }
     if (fixed >= budget_bytes)

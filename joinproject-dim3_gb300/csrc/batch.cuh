@@ -464,8 +464,9 @@ static __global__ void k_q_row_work(QueryPools Q, uint32_t cap_w, uint32_t cap_b
         const uint32_t m = Q.res[qi].nz;
         const uint32_t u = (uint32_t)(w < m ? w : m);
         Q.ucap[g] = u;
-        uint32_t k = row_class(w, u, cap_w, cap_b, true);
-        if (k && Q.qin[qi].op == kOpCount) {
+        const bool count = Q.qin[qi].op == kOpCount;
+        uint32_t k = row_class(w, u, cap_w, count ? agg_cap_b(m, cap_b) : cap_b, true);
+        if (k && count) {
             k += 8;
             if (w >= 0xFFFFFFFFull) raise_error(&Q.res[qi].err, kErrCountRange);
         }
@@ -708,6 +709,23 @@ static __global__ void __launch_bounds__(256) k_b_single_warp(QueryPools Q, Batc
     sink.flush();
 }
 
+// The query of the pack list's row in lane `lo` (g: the lanes' rows), tried
+// against the warp's current query first.
+__device__ __forceinline__ uint32_t pack_query_of(const QueryPools& Q, uint32_t g, uint32_t lo, uint32_t cur_q) {
+    const uint32_t g0 = __shfl_sync(0xffffffffu, g, lo);
+    if (cur_q != 0xFFFFFFFFu && g0 >= (uint32_t)Q.qrow_off[cur_q] && g0 < (uint32_t)Q.qrow_off[cur_q + 1]) return cur_q;
+    return seg_find(Q.qrow_off, Q.nq, g0);
+}
+// The end of the run of lanes [lo, end) whose rows belong to query qi, whose
+// rows start at *q_lo.
+__device__ __forceinline__ uint32_t pack_query_end(const QueryPools& Q, uint32_t g, uint32_t lo, uint32_t n, uint32_t qi,
+                                                   uint32_t* q_lo) {
+    *q_lo = (uint32_t)Q.qrow_off[qi];
+    const uint32_t q_hi = (uint32_t)Q.qrow_off[qi + 1], lane = lane_id();
+    const uint32_t other = __ballot_sync(0xffffffffu, lane >= lo && lane < n && (g < *q_lo || g >= q_hi));
+    return other ? __ffs(other) - 1 : n;
+}
+
 // Tiny rows: packs of rows of one query (packed.cuh), at most 8 warps a CTA
 // with a context slot each.  A pack ends where the list goes on to another
 // query.
@@ -725,14 +743,9 @@ static __global__ void __launch_bounds__(256, 4) k_b_single_pack(QueryPools Q, B
         const uint32_t n = (uint32_t)min((uint64_t)take, nrows - r0);
         const uint32_t g = lane < n ? L.list[r0 + lane] : 0xFFFFFFFFu;
         for (uint32_t lo = 0; lo < n;) {
-            const uint32_t g0 = __shfl_sync(0xffffffffu, g, lo);
-            const uint32_t qi = cur_q != 0xFFFFFFFFu && g0 >= (uint32_t)Q.qrow_off[cur_q] &&
-                                        g0 < (uint32_t)Q.qrow_off[cur_q + 1]
-                                    ? cur_q
-                                    : seg_find(Q.qrow_off, Q.nq, g0);
-            const uint32_t q_lo = (uint32_t)Q.qrow_off[qi], q_hi = (uint32_t)Q.qrow_off[qi + 1];
-            const uint32_t other = __ballot_sync(0xffffffffu, lane >= lo && lane < n && (g < q_lo || g >= q_hi));
-            const uint32_t hi = other ? __ffs(other) - 1 : n;
+            const uint32_t qi = pack_query_of(Q, g, lo, cur_q);
+            uint32_t q_lo;
+            const uint32_t hi = pack_query_end(Q, g, lo, n, qi, &q_lo);
             if (qi != cur_q) {
                 sink.flush();
                 __syncwarp();
@@ -749,261 +762,98 @@ static __global__ void __launch_bounds__(256, 4) k_b_single_pack(QueryPools Q, B
     sink.flush();
 }
 
-// ---- COUNT, single pass: rows reserve output ranges from their query's
-// cursor, one atomic per 32 emitted groups.
-__device__ __forceinline__ void emit_groups(const RowCtx& c, const Reserve& rs, unsigned long long* out_cnt,
-                                            bool have, uint32_t xv, uint32_t zv, uint32_t cnt) {
-    const uint32_t b = __ballot_sync(0xffffffffu, have);
-    if (!b) return;
-    unsigned long long base = 0;
-    if (lane_id() == 0) base = atomicAdd(rs.cursor, (unsigned long long)__popc(b));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (have) {
-        const unsigned long long pos = base + __popc(b & lanemask_lt());
-        if (pos < rs.cap) {
-            c.out[pos] = make_uint2(xv, zv);
-            out_cnt[pos] = cnt;
-        }
-    }
+// ---- COUNT, single pass: the row forms of aggregate.cuh, groups to each
+// query's cursor.
+__device__ __forceinline__ AggOut query_agg(const QueryPools& Q, uint32_t qi) {
+    return AggOut{Q.qin[qi].out_cnt, SumAcc{}, Q.rs[qi]};
 }
 
-// (x, z, count) groups staged across the rows of one warp and one query,
-// reserved once per kStage groups (see PairStageSink).
-struct GroupStage {
-    uint2* pairs;      // cap (x value, z value)
-    uint32_t* counts;  // cap counts
-    uint2* out;
-    unsigned long long* out_cnt;
-    Reserve rs;
-    uint32_t cap;      // at least 32
-    uint32_t n = 0;
-    __device__ __forceinline__ void flush() {
-        if (n == 0) return;
-        unsigned long long base = 0;
-        if (lane_id() == 0) base = atomicAdd(rs.cursor, (unsigned long long)n);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        __syncwarp();
-        if (base + n <= rs.cap)
-            for (uint32_t i = lane_id(); i < n; i += 32) {
-                out[base + i] = pairs[i];
-                out_cnt[base + i] = counts[i];
-            }
-        __syncwarp();
-        n = 0;
-    }
-    // warp-collective: the lanes with `have` add one group each
-    __device__ __forceinline__ void add(bool have, uint32_t xv, uint32_t zv, uint32_t cnt) {
-        const uint32_t b = __ballot_sync(0xffffffffu, have);
-        if (!b) return;
-        if (n + __popc(b) > cap) flush();
-        if (have) {
-            const uint32_t pos = n + __popc(b & lanemask_lt());
-            pairs[pos] = make_uint2(xv, zv);
-            counts[pos] = cnt;
-        }
-        n += __popc(b);
-        __syncwarp();
-    }
-};
-
-// Per-warp shared memory of the COUNT warp classes: 2^(warp_lg+1) map
-// words, then `stage` staged groups (3 words each).
-__host__ __device__ constexpr size_t agg_warp_words(uint32_t warp_lg, uint32_t stage) {
-    return ((size_t)2 << warp_lg) + 3 * (size_t)stage;
-}
-
-static __global__ void __launch_bounds__(256) k_b_agg_warp(QueryPools Q, BatchRows L, uint32_t warp_lg,
-                                                           uint32_t stage) {
+static __global__ void __launch_bounds__(256, 4) k_b_agg_pack(QueryPools Q, BatchRows L) {
     extern __shared__ uint32_t smem[];
     __shared__ RowCtx s_c[8];
     const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
-    uint32_t* keys = smem + (size_t)wib * agg_warp_words(warp_lg, stage);
-    uint32_t* vals = keys + (1u << warp_lg);
-    GroupStage gs{reinterpret_cast<uint2*>(keys + (2u << warp_lg)), keys + (2u << warp_lg) + 2 * stage, nullptr,
-                  nullptr, Reserve{nullptr, 0}, stage};
-    uint32_t cur_q = 0xFFFFFFFFu, q_lo = 1, q_hi = 0;
-    const uint32_t nrows = (uint32_t)*L.n_a;
-    for (uint32_t ri = blockIdx.x * nw + wib; ri < nrows; ri += gridDim.x * nw) {
-        // rows of one query are contiguous in the list: look the query up
-        // only when the row leaves the current query's row range
-        const uint32_t g = L.list[ri];
-        uint32_t qi = cur_q;
-        if (g < q_lo || g >= q_hi) {
-            qi = seg_find(Q.qrow_off, Q.nq, g);
-            q_lo = (uint32_t)Q.qrow_off[qi];
-            q_hi = (uint32_t)Q.qrow_off[qi + 1];
-        }
-        const uint32_t x = g - q_lo;
-        if (qi != cur_q) {
-            gs.flush();
-            __syncwarp();
-            if (lane == 0) s_c[wib] = Q.rc[qi];
-            __syncwarp();
-            gs.rs = Q.rs[qi];
-            gs.out = s_c[wib].out;
-            gs.out_cnt = Q.qin[qi].out_cnt;
-            cur_q = qi;
-        }
-        const RowCtx& c = s_c[wib];
-        const uint32_t u = c.ucap[x];
-        const uint32_t xv = c.id2x[x];
-        NullSink sink;
-        if (use_row_counters(c.m, u, warp_lg + 1)) {
-            for (uint32_t s = lane; s < c.m; s += 32) keys[s] = 0;
-            __syncwarp();
-            CountTile set{keys, 0};
-            warp_expand(c, c.JR_R[x], c.JR_R[x + 1], 0, 0, 0, c.T, set, sink);
-            __syncwarp();
-            for (uint32_t sb = 0; sb < c.m; sb += 32) {
-                const uint32_t z = sb + lane;
-                const uint32_t v = z < c.m ? keys[z] : 0u;
-                gs.add(v != 0, xv, v ? __ldg(&c.id2z[z]) : 0u, v);
+    uint32_t* keys = smem + (size_t)wib * kAggPackWords;
+    uint32_t* stage = keys + (2u << kAggPackLg);
+    GroupStage gs{reinterpret_cast<uint2*>(stage), stage + 2 * kAggPackStage, nullptr, nullptr, Reserve{nullptr, 0},
+                  kAggPackStage};
+    uint32_t cur_q = 0xFFFFFFFFu;
+    const uint32_t nrows = (uint32_t)*L.n_a, warps = gridDim.x * nw;
+    uint32_t take = (nrows + warps - 1) / warps;
+    take = take > 32 ? 32 : take;
+    for (uint64_t r0 = (uint64_t)(blockIdx.x * nw + wib) * take; r0 < nrows; r0 += (uint64_t)warps * take) {
+        const uint32_t n = (uint32_t)min((uint64_t)take, nrows - r0);
+        const uint32_t g = lane < n ? L.list[r0 + lane] : 0xFFFFFFFFu;
+        for (uint32_t lo = 0; lo < n;) {
+            const uint32_t qi = pack_query_of(Q, g, lo, cur_q);
+            uint32_t q_lo;
+            const uint32_t hi = pack_query_end(Q, g, lo, n, qi, &q_lo);
+            if (qi != cur_q) {
+                gs.flush();
+                __syncwarp();
+                if (lane == 0) s_c[wib] = Q.rc[qi];
+                __syncwarp();
+                const AggOut ao = query_agg(Q, qi);
+                gs.rs = ao.rs;
+                gs.out = s_c[wib].out;
+                gs.out_cnt = ao.cnt;
+                cur_q = qi;
             }
-            __syncwarp();
-            continue;
+            agg_pack_rows(s_c[wib], lane >= lo && lane < hi ? g - q_lo : 0u, lo, hi, keys, gs);
+            lo = hi;
         }
-        uint32_t lg = ceil_log2(2 * u);
-        lg = lg < 5 ? 5 : (lg > warp_lg ? warp_lg : lg);
-        for (uint32_t s = lane; s < (1u << lg); s += 32) {
-            keys[s] = kEmpty32;
-            vals[s] = 0;
-        }
-        __syncwarp();
-        CountMap set{keys, vals, lg, c.err};
-        warp_expand(c, c.JR_R[x], c.JR_R[x + 1], 0, 0, 0, c.T, set, sink);
-        __syncwarp();
-        for (uint32_t sb = 0; sb < (1u << lg); sb += 32) {
-            const uint32_t key = keys[sb + lane];
-            const bool have = key != kEmpty32;
-            gs.add(have, xv, have ? __ldg(&c.id2z[key]) : 0u, have ? vals[sb + lane] : 0u);
-        }
-        __syncwarp();
     }
     gs.flush();
 }
 
-static __global__ void __launch_bounds__(256) k_b_agg_block(QueryPools Q, BatchRows L, uint32_t block_lg) {
+static __global__ void __launch_bounds__(1024, 1) k_b_agg_map(QueryPools Q, BatchRows L, uint32_t lg) {
     extern __shared__ uint32_t smem[];
-    __shared__ uint32_t s_row, s_x, s_q;
+    __shared__ uint32_t s_row, s_x, s_q, s_pos;
     __shared__ RowCtx s_c;
-    const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
-    const uint32_t nw_lg = 31 - __clz(nw);
-    uint32_t* keys = smem;
-    uint32_t* vals = smem + (1u << block_lg);
+    __shared__ CtaChunks s_cc;
     const uint32_t nrows = (uint32_t)*L.n_a;
+    const uint32_t* rows = L.rows();
     for (uint32_t ri = cta_next_row(L.next, &s_row); ri < nrows; ri = cta_next_row(L.next, &s_row)) {
         if (threadIdx.x == 0) {
             uint32_t x;
-            s_q = query_of_row(Q, L.list[ri], &x);
+            s_q = query_of_row(Q, rows[ri], &x);
             s_x = x;
             s_c = Q.rc[s_q];
         }
         __syncthreads();
-        const RowCtx& c = s_c;
-        const uint32_t x = s_x;
-        const uint32_t u = c.ucap[x];
-        const bool direct = use_row_counters(c.m, u, block_lg + 1);
-        uint32_t lg = ceil_log2(2 * u);
-        lg = lg < 5 ? 5 : (lg > block_lg ? block_lg : lg);
-        if (direct) {
-            for (uint32_t s = threadIdx.x; s < c.m; s += blockDim.x) keys[s] = 0;
-        } else {
-            for (uint32_t s = threadIdx.x; s < (1u << lg); s += blockDim.x) {
-                keys[s] = kEmpty32;
-                vals[s] = 0;
-            }
-        }
-        __syncthreads();
-        NullSink sink;
-        if (direct) {
-            CountTile set{keys, 0};
-            warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, 0, c.T, set, sink);
-        } else {
-            CountMap set{keys, vals, lg, c.err};
-            warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, 0, c.T, set, sink);
-        }
-        __syncthreads();
-        const Reserve rs = Q.rs[s_q];
-        const uint32_t xv = c.id2x[x];
-        unsigned long long* oc = Q.qin[s_q].out_cnt;
-        const uint32_t span = direct ? c.m : (1u << lg);
-        for (uint32_t sb = wib * 32; sb < span; sb += nw * 32) {
-            const uint32_t s = sb + lane;
-            uint32_t zid = kEmpty32, v = 0;
-            if (s < span) {
-                if (direct) {
-                    v = keys[s];
-                    zid = v ? s : kEmpty32;
-                } else {
-                    zid = keys[s];
-                    v = vals[s];
-                }
-            }
-            const bool have = zid != kEmpty32;
-            emit_groups(c, rs, oc, have, xv, have ? __ldg(&c.id2z[zid]) : 0u, have ? v : 0u);
-        }
+        agg_map_row(s_c, query_agg(Q, s_q), s_x, smem, lg, &s_cc, &s_pos);
     }
 }
 
-// Classes 3/4 of COUNT: one CTA per row with a private counter array over
-// one z tile in global memory (L2-resident), plus a list of the z touched
-// in the tile, so emission and reset cost O(distinct z).
-struct TouchCountTile {
-    uint32_t* ctr;
-    uint32_t* touched;
-    uint32_t* n_touched;  // shared
-    uint32_t lo;
-    __device__ __forceinline__ bool insert(uint32_t z, bool act) {
-        if (act) {
-            const uint32_t zl = z - lo;
-            if (atomicAdd(&ctr[zl], 1u) == 0) touched[atomicAdd(n_touched, 1u)] = zl;
-        }
-        return false;
-    }
-};
-
-static __global__ void __launch_bounds__(512) k_b_agg_tile(QueryPools Q, BatchRows L, uint32_t* scratch, uint32_t tile_cap) {
-    __shared__ uint32_t s_row, s_x, s_q, s_nt;
-    __shared__ RowCtx s_c;
-    const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
-    const uint32_t nw_lg = 31 - __clz(nw);
-    uint32_t* ctr = scratch + (size_t)blockIdx.x * 2 * tile_cap;
-    uint32_t* touched = ctr + tile_cap;
+// Ranked rows: a row's z tiles are taken in turn; the next row is claimed, and
+// its query and header looked up, during the current one.
+static __global__ void __launch_bounds__(1024, 1) k_b_agg_ranked(QueryPools Q, BatchRows L, size_t smem_bytes) {
+    extern __shared__ uint32_t smem[];
+    __shared__ uint32_t s_q[2], s_pos, s_wbase[33];
+    __shared__ unsigned long long s_base;
+    __shared__ RankHead s_head[2];
+    __shared__ RowCtx s_c[2];
+    __shared__ CtaChunks s_cc;
     const uint32_t nrows = (uint32_t)(*L.n_a + *L.n_b);
-    for (uint32_t ri = cta_next_row(L.next, &s_row); ri < nrows; ri = cta_next_row(L.next, &s_row)) {
-        if (threadIdx.x == 0) {
-            uint32_t x;
-            s_q = query_of_row(Q, L.list[ri], &x);
-            s_x = x;
-            s_c = Q.rc[s_q];
-        }
-        __syncthreads();
-        const RowCtx& c = s_c;
-        const uint32_t x = s_x;
-        const Reserve rs = Q.rs[s_q];
-        const uint32_t xv = c.id2x[x];
-        unsigned long long* oc = Q.qin[s_q].out_cnt;
+    auto claim = [&](uint32_t k) {
+        const uint32_t i = atomicAdd(L.next, 1u);
+        s_head[k].item = i;
+        if (i >= nrows) return;
+        uint32_t x;
+        s_q[k] = query_of_row(Q, L.list[i], &x);
+        s_c[k] = Q.rc[s_q[k]];
+        s_head[k] = rank_head(s_c[k], i, x);
+    };
+    if (threadIdx.x == 0) claim(0);
+    __syncthreads();
+    for (uint32_t k = 0; s_head[k].item < nrows; k ^= 1) {
+        const RowCtx& c = s_c[k];
+        const AggOut ao = query_agg(Q, s_q[k]);
+        const RankHead h = s_head[k];
+        const RankLayout l = rank_layout(c.tile_width, blockDim.x >> 5, smem_bytes);
         for (uint32_t t = 0; t < c.T; t++) {
-            const uint32_t lo = t * c.tile_width;
-            if (threadIdx.x == 0) s_nt = 0;
-            __syncthreads();
-            TouchCountTile set{ctr, touched, &s_nt, lo};
-            NullSink sink;
-            warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, t, t + 1, set, sink);
-            __threadfence_block();
-            __syncthreads();
-            const uint32_t nt = s_nt;
-            for (uint32_t jb = wib * 32; jb < nt; jb += nw * 32) {
-                const uint32_t j = jb + lane;
-                const bool have = j < nt;
-                uint32_t zl = 0, v = 0;
-                if (have) {
-                    zl = __ldcg(&touched[j]);
-                    v = __ldcg(&ctr[zl]);
-                    ctr[zl] = 0;
-                }
-                emit_groups(c, rs, oc, have, xv, have ? __ldg(&c.id2z[lo + zl]) : 0u, v);
-            }
+            agg_ranked_tile(c, ao, h, t, smem, l, &s_cc, &s_pos, s_wbase, &s_base, [&] {
+                if (t == 0) claim(k ^ 1);
+            });
             __syncthreads();
         }
     }

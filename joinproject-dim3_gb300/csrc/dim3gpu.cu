@@ -106,7 +106,7 @@ struct Params {
 
 constexpr size_t kMaxSmemOptin = 227 * 1024;  // dynamic shared memory a CTA may opt into
 constexpr uint32_t kFlatAvgBitmap = 160, kFlatAvgBlock = 560, kFlatAvgWarp = 160;  // single pass, per row class
-constexpr uint32_t kAggTileLg = 15;  // join-aggregate class-3 tile: 32K counters (128 KB)
+constexpr uint32_t kAggTileLgMax = 19;  // join-aggregate z tile (its bitmap and ranks are 96 KB)
 
 struct Scalars {
     unsigned long long nx, ny, nz, nkept, total, outj;
@@ -216,7 +216,7 @@ T* ws_get(dim3g_ctx* c, uint64_t count) {
 // single pass writes into whatever is there and reports the size needed).
 struct OutPrep {
     int (*fn)(dim3g_ctx* c, void* user, uint64_t total, uint2** out, unsigned long long** cnt);
-    void (*peek)(dim3g_ctx* c, void* user, uint2** out, uint64_t* capacity);
+    void (*peek)(dim3g_ctx* c, void* user, uint2** out, unsigned long long** cnt, uint64_t* capacity);
     void* user;
 };
 
@@ -239,7 +239,7 @@ struct RowLists {
     const uint32_t *w, *b, *m;                          // class 1, class 2, classes 4 then 3
     const unsigned long long *nw, *nb, *n3, *n4;        // their sizes (device)
 };
-int run_aggregate_write(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L);
+int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc, const uint32_t* list_t);
 
 // Warps per CTA of a warp-per-row kernel whose warps each own per_warp
 // bytes of shared memory: up to 8, within about half an SM's shared memory
@@ -684,7 +684,8 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         return fail(c, DIM3G_ERR_UNSUPPORTED, "key domains of 2^31 or more distinct values are not supported");
 
     // z tiles for the bitmap class
-    uint32_t tile_lg = jp.aggregate ? kAggTileLg : c->prm.tile_lg;
+    uint32_t tile_lg = c->prm.tile_lg;
+    if (jp.aggregate && tile_lg > kAggTileLgMax) tile_lg = kAggTileLgMax;
     uint32_t T = 1, tile_shift = 31, tile_width = m;
     if (m > (1u << tile_lg)) {
         tile_shift = tile_lg;
@@ -705,10 +706,10 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     uint32_t* IC_R = ws_get<uint32_t>(c, jp.nP);
     uint32_t* cur_yt = ws_get<uint32_t>(c, k1);
     uint32_t* JR_S = ws_get<uint32_t>(c, k1);
-    // S's entries: the single pass reads (z id, z value) pairs, COUNT and the
-    // count pass ids, ordered output and the join-project summaries both
-    const bool single = jp.single_pass && !jp.aggregate && !jp.count_only;
-    const bool want_ids = !single, want_pairs = !jp.aggregate && !jp.count_only;
+    // S's entries: the join-project's single pass reads (z id, z value) pairs,
+    // COUNT and the count pass ids, ordered output and summaries both
+    const bool single = jp.single_pass && !jp.count_only;
+    const bool want_ids = !single || jp.aggregate, want_pairs = !jp.aggregate && !jp.count_only;
     uint32_t* IC_S = want_ids ? ws_get<uint32_t>(c, nq) : nullptr;
     uint32_t* VS = nullptr;  // the value paths read the pairs in ISV
     // +2: the streamed bitmap rows copy 16-byte-aligned supersets of S
@@ -759,11 +760,11 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     rc.id2z = id2z;
     rc.out = nullptr;
     rc.err = &sc->err;
-    // tiny rows get their own warp launch, and the block class is split by
-    // hash-set size (2^lg slots for 2u keys), in the single pass only
-    const bool block_split = single && !jp.sum.tiles && c->prm.block_split &&
-                             !(c->prm.prefetch_rows && c->prm.cta_rr == 3);
-    const RowBuckets rb{1u << (c->prm.warp_lg - 1), 1u << (c->prm.block_lg - 1), single, block_split,
+    // tiny rows go many to a warp in the single pass, and the block class is
+    // split by hash-set size (2^lg slots for 2u keys) there and for COUNT
+    const bool block_split = c->prm.block_split && (jp.aggregate || (single && !(c->prm.prefetch_rows && c->prm.cta_rr == 3)));
+    const uint32_t cap_w = 1u << (c->prm.warp_lg - 1), cap_b = 1u << (c->prm.block_lg - 1);
+    const RowBuckets rb{cap_w, jp.aggregate ? agg_cap_b(m, cap_b) : cap_b, single, block_split,
                         1u << (c->prm.block_lg - 3), 1u << (c->prm.block_lg - 2)};
     const uint32_t lanes = row_work_lanes((double)jp.nP / n);
     k_row_work<<<grid_for((uint64_t)n << lanes, sm), 256, 0, st>>>(rc, n, lanes, rb, jp.aggregate, jp.sum, ucap, bucket,
@@ -802,7 +803,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         // needs no count pass (nothing is placed)
         CU(cudaEventRecord(c->evc[4], st));
         if (jp.aggregate) {
-            int r = run_aggregate_write(c, rc, AggOut{nullptr, jp.sum}, L);
+            int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, nullptr);
             if (r) return r;
         } else {
             k_sum_bitmap<<<resident_grid(k_sum_bitmap, blk_m, smem_m, sm), blk_m, smem_m, st>>>(rc, jp.sum, L.m,
@@ -835,12 +836,42 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         S.ms_total = a + b + e;
         return DIM3G_OK;
     }
-    if (jp.single_pass && !jp.aggregate && !jp.count_only) {
-        uint2* out = nullptr;
-        uint64_t cap = 0;
-        jp.prep.peek(c, jp.prep.user, &out, &cap);
-        if (!out) cap = 0;
-        rc.out = out;
+    uint2* sp_out = nullptr;
+    unsigned long long* sp_cnt = nullptr;
+    uint64_t cap = 0;
+    if (single) {
+        jp.prep.peek(c, jp.prep.user, &sp_out, &sp_cnt, &cap);
+        if (!sp_out) cap = 0;
+        rc.out = sp_out;
+    }
+    if (single && jp.aggregate) {
+        int r = run_aggregate(c, rc, AggOut{sp_cnt, SumAcc{}, Reserve{&sc->cursor, cap}}, L, sc, list_t);
+        if (r) return r;
+        CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
+        CU(cudaEventRecord(c->ev[3], st));
+        CU(cudaStreamSynchronize(st));
+        if (c->h_sc->err) return fail(c, DIM3G_ERR_DEVICE, "device bound violated in write pass (flags %u)", c->h_sc->err);
+        const uint64_t total = c->h_sc->cursor;
+        S.out_j = c->h_sc->outj;
+        S.n_out = total;
+        S.rows_warp = (uint32_t)(c->h_sc->nrows[1] + c->h_sc->nrows[5]);
+        S.rows_block = (uint32_t)c->h_sc->nrows[2];
+        S.rows_bitmap = (uint32_t)(c->h_sc->nrows[3] + c->h_sc->nrows[4]);
+        S.out_j_cls[0] = c->h_sc->outj_cls[3] + c->h_sc->outj_cls[4];
+        S.out_j_cls[1] = c->h_sc->outj_cls[2];
+        S.out_j_cls[2] = c->h_sc->outj_cls[1] + c->h_sc->outj_cls[5];
+        *n_out = total;
+        cudaEventElapsedTime(&S.ms_map, c->ev[0], c->ev[1]);
+        cudaEventElapsedTime(&S.ms_csr, c->ev[1], c->ev[2]);
+        cudaEventElapsedTime(&S.ms_write, c->ev[2], c->ev[3]);
+        S.ms_total = S.ms_map + S.ms_csr + S.ms_write;
+        if (total > cap)
+            return fail(c, DIM3G_ERR_CAPACITY, "output needs %llu pairs, capacity is %llu", (unsigned long long)total,
+                        (unsigned long long)cap);
+        return DIM3G_OK;
+    }
+    if (single) {
+        uint2* const out = sp_out;
         const Reserve rs{&sc->cursor, cap};
         CU(cudaEventRecord(c->evc[4], st));
         // single-pass kernels add one kStage-entry staging buffer per warp
@@ -1006,7 +1037,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     CU(cudaMemsetAsync(sc->next_row, 0, sizeof(sc->next_row), st));
     if (total > 0) {
         if (jp.aggregate) {
-            int r = run_aggregate_write(c, rc, AggOut{out_cnt}, L);
+            int r = run_aggregate(c, rc, AggOut{out_cnt, SumAcc{}, Reserve{nullptr, 0}}, L, sc, nullptr);
             if (r) return r;
         } else {
             CU(cudaEventRecord(c->evc[4], st));
@@ -1045,30 +1076,56 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     return DIM3G_OK;
 }
 
-int run_aggregate_write(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L) {
+// COUNT's row kernels (aggregate.cuh): the ranked rows first, then the map
+// rows from the largest maps down, then the tiny rows (list_t; null: none).
+// CTAs by map size, so that small maps run many rows an SM.
+int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc,
+                  const uint32_t* list_t) {
     cudaStream_t st = c->stream;
     const int sm = c->sm_count;
-    const uint32_t wpa = warps_per_cta((size_t)8 << c->prm.warp_lg);
-    const size_t smem_w = (size_t)wpa << (c->prm.warp_lg + 1) << 2;
-    const size_t smem_b = (size_t)2 << c->prm.block_lg << 2;
-    const size_t smem_m = (size_t)rc.tile_width * 4;
-    k_agg_tile<<<resident_grid(k_agg_tile, 1024, smem_m, sm), 1024, smem_m, st>>>(rc, ao, L.m, L.n3, L.n4);
+    // one ranked CTA an SM with all of its shared memory, or two where a
+    // half leaves 60 KB for the counters
+    const bool half = rank_layout(rc.tile_width, 16, 0).words * 6 + (60u << 10) <= (102u << 10);
+    const int thr_m = half ? 512 : 1024;
+    const size_t smem_m = half ? 102 << 10 : 200 << 10;
+    k_agg_ranked<<<resident_grid(k_agg_ranked, thr_m, smem_m, sm), thr_m, smem_m, st>>>(
+        rc, ao, L.m, L.n3, L.n4, rank_layout(rc.tile_width, thr_m / 32, smem_m));
     CHECK_LAUNCH();
-    k_agg_block<<<resident_grid(k_agg_block, 256, smem_b, sm), 256, smem_b, st>>>(rc, ao, L.b, L.nb, c->prm.block_lg);
-    CHECK_LAUNCH();
-    k_agg_warp<<<resident_grid(k_agg_warp, 32 * wpa, smem_w, sm), 32 * wpa, smem_w, st>>>(rc, ao, L.w, L.nw,
-                                                                                         c->prm.warp_lg);
-    CHECK_LAUNCH();
+    auto map_rows = [&](const uint32_t* rows, const unsigned long long* n, uint32_t lg, const unsigned long long* s0,
+                        const unsigned long long* s1, uint32_t ctr) -> int {
+        const int thr = lg >= 14 ? 1024 : (lg == 13 ? 512 : (lg == 12 ? 256 : 128));
+        const size_t smem = (size_t)8 << lg;
+        k_agg_map<<<resident_grid(k_agg_map, thr, smem, sm), thr, smem, st>>>(rc, ao, rows, n, lg, s0, s1, ctr);
+        CHECK_LAUNCH();
+        return DIM3G_OK;
+    };
+    const uint32_t b = c->prm.block_lg;
+    int r = DIM3G_OK;
+    if (c->prm.block_split) {
+        r = map_rows(L.b, &sc->nrows_b[2], b, &sc->nrows_b[0], &sc->nrows_b[1], 6);
+        if (!r) r = map_rows(L.b, &sc->nrows_b[1], b - 1, &sc->nrows_b[0], nullptr, 5);
+        if (!r) r = map_rows(L.b, &sc->nrows_b[0], b - 2, nullptr, nullptr, 4);
+    } else {
+        r = map_rows(L.b, L.nb, b, nullptr, nullptr, 4);
+    }
+    if (!r) r = map_rows(L.w, L.nw, c->prm.warp_lg, nullptr, nullptr, 2);
+    if (r) return r;
+    if (list_t) {
+        const size_t smem = 8 * kAggPackWords * 4;
+        k_agg_pack<<<resident_grid(k_agg_pack, 256, smem, sm), 256, smem, st>>>(rc, ao, list_t, &sc->nrows[5]);
+        CHECK_LAUNCH();
+    }
     return DIM3G_OK;
 }
 
 bool set_aggregate_attributes() {
-    return cudaFuncSetAttribute(k_agg_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess &&
+    return cudaFuncSetAttribute(k_agg_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * kAggPackWords * 4)) ==
+               cudaSuccess &&
            cudaFuncSetAttribute(k_sum_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess &&
            cudaFuncSetAttribute(k_sum_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 1 << 14 << 2) == cudaSuccess &&
            cudaFuncSetAttribute(k_sum_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, (1 << 20) / 8) == cudaSuccess &&
-           cudaFuncSetAttribute(k_agg_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 << 14 << 2) == cudaSuccess &&
-           cudaFuncSetAttribute(k_agg_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (1 << kAggTileLg) * 4) == cudaSuccess;
+           cudaFuncSetAttribute(k_agg_map, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 << 14) == cudaSuccess &&
+           cudaFuncSetAttribute(k_agg_ranked, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10) == cudaSuccess;
 }
 
 int ensure_dev(dim3g_ctx* c, void** p, size_t* have, size_t need) {
@@ -1103,9 +1160,10 @@ int prep_device(dim3g_ctx* c, void* user, uint64_t total, uint2** out, unsigned 
     *cnt = d->cnt;
     return DIM3G_OK;
 }
-void peek_device(dim3g_ctx*, void* user, uint2** out, uint64_t* capacity) {
+void peek_device(dim3g_ctx*, void* user, uint2** out, unsigned long long** cnt, uint64_t* capacity) {
     DeviceOut* d = (DeviceOut*)user;
     *out = d->out;
+    *cnt = d->cnt;
     *capacity = d->capacity;
 }
 
@@ -1121,9 +1179,12 @@ int prep_staging(dim3g_ctx* c, void* user, uint64_t total, uint2** out, unsigned
     *cnt = agg ? (unsigned long long*)((char*)c->d_out + total * 8) : nullptr;
     return DIM3G_OK;
 }
-void peek_staging(dim3g_ctx* c, void*, uint2** out, uint64_t* capacity) {
+// The staging buffer as it is: pairs, then (COUNT) as many counts.
+void peek_staging(dim3g_ctx* c, void* user, uint2** out, unsigned long long** cnt, uint64_t* capacity) {
+    const bool agg = ((StagingOut*)user)->aggregate;
+    *capacity = c->d_out ? c->d_out_bytes / (agg ? 16 : 8) : 0;
     *out = (uint2*)c->d_out;
-    *capacity = c->d_out ? c->d_out_bytes / 8 : 0;
+    *cnt = agg ? (unsigned long long*)((char*)c->d_out + *capacity * 8) : nullptr;
 }
 
 // Host-input join: stage R and S on the device, run, copy the result back
@@ -1164,19 +1225,20 @@ int host_join(dim3g_ctx* c, const uint32_t* R, uint64_t nR, const uint32_t* S, u
     StagingOut so{aggregate};
     // single pass once the staging buffer exists; a result larger than it
     // grows the buffer and runs again
-    const bool single = !aggregate && !c->prm.ordered && c->d_out != nullptr;
+    const bool single = !c->prm.ordered && c->d_out != nullptr;
     JoinPlan jp{dP, nP, dQ, nQ, swap, aggregate, false, single, OutPrep{prep_staging, peek_staging, &so}};
     uint64_t n = 0;
     r = run_join(c, jp, &n);
     if (r == DIM3G_ERR_CAPACITY && single) {
-        r = ensure_dev(c, &c->d_out, &c->d_out_bytes, n * 8);
+        r = ensure_dev(c, &c->d_out, &c->d_out_bytes, n * (aggregate ? 16 : 8));
         if (r) return r;
         r = run_join(c, jp, &n);
     }
     if (r) return r;
     *n_out = n;
     const uint2* dout = (const uint2*)c->d_out;
-    const unsigned long long* dcnt = aggregate ? (const unsigned long long*)((const char*)c->d_out + n * 8) : nullptr;
+    const uint64_t cnt_at = single ? c->d_out_bytes / 16 : n;  // the counts follow the pairs' room
+    const unsigned long long* dcnt = aggregate ? (const unsigned long long*)((const char*)c->d_out + cnt_at * 8) : nullptr;
     if (out_into) {
         if (n > capacity)
             return fail(c, DIM3G_ERR_CAPACITY, "output needs %llu pairs, capacity is %llu", (unsigned long long)n,
@@ -1475,7 +1537,7 @@ int dim3g_join_count_device(dim3g_ctx* c, const uint32_t* dR, uint64_t nR, const
     const bool swap = !c->prm.keep_roles && nR < nS;
     DeviceOut d{(uint2*)d_out_xz, (unsigned long long*)d_out_cnt, capacity};
     JoinPlan jp{(const uint2*)(swap ? dS : dR), swap ? nS : nR, (const uint2*)(swap ? dR : dS), swap ? nR : nS,
-                swap, true, false, false, OutPrep{prep_device, peek_device, &d}};
+                swap, true, false, !c->prm.ordered, OutPrep{prep_device, peek_device, &d}};
     return run_join(c, jp, n_out);
 }
 

@@ -47,6 +47,14 @@ __device__ __forceinline__ uint32_t row_class(unsigned long long w, uint32_t u, 
     if (u <= cap_b) return 2;
     return u <= kHugeRow ? 3 : 4;
 }
+// The block class's distinct bound for COUNT rows: larger rows are ranked over
+// a bitmap (aggregate.cuh), which costs by the z domain where a map costs by
+// its slots; below 128 z a distinct z the ranks are cheaper than the larger
+// maps (1M-tuple COUNT, m = 196K: rows of 2K to 8K distinct z 2.6 ms in maps
+// of 2^13 and 2^14).
+__host__ __device__ __forceinline__ uint32_t agg_cap_b(uint64_t m, uint32_t cap_b) {
+    return m <= 128ull * (cap_b / 4) ? cap_b / 4 : (m <= 128ull * (cap_b / 2) ? cap_b / 2 : cap_b);
+}
 // Words of a whole-domain bitmap, rounded to uint4 and at least 32 (idle
 // lanes of TileBitmap touch words 0..31).
 __device__ __forceinline__ uint32_t row_bitmap_words(uint32_t m) {
