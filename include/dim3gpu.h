@@ -181,7 +181,7 @@ int dim3g_join_count_summary(dim3g_ctx* ctx, const uint32_t* d_R, uint64_t nR, c
  * fixed-budget allocator, hosts that preallocate everything at start-up,
  * and pipelines that cannot afford the synchronisation an allocation may
  * bring.  Device inputs, the caller's output buffer, and all scratch in one
- * fixed array inside the library (about 19 MB, held on every GPU that loads
+ * fixed array inside the library (about 20 MB, held on every GPU that loads
  * the library until the process exits); it calls no allocating routine.
  * Limits: the larger relation holds at most DIM3G_NOALLOC_MAX_TUPLES tuples
  * and the result at most DIM3G_NOALLOC_MAX_PAIRS distinct pairs; beyond

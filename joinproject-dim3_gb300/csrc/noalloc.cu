@@ -10,7 +10,7 @@
 // so it never calls cudaMalloc, cudaFree or any allocating routine.
 //
 // Costs and limits (stated in include/dim3gpu.h):
-//   - every GPU that loads this library holds kScratchBytes (about 19 MB)
+//   - every GPU that loads this library holds kScratchBytes (about 20 MB)
 //     for the life of the process;
 //   - the larger relation may hold at most DIM3G_NOALLOC_MAX_TUPLES tuples
 //     and the result at most DIM3G_NOALLOC_MAX_PAIRS distinct pairs;
@@ -32,27 +32,45 @@ namespace {
 
 constexpr uint32_t kMaxTuples = DIM3G_NOALLOC_MAX_TUPLES;  // larger relation
 constexpr uint32_t kMaxPairs = DIM3G_NOALLOC_MAX_PAIRS;    // distinct output pairs
-constexpr uint32_t kBuckets = 1u << 19;                     // chain heads on the join key
+constexpr uint32_t kBuckets = 1u << 17;                     // buckets on the join key
 constexpr uint32_t kPairSlots = 2 * kMaxPairs;              // pair set, load factor <= ~1/2
-constexpr uint32_t kNil = 0xFFFFFFFFu;
 constexpr unsigned long long kEmptyPair = ~0ull;
+// The probe's tasks: a run of 32 probe tuples is cut into pieces of at least
+// kPiece candidates (as many as the task list has room for), so that a few
+// join values with long buckets do not leave their candidates to one warp.
+constexpr uint32_t kPiece = 1024, kMaxTasks = kMaxTuples / 32 * 16;
+constexpr int kThreads = 512, kCtasPerSm = 3;
+constexpr uint32_t kBarrierPolls = 1u << 22;  // a grid barrier gives up after this many (seconds)
 
-// Layout of the scratch array (byte offsets, 256-aligned).
-constexpr size_t kOffHead = 0;
-constexpr size_t kOffNext = kOffHead + (size_t)kBuckets * 4;
-constexpr size_t kOffPairs = kOffNext + (size_t)kMaxTuples * 4;
-constexpr size_t kOffCounters = kOffPairs + (size_t)kPairSlots * 8;
-constexpr size_t kScratchBytes = kOffCounters + 256;
+// Layout of the scratch array (byte offsets, 256-aligned).  The counters and
+// bucket counts are zeroed together.
+constexpr size_t kOffCounters = 0;
+constexpr size_t kOffCount = kOffCounters + 256;
+constexpr size_t kOffBase = kOffCount + (size_t)kBuckets * 4;
+constexpr size_t kOffSorted = kOffBase + (size_t)kBuckets * 4;
+constexpr size_t kOffTasks = kOffSorted + (size_t)kMaxTuples * 8;
+constexpr size_t kOffPairs = kOffTasks + (size_t)kMaxTasks * 4;
+constexpr size_t kScratchBytes = kOffPairs + (size_t)kPairSlots * 8;
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
-// counters: [0] distinct pairs found, [1] flags (bit 1: a probe walked the
-// whole pair table), [2] the all-ones pair seen
+struct Counters {
+    unsigned long long n_out;    // distinct pairs found
+    unsigned long long flags;    // bit 1: a probe walked the whole pair table; bit 2: a grid barrier gave up
+    unsigned long long all_ones; // the all-ones pair seen
+    uint32_t placed;             // sorted tuples given to buckets
+    uint32_t n_tasks, next_task;
+    uint32_t barrier[4];         // CTAs arrived
+};
+static_assert(sizeof(Counters) <= 256, "counters' room");
+
 struct Scratch {
-    uint32_t* head;
-    uint32_t* next;
+    Counters* c;
+    uint32_t* count;  // tuples per bucket (counted down again as they are placed)
+    uint32_t* base;   // first sorted tuple of each bucket; its end once placed
+    uint2* sorted;    // the larger relation, bucket by bucket
+    uint32_t* tasks;  // run of 32 probe tuples * pieces a run + piece
     unsigned long long* pairs;
-    unsigned long long* counters;
 };
 
 __device__ __forceinline__ uint32_t mix32(uint32_t h) {
@@ -69,59 +87,185 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long v) {
     return v ^ (v >> 31);
 }
 
-// Chained hash table on the larger relation's join key: next[i] links tuple
-// i to the previous head of its bucket.
-__global__ void k_na_build(const uint2* __restrict__ P, uint32_t nP, Scratch s) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nP; i += gridDim.x * blockDim.x)
-        s.next[i] = atomicExch(&s.head[mix32(P[i].y) & (kBuckets - 1)], i);
+__device__ __forceinline__ uint32_t bucket_of(uint32_t y) { return mix32(y) & (kBuckets - 1); }
+__device__ __forceinline__ uint32_t lane() { return threadIdx.x & 31; }
+__device__ __forceinline__ uint32_t warp_scan(uint32_t v) {  // inclusive
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
+        if ((int)lane() >= o) v += t;
+    }
+    return v;
 }
 
-__device__ __forceinline__ void emit(Scratch s, uint2* out, unsigned long long cap, uint32_t px, uint32_t qc) {
-    unsigned long long pos = atomicAdd(&s.counters[0], 1ull);
-    if (pos < cap) out[pos] = make_uint2(px, qc);
+// All CTAs of the grid (co-resident: a cooperative launch).  False once a
+// wait has given up; the caller returns.
+__device__ bool grid_barrier(const Scratch& s, uint32_t k) {
+    __shared__ bool ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&s.c->barrier[k], 1u);
+        uint32_t polls = 0;
+        while (*(volatile uint32_t*)&s.c->barrier[k] < gridDim.x && ++polls < kBarrierPolls) {
+        }
+        ok = polls < kBarrierPolls;
+        if (!ok) atomicOr(&s.c->flags, 4ull);
+        __threadfence();
+    }
+    __syncthreads();
+    return ok;
 }
 
 // Distinct-pair set: 64-bit keys (P.first << 32 | Q.first) with linear
-// probing; the all-ones key is tracked by a flag.  New pairs are counted
-// and, while they fit, written straight to the caller's buffer.
-__device__ void insert_pair(Scratch s, uint2* out, unsigned long long cap, uint32_t px, uint32_t qc) {
-    const unsigned long long key = ((unsigned long long)px << 32) | qc;
-    if (key == kEmptyPair) {
-        if (atomicExch(&s.counters[2], 1ull) == 0ull) emit(s, out, cap, px, qc);
-        return;
-    }
-    uint32_t h = (uint32_t)mix64(key) & (kPairSlots - 1);
-    for (uint32_t p = 0; p < kPairSlots; p++) {
-        unsigned long long cur = ((volatile unsigned long long*)s.pairs)[h];
-        if (cur == key) return;
+// probing; the all-ones key is tracked by a flag.  `cur`: the key's first
+// slot h, already loaded.  True for a pair's first insertion.
+__device__ bool insert_pair(const Scratch& s, unsigned long long key, uint32_t h, unsigned long long cur) {
+    if (key == kEmptyPair) return atomicExch(&s.c->all_ones, 1ull) == 0ull;
+    for (uint32_t p = 0;;) {
+        if (cur == key) return false;
         if (cur == kEmptyPair) {
-            // The limit is decided after the fact: the counter only counts
-            // pairs that were claimed, so once it is above the limit the
-            // result is known to be too large and no more pairs are claimed
-            // (the host reports it from the final count).  Threads that pass
-            // this test together overshoot by at most the threads in flight,
-            // which the table's 2x slot count absorbs.
-            if (((volatile unsigned long long*)s.counters)[0] > kMaxPairs) return;
-            unsigned long long prev = atomicCAS(&s.pairs[h], kEmptyPair, key);
-            if (prev == kEmptyPair) {
-                emit(s, out, cap, px, qc);
-                return;
-            }
-            if (prev == key) return;
+            cur = atomicCAS(&s.pairs[h], kEmptyPair, key);
+            if (cur == kEmptyPair) return true;
+            if (cur == key) return false;
         }
+        if (++p == kPairSlots) break;
         h = (h + 1) & (kPairSlots - 1);
+        cur = __ldcg(&s.pairs[h]);
     }
-    atomicOr(&s.counters[1], 2ull);
+    atomicOr(&s.c->flags, 2ull);
+    return false;
 }
 
-// Probe with the smaller relation: every P tuple on the chain of q's key
-// with the same key forms the candidate (P.first, q.first).
-__global__ void k_na_probe(const uint2* __restrict__ P, const uint2* __restrict__ Q, uint32_t nQ, Scratch s,
-                           uint2* out, unsigned long long cap) {
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nQ; j += gridDim.x * blockDim.x) {
-        const uint2 q = Q[j];
-        for (uint32_t i = s.head[mix32(q.y) & (kBuckets - 1)]; i != kNil; i = s.next[i])
-            if (P[i].y == q.y) insert_pair(s, out, cap, P[i].x, q.x);
+// The run of 32 probe tuples from q0: the lane's tuple and its bucket.
+struct Run {
+    uint2 q;
+    uint32_t end, len;  // the bucket's end and length
+};
+__device__ __forceinline__ Run load_run(const uint2* __restrict__ Q, uint32_t nQ, uint32_t q0, const Scratch& s) {
+    Run r{make_uint2(0, 0), 0, 0};
+    const uint32_t i = q0 + lane();
+    if (i < nQ) {
+        r.q = __ldg(&Q[i]);
+        const uint32_t b = bucket_of(r.q.y);
+        r.end = __ldcg(&s.base[b]);
+        r.len = __ldcg(&s.count[b]);
+    }
+    return r;
+}
+
+// The whole join in one cooperative launch.  The larger relation P is placed
+// bucket by bucket of its join key (count, give every bucket a range, place;
+// the ranges are in no order, so no prefix sum), then the smaller one, Q,
+// probes: the candidates of 32 probe tuples are flattened over a warp, each
+// lane comparing one sorted tuple's key, and new pairs take one reservation
+// per group of 128 candidates.
+//
+// Bound by the latency of dependent accesses.  A linked list per bucket,
+// walked by one thread a probe tuple, with a reservation a pair, took 205 us
+// in the probe alone for 150K x 90K tuples.
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+    k_na_join(const uint2* __restrict__ P, uint32_t nP, const uint2* __restrict__ Q, uint32_t nQ, Scratch s, uint2* out,
+              unsigned long long cap) {
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    const uint32_t warp = tid >> 5, warps = stride >> 5, ln = lane();
+    const uint32_t lt = (1u << ln) - 1u;
+    // count
+    for (uint32_t i = tid; i < nP; i += stride) atomicAdd(&s.count[bucket_of(__ldg(&P[i]).y)], 1u);
+    if (!grid_barrier(s, 0)) return;
+    // ranges: a warp's 128 buckets take one range, four buckets a lane
+    for (uint32_t b0 = warp * 128; b0 < kBuckets; b0 += warps * 128) {
+        const uint4 n = __ldcg(reinterpret_cast<const uint4*>(s.count + b0) + ln);
+        const uint32_t sum = n.x + n.y + n.z + n.w, inc = warp_scan(sum);
+        const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
+        if (tot == 0) continue;
+        uint32_t at = 0;
+        if (ln == 0) at = atomicAdd(&s.c->placed, tot);
+        at = __shfl_sync(0xffffffffu, at, 0) + inc - sum;
+        reinterpret_cast<uint4*>(s.base + b0)[ln] = make_uint4(at, at + n.x, at + n.x + n.y, at + n.x + n.y + n.z);
+    }
+    if (!grid_barrier(s, 1)) return;
+    // place (base becomes the bucket's end)
+    for (uint32_t i = tid; i < nP; i += stride) {
+        const uint2 p = __ldg(&P[i]);
+        s.sorted[atomicAdd(&s.base[bucket_of(p.y)], 1u)] = p;
+    }
+    if (!grid_barrier(s, 2)) return;
+    // tasks: the pieces of every run of 32 probe tuples
+    const uint32_t runs = (nQ + 31) / 32, most = kMaxTasks / runs;
+    for (uint32_t r = warp; r < runs; r += warps) {
+        const Run run = load_run(Q, nQ, r * 32, s);
+        unsigned long long w = run.len;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+        if (w == 0) continue;
+        const uint32_t n = (uint32_t)min((w + kPiece - 1) / kPiece, (unsigned long long)most);
+        uint32_t at = 0;
+        if (ln == 0) at = atomicAdd(&s.c->n_tasks, n);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        for (uint32_t k = ln; k < n; k += 32) s.tasks[at + k] = r * most + k;
+    }
+    if (!grid_barrier(s, 3)) return;
+    const uint32_t tasks = __ldcg(&s.c->n_tasks);
+    for (;;) {
+        uint32_t t = 0;
+        if (ln == 0) t = atomicAdd(&s.c->next_task, 1u);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= tasks) break;
+        const uint32_t task = __ldcg(&s.tasks[t]), piece = task % most;
+        const Run run = load_run(Q, nQ, task / most * 32, s);
+        // 32 buckets of at most 2^18 tuples: the prefix fits 32 bits
+        const uint32_t inc = warp_scan(run.len);
+        const uint32_t w = __shfl_sync(0xffffffffu, inc, 31);
+        const uint32_t n = min((w + kPiece - 1) / kPiece, most), share = (w + n - 1) / n;
+        const uint32_t lo = min(w, piece * share), hi = min(w, lo + share);
+        for (uint32_t cb = lo; cb < hi; cb += 128) {
+            // a result past the limit is already known: no more pairs are
+            // claimed (those in flight fit the table's second half)
+            unsigned long long found = 0;
+            if (ln == 0) found = *(volatile unsigned long long*)&s.c->n_out;
+            if (__shfl_sync(0xffffffffu, found, 0) > kMaxPairs) return;
+            uint2 p[4], q[4];
+            uint32_t b[4], tot = 0;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                const uint32_t ci = min(cb + u * 32 + ln, hi - 1);
+                uint32_t k = 0;  // the probe tuple holding candidate ci
+#pragma unroll
+                for (uint32_t step = 16; step >= 1; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, inc, k + step - 1) <= ci) k += step;
+                const uint32_t j = __shfl_sync(0xffffffffu, run.end - inc, k) + ci;
+                q[u].x = __shfl_sync(0xffffffffu, run.q.x, k);
+                q[u].y = __shfl_sync(0xffffffffu, run.q.y, k);
+                p[u] = __ldcg(&s.sorted[j]);
+            }
+            unsigned long long key[4], cur[4];
+            uint32_t h[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                key[u] = ((unsigned long long)p[u].x << 32) | q[u].x;
+                h[u] = (uint32_t)mix64(key[u]) & (kPairSlots - 1);
+                if (p[u].y == q[u].y) cur[u] = __ldcg(&s.pairs[h[u]]);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                const bool fresh = cb + u * 32 + ln < hi && p[u].y == q[u].y && insert_pair(s, key[u], h[u], cur[u]);
+                b[u] = __ballot_sync(0xffffffffu, fresh);
+                tot += __popc(b[u]);
+            }
+            if (tot == 0) continue;
+            unsigned long long pos = 0;
+            if (ln == 0) pos = atomicAdd(&s.c->n_out, (unsigned long long)tot);
+            pos = __shfl_sync(0xffffffffu, pos, 0);
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                if (b[u] >> ln & 1u) {
+                    const unsigned long long at = pos + __popc(b[u] & lt);
+                    if (at < cap) out[at] = make_uint2(p[u].x, q[u].x);
+                }
+                pos += __popc(b[u]);
+            }
+        }
     }
 }
 
@@ -149,7 +293,13 @@ int scratch_for_device(int dev, unsigned char** base, int* grid) {
                 cudaGetLastError();
                 return DIM3G_ERR_CUDA;
             }
-            g_grid[dev] = 4 * sms;  // 4 CTAs of 256 threads per SM
+            int per_sm = 0;  // the CTAs wait on one another, so all must be resident
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_na_join, kThreads, 0) != cudaSuccess ||
+                per_sm < 1) {
+                cudaGetLastError();
+                return DIM3G_ERR_CUDA;
+            }
+            g_grid[dev] = sms * (per_sm < kCtasPerSm ? per_sm : kCtasPerSm);
             p = (unsigned char*)addr;
             g_base[dev].store(p, std::memory_order_release);
         }
@@ -188,27 +338,35 @@ extern "C" int dim3g_join_project_noalloc(const uint32_t* d_R, uint64_t nR, cons
     int grid = 0;
     int r = scratch_for_device(dev, &base, &grid);
     if (r) return r;
-    Scratch s{(uint32_t*)(base + kOffHead), (uint32_t*)(base + kOffNext), (unsigned long long*)(base + kOffPairs),
-              (unsigned long long*)(base + kOffCounters)};
+    Scratch s{(Counters*)(base + kOffCounters), (uint32_t*)(base + kOffCount), (uint32_t*)(base + kOffBase),
+              (uint2*)(base + kOffSorted), (uint32_t*)(base + kOffTasks), (unsigned long long*)(base + kOffPairs)};
     cudaStream_t st = (cudaStream_t)cuda_stream;
     // the previous call's contents stay in the array: reset what must start
-    // empty (chain heads, pair set, counters)
-    if (cudaMemsetAsync(s.head, 0xff, (size_t)kBuckets * 4, st) != cudaSuccess ||
-        cudaMemsetAsync(s.pairs, 0xff, (size_t)kPairSlots * 8, st) != cudaSuccess ||
-        cudaMemsetAsync(s.counters, 0, 256, st) != cudaSuccess) {
+    // empty (counters, bucket counts, pair set)
+    if (cudaMemsetAsync(s.c, 0, kOffBase - kOffCounters, st) != cudaSuccess ||
+        cudaMemsetAsync(s.pairs, 0xff, (size_t)kPairSlots * 8, st) != cudaSuccess) {
         cudaGetLastError();
         return DIM3G_ERR_CUDA;
     }
-    k_na_build<<<grid, 256, 0, st>>>(P, (uint32_t)nP, s);
-    k_na_probe<<<grid, 256, 0, st>>>(P, Q, (uint32_t)nQ, s, (uint2*)d_out, capacity);
-    unsigned long long h[2] = {0, 0};
-    if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(h, s.counters, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    // a CTA per 512 tuples (the barriers cost by the CTAs), at least one an SM
+    // (the candidates are not known), at most what is resident
+    const uint2* out = (const uint2*)d_out;
+    uint32_t n_p = (uint32_t)nP, n_q = (uint32_t)nQ;
+    unsigned long long cap = capacity;
+    int ctas = (int)((nP + nQ + kThreads - 1) / kThreads);
+    if (ctas < grid / kCtasPerSm) ctas = grid / kCtasPerSm;
+    if (ctas > grid) ctas = grid;
+    void* args[] = {&P, &n_p, &Q, &n_q, &s, &out, &cap};
+    unsigned long long h[2] = {0, 0};  // n_out, flags
+    if (cudaLaunchCooperativeKernel((const void*)k_na_join, dim3((unsigned)ctas), dim3(kThreads), args, 0, st) !=
+            cudaSuccess ||
+        cudaMemcpyAsync(h, s.c, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {
         cudaGetLastError();
         return DIM3G_ERR_CUDA;
     }
     if (h[0] > kMaxPairs) return DIM3G_ERR_UNSUPPORTED;  // more distinct pairs than DIM3G_NOALLOC_MAX_PAIRS
-    if (h[1] & 2ull) return DIM3G_ERR_DEVICE;
+    if (h[1]) return DIM3G_ERR_DEVICE;
     *n_out = h[0];
     return h[0] > capacity ? DIM3G_ERR_CAPACITY : DIM3G_OK;
 }
