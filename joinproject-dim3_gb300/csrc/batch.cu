@@ -130,6 +130,7 @@ struct dim3g_relset {
     std::vector<RelIn> h_in;
     std::vector<uint64_t> h_tup_off, h_tab_off;
     std::vector<uint64_t> h_cap;  // sketch-sized table slots per relation (when sized)
+    std::vector<uint64_t> h_nf;   // distinct first values per relation, once built (empty: not known to the host)
     std::vector<uint8_t> h_roles; // CSRs each relation needs (RelRole bits; empty: both for every relation)
     bool sized = false;           // tables from h_cap (else from the tuple counts)
     uint64_t ntot = 0, tabtot = 0, yt_cap = 0;
@@ -182,7 +183,7 @@ int relset_plan(dim3g_relset* s, const dim3g_relation* rels, uint32_t n, uint64_
                  o_ny = L.add<unsigned long long>(n), o_id2f = L.add<uint32_t>(s->ntot),
                  o_id2y = L.add<uint32_t>(s->ntot), o_Pm = L.add<uint2>(s->ntot), o_deg = L.add<uint32_t>(s->ntot + 1),
                  o_JRf = L.add<uint32_t>(s->ntot + 1), o_curF = L.add<uint32_t>(s->ntot + 1),
-                 o_ICf = L.add<uint32_t>(s->ntot), o_ICr = L.add<uint32_t>(s->ntot), o_cyt = L.add<uint32_t>(s->yt_cap),
+                 o_ICf = L.add<uint32_t>(s->ntot), o_cyt = L.add<uint32_t>(s->yt_cap),
                  o_JRy = L.add<uint32_t>(s->yt_cap), o_curY = L.add<uint32_t>(s->yt_cap),
                  o_ICy = L.add<uint32_t>(s->ntot), o_VSy = L.add<uint32_t>(s->ntot), o_err = L.add<uint32_t>(4),
                  o_need = L.add<unsigned long long>(2), o_yoff = L.add<uint64_t>(n + 1),
@@ -223,7 +224,6 @@ int relset_plan(dim3g_relset* s, const dim3g_relation* rels, uint32_t n, uint64_
     P.JRf = (uint32_t*)(m + o_JRf);
     P.curF = (uint32_t*)(m + o_curF);
     P.ICf = (uint32_t*)(m + o_ICf);
-    P.ICr = (uint32_t*)(m + o_ICr);
     P.cnt_yt = (uint32_t*)(m + o_cyt);
     P.JRy = (uint32_t*)(m + o_JRy);
     P.curY = (uint32_t*)(m + o_curY);
@@ -379,16 +379,14 @@ struct QueryPlan {
     bool has_project = false, has_count = false;
     QueryPools Q{};
     uint32_t* lists = nullptr;             // 3 x nrows
-    unsigned long long* ncls = nullptr;    // rows per class 0..8
+    unsigned long long* ncls = nullptr;    // per op 32 words: class counts, split counts, bucket counts, list cursors
     uint32_t* next_row = nullptr;          // 8 dynamic counters (4..6: split block launches)
-    uint32_t* part = nullptr;              // class-list partition: per-tile bucket offsets
-    unsigned long long* pbase = nullptr;   // its bucket starts (8)
 };
 
 // Device layout of a query pass's scratch (every size monotone in the
 // arguments, so scratch laid out for maxima fits every smaller pass).
 struct QLayout {
-    size_t qin, qt, qr, ymap, ICq, JRq, ucap, cls, wrow, rc, rs, res, lists, ncls, next, part, pbase, total;
+    size_t qin, qt, qr, ymap, step, ICq, JRq, ucap, bucket, rc, rs, res, lists, ncls, next, total;
 };
 QLayout query_layout(uint32_t nq, uint64_t ntot, uint64_t nrows) {
     Layout L;
@@ -396,20 +394,18 @@ QLayout query_layout(uint32_t nq, uint64_t ntot, uint64_t nrows) {
     o.qin = L.add<QueryIn>(nq);
     o.qt = L.add<uint64_t>(nq + 1);
     o.qr = L.add<uint64_t>(nq + 1);
-    o.ymap = L.add<uint32_t>(ntot);
+    o.ymap = L.add<uint2>(ntot);
+    o.step = L.add<uint64_t>(nq + 1);
     o.ICq = L.add<uint32_t>(ntot);
     o.JRq = L.add<uint32_t>(nrows);
     o.ucap = L.add<uint32_t>(nrows);
-    o.cls = L.add<uint8_t>(nrows);
-    o.wrow = L.add<unsigned long long>(nrows);
+    o.bucket = L.add<uint8_t>(nrows);
     o.rc = L.add<RowCtx>(nq);
     o.rs = L.add<Reserve>(nq);
     o.res = L.add<QueryRes>(nq);
     o.lists = L.add<uint32_t>(4 * nrows);
-    o.ncls = L.add<unsigned long long>(24);  // [16..18]: block-class rows by hash-set size
-    o.next = L.add<uint32_t>(8);
-    o.part = L.add<uint32_t>(8 * ((nrows + kPartTile - 1) / kPartTile));
-    o.pbase = L.add<unsigned long long>(8);
+    o.ncls = L.add<unsigned long long>(64);
+    o.next = L.add<uint32_t>(16);
     o.total = L.total;
     return o;
 }
@@ -444,7 +440,9 @@ int query_plan(dim3g_relset* s, QueryScratch& qs, const dim3g_query* q, uint32_t
         qp.h_qin[i] = qi;
         qp.swapped[i] = sw;
         qp.h_qt_off[i + 1] = qp.h_qt_off[i] + np;
-        qp.h_qrow_off[i + 1] = qp.h_qrow_off[i] + np + 1;
+        // rows: the driving relation's distinct first values, at most its tuples
+        const uint64_t rows = np && !s->h_nf.empty() && s->h_nf[qi.p] < np ? s->h_nf[qi.p] : np;
+        qp.h_qrow_off[i + 1] = qp.h_qrow_off[i] + rows + 1;
         if (qi.op == kOpCount) qp.has_count = true;
         else qp.has_project = true;
     }
@@ -491,26 +489,24 @@ int query_plan(dim3g_relset* s, QueryScratch& qs, const dim3g_query* q, uint32_t
     Q.id2y = P.id2y;
     Q.JRf = P.JRf;
     Q.ICf = P.ICf;
-    Q.ICr = P.ICr;
     Q.JRy = P.JRy;
     Q.ICy = P.ICy;
     Q.VSy = P.VSy;
     Q.yt_need = P.yt_need;
     Q.yt_cap = P.yt_cap;
-    Q.ymap = (uint32_t*)(m + o.ymap);
+    Q.ymap = (uint2*)(m + o.ymap);
+    Q.step_off = (uint64_t*)(m + o.step);
     Q.ICq = (uint32_t*)(m + o.ICq);
     Q.JRq = (uint32_t*)(m + o.JRq);
     Q.ucap = (uint32_t*)(m + o.ucap);
-    Q.cls = (uint8_t*)(m + o.cls);
-    Q.wrow = (unsigned long long*)(m + o.wrow);
+    Q.bucket = (uint8_t*)(m + o.bucket);
     Q.rc = (RowCtx*)(m + o.rc);
     Q.rs = (Reserve*)(m + o.rs);
     Q.res = (QueryRes*)(m + o.res);
     qp.lists = (uint32_t*)(m + o.lists);
     qp.ncls = (unsigned long long*)(m + o.ncls);
     qp.next_row = (uint32_t*)(m + o.next);
-    qp.part = (uint32_t*)(m + o.part);
-    qp.pbase = (unsigned long long*)(m + o.pbase);
+    for (int op = 0; op < 2; op++) Q.nbucket[op] = qp.ncls + 32 * op + 16;
     return DIM3G_OK;
 }
 
@@ -536,22 +532,18 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
     const Tuning tu = tuning_of(ctx);
     const uint32_t nq = qp.nq;
     Q.cta_rr = tu.cta_rr;
-    BCU(cudaMemsetAsync(qp.ncls, 0, 24 * 8, st));
-    BCU(cudaMemsetAsync(Q.cls, 0, qp.nrows, st));
-    BCU(cudaMemsetAsync(Q.wrow, 0, qp.nrows * 8, st));
-    BCU(cudaMemsetAsync(qp.next_row, 0, 8 * 4, st));
-    k_q_setup<<<(nq + 127) / 128, 128, 0, st>>>(Q);
+    BCU(cudaMemsetAsync(qp.ncls, 0, 64 * 8, st));
+    BCU(cudaMemsetAsync(qp.next_row, 0, 16 * 4, st));
+    BCU(cudaMemsetAsync(Q.bucket, kNoBucket, qp.nrows, st));
+    k_q_setup<<<1, 1024, 0, st>>>(Q);
     BLAUNCH();
     if (qp.ntot) {
         k_q_ymap<<<elem_grid(qp.ntot, sm), 256, 0, st>>>(Q);
         BLAUNCH();
-        k_q_entries<<<elem_grid(qp.ntot, sm), 256, 0, st>>>(Q);
-        BLAUNCH();
     }
-    k_q_rows<<<elem_grid(qp.nrows, sm), 256, 0, st>>>(Q);
-    BLAUNCH();
-    const uint32_t cap_w = 1u << (tu.warp_lg - 1), cap_b = 1u << (tu.block_lg - 1);
-    k_q_row_work<<<elem_grid(qp.nrows, sm), 256, 0, st>>>(Q, cap_w, cap_b);
+    const RowBuckets rb{1u << (tu.warp_lg - 1), 1u << (tu.block_lg - 1), true, tu.block_split != 0,
+                        1u << (tu.block_lg - 3), 1u << (tu.block_lg - 2)};
+    k_q_work<<<elem_grid(qp.ntot + 32 * (uint64_t)nq, sm), 256, 0, st>>>(Q, rb);
     BLAUNCH();
     uint32_t* lw = qp.lists;
     uint32_t* lb = qp.lists + qp.nrows;
@@ -561,31 +553,17 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
     for (int op = 0; op < 2; op++) {
         if (op == 0 && !qp.has_project) continue;
         if (op == 1 && !qp.has_count) continue;
-        const uint8_t k0 = op ? 8 : 0;
-        unsigned long long* n = qp.ncls + 8 * op;  // n[1..5]: rows of classes k0+1..k0+5
-        unsigned long long* nb = qp.ncls + 16 + 4 * op;  // block-class rows by hash-set size (split)
+        unsigned long long* n = qp.ncls + 32 * op;  // n[1..5]: rows per class
+        unsigned long long* nb = n + 8;             // block-class rows by hash-set size
+        uint32_t* next = qp.next_row + 8 * op;
         const bool split = tu.block_split;
-        {
-            // the class lists (and the CTA class by hash-set size) in one partition
-            const uint32_t b = tu.block_lg;
-            const PartSpec ps{k0, split ? 1u : 0u, 1u << (b - 3), 1u << (b - 2)};
-            const uint64_t ntiles = (qp.nrows + kPartTile - 1) / kPartTile;
-            if (ntiles) {
-                k_part_count<<<(unsigned)ntiles, 256, 0, st>>>(Q.cls, Q.ucap, qp.nrows, ps, qp.part);
-                BLAUNCH();
-                k_part_offsets<<<1, 1024, 0, st>>>(qp.part, (uint32_t)ntiles, n, split ? nb : nullptr, qp.pbase);
-                BLAUNCH();
-                k_part_scatter<<<(unsigned)ntiles, 256, 0, st>>>(Q.cls, Q.ucap, qp.nrows, ps, qp.part, qp.pbase, lw, lb,
-                                                                 lm, lt);
-                BLAUNCH();
-            }
-        }
-        BCU(cudaGetLastError());
-        BCU(cudaMemsetAsync(qp.next_row, 0, 8 * 4, st));
+        k_row_lists<<<(unsigned)((qp.nrows + kListTile - 1) / kListTile), 256, 0, st>>>(
+            Q.bucket, (uint32_t)qp.nrows, op ? kCountBuckets : 0, n + 16, n + 24, qp.lists, n, nb);
+        BLAUNCH();
         if (op == 0) {
             const size_t ss_m = (size_t)bm_words * 4 + 16 * kStage * 4;
             k_b_single_bitmap<<<resident(k_b_single_bitmap, 512, ss_m, sm), 512, ss_m, st>>>(
-                Q, BatchRows{lm, &n[4], &n[3], &qp.next_row[0]}, bm_words);
+                Q, BatchRows{lm, &n[4], &n[3], &next[0]}, bm_words);
             BLAUNCH();
             const int blk_b = (int)tu.block_threads;
             if (split) {
@@ -595,13 +573,13 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
                     const uint32_t lg = tu.block_lg - 2 + k;
                     const size_t ss = ((size_t)1 << lg) * 4 + (size_t)(thr / 32) * kStage * 4;
                     k_b_single_block<<<resident(k_b_single_block, thr, ss, sm), thr, ss, st>>>(
-                        Q, BatchRows{lb, &nb[k], nullptr, &qp.next_row[4 + k], skip[k][0], skip[k][1]}, lg);
+                        Q, BatchRows{lb, &nb[k], nullptr, &next[4 + k], skip[k][0], skip[k][1]}, lg);
                     BLAUNCH();
                 }
             } else {
                 const size_t ss_b = ((size_t)1 << tu.block_lg) * 4 + (size_t)(blk_b / 32) * kStage * 4;
                 k_b_single_block<<<resident(k_b_single_block, blk_b, ss_b, sm), blk_b, ss_b, st>>>(
-                    Q, BatchRows{lb, &n[2], nullptr, &qp.next_row[1]}, tu.block_lg);
+                    Q, BatchRows{lb, &n[2], nullptr, &next[1]}, tu.block_lg);
                 BLAUNCH();
             }
             const uint32_t wps = warps_for(warp_row_words(tu.warp_lg, kStage) * 4);
@@ -616,7 +594,7 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
         } else {
             const size_t ss_m = 200 << 10;
             k_b_agg_ranked<<<resident(k_b_agg_ranked, 1024, ss_m, sm), 1024, ss_m, st>>>(
-                Q, BatchRows{lm, &n[4], &n[3], &qp.next_row[2]}, ss_m);
+                Q, BatchRows{lm, &n[4], &n[3], &next[2]}, ss_m);
             BLAUNCH();
             auto map_rows = [&](const BatchRows& rows, uint32_t lg) -> int {
                 const int thr = lg >= 14 ? 1024 : (lg == 13 ? 512 : (lg == 12 ? 256 : 128));
@@ -628,13 +606,13 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
             int r = DIM3G_OK;
             const uint32_t b = tu.block_lg;
             if (split) {
-                r = map_rows(BatchRows{lb, &nb[2], nullptr, &qp.next_row[6], &nb[0], &nb[1]}, b);
-                if (!r) r = map_rows(BatchRows{lb, &nb[1], nullptr, &qp.next_row[5], &nb[0], nullptr}, b - 1);
-                if (!r) r = map_rows(BatchRows{lb, &nb[0], nullptr, &qp.next_row[4]}, b - 2);
+                r = map_rows(BatchRows{lb, &nb[2], nullptr, &next[6], &nb[0], &nb[1]}, b);
+                if (!r) r = map_rows(BatchRows{lb, &nb[1], nullptr, &next[5], &nb[0], nullptr}, b - 1);
+                if (!r) r = map_rows(BatchRows{lb, &nb[0], nullptr, &next[4]}, b - 2);
             } else {
-                r = map_rows(BatchRows{lb, &n[2], nullptr, &qp.next_row[3]}, b);
+                r = map_rows(BatchRows{lb, &n[2], nullptr, &next[3]}, b);
             }
-            if (!r) r = map_rows(BatchRows{lw, &n[1], nullptr, &qp.next_row[0]}, tu.warp_lg);
+            if (!r) r = map_rows(BatchRows{lw, &n[1], nullptr, &next[0]}, tu.warp_lg);
             if (r) return r;
             const size_t ss_t = 8 * kAggPackWords * 4;
             k_b_agg_pack<<<resident(k_b_agg_pack, 256, ss_t, sm), 256, ss_t, st>>>(
@@ -700,6 +678,8 @@ int relset_build_sync(dim3g_relset* s, const dim3g_relation* rels) {
         const uint32_t err = (uint32_t)s->h_need[1];
         if (need <= s->yt_cap) {
             if (err) return I::fail(ctx, DIM3G_ERR_DEVICE, "relation set build: device bound violated (flags %u)", err);
+            s->h_nf.resize(s->nrel);
+            BCU(cudaMemcpy(s->h_nf.data(), s->P.nf_cnt, s->nrel * 8, cudaMemcpyDeviceToHost));
             return DIM3G_OK;
         }
         r = relset_plan(s, rels, s->nrel, need);  // regrow the (y, tile) pool

@@ -123,7 +123,6 @@ struct RelPools {
     uint32_t* JRf;            // ntot + 1, global positions
     uint32_t* curF;
     uint32_t* ICf;            // global y ids
-    uint32_t* ICr;            // the row (local f id) of each ICf entry
     uint32_t* cnt_yt;         // yt_cap
     uint32_t* JRy;            // yt_cap, global positions
     uint32_t* curY;
@@ -276,7 +275,6 @@ static __global__ void k_ix_scatter(RelPools P) {
         if (ro & kRoleRows) {
             const uint32_t pos = atomicAdd(&P.curF[pm.x], 1u);
             P.ICf[pos] = pm.y;
-            P.ICr[pos] = fl;
         }
         if (ro & kRoleCols) {
             const uint64_t key = d.yt_base + (uint64_t)(pm.y - d.ybase) * d.T + (fl >> d.tile_shift);
@@ -343,16 +341,16 @@ struct QueryPools {
     const uint32_t* id2y;
     const uint32_t* JRf;
     const uint32_t* ICf;
-    const uint32_t* ICr;
     const uint32_t* JRy;
     const uint32_t* ICy;
     const uint32_t* VSy;
-    uint32_t* ymap;   // ntot
+    uint2* ymap;      // ntot: per y id of P, Q's y id and its tuples
+    uint64_t* step_off;  // nq + 1: prefix of the queries' warp steps (k_q_work)
     uint32_t* ICq;    // ntot: P entries as Q y ids
     uint32_t* JRq;    // nrows: P row pointers, relative
     uint32_t* ucap;   // nrows
-    uint8_t* cls;     // nrows
-    unsigned long long* wrow;  // nrows: candidates per row
+    uint8_t* bucket;  // nrows: RowBuckets, COUNT rows from kCountBuckets on
+    unsigned long long* nbucket[2];  // rows per bucket: join-project, COUNT
     RowCtx* rc;       // nq
     Reserve* rs;      // nq
     QueryRes* res;    // nq
@@ -377,47 +375,20 @@ static __global__ void k_q_ymap(QueryPools Q) {
         const uint64_t y = i - sc.lo;
         if (y >= p.ny) continue;
         const uint32_t g = table_find(rel_table((unsigned long long*)Q.TY, q), Q.id2y[p.ybase + y]);
-        Q.ymap[i] = g == kNotFound ? (uint32_t)q.ny : g - (uint32_t)q.ybase;
-    }
-}
-
-// P's CSR entries as Q y ids.
-static __global__ void k_q_entries(QueryPools Q) {
-    if (!layout_ok(Q)) return;
-    SegCursor sc{Q.qt_off, Q.nq};
-    DIM3G_FOR_CHUNK(i, Q.ntot) {
-        const uint32_t qi = sc.at(i);
-        const RelDev& p = Q.rel[Q.qin[qi].p];
-        const uint64_t e = i - sc.lo;
-        const uint32_t yg = Q.ICf[p.tup_off + e];
-        const uint32_t yq = Q.ymap[sc.lo + (yg - p.ybase)];
-        Q.ICq[i] = yq;
-        // candidates of the entry: its S segment over all z tiles
-        const RelDev& q = Q.rel[Q.qin[qi].q];
+        const uint32_t yq = g == kNotFound ? (uint32_t)q.ny : g - (uint32_t)q.ybase;
         const uint32_t* jr = Q.JRy + q.yt_base + (uint64_t)yq * q.T;
-        const uint32_t len = jr[q.T] - jr[0];
-        // entries of one row are contiguous: one atomic per run of a row
-        const uint64_t g = Q.qrow_off[qi] + Q.ICr[p.tup_off + e];
-        atomic_add_grouped(&Q.wrow[g], g, len);
+        Q.ymap[i] = make_uint2(yq, jr[q.T] - jr[0]);
     }
 }
 
-// P's row pointers relative to P's first entry.
-static __global__ void k_q_rows(QueryPools Q) {
-    if (!layout_ok(Q)) return;
-    SegCursor sc{Q.qrow_off, Q.nq};
-    DIM3G_FOR_CHUNK(i, Q.nrows) {
-        const uint32_t qi = sc.at(i);
-        const RelDev& p = Q.rel[Q.qin[qi].p];
-        const uint64_t x = i - sc.lo;
-        if (x <= Q.res[qi].nx) Q.JRq[i] = Q.JRf[p.fbase + x] - (uint32_t)p.tup_off;
-    }
+// Lanes a row (log2) of a query's k_q_work steps.
+__device__ __forceinline__ uint32_t query_lanes(const RelDev& p) {
+    const uint64_t per_row = p.nf ? p.nt / p.nf : 0;
+    return per_row > 64 ? 5u : (per_row > 24 ? 4u : (per_row > 8 ? 3u : 2u));
 }
 
-// One thread per query: its row context and output reservation.
-static __global__ void k_q_setup(QueryPools Q) {
-    const uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (qi >= Q.nq) return;
+// A query's row context and output reservation.
+__device__ __forceinline__ void query_setup(const QueryPools& Q, uint32_t qi) {
     const QueryIn qn = Q.qin[qi];
     const RelDev& p = Q.rel[qn.p];
     const RelDev& q = Q.rel[qn.q];
@@ -451,158 +422,124 @@ static __global__ void k_q_setup(QueryPools Q) {
     Q.res[qi] = r;
 }
 
-// Per-row class (1..5 project, 9..13 COUNT) from the candidates counted per
-// row by k_q_entries; one thread per row of the row space.
-static __global__ void k_q_row_work(QueryPools Q, uint32_t cap_w, uint32_t cap_b) {
-    if (!layout_ok(Q)) return;
-    SegCursor sc{Q.qrow_off, Q.nq};
-    DIM3G_FOR_CHUNK(g, Q.nrows) {
-        const uint32_t qi = sc.at(g);
-        const uint64_t x = g - sc.lo;
-        if (x >= Q.res[qi].nx) continue;
-        const unsigned long long w = Q.wrow[g];
-        const uint32_t m = Q.res[qi].nz;
-        const uint32_t u = (uint32_t)(w < m ? w : m);
-        Q.ucap[g] = u;
-        const bool count = Q.qin[qi].op == kOpCount;
-        uint32_t k = row_class(w, u, cap_w, count ? agg_cap_b(m, cap_b) : cap_b, true);
-        if (k && count) {
-            k += 8;
-            if (w >= 0xFFFFFFFFull) raise_error(&Q.res[qi].err, kErrCountRange);
-        }
-        Q.cls[g] = (uint8_t)k;
-        atomic_add_grouped(&Q.res[qi].out_j, qi, w);  // one atomic per query run
-    }
-}
-
-// ---- class lists in one partition of the row space (instead of one
-// prefix sum per class).  A row's bucket: 0 warp class (k0+1); 1..3 CTA
-// class (k0+2), by distinct bound u <= capS, u <= capM, larger when split
-// (else all 1); 4 huge bitmap rows (k0+4); 5 bitmap rows (k0+3); 6 tiny
-// rows (k0+5); 7 none.  Three launches: per-tile bucket counts, their
-// prefix per bucket (one CTA), the scatter into the lists.  Order within a
-// list is unspecified (rows are claimed dynamically anyway).
-constexpr uint32_t kPartItems = 16;
-constexpr uint32_t kPartTile = 256 * kPartItems;  // rows a CTA tile
-constexpr uint32_t kPartBuckets = 7;
-struct PartSpec {
-    uint32_t k0, split, capS, capM;
-};
-__device__ __forceinline__ uint32_t row_bucket(const uint8_t* __restrict__ cls, const uint32_t* __restrict__ ucap,
-                                               uint64_t i, const PartSpec& ps) {
-    const uint32_t c = cls[i];
-    if (c == ps.k0 + 1u) return 0;
-    if (c == ps.k0 + 2u) {
-        if (!ps.split) return 1;
-        const uint32_t u = ucap[i];
-        return u <= ps.capS ? 1u : (u <= ps.capM ? 2u : 3u);
-    }
-    if (c == ps.k0 + 4u) return 4;
-    if (c == ps.k0 + 3u) return 5;
-    if (c == ps.k0 + 5u) return 6;
-    return 7;
-}
-
-// hist[tile * 8 + b] = rows of bucket b in the tile.
-static __global__ void __launch_bounds__(256) k_part_count(const uint8_t* __restrict__ cls,
-                                                           const uint32_t* __restrict__ ucap, uint64_t n, PartSpec ps,
-                                                           uint32_t* __restrict__ hist) {
-    __shared__ uint32_t s[8];
-    if (threadIdx.x < 8) s[threadIdx.x] = 0;
-    __syncthreads();
-    const uint64_t base = (uint64_t)blockIdx.x * kPartTile;
-    uint32_t c[kPartBuckets];
-#pragma unroll
-    for (uint32_t b = 0; b < kPartBuckets; b++) c[b] = 0;
-#pragma unroll 4
-    for (uint32_t k = 0; k < kPartItems; k++) {
-        const uint64_t i = base + (uint64_t)k * 256 + threadIdx.x;
-        const uint32_t b = i < n ? row_bucket(cls, ucap, i, ps) : 7u;
-#pragma unroll
-        for (uint32_t q = 0; q < kPartBuckets; q++) c[q] += b == q ? 1u : 0u;
-    }
-#pragma unroll
-    for (uint32_t q = 0; q < kPartBuckets; q++) {
-        const uint32_t v = warp_sum(c[q]);
-        if ((threadIdx.x & 31) == 0 && v) atomicAdd(&s[q], v);
-    }
-    __syncthreads();
-    if (threadIdx.x < kPartBuckets) hist[(uint64_t)blockIdx.x * 8 + threadIdx.x] = s[threadIdx.x];
-}
-
-// One CTA: hist becomes each tile's first position in its bucket; the
-// bucket totals go to the class counts (n[1..5] as the class prefix sums
-// gave them; nb[0..2] the split CTA class), base[b] = where bucket b starts
-// in its list.
-static __global__ void __launch_bounds__(1024) k_part_offsets(uint32_t* __restrict__ hist, uint32_t ntiles,
-                                                              unsigned long long* n, unsigned long long* nb,
-                                                              unsigned long long* base) {
+// One CTA: every query's setup, and the warp steps of its rows (the rows of a
+// step share a warp; nx + 1 row pointers).
+static __global__ void __launch_bounds__(1024) k_q_setup(QueryPools Q) {
     __shared__ uint64_t sm[1024 / 32 + 1];
-    __shared__ unsigned long long tot[8];
-    for (uint32_t b = 0; b < kPartBuckets; b++) {
-        uint64_t carry = 0;
-        for (uint32_t t0 = 0; t0 < ntiles; t0 += 1024) {
-            const uint32_t t = t0 + threadIdx.x;
-            const uint64_t v = t < ntiles ? hist[(uint64_t)t * 8 + b] : 0u;
-            uint64_t sum;
-            const uint64_t e = block_excl_scan<1024>(v, sm, &sum);
-            if (t < ntiles) hist[(uint64_t)t * 8 + b] = (uint32_t)(carry + e);
-            carry += sum;
+    uint64_t carry = 0;
+    for (uint32_t b = 0; b < Q.nq; b += 1024) {
+        const uint32_t qi = b + threadIdx.x;
+        uint64_t steps = 0;
+        if (qi < Q.nq) {
+            query_setup(Q, qi);
+            const uint32_t per = 32u >> query_lanes(Q.rel[Q.qin[qi].p]);
+            steps = layout_ok(Q) ? (Q.res[qi].nx + per) / per : 0;
         }
-        if (threadIdx.x == 0) tot[b] = carry;
+        uint64_t sum;
+        const uint64_t e = block_excl_scan<1024>(steps, sm, &sum);
+        if (qi < Q.nq) Q.step_off[qi] = carry + e;
+        carry += sum;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        n[1] = tot[0];
-        n[2] = tot[1] + tot[2] + tot[3];
-        if (nb) {
-            nb[0] = tot[1];
-            nb[1] = tot[2];
-            nb[2] = tot[3];
-        }
-        n[4] = tot[4];
-        n[3] = tot[5];
-        n[5] = tot[6];
-        base[0] = 0;
-        base[1] = 0;
-        base[2] = tot[1];
-        base[3] = tot[1] + tot[2];
-        base[4] = 0;
-        base[5] = tot[4];
-        base[6] = 0;
-    }
+    if (threadIdx.x == 0) Q.step_off[Q.nq] = carry;
 }
 
-// Each row of a bucket to list[base[b] + its tile's offset + its rank in the
-// tile] (one shared atomic per group of lanes with the same bucket).
-static __global__ void __launch_bounds__(256) k_part_scatter(const uint8_t* __restrict__ cls,
-                                                             const uint32_t* __restrict__ ucap, uint64_t n,
-                                                             PartSpec ps, const uint32_t* __restrict__ off,
-                                                             const unsigned long long* __restrict__ base,
-                                                             uint32_t* lw, uint32_t* lb, uint32_t* lm,
-                                                             uint32_t* lt) {
-    __shared__ uint32_t s[8];
-    __shared__ unsigned long long s_at[8];
-    if (threadIdx.x < kPartBuckets) {
-        s[threadIdx.x] = 0;
-        s_at[threadIdx.x] = base[threadIdx.x] + off[(uint64_t)blockIdx.x * 8 + threadIdx.x];
-    }
+// The rows of all queries: P's entries as Q's y ids, P's row pointers, the
+// row's candidates and its bucket.  A warp step is 32 >> lg rows of one query,
+// 2^lg lanes a row, about as many as its rows have entries on average (a row
+// of more than 4 x 2^lg is finished by the whole warp; see k_row_work).  Row
+// space planned from tuple counts, past a query's distinct first values, is
+// not visited.  An entry costs one random sector (its y id's ymap pair).
+// In place of three passes with a per-entry atomic on the row's candidates
+// (16 resident queries of 35M entries: 1020 us; 48-join batch: 345 us).
+constexpr uint32_t kCountBuckets = 8, kNoBucket = 0xFF;
+static __global__ void __launch_bounds__(256) k_q_work(QueryPools Q, RowBuckets rb) {
+    __shared__ uint32_t s_n[2][kRowBuckets + 1];
+    if (threadIdx.x < 2 * (kRowBuckets + 1)) s_n[threadIdx.x / (kRowBuckets + 1)][threadIdx.x % (kRowBuckets + 1)] = 0;
     __syncthreads();
-    const uint64_t t0 = (uint64_t)blockIdx.x * kPartTile;
     const uint32_t lane = lane_id();
-    for (uint32_t k = 0; k < kPartItems; k++) {
-        const uint64_t i = t0 + (uint64_t)k * 256 + threadIdx.x;
-        const uint32_t b = i < n ? row_bucket(cls, ucap, i, ps) : 7u;
-        const unsigned grp = __match_any_sync(0xffffffffu, b);
-        const int leader = __ffs(grp) - 1;
-        uint32_t r0 = 0;
-        if ((int)lane == leader && b < kPartBuckets) r0 = atomicAdd(&s[b], (uint32_t)__popc(grp));
-        r0 = __shfl_sync(0xffffffffu, r0, leader);
-        if (b < kPartBuckets) {
-            const unsigned long long pos = s_at[b] + r0 + __popc(grp & lanemask_lt());
-            uint32_t* list = b == 0 ? lw : (b <= 3 ? lb : (b <= 5 ? lm : lt));
-            list[pos] = (uint32_t)i;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t steps = layout_ok(Q) ? Q.step_off[Q.nq] : 0;
+    uint64_t lo = 1, hi = 0;  // steps of the warp's query
+    uint32_t qi = 0, nx = 0, m = 0, fam = 0, lg = 5, tup_off = 0;
+    const uint32_t* jp = nullptr;  // P's row pointers (from tup_off on)
+    const uint32_t* icf = nullptr;  // P's entries (global y ids)
+    const uint2* ymap = nullptr;    // indexed by P's global y id
+    uint32_t* icq = nullptr;
+    unsigned long long acc = 0;  // candidates of the warp's query, lane's share
+    for (uint64_t s = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < steps; s += nwarps) {
+        if (s < lo || s >= hi) {
+            acc = warp_sum(acc);
+            if (lane == 0 && acc) atomicAdd(&Q.res[qi].out_j, acc);
+            acc = 0;
+            qi = seg_find(Q.step_off, Q.nq, s);
+            lo = Q.step_off[qi];
+            hi = Q.step_off[qi + 1];
+            const QueryIn qn = Q.qin[qi];
+            const RelDev& p = Q.rel[qn.p];
+            nx = Q.res[qi].nx;
+            m = Q.res[qi].nz;
+            fam = qn.op == kOpCount;
+            lg = query_lanes(p);
+            tup_off = (uint32_t)p.tup_off;
+            jp = Q.JRf + p.fbase;
+            icf = Q.ICf + p.tup_off;
+            ymap = Q.ymap + Q.qt_off[qi] - p.ybase;
+            icq = Q.ICq + Q.qt_off[qi];
         }
+        const uint32_t G = 1u << lg, gl = lane & (G - 1);
+        const uint64_t x = ((s - lo) << (5 - lg)) + (lane >> lg), g = Q.qrow_off[qi] + x;
+        const bool live = x < nx;
+        uint32_t e0 = 0, e1 = 0;
+        if (x <= nx) {
+            e0 = jp[x] - tup_off;
+            if (gl == 0) Q.JRq[g] = e0;
+            e1 = live ? jp[x + 1] - tup_off : e0;
+        }
+        unsigned long long w = 0;
+        const uint32_t head = min(e1, e0 + 4 * G);
+        uint32_t y[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) y[k] = e0 + gl + k * G < head ? __ldg(&icf[e0 + gl + k * G]) : kEmpty32;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++)
+            if (y[k] != kEmpty32) {
+                const uint2 t = __ldg(&ymap[y[k]]);
+                icq[e0 + gl + k * G] = t.x;
+                w += t.y;
+            }
+        // the rest of the warp's long rows, all lanes on one row at a time
+        for (uint32_t longs = __ballot_sync(0xffffffffu, gl == 0 && head < e1); longs; longs &= longs - 1) {
+            const int src = __ffs(longs) - 1;
+            const uint32_t b0 = __shfl_sync(0xffffffffu, head, src), b1 = __shfl_sync(0xffffffffu, e1, src);
+            unsigned long long v = 0;
+#pragma unroll 4
+            for (uint32_t e = b0 + lane; e < b1; e += 32) {
+                const uint2 t = __ldg(&ymap[__ldg(&icf[e])]);
+                icq[e] = t.x;
+                v += t.y;
+            }
+            v = warp_sum(v);
+            if ((int)lane == src) w += v;
+        }
+        for (uint32_t o = G >> 1; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+        if (gl == 0 && live) {
+            const uint32_t u = (uint32_t)(w < m ? w : m);
+            const uint32_t k = rb.of(row_class(w, u, rb.cap_w, fam ? agg_cap_b(m, rb.cap_b) : rb.cap_b, rb.tiny), u);
+            Q.ucap[g] = u;
+            if (fam && w >= 0xFFFFFFFFull) raise_error(&Q.res[qi].err, kErrCountRange);
+            acc += w;
+            if (k < kRowBuckets) {
+                Q.bucket[g] = (uint8_t)(fam * kCountBuckets + k);
+                atomicAdd(&s_n[fam][k], 1u);
+            }
+        }
+    }
+    acc = warp_sum(acc);
+    if (lane == 0 && acc) atomicAdd(&Q.res[qi].out_j, acc);
+    __syncthreads();
+    if (threadIdx.x < 2 * (kRowBuckets + 1)) {
+        const uint32_t fam = threadIdx.x / (kRowBuckets + 1), k = threadIdx.x % (kRowBuckets + 1);
+        if (k < kRowBuckets && s_n[fam][k]) atomicAdd(&Q.nbucket[fam][k], (unsigned long long)s_n[fam][k]);
     }
 }
 

@@ -774,7 +774,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     uint32_t* list_b = lists + n;
     uint32_t* list_m = lists + 2 * (uint64_t)n;
     uint32_t* list_t = lists + 3 * (uint64_t)n;
-    k_row_lists<<<(unsigned)((n + kListTile - 1) / kListTile), 256, 0, st>>>(bucket, n, sc->nbucket, sc->list_cur, lists,
+    k_row_lists<<<(unsigned)((n + kListTile - 1) / kListTile), 256, 0, st>>>(bucket, n, 0, sc->nbucket, sc->list_cur, lists,
                                                                              sc->nrows, sc->nrows_b);
     CHECK_LAUNCH();
     CU(cudaEventRecord(c->ev[2], st));

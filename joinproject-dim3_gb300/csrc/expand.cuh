@@ -853,9 +853,10 @@ inline uint32_t row_work_lanes(double per_row) { return per_row > 64 ? 5 : (per_
 // its kListTile rows in shared memory and takes one range of each bucket from
 // its cursor.  One launch (a prefix sum per bucket was three each).  Rows of
 // a tile stay in order and together; the order of tiles is unspecified.  The
-// class counts go to n[1..5] and nb[0..2].
+// class counts go to n[1..5] and nb[0..2].  Buckets are stored from k0 on
+// (many-query passes keep two families of rows in one array).
 constexpr uint32_t kListItems = 8, kListTile = 256 * kListItems;
-static __global__ void __launch_bounds__(256) k_row_lists(const uint8_t* __restrict__ bucket, uint32_t n,
+static __global__ void __launch_bounds__(256) k_row_lists(const uint8_t* __restrict__ bucket, uint32_t n, uint32_t k0,
                                                           const unsigned long long* __restrict__ nbucket,
                                                           unsigned long long* cursor, uint32_t* __restrict__ lists,
                                                           unsigned long long* nrows, unsigned long long* nrows_b) {
@@ -869,7 +870,8 @@ static __global__ void __launch_bounds__(256) k_row_lists(const uint8_t* __restr
 #pragma unroll
     for (uint32_t k = 0; k < kListItems; k++) {
         const uint64_t x = t0 + k * 256 + threadIdx.x;
-        b[k] = x < n ? bucket[x] : kRowBuckets;
+        b[k] = x < n ? bucket[x] - k0 : kRowBuckets;
+        b[k] = b[k] < kRowBuckets ? b[k] : kRowBuckets;
     }
 #pragma unroll
     for (uint32_t k = 0; k < kListItems; k++) {
