@@ -19,6 +19,7 @@
 #include <string.h>
 
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/dim3gpu.h"
@@ -32,6 +33,7 @@
 #include "scan.cuh"
 #include "single.cuh"
 #include "stream.cuh"
+#include "ordered.cuh"
 #include "packed.cuh"
 #include "prefetch.cuh"
 
@@ -259,6 +261,38 @@ unsigned resident_grid(K kernel, int block, size_t smem, int sm) {
         per = 1;
     }
     return (unsigned)(per * sm);
+}
+
+// The block class's launches: its rows in three lists by distinct bound u (<=
+// 2^(b-3), <= 2^(b-2), the rest; b = block_slots_log2), 2^lg table words each:
+// a set of 2u slots, or the bitmap of the whole domain where every row of the
+// list takes that (use_row_bitmap) and it is smaller -- 15 KB instead of 64
+// for m = 121K, so four CTAs an SM instead of two.  The smaller tables run in
+// 256-thread CTAs.  Lists of one size are one launch.
+struct BlockPart {
+    uint32_t lg;
+    int threads;
+};
+struct BlockParts {
+    uint32_t n;
+    BlockPart p[3];
+    const unsigned long long* rows(const Scalars* sc, uint32_t k) const { return n == 1 ? &sc->nrows[2] : &sc->nrows_b[k]; }
+    const unsigned long long* skip0(const Scalars* sc, uint32_t k) const { return k > 0 ? &sc->nrows_b[0] : nullptr; }
+    const unsigned long long* skip1(const Scalars* sc, uint32_t k) const { return k > 1 ? &sc->nrows_b[1] : nullptr; }
+};
+BlockParts block_parts(const dim3g_ctx* c, uint32_t m, int threads, bool split) {
+    const uint32_t b = c->prm.block_lg;
+    if (!split) return BlockParts{1, {{b, threads}}};
+    uint32_t words_lg = 0;
+    while ((1ull << words_lg) < row_bitmap_words(m)) words_lg++;
+    BlockParts r{3, {}};
+    for (uint32_t k = 0; k < 3; k++) {
+        uint32_t lg = b - 2 + k;
+        if (k && (uint64_t)m <= kBitmapPerZ * (1u << (b - 4 + k)) && words_lg < lg) lg = words_lg > b - 2 ? words_lg : b - 2;
+        r.p[k] = BlockPart{lg, lg < b ? (int)kBlockSplitThreads : threads};
+    }
+    if (r.p[0].lg == r.p[2].lg) r.n = 1;
+    return r;
 }
 
 // ------------------------------------------------------------ dense block
@@ -760,11 +794,13 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     rc.id2z = id2z;
     rc.out = nullptr;
     rc.err = &sc->err;
-    // tiny rows go many to a warp in the single pass, and the block class is
-    // split by hash-set size (2^lg slots for 2u keys) there and for COUNT
-    const bool block_split = c->prm.block_split && (jp.aggregate || (single && !(c->prm.prefetch_rows && c->prm.cta_rr == 3)));
+    // tiny rows go many to a warp but in summaries and COUNT at exact
+    // offsets; the block class is split by hash-set size (2^lg slots for 2u
+    // keys)
+    const bool block_split = c->prm.block_split && !(single && !jp.aggregate && c->prm.prefetch_rows && c->prm.cta_rr == 3);
+    const bool tiny = single || (!jp.aggregate && !jp.sum.tiles);
     const uint32_t cap_w = 1u << (c->prm.warp_lg - 1), cap_b = 1u << (c->prm.block_lg - 1);
-    const RowBuckets rb{cap_w, jp.aggregate ? agg_cap_b(m, cap_b) : cap_b, single, block_split,
+    const RowBuckets rb{cap_w, jp.aggregate ? agg_cap_b(m, cap_b) : cap_b, tiny, block_split,
                         1u << (c->prm.block_lg - 3), 1u << (c->prm.block_lg - 2)};
     const uint32_t lanes = row_work_lanes((double)jp.nP / n);
     k_row_work<<<grid_for((uint64_t)n << lanes, sm), 256, 0, st>>>(rc, n, lanes, rb, jp.aggregate, jp.sum, ucap, bucket,
@@ -793,10 +829,17 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     size_t smem_m = (size_t)((((tile_width + 31) / 32) + 3) / 4) * 16;  // whole uint4 words (cleared as uint4)
     if (smem_m < 128) smem_m = 128;  // idle lanes touch words 0..31
     const int blk_m = tile_width > (1u << 19) ? 1024 : DIM3G_BM_THREADS;
-    const unsigned g_w = resident_grid(k_rows_warp<true>, 32 * wpc, smem_w, sm);
     const int blk_b = (int)c->prm.block_threads;
-    const unsigned g_b = resident_grid(k_rows_block<true>, blk_b, smem_b, sm);
-    const unsigned g_m = resident_grid(k_rows_bitmap<true>, blk_m, smem_m, sm);
+    const BlockParts parts = block_parts(c, m, blk_b, block_split);
+    // Launches whose class holds no row are left out: from the class
+    // counts where the host has them, else from u <= m (a launch over an
+    // empty list is about 3 us of a small join).
+    const Scalars& h = *c->h_sc;
+    const bool has_m = dp.counted ? h.nrows[3] + h.nrows[4] != 0 : m > rb.cap_b;
+    const bool has_b[3] = {!dp.counted || h.nrows_b[0], dp.counted ? h.nrows_b[1] != 0 : m > rb.cap_s,
+                           dp.counted ? h.nrows_b[2] != 0 : m > rb.cap_m};
+    const bool has_any_b = !dp.counted || h.nrows[2], has_w = !dp.counted || h.nrows[1],
+               has_t = !dp.counted || h.nrows[5];
 
     if (jp.sum.tiles) {
         // summaries: the expansion kernels hash instead of writing; COUNT
@@ -888,15 +931,6 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
                 list_m, dp.nd, dp.D, dp.Wd, dp.Wm, dp.cpr, dp.coff, id2x, id2z, out, nullptr, &sc->dense_base);
             CHECK_LAUNCH();
         }
-        // Launches whose class holds no row are left out: from the class
-        // counts where the host has them, else from u <= m (a launch over an
-        // empty list is about 3 us of a small join).
-        const Scalars& h = *c->h_sc;
-        const bool has_m = dp.counted ? h.nrows[3] + h.nrows[4] != 0 : m > rb.cap_b;
-        const bool has_b[3] = {!dp.counted || h.nrows_b[0], dp.counted ? h.nrows_b[1] != 0 : m > rb.cap_s,
-                               dp.counted ? h.nrows_b[2] != 0 : m > rb.cap_m};
-        const bool has_any_b = !dp.counted || h.nrows[2], has_w = !dp.counted || h.nrows[1],
-                   has_t = !dp.counted || h.nrows[5];
         // the cross-segment gather's threshold per row class, measured on
         // the 2-hop (bitmap rows 45.5 -> 44.7 ms at 160, block rows 26.3 ->
         // 25.7 at 560, warp rows 2.62 -> 2.58 at 160; every setting exact)
@@ -921,24 +955,15 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
             k_single_block_pf<<<resident_grid(k_single_block_pf, kPfThreads, ss_p, sm), kPfThreads, ss_p, st>>>(
                 rc, rs, L.b, L.nb, c->prm.block_lg);
             CHECK_LAUNCH();
-        } else if (block_split) {
-            // three launches over list_b's three parts, smallest sets first
-            const uint32_t b = c->prm.block_lg;
-            const unsigned long long* skip[3][2] = {{nullptr, nullptr}, {&sc->nrows_b[0], nullptr},
-                                                    {&sc->nrows_b[0], &sc->nrows_b[1]}};
-            for (uint32_t k = 0; k < 3; k++) {
-                if (!has_b[k]) continue;
-                const int thr = k < 2 ? (int)kBlockSplitThreads : blk_b;
-                const uint32_t lg = b - 2 + k;
-                const size_t ss = ((size_t)1 << lg << 2) + (size_t)(thr / 32) * kStage * 4;
-                k_single_block<<<resident_grid(k_single_block, thr, ss, sm), thr, ss, st>>>(
-                    rc, rs, L.b, &sc->nrows_b[k], lg, skip[k][0], skip[k][1], 4 + k);
+        } else {
+            for (uint32_t k = 0; k < parts.n; k++) {
+                if (parts.n > 1 && !has_b[k]) continue;
+                const BlockPart& p = parts.p[k];
+                const size_t ss = ((size_t)1 << p.lg << 2) + (size_t)(p.threads / 32) * kStage * 4;
+                k_single_block<<<resident_grid(k_single_block, p.threads, ss, sm), p.threads, ss, st>>>(
+                    rc, rs, L.b, parts.rows(sc, k), p.lg, parts.skip0(sc, k), parts.skip1(sc, k), 4 + k);
                 CHECK_LAUNCH();
             }
-        } else {
-            k_single_block<<<resident_grid(k_single_block, blk_b, ss_b, sm), blk_b, ss_b, st>>>(
-                rc, rs, L.b, L.nb, c->prm.block_lg, nullptr, nullptr, 2);
-            CHECK_LAUNCH();
         }
         CU(cudaEventRecord(c->evc[6], st));
         CU(cudaMemcpyAsync(&sc->cursor_at[1], &sc->cursor, 8, cudaMemcpyDeviceToDevice, st));
@@ -992,14 +1017,39 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         k_dense_rowcnt<<<grid_for(dp.nd, sm), 256, 0, st>>>(list_m, dp.nd, dp.cpr, dp.coff, cnt);
         CHECK_LAUNCH();
     }
-    k_rows_bitmap<false><<<g_m, blk_m, smem_m, st>>>(rc, L.m, L.n3, L.n4);
-    CHECK_LAUNCH();
-    CU(cudaEventRecord(c->evc[1], st));
-    k_rows_block<false><<<g_b, blk_b, smem_b, st>>>(rc, L.b, L.nb, c->prm.block_lg);
-    CHECK_LAUNCH();
-    CU(cudaEventRecord(c->evc[2], st));
-    k_rows_warp<false><<<g_w, 32 * wpc, smem_w, st>>>(rc, L.w, L.nw, c->prm.warp_lg);
-    CHECK_LAUNCH();
+    // the row kernels of one pass over the classes, with an event after each
+    auto pass = [&](auto write, cudaEvent_t* ev) -> int {
+        constexpr bool W = decltype(write)::value;
+        if (has_m) {
+            k_rows_bitmap<W><<<resident_grid(k_rows_bitmap<W>, blk_m, smem_m, sm), blk_m, smem_m, st>>>(rc, L.m, L.n3, L.n4);
+            CHECK_LAUNCH();
+        }
+        CU(cudaEventRecord(ev[1], st));
+        for (uint32_t k = 0; k < parts.n; k++) {
+            if (!has_any_b || (parts.n > 1 && !has_b[k])) continue;
+            const BlockPart& p = parts.p[k];
+            const size_t ss = (size_t)1 << p.lg << 2;
+            k_rows_block<W><<<resident_grid(k_rows_block<W>, p.threads, ss, sm), p.threads, ss, st>>>(
+                rc, L.b, parts.rows(sc, k), p.lg, parts.skip0(sc, k), parts.skip1(sc, k), 4 + k);
+            CHECK_LAUNCH();
+        }
+        CU(cudaEventRecord(ev[2], st));
+        if (has_w) {
+            k_rows_warp<W><<<resident_grid(k_rows_warp<W>, 32 * wpc, smem_w, sm), 32 * wpc, smem_w, st>>>(
+                rc, L.w, L.nw, c->prm.warp_lg);
+            CHECK_LAUNCH();
+        }
+        if (tiny && has_t) {
+            const size_t ss = 8 * kRowsPackWords * 4;
+            k_rows_pack<W><<<resident_grid(k_rows_pack<W>, 256, ss, sm), 256, ss, st>>>(rc, list_t, &sc->nrows[5]);
+            CHECK_LAUNCH();
+        }
+        return DIM3G_OK;
+    };
+    {
+        int r = pass(std::false_type{}, &c->evc[0]);
+        if (r) return r;
+    }
     CU(cudaEventRecord(c->evc[3], st));
     SCAN(U32Src{cnt}, OffDst{off}, (uint64_t)n + 1, bsum2, &sc->total, &sc->err);
     CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
@@ -1011,12 +1061,12 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     for (int i = 0; i < 3; i++) cudaEventElapsedTime(&S.ms_count_cls[i], c->evc[i], c->evc[i + 1]);
     S.out_j = c->h_sc->outj;
     S.n_out = total;
-    S.rows_warp = (uint32_t)c->h_sc->nrows[1];
+    S.rows_warp = (uint32_t)(c->h_sc->nrows[1] + c->h_sc->nrows[5]);
     S.rows_block = (uint32_t)c->h_sc->nrows[2];
     S.rows_bitmap = (uint32_t)(c->h_sc->nrows[3] + c->h_sc->nrows[4]);
     S.out_j_cls[0] = c->h_sc->outj_cls[3] + c->h_sc->outj_cls[4];
     S.out_j_cls[1] = c->h_sc->outj_cls[2];
-    S.out_j_cls[2] = c->h_sc->outj_cls[1];
+    S.out_j_cls[2] = c->h_sc->outj_cls[1] + c->h_sc->outj_cls[5];
     *n_out = total;
     if (jp.count_only) {
         float a, b, d;
@@ -1046,14 +1096,8 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
                     list_m, dp.nd, dp.D, dp.Wd, dp.Wm, dp.cpr, dp.coff, id2x, id2z, out, off, nullptr);
                 CHECK_LAUNCH();
             }
-            k_rows_bitmap<true><<<g_m, blk_m, smem_m, st>>>(rc, L.m, L.n3, L.n4);
-            CHECK_LAUNCH();
-            CU(cudaEventRecord(c->evc[5], st));
-            k_rows_block<true><<<g_b, blk_b, smem_b, st>>>(rc, L.b, L.nb, c->prm.block_lg);
-            CHECK_LAUNCH();
-            CU(cudaEventRecord(c->evc[6], st));
-            k_rows_warp<true><<<g_w, 32 * wpc, smem_w, st>>>(rc, L.w, L.nw, c->prm.warp_lg);
-            CHECK_LAUNCH();
+            int r = pass(std::true_type{}, &c->evc[4]);
+            if (r) return r;
             CU(cudaEventRecord(c->evc[7], st));
         }
     }
@@ -1328,6 +1372,10 @@ int dim3g_create(int device, dim3g_ctx** out) {
               cudaFuncSetAttribute(k_rows_bitmap<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_m) == cudaSuccess &&
               cudaFuncSetAttribute(k_rows_bitmap<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_m) == cudaSuccess &&
               cudaFuncSetAttribute(k_single_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_wmax) == cudaSuccess &&
+              cudaFuncSetAttribute(k_rows_pack<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(8 * kRowsPackWords * 4)) == cudaSuccess &&
+              cudaFuncSetAttribute(k_rows_pack<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(8 * kRowsPackWords * 4)) == cudaSuccess &&
               cudaFuncSetAttribute(k_single_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * kPackWords * 4)) ==
                   cudaSuccess &&
               cudaFuncSetAttribute(k_single_block, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -9,11 +9,9 @@
 //   class 3/4 (u > cap_b): one CTA per row, a shared-memory bitmap over one
 //                          z tile at a time (S is bucketed by (y, z tile));
 //                          class 4 (u > kHugeRow) rows are scheduled first.
-// CTA classes take rows dynamically from an atomic counter.  Each kernel
-// runs twice: a count pass writes cnt[x] = |distinct z|; after a prefix sum
-// over cnt the write pass repeats the expansion and every first insertion of
-// a z emits (x value, z value) at off[x] + a row-local slot, so each row's
-// pairs are contiguous and the whole output is dense.
+// CTA classes take rows dynamically from an atomic counter.  The single pass
+// (single.cuh, packed.cuh) expands each row once; ordered output (ordered.cuh)
+// expands it twice, counting and then writing at exact offsets.
 #pragma once
 #include "common.cuh"
 
@@ -28,11 +26,13 @@ constexpr uint32_t kTinyU = 256, kTinyW = 4096;
 
 // A hash-class row dedups with a bitmap over the whole z domain instead of
 // a hash set when that bitmap fits the kernel's table memory (2^slots_lg
-// words) and clearing it costs no more than the row's candidates
-// (m <= 32 u, u = min(candidates, m)): no probing, one atomicOr per
-// candidate.  Small z domains with many duplicate candidates take this path.
+// words) and holds at most kBitmapPerZ ids per distinct z (m <= 128 u, u =
+// min(candidates, m)): no probing, one atomicOr per candidate, at m / 32
+// words to clear against 2u to 4u.  (1.2M-edge 2-hop, m = 121K: block rows
+// 983 us at 32 ids per distinct z, 677 at 128.)
+constexpr uint64_t kBitmapPerZ = 128;
 __device__ __forceinline__ bool use_row_bitmap(uint32_t m, uint32_t u, uint32_t slots_lg) {
-    return (uint64_t)m <= (32ull << slots_lg) && (uint64_t)m <= 32ull * u;
+    return (uint64_t)m <= (32ull << slots_lg) && (uint64_t)m <= kBitmapPerZ * u;
 }
 // Row class from its candidates w and u = min(w, m): 5 (one warp, small
 // table; only where the caller runs that kernel) for tiny rows, 1 (one warp)
@@ -57,7 +57,7 @@ __host__ __device__ __forceinline__ uint32_t agg_cap_b(uint64_t m, uint32_t cap_
 }
 // Words of a whole-domain bitmap, rounded to uint4 and at least 32 (idle
 // lanes of TileBitmap touch words 0..31).
-__device__ __forceinline__ uint32_t row_bitmap_words(uint32_t m) {
+__host__ __device__ __forceinline__ uint32_t row_bitmap_words(uint32_t m) {
     const uint32_t w = (((m + 31) >> 5) + 3) & ~3u;
     return w < 32 ? 32 : w;
 }
@@ -629,129 +629,6 @@ __device__ __forceinline__ uint32_t cta_next_row(uint32_t* counter, uint32_t* s_
     if (threadIdx.x == 0) *s_row = atomicAdd(counter, 1u);
     __syncthreads();
     return *s_row;
-}
-
-// Class 1: one warp per row, 2^warp_lg slots per warp.
-template <bool WRITE>
-static __global__ void __launch_bounds__(256) k_rows_warp(RowCtx c, const uint32_t* __restrict__ rows,
-                                                   const unsigned long long* __restrict__ nrows_p, uint32_t warp_lg) {
-    extern __shared__ uint32_t smem[];
-    const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
-    uint32_t* tab = smem + ((size_t)wib << warp_lg);
-    const uint32_t nrows = (uint32_t)*nrows_p;
-    for (uint32_t ri = blockIdx.x * nw + wib; ri < nrows; ri += gridDim.x * nw) {
-        const uint32_t x = rows[ri];
-        const uint32_t u = c.ucap[x];
-        const bool bm = use_row_bitmap(c.m, u, warp_lg);
-        uint32_t lg = ceil_log2(2 * u);
-        lg = lg < 5 ? 5 : (lg > warp_lg ? warp_lg : lg);
-        const uint32_t nclr = bm ? row_bitmap_words(c.m) : (1u << lg);
-        const uint32_t fill = bm ? 0u : kEmpty32;
-        for (uint32_t s = lane; s < nclr; s += 32) tab[s] = fill;
-        __syncwarp();
-        WriteSink wsink{c.out, c.err, 0, 0, 0, nullptr};
-        CountSink csink;
-        if (WRITE) {
-            wsink.base = c.off[x];
-            wsink.lim = c.cnt[x];
-            wsink.xv = c.id2x[x];
-        }
-        if (bm) {
-            TileBitmap set{tab, 0};
-            if (WRITE) warp_expand(c, c.JR_R[x], c.JR_R[x + 1], 0, 0, 0, c.T, set, wsink);
-            else warp_expand(c, c.JR_R[x], c.JR_R[x + 1], 0, 0, 0, c.T, set, csink);
-        } else {
-            HashSet set{tab, lg, c.err};
-            if (WRITE) warp_expand(c, c.JR_R[x], c.JR_R[x + 1], 0, 0, 0, c.T, set, wsink);
-            else warp_expand(c, c.JR_R[x], c.JR_R[x + 1], 0, 0, 0, c.T, set, csink);
-        }
-        if (!WRITE && lane == 0) c.cnt[x] = csink.count;
-        __syncwarp();
-    }
-}
-
-// Class 2: one CTA per row, 2^block_lg slots.
-template <bool WRITE>
-static __global__ void __launch_bounds__(1024) k_rows_block(RowCtx c, const uint32_t* __restrict__ rows,
-                                                    const unsigned long long* __restrict__ nrows_p, uint32_t block_lg) {
-    extern __shared__ uint32_t smem[];
-    __shared__ uint32_t s_count, s_row;
-    const uint32_t wib = threadIdx.x >> 5, lane = lane_id();
-    const uint32_t nw_lg = 31 - __clz(blockDim.x >> 5);
-    const uint32_t nrows = (uint32_t)*nrows_p;
-    for (uint32_t ri = cta_next_row(&c.next_row[2], &s_row); ri < nrows; ri = cta_next_row(&c.next_row[2], &s_row)) {
-        const uint32_t x = rows[ri];
-        const uint32_t u = c.ucap[x];
-        const bool bm = use_row_bitmap(c.m, u, block_lg);
-        uint32_t lg = ceil_log2(2 * u);
-        lg = lg < 5 ? 5 : (lg > block_lg ? block_lg : lg);
-        const uint32_t fill = bm ? 0u : kEmpty32;
-        const uint32_t n4 = (bm ? row_bitmap_words(c.m) : (1u << lg)) / 4;
-        uint4* t4 = reinterpret_cast<uint4*>(smem);
-        for (uint32_t s = threadIdx.x; s < n4; s += blockDim.x) t4[s] = make_uint4(fill, fill, fill, fill);
-        if (threadIdx.x == 0) s_count = 0;
-        __syncthreads();
-        WriteSink wsink{c.out, c.err, 0, 0, 0, &s_count};
-        CountSink csink;
-        if (WRITE) {
-            wsink.base = c.off[x];
-            wsink.lim = c.cnt[x];
-            wsink.xv = c.id2x[x];
-        }
-        if (bm) {
-            TileBitmap set{smem, 0};
-            if (WRITE) warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, 0, c.T, set, wsink);
-            else warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, 0, c.T, set, csink);
-        } else {
-            HashSet set{smem, lg, c.err};
-            if (WRITE) warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, 0, c.T, set, wsink);
-            else warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, 0, c.T, set, csink);
-        }
-        if (!WRITE && lane == 0 && csink.count) atomicAdd(&s_count, csink.count);
-        __syncthreads();
-        if (!WRITE && threadIdx.x == 0) c.cnt[x] = s_count;
-    }
-}
-
-// Classes 3 and 4: one CTA per row, a bitmap over one z tile at a time.  The
-// row list holds the class-4 rows first; nrows = *n4 + *n3.
-template <bool WRITE>
-static __global__ void __launch_bounds__(1024) k_rows_bitmap(RowCtx c, const uint32_t* __restrict__ rows,
-                                                      const unsigned long long* __restrict__ n3,
-                                                      const unsigned long long* __restrict__ n4) {
-    extern __shared__ uint32_t bm[];
-    __shared__ uint32_t s_count, s_row;
-    const uint32_t wib = threadIdx.x >> 5, lane = lane_id();
-    const uint32_t nw_lg = 31 - __clz(blockDim.x >> 5);
-    const uint32_t nrows = (uint32_t)(*n3 + *n4);
-    for (uint32_t ri = cta_next_row(&c.next_row[3], &s_row); ri < nrows; ri = cta_next_row(&c.next_row[3], &s_row)) {
-        const uint32_t x = rows[ri];
-        if (threadIdx.x == 0) s_count = 0;
-        WriteSink wsink{c.out, c.err, 0, 0, 0, &s_count};
-        if (WRITE) {
-            wsink.base = c.off[x];
-            wsink.lim = c.cnt[x];
-            wsink.xv = c.id2x[x];
-        }
-        CountSink csink;
-        for (uint32_t t = 0; t < c.T; t++) {
-            const uint32_t lo = t * c.tile_width;
-            const uint32_t width = min(c.tile_width, c.m - lo);
-            const uint32_t words4 = (((width + 31) >> 5) + 3) >> 2;
-            uint4* b4 = reinterpret_cast<uint4*>(bm);
-            for (uint32_t w = threadIdx.x; w < words4; w += blockDim.x) b4[w] = make_uint4(0, 0, 0, 0);
-            __syncthreads();
-            TileBitmap set{bm, lo};
-            if (WRITE) warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, t, t + 1, set, wsink);
-            else warp_expand(c, c.JR_R[x], c.JR_R[x + 1], wib, nw_lg, t, t + 1, set, csink);
-            __syncthreads();
-        }
-        if (!WRITE) {
-            if (lane == 0 && csink.count) atomicAdd(&s_count, csink.count);
-            __syncthreads();
-            if (threadIdx.x == 0) c.cnt[x] = s_count;
-        }
-    }
 }
 
 // The rows' lists.  A row's bucket: 0 warp class; 1..3 block class, by

@@ -39,8 +39,8 @@ __device__ __forceinline__ uint32_t pack_end(uint32_t u, uint32_t first, uint32_
 }
 
 // Candidates of the pack: the lane's row has entries [e0, e0 + ne) (ne 0:
-// none), keys from key0 on and first value xv.
-//   set.insert(key, active) -> bool; sink.take(b[], xv[], v[], z[])
+// none), keys from key0 on and tag xv.
+//   set.insert(key, active) -> bool; sink.take(b[], xv[], v[])
 template <bool kPair, class Set, class Sink>
 __device__ __forceinline__ void pack_expand(const RowCtx& c, uint32_t e0, uint32_t ne, uint32_t key0, uint32_t xv,
                                             Set& set, Sink& sink) {
@@ -90,19 +90,19 @@ __device__ __forceinline__ void pack_expand(const RowCtx& c, uint32_t e0, uint32
     }
 }
 
-// The rows list[base .. min(base + 32, n)) of a warp as packs into the
-// warp's table and pair stage.  row(i): the row index of list entry i; rows
-// beyond *stop rows belong to another context (many-query lists).
+// The rows of lanes [lo, hi) (x: the lane's row) as packs through the warp's
+// table into the sink.  sink.tag(c, x): what the sink is given with each of
+// the row's candidates.
 template <class Sink>
 __device__ __forceinline__ void pack_rows(const RowCtx& c, uint32_t x, uint32_t lo, uint32_t hi, uint32_t* tab,
                                           Sink& sink) {
     const uint32_t lane = lane_id();
-    uint32_t u = 0, e0 = 0, ne = 0, xv = 0;
+    uint32_t u = 0, e0 = 0, ne = 0, tag = 0;
     if (lane >= lo && lane < hi) {
         u = c.ucap[x];
         e0 = c.JR_R[x];
         ne = c.JR_R[x + 1] - e0;
-        xv = c.id2x[x];
+        tag = sink.tag(c, x);
     }
     for (uint32_t first = lo; first < hi;) {
         uint32_t sum;
@@ -120,12 +120,12 @@ __device__ __forceinline__ void pack_rows(const RowCtx& c, uint32_t x, uint32_t 
         __syncwarp();
         if (bm) {
             TileBitmap set{tab, 0};
-            if (c.ISV) pack_expand<true>(c, e0, n, key0, xv, set, sink);
-            else pack_expand<false>(c, e0, n, key0, xv, set, sink);
+            if (Sink::kValues && c.ISV) pack_expand<true>(c, e0, n, key0, tag, set, sink);
+            else pack_expand<false>(c, e0, n, key0, tag, set, sink);
         } else {
             HashSet set{tab, lg, c.err};
-            if (c.ISV) pack_expand<true>(c, e0, n, key0, xv, set, sink);
-            else pack_expand<false>(c, e0, n, key0, xv, set, sink);
+            if (Sink::kValues && c.ISV) pack_expand<true>(c, e0, n, key0, tag, set, sink);
+            else pack_expand<false>(c, e0, n, key0, tag, set, sink);
         }
         __syncwarp();
         first = end;
@@ -140,6 +140,7 @@ struct PackSink {
     Reserve rs;
     uint32_t n = 0;
 
+    __device__ __forceinline__ uint32_t tag(const RowCtx& c, uint32_t x) const { return c.id2x[x]; }
     __device__ __forceinline__ void flush() {
         if (n == 0) return;
         unsigned long long base = 0;
