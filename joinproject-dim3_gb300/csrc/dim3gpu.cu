@@ -927,7 +927,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         if (dp.on) {
             k_dense_reserve<<<1, 1, 0, st>>>(dp.coff + (uint64_t)dp.nd * dp.cpr, &sc->cursor, cap, &sc->dense_base);
             CHECK_LAUNCH();
-            k_dense_emit<<<resident_grid(k_dense_emit, 256, kDenseEmitSmem, sm), 256, kDenseEmitSmem, st>>>(
+            k_dense_emit<<<resident_grid(k_dense_emit, 256, 0, sm), 256, 0, st>>>(
                 list_m, dp.nd, dp.D, dp.Wd, dp.Wm, dp.cpr, dp.coff, id2x, id2z, out, nullptr, &sc->dense_base);
             CHECK_LAUNCH();
         }
@@ -1092,7 +1092,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         } else {
             CU(cudaEventRecord(c->evc[4], st));
             if (dp.on) {
-                k_dense_emit<<<resident_grid(k_dense_emit, 256, kDenseEmitSmem, sm), 256, kDenseEmitSmem, st>>>(
+                k_dense_emit<<<resident_grid(k_dense_emit, 256, 0, sm), 256, 0, st>>>(
                     list_m, dp.nd, dp.D, dp.Wd, dp.Wm, dp.cpr, dp.coff, id2x, id2z, out, off, nullptr);
                 CHECK_LAUNCH();
             }
@@ -1393,8 +1393,6 @@ int dim3g_create(int device, dim3g_ctx** out) {
                                    (int)kDenseSmem) == cudaSuccess &&
               cudaFuncSetAttribute(k_dense_mma<kDenseSumCount>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kDenseSmem) == cudaSuccess &&
-              cudaFuncSetAttribute(k_dense_emit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseEmitSmem) ==
-                  cudaSuccess &&
               set_aggregate_attributes();
     if (!ok) {
         cudaGetLastError();
