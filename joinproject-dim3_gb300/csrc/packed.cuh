@@ -18,9 +18,11 @@
 
 namespace dim3g {
 
-// Slots (log2) of a warp's table, twice the distinct bound of a pack; pairs a
-// warp stages.  6 KB a warp, so the registers bound the warps in flight.
-constexpr uint32_t kPackLg = 10, kPackCap = 1u << (kPackLg - 1), kPackStage = 256;
+// Slots (log2) of a warp's table, three times the distinct bound of a pack (a
+// probe loop runs as long as its longest lane: 1M rows of 100 candidates 930
+// us at twice, 865 at three times, 877 at four times and smaller packs); pairs
+// a warp stages.  6 KB a warp, so the registers bound the warps in flight.
+constexpr uint32_t kPackLg = 10, kPackCap = 340, kPackStage = 256;
 static_assert(kTinyU <= kPackCap, "a small row fits a pack");
 constexpr size_t kPackWords = ((size_t)1 << kPackLg) + 2 * kPackStage;  // shared words a warp
 
@@ -110,13 +112,15 @@ __device__ __forceinline__ void pack_rows(const RowCtx& c, uint32_t x, uint32_t 
         const bool in = lane >= first && lane < end;
         const uint32_t key0 = in ? (lane - first) * c.m : 0u, n = in ? ne : 0u;
         const uint32_t rows = end - first;
-        uint32_t lg = ceil_log2(2 * sum);
+        uint32_t lg = ceil_log2(3 * sum);
         lg = lg < 5 ? 5 : lg;
         // a bitmap over the pack's rows x z domain where it is no larger
         const uint64_t bits = (uint64_t)rows * c.m;
         const bool bm = bits <= (32ull << lg);
         const uint32_t nclr = bm ? row_bitmap_words((uint32_t)bits) : 1u << lg;
-        for (uint32_t s = lane; s < nclr; s += 32) tab[s] = bm ? 0u : kEmpty32;
+        const uint32_t fill = bm ? 0u : kEmpty32;
+        uint4* t4 = reinterpret_cast<uint4*>(tab);
+        for (uint32_t s = lane; s < nclr / 4; s += 32) t4[s] = make_uint4(fill, fill, fill, fill);
         __syncwarp();
         if (bm) {
             TileBitmap set{tab, 0};
