@@ -18,7 +18,9 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <map>
 #include <string>
+#include <tuple>
 #include <type_traits>
 #include <vector>
 
@@ -106,6 +108,7 @@ struct Params {
     uint32_t block_split = 1;    // single pass: block-class rows in three launches by hash-set size
 };
 
+constexpr uint64_t kSmallSlots = (uint64_t)1 << 17;  // tuple-sized tables this small are not sized by a sketch
 constexpr size_t kMaxSmemOptin = 227 * 1024;  // dynamic shared memory a CTA may opt into
 constexpr uint32_t kFlatAvgBitmap = 160, kFlatAvgBlock = 560, kFlatAvgWarp = 160;  // single pass, per row class
 constexpr uint32_t kAggTileLgMax = 19;  // join-aggregate z tile (its bitmap and ranks are 96 KB)
@@ -148,6 +151,9 @@ struct dim3g_ctx {
     cudaEvent_t evc[8] = {};  // per row-class kernel timing
     cudaEvent_t evd[4] = {};  // dense block: selection, operands, product, light pass
     uint64_t launches = 0;  // kernels launched on this context since creation
+    // resident CTAs per SM by (kernel, CTA width, shared memory): the query
+    // costs about a microsecond, for each of a join's persistent launches
+    std::map<std::tuple<const void*, int, size_t>, int> occupancy;
 };
 
 struct dim3g_mapper {
@@ -254,13 +260,13 @@ inline uint32_t warps_per_cta(size_t per_warp) {
 
 // Grid of a persistent / grid-stride kernel: resident CTAs per SM x SMs.
 template <class K>
-unsigned resident_grid(K kernel, int block, size_t smem, int sm) {
-    int per = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, smem) != cudaSuccess || per < 1) {
+unsigned resident_grid(dim3g_ctx* c, K kernel, int block, size_t smem) {
+    int& per = c->occupancy[{(const void*)kernel, block, smem}];
+    if (per == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, smem) != cudaSuccess || per < 1)) {
         cudaGetLastError();
         per = 1;
     }
-    return (unsigned)(per * sm);
+    return (unsigned)(per * c->sm_count);
 }
 
 // The block class's launches: its rows in three lists by distinct bound u (<=
@@ -645,9 +651,23 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     unsigned long long* states = (unsigned long long*)(zero + sc_bytes + regs_bytes);
     CU(cudaMemsetAsync(zero, 0, zero_bytes, st));
 
+    // A small join is latency: kernels of a few microseconds and host round
+    // trips between them.  Tuple-sized tables of up to kSmallSlots slots (1 MB
+    // each) sit in L2 as they are, so they need no sketch.  And where they do,
+    // one z tile covers Q and the dense block cannot pay -- too few candidates
+    // (at most |P| |Q|), or no row can pass the block class -- the single pass
+    // runs on the tuple counts as bounds of the id counts, with nothing to wait
+    // for before its end: 1.2K x 0.9K tuples 175 us with four round trips, 98
+    // with one.  (A slack below 100 % asks for tables smaller than the keys,
+    // which only the sketch gives.)
+    const bool small_tables = fullP <= kSmallSlots && fullQ <= kSmallSlots && c->prm.table_slack_pct >= 100;
+    const uint32_t dense_mode = jp.aggregate ? 0 : c->prm.dense;
+    const bool small = small_tables && jp.single_pass && !jp.count_only && jp.nQ <= (1ull << c->prm.tile_lg) &&
+                       (dense_mode == 0 || (dense_mode == 1 && (jp.nP * jp.nQ < kDenseMinCand ||
+                                                                jp.nQ <= (1ull << (c->prm.block_lg - 1)))));
     // table capacities from the distinct-key sketch (see mapping.cuh)
     uint64_t capX = fullP, capY = fullP, capZ = fullQ;
-    if (c->prm.sized_tables) {
+    if (c->prm.sized_tables && !small_tables) {
         k_sketch<<<grid_for(jp.nP > jp.nQ ? jp.nP : jp.nQ, sm, 4, kSketchThreads), kSketchThreads, 0, st>>>(
             jp.P, jp.nP, jp.Q, jp.nQ, regs);
         CHECK_LAUNCH();
@@ -690,6 +710,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         device_scan(IdJob{OccupiedSrc{tz.slots}, AssignIdDst{tz.slots, id2z}, capZ, states + 2 * sP, &sc->nz}, &sc->err,
                     st);
         CHECK_LAUNCH();
+        if (small) break;
         CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
         if (sized && attempt == 0 && c->h_sc->err == kErrProbeLimit) {
@@ -701,14 +722,20 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         }
         break;
     }
-    if (c->h_sc->err) return fail(c, DIM3G_ERR_DEVICE, "device bound violated in mapping (flags %u)", c->h_sc->err);
+    if (!small && c->h_sc->err)
+        return fail(c, DIM3G_ERR_DEVICE, "device bound violated in mapping (flags %u)", c->h_sc->err);
     S.table_slots = capX + capY + capZ;
-    const uint32_t n = (uint32_t)c->h_sc->nx, k = (uint32_t)c->h_sc->ny, m = (uint32_t)c->h_sc->nz;
-    const uint64_t nq = c->h_sc->nkept;
-    S.nx = n;
-    S.ny = k;
-    S.nz = m;
-    S.n_small_kept = nq;
+    auto id_counts = [&] {
+        S.nx = (uint32_t)c->h_sc->nx;
+        S.ny = (uint32_t)c->h_sc->ny;
+        S.nz = (uint32_t)c->h_sc->nz;
+        S.n_small_kept = c->h_sc->nkept;
+    };
+    if (!small) id_counts();
+    const uint32_t n = small ? (uint32_t)jp.nP : S.nx, k = small ? (uint32_t)jp.nP : S.ny,
+                   m = small ? (uint32_t)jp.nQ : S.nz;
+    const uint64_t nq = small ? jp.nQ : S.n_small_kept;
+    const unsigned long long* nkept = small ? &sc->nkept : nullptr;
     CU(cudaEventRecord(c->ev[1], st));
     if (nq == 0) {
         S.ms_total = 0;
@@ -766,14 +793,14 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     // latency-bound, so each step builds both in one launch.
     CU(cudaMemsetAsync(degx, 0, zero2, st));
     const unsigned g_csr = grid_for(jp.nP > nq ? jp.nP : nq, sm);
-    k_map<<<dim3(g_csr, 2), 256, 0, st>>>(MapArgs{jp.P, jp.nP, tx, ty, Pm, degx, Qk, nq, tz, T, tile_shift, Zq, cnt_yt});
+    k_map<<<dim3(g_csr, 2), 256, 0, st>>>(MapArgs{jp.P, jp.nP, tx, ty, Pm, degx, Qk, nq, nkept, tz, T, tile_shift, Zq, cnt_yt});
     CHECK_LAUNCH();
     using PtrJob = ScanJob<U32Src, RowPtrDst>;
     device_scan2(PtrJob{U32Src{degx}, RowPtrDst{JR_R, curx}, n1, st_r, nullptr},
                  PtrJob{U32Src{cnt_yt}, RowPtrDst{JR_S, cur_yt}, k1, st_r + sR, nullptr}, &sc->err, st);
     CHECK_LAUNCH();
     k_scatter<<<dim3(g_csr, 2), 256, 0, st>>>(
-        ScatterArgs{Pm, jp.nP, curx, IC_R, Qk, Zq, nq, T, tile_shift, cur_yt, IC_S, ISV});
+        ScatterArgs{Pm, jp.nP, curx, IC_R, Qk, Zq, nq, nkept, T, tile_shift, cur_yt, IC_S, ISV});
     CHECK_LAUNCH();
 
     RowCtx rc{};
@@ -816,7 +843,8 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     CU(cudaEventRecord(c->ev[2], st));
     DensePlan dp;
     {
-        int r = run_dense(c, jp, rc, sc, list_m, k, m, &dp);
+        S.dense_skip = dense_mode == 0 ? 1 : 2;  // off, or too little heavy work
+        int r = small ? DIM3G_OK : run_dense(c, jp, rc, sc, list_m, k, m, &dp);
         if (r) return r;
     }
 
@@ -849,14 +877,14 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
             int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, nullptr);
             if (r) return r;
         } else {
-            k_sum_bitmap<<<resident_grid(k_sum_bitmap, blk_m, smem_m, sm), blk_m, smem_m, st>>>(rc, jp.sum, L.m,
+            k_sum_bitmap<<<resident_grid(c, k_sum_bitmap, blk_m, smem_m), blk_m, smem_m, st>>>(rc, jp.sum, L.m,
                                                                                             L.n3, L.n4);
             CHECK_LAUNCH();
-            k_sum_block<<<resident_grid(k_sum_block, blk_b, smem_b, sm), blk_b, smem_b, st>>>(rc, jp.sum, L.b, L.nb,
+            k_sum_block<<<resident_grid(c, k_sum_block, blk_b, smem_b), blk_b, smem_b, st>>>(rc, jp.sum, L.b, L.nb,
                                                                                           c->prm.block_lg);
             CHECK_LAUNCH();
             const size_t sw = (size_t)wpc << c->prm.warp_lg << 2;
-            k_sum_warp<<<resident_grid(k_sum_warp, 32 * wpc, sw, sm), 32 * wpc, sw, st>>>(rc, jp.sum, L.w, L.nw,
+            k_sum_warp<<<resident_grid(c, k_sum_warp, 32 * wpc, sw), 32 * wpc, sw, st>>>(rc, jp.sum, L.w, L.nw,
                                                                                       c->prm.warp_lg);
             CHECK_LAUNCH();
         }
@@ -895,6 +923,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         CU(cudaStreamSynchronize(st));
         if (c->h_sc->err) return fail(c, DIM3G_ERR_DEVICE, "device bound violated in write pass (flags %u)", c->h_sc->err);
         const uint64_t total = c->h_sc->cursor;
+        if (small) id_counts();
         S.out_j = c->h_sc->outj;
         S.n_out = total;
         S.rows_warp = (uint32_t)(c->h_sc->nrows[1] + c->h_sc->nrows[5]);
@@ -927,7 +956,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         if (dp.on) {
             k_dense_reserve<<<1, 1, 0, st>>>(dp.coff + (uint64_t)dp.nd * dp.cpr, &sc->cursor, cap, &sc->dense_base);
             CHECK_LAUNCH();
-            k_dense_emit<<<resident_grid(k_dense_emit, 256, 0, sm), 256, 0, st>>>(
+            k_dense_emit<<<resident_grid(c, k_dense_emit, 256, 0), 256, 0, st>>>(
                 list_m, dp.nd, dp.D, dp.Wd, dp.Wm, dp.cpr, dp.coff, id2x, id2z, out, nullptr, &sc->dense_base);
             CHECK_LAUNCH();
         }
@@ -938,11 +967,11 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         if (!has_m) {
         } else if (c->prm.stream_rows && stream_smem_bytes(bm_words) <= kMaxSmemOptin) {
             const size_t ss_s = stream_smem_bytes(bm_words);
-            k_stream_bitmap<<<resident_grid(k_stream_bitmap, kStreamThreads, ss_s, sm), kStreamThreads, ss_s, st>>>(
+            k_stream_bitmap<<<resident_grid(c, k_stream_bitmap, kStreamThreads, ss_s), kStreamThreads, ss_s, st>>>(
                 rc, rs, L.m, L.n3, L.n4, bm_words);
             CHECK_LAUNCH();
         } else {
-            k_single_bitmap<<<resident_grid(k_single_bitmap, blk_m, ss_m, sm), blk_m, ss_m, st>>>(rc, rs, L.m, L.n3,
+            k_single_bitmap<<<resident_grid(c, k_single_bitmap, blk_m, ss_m), blk_m, ss_m, st>>>(rc, rs, L.m, L.n3,
                                                                                              L.n4, bm_words);
             CHECK_LAUNCH();
         }
@@ -952,7 +981,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         if (!has_any_b) {
         } else if (c->prm.prefetch_rows && c->prm.cta_rr == 3) {
             const size_t ss_p = (((size_t)1 << c->prm.block_lg) + (size_t)kPfWorkers * kStage) * 4;
-            k_single_block_pf<<<resident_grid(k_single_block_pf, kPfThreads, ss_p, sm), kPfThreads, ss_p, st>>>(
+            k_single_block_pf<<<resident_grid(c, k_single_block_pf, kPfThreads, ss_p), kPfThreads, ss_p, st>>>(
                 rc, rs, L.b, L.nb, c->prm.block_lg);
             CHECK_LAUNCH();
         } else {
@@ -960,7 +989,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
                 if (parts.n > 1 && !has_b[k]) continue;
                 const BlockPart& p = parts.p[k];
                 const size_t ss = ((size_t)1 << p.lg << 2) + (size_t)(p.threads / 32) * kStage * 4;
-                k_single_block<<<resident_grid(k_single_block, p.threads, ss, sm), p.threads, ss, st>>>(
+                k_single_block<<<resident_grid(c, k_single_block, p.threads, ss), p.threads, ss, st>>>(
                     rc, rs, L.b, parts.rows(sc, k), p.lg, parts.skip0(sc, k), parts.skip1(sc, k), 4 + k);
                 CHECK_LAUNCH();
             }
@@ -969,12 +998,12 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         CU(cudaMemcpyAsync(&sc->cursor_at[1], &sc->cursor, 8, cudaMemcpyDeviceToDevice, st));
         rc.flat_avg = kFlatAvgWarp;
         if (has_w) {
-            k_single_warp<<<resident_grid(k_single_warp, 32 * wps, ss_w, sm), 32 * wps, ss_w, st>>>(
+            k_single_warp<<<resident_grid(c, k_single_warp, 32 * wps, ss_w), 32 * wps, ss_w, st>>>(
                 rc, rs, L.w, L.nw, c->prm.warp_lg, kStage);
             CHECK_LAUNCH();
         }
         if (has_t) {
-            k_single_pack<<<resident_grid(k_single_pack, 256, ss_t, sm), 256, ss_t, st>>>(rc, rs, list_t, &sc->nrows[5]);
+            k_single_pack<<<resident_grid(c, k_single_pack, 256, ss_t), 256, ss_t, st>>>(rc, rs, list_t, &sc->nrows[5]);
             CHECK_LAUNCH();
         }
         CU(cudaEventRecord(c->evc[7], st));
@@ -984,6 +1013,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         if (c->h_sc->err) return fail(c, DIM3G_ERR_DEVICE, "device bound violated in single pass (flags %u)", c->h_sc->err);
         dense_times(c, dp);
         const uint64_t total = c->h_sc->cursor;
+        if (small) id_counts();
         S.out_j = c->h_sc->outj;
         S.n_out_cls[0] = c->h_sc->cursor_at[0];
         S.n_out_cls[1] = c->h_sc->cursor_at[1] - c->h_sc->cursor_at[0];
@@ -1021,7 +1051,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     auto pass = [&](auto write, cudaEvent_t* ev) -> int {
         constexpr bool W = decltype(write)::value;
         if (has_m) {
-            k_rows_bitmap<W><<<resident_grid(k_rows_bitmap<W>, blk_m, smem_m, sm), blk_m, smem_m, st>>>(rc, L.m, L.n3, L.n4);
+            k_rows_bitmap<W><<<resident_grid(c, k_rows_bitmap<W>, blk_m, smem_m), blk_m, smem_m, st>>>(rc, L.m, L.n3, L.n4);
             CHECK_LAUNCH();
         }
         CU(cudaEventRecord(ev[1], st));
@@ -1029,19 +1059,19 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
             if (!has_any_b || (parts.n > 1 && !has_b[k])) continue;
             const BlockPart& p = parts.p[k];
             const size_t ss = (size_t)1 << p.lg << 2;
-            k_rows_block<W><<<resident_grid(k_rows_block<W>, p.threads, ss, sm), p.threads, ss, st>>>(
+            k_rows_block<W><<<resident_grid(c, k_rows_block<W>, p.threads, ss), p.threads, ss, st>>>(
                 rc, L.b, parts.rows(sc, k), p.lg, parts.skip0(sc, k), parts.skip1(sc, k), 4 + k);
             CHECK_LAUNCH();
         }
         CU(cudaEventRecord(ev[2], st));
         if (has_w) {
-            k_rows_warp<W><<<resident_grid(k_rows_warp<W>, 32 * wpc, smem_w, sm), 32 * wpc, smem_w, st>>>(
+            k_rows_warp<W><<<resident_grid(c, k_rows_warp<W>, 32 * wpc, smem_w), 32 * wpc, smem_w, st>>>(
                 rc, L.w, L.nw, c->prm.warp_lg);
             CHECK_LAUNCH();
         }
         if (tiny && has_t) {
             const size_t ss = 8 * kRowsPackWords * 4;
-            k_rows_pack<W><<<resident_grid(k_rows_pack<W>, 256, ss, sm), 256, ss, st>>>(rc, list_t, &sc->nrows[5]);
+            k_rows_pack<W><<<resident_grid(c, k_rows_pack<W>, 256, ss), 256, ss, st>>>(rc, list_t, &sc->nrows[5]);
             CHECK_LAUNCH();
         }
         return DIM3G_OK;
@@ -1092,7 +1122,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         } else {
             CU(cudaEventRecord(c->evc[4], st));
             if (dp.on) {
-                k_dense_emit<<<resident_grid(k_dense_emit, 256, 0, sm), 256, 0, st>>>(
+                k_dense_emit<<<resident_grid(c, k_dense_emit, 256, 0), 256, 0, st>>>(
                     list_m, dp.nd, dp.D, dp.Wd, dp.Wm, dp.cpr, dp.coff, id2x, id2z, out, off, nullptr);
                 CHECK_LAUNCH();
             }
@@ -1132,14 +1162,14 @@ int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, 
     const bool half = rank_layout(rc.tile_width, 16, 0).words * 6 + (60u << 10) <= (102u << 10);
     const int thr_m = half ? 512 : 1024;
     const size_t smem_m = half ? 102 << 10 : 200 << 10;
-    k_agg_ranked<<<resident_grid(k_agg_ranked, thr_m, smem_m, sm), thr_m, smem_m, st>>>(
+    k_agg_ranked<<<resident_grid(c, k_agg_ranked, thr_m, smem_m), thr_m, smem_m, st>>>(
         rc, ao, L.m, L.n3, L.n4, rank_layout(rc.tile_width, thr_m / 32, smem_m));
     CHECK_LAUNCH();
     auto map_rows = [&](const uint32_t* rows, const unsigned long long* n, uint32_t lg, const unsigned long long* s0,
                         const unsigned long long* s1, uint32_t ctr) -> int {
         const int thr = lg >= 14 ? 1024 : (lg == 13 ? 512 : (lg == 12 ? 256 : 128));
         const size_t smem = (size_t)8 << lg;
-        k_agg_map<<<resident_grid(k_agg_map, thr, smem, sm), thr, smem, st>>>(rc, ao, rows, n, lg, s0, s1, ctr);
+        k_agg_map<<<resident_grid(c, k_agg_map, thr, smem), thr, smem, st>>>(rc, ao, rows, n, lg, s0, s1, ctr);
         CHECK_LAUNCH();
         return DIM3G_OK;
     };
@@ -1156,7 +1186,7 @@ int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, 
     if (r) return r;
     if (list_t) {
         const size_t smem = 8 * kAggPackWords * 4;
-        k_agg_pack<<<resident_grid(k_agg_pack, 256, smem, sm), 256, smem, st>>>(rc, ao, list_t, &sc->nrows[5]);
+        k_agg_pack<<<resident_grid(c, k_agg_pack, 256, smem), 256, smem, st>>>(rc, ao, list_t, &sc->nrows[5]);
         CHECK_LAUNCH();
     }
     return DIM3G_OK;

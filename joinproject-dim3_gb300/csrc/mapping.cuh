@@ -242,7 +242,8 @@ struct MapArgs {
     uint2* Pm;
     uint32_t* degx;
     const uint2* Qk;
-    uint64_t nQ;
+    uint64_t nQ;  // kept tuples, or a bound on them with the count in *nkept
+    const unsigned long long* nkept;
     DevTable tz;
     uint32_t T, tile_shift;
     uint32_t* zid;
@@ -259,7 +260,8 @@ static __global__ void __launch_bounds__(256) k_map(MapArgs a) {
             atomicAdd(&a.degx[xi], 1u);
         }
     } else {
-        for (uint64_t i = first; i < a.nQ; i += stride) {
+        const uint64_t nQ = a.nkept ? *a.nkept : a.nQ;
+        for (uint64_t i = first; i < nQ; i += stride) {
             const uint2 q = __ldg(&a.Qk[i]);
             const uint32_t zi = table_find(a.tz, q.x);
             a.zid[i] = zi;
@@ -296,6 +298,7 @@ struct ScatterArgs {
     const uint2* Qk;
     const uint32_t* zid;
     uint64_t nQ;
+    const unsigned long long* nkept;
     uint32_t T, tile_shift;
     uint32_t* cur_yt;
     uint32_t* ic_s;
@@ -309,7 +312,8 @@ static __global__ void __launch_bounds__(256) k_scatter(ScatterArgs a) {
             a.ic_r[atomicAdd(&a.curx[p.x], 1u)] = p.y;
         }
     } else {
-        for (uint64_t i = first; i < a.nQ; i += stride) {
+        const uint64_t nQ = a.nkept ? *a.nkept : a.nQ;
+        for (uint64_t i = first; i < nQ; i += stride) {
             const uint2 q = __ldg(&a.Qk[i]);
             const uint32_t zi = __ldg(&a.zid[i]);
             const uint32_t pos = atomicAdd(&a.cur_yt[(uint64_t)q.y * a.T + (zi >> a.tile_shift)], 1u);
