@@ -5,7 +5,7 @@
 // Relation set creation: a distinct-key sketch of every relation's columns
 // sizes its value -> id tables (k_rel_sketch, synchronised once).
 // Relation set build (one stream, no host synchronisation inside):
-//   memsets -> k_ix_insert -> k_ix_layout -> id scans (TF, TY) -> k_ix_map
+//   memsets -> k_ix_insert -> id scans (TF, TY) -> k_ix_layout -> k_ix_map
 //   -> CSR scans (by f, by (y, f tile); bounded by the layout's counts)
 //   -> k_ix_scatter (a batch builds only the CSR each relation's query reads)
 // Query pass over queries (P, Q) of a set:
@@ -99,9 +99,9 @@ Tuning tuning_of(const dim3g_ctx* ctx) {
     return Tuning{(uint32_t)w, (uint32_t)b, (uint32_t)t, (uint32_t)tl, (uint32_t)rr, (uint32_t)bs};
 }
 
-// Warps per CTA of the warp-class kernels (about half an SM's shared memory).
+// Warps per CTA of the warp-class kernels (about a third of an SM's shared memory).
 uint32_t warps_for(size_t per_warp) {
-    size_t w = (size_t)112 * 1024 / per_warp;
+    size_t w = (size_t)74 * 1024 / per_warp;
     return (uint32_t)(w < 1 ? 1 : (w > 8 ? 8 : w));
 }
 
@@ -187,7 +187,9 @@ int relset_plan(dim3g_relset* s, const dim3g_relation* rels, uint32_t n, uint64_
                  o_JRy = L.add<uint32_t>(s->yt_cap), o_curY = L.add<uint32_t>(s->yt_cap),
                  o_ICy = L.add<uint32_t>(s->ntot), o_VSy = L.add<uint32_t>(s->ntot), o_err = L.add<uint32_t>(4),
                  o_need = L.add<unsigned long long>(2), o_yoff = L.add<uint64_t>(n + 1),
-                 o_roles = L.add<uint8_t>(n), o_fneed = L.add<unsigned long long>(1);
+                 o_roles = L.add<uint8_t>(n), o_fneed = L.add<unsigned long long>(1),
+                 o_tabF = L.add<unsigned long long>(s->tabtot / kTabMark + 1),
+                 o_tabY = L.add<unsigned long long>(s->tabtot / kTabMark + 1);
     s->scan_words[0] = s->scan_words[1] = scan_storage(s->tabtot);
     s->scan_words[2] = scan_storage(s->ntot + 1);
     s->scan_words[3] = scan_storage(s->yt_cap);
@@ -235,6 +237,9 @@ int relset_plan(dim3g_relset* s, const dim3g_relation* rels, uint32_t n, uint64_
     P.yoff = (uint64_t*)(m + o_yoff);
     P.roles = (const uint8_t*)(m + o_roles);
     P.f_need = (unsigned long long*)(m + o_fneed);
+    P.tabF = (unsigned long long*)(m + o_tabF);
+    P.tabY = (unsigned long long*)(m + o_tabY);
+    P.tab_marks = s->tabtot / kTabMark;
     s->scan_state = (unsigned long long*)(m + o_scan);
     BCU(cudaMemcpy((void*)P.in, s->h_in.data(), n * sizeof(RelIn), cudaMemcpyHostToDevice));
     BCU(cudaMemcpy((void*)P.tup_off, s->h_tup_off.data(), (n + 1) * 8, cudaMemcpyHostToDevice));
@@ -332,8 +337,6 @@ int relset_enqueue_build(dim3g_relset* s, cudaStream_t st, uint64_t& launches) {
     const int sm = I::sm_count(ctx);
     BCU(cudaMemsetAsync(P.TF, 0xff, s->tabtot * 8, st));
     BCU(cudaMemsetAsync(P.TY, 0xff, s->tabtot * 8, st));
-    BCU(cudaMemsetAsync(P.nf_cnt, 0, s->nrel * 8, st));
-    BCU(cudaMemsetAsync(P.ny_cnt, 0, s->nrel * 8, st));
     BCU(cudaMemsetAsync(P.degF, 0, (s->ntot + 1) * 4, st));
     BCU(cudaMemsetAsync(P.cnt_yt, 0, s->yt_cap * 4, st));
     BCU(cudaMemsetAsync(P.err, 0, 16, st));
@@ -343,13 +346,13 @@ int relset_enqueue_build(dim3g_relset* s, cudaStream_t st, uint64_t& launches) {
         k_ix_insert<<<elem_grid(s->ntot, sm), 256, 0, st>>>(P);
         BLAUNCH();
     }
-    k_ix_layout<<<1, 1024, 0, st>>>(P, s->tile_lg);
-    BLAUNCH();
-    using IdJob = ScanJob<OccupiedSrc, AssignIdDst>;
+    using IdJob = ScanJob<OccupiedSrc, AssignPoolIdDst>;
     using PtrJob = ScanJob<U32Src, RowPtrDst>;
     unsigned long long* w[4] = {s->scan_state, w[0] + s->scan_words[0], w[1] + s->scan_words[1], w[2] + s->scan_words[2]};
-    device_scan2(IdJob{OccupiedSrc{P.TF}, AssignIdDst{P.TF, P.id2f}, s->tabtot, w[0], nullptr},
-                 IdJob{OccupiedSrc{P.TY}, AssignIdDst{P.TY, P.id2y}, s->tabtot, w[1], nullptr}, P.err, st);
+    device_scan2(IdJob{OccupiedSrc{P.TF}, {{P.TF, P.id2f}, P.tabF}, s->tabtot, w[0], P.tabF + P.tab_marks},
+                 IdJob{OccupiedSrc{P.TY}, {{P.TY, P.id2y}, P.tabY}, s->tabtot, w[1], P.tabY + P.tab_marks}, P.err, st);
+    BLAUNCH();
+    k_ix_layout<<<1, 1024, 0, st>>>(P, s->tile_lg);
     BLAUNCH();
     if (s->ntot) {
         k_ix_map<<<elem_grid(s->ntot, sm), 256, 0, st>>>(P);
@@ -582,10 +585,10 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
                     Q, BatchRows{lb, &n[2], nullptr, &next[1]}, tu.block_lg);
                 BLAUNCH();
             }
-            const uint32_t wps = warps_for(warp_row_words(tu.warp_lg, kStage) * 4);
-            const size_t ss_w = (size_t)wps * warp_row_words(tu.warp_lg, kStage) * 4;
+            const uint32_t wps = warps_for(warp_row_words(tu.warp_lg, kWarpStage) * 4);
+            const size_t ss_w = (size_t)wps * warp_row_words(tu.warp_lg, kWarpStage) * 4;
             k_b_single_warp<<<resident(k_b_single_warp, 32 * wps, ss_w, sm), 32 * wps, ss_w, st>>>(
-                Q, BatchRows{lw, &n[1], nullptr, nullptr}, tu.warp_lg, kStage);
+                Q, BatchRows{lw, &n[1], nullptr, nullptr}, tu.warp_lg, kWarpStage);
             BLAUNCH();
             const size_t ss_t = 8 * kPackWords * 4;
             k_b_single_pack<<<resident(k_b_single_pack, 256, ss_t, sm), 256, ss_t, st>>>(

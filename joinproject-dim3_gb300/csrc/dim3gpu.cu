@@ -250,9 +250,9 @@ struct RowLists {
 int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc, const uint32_t* list_t);
 
 // Warps per CTA of a warp-per-row kernel whose warps each own per_warp
-// bytes of shared memory: up to 8, within about half an SM's shared memory
-// so two CTAs fit per SM.
-constexpr size_t kWarpCtaSmem = 112 * 1024;
+// bytes of shared memory: up to 8, within about a third of an SM's shared
+// memory so three CTAs fit per SM.
+constexpr size_t kWarpCtaSmem = 74 * 1024;
 inline uint32_t warps_per_cta(size_t per_warp) {
     size_t w = kWarpCtaSmem / per_warp;
     return (uint32_t)(w < 1 ? 1 : (w > 8 ? 8 : w));
@@ -950,8 +950,8 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         const uint32_t bm_words = (uint32_t)(smem_m / 4);
         const size_t ss_m = smem_m + (size_t)(blk_m / 32) * kStage * 4;
         const size_t ss_b = smem_b + (size_t)(blk_b / 32) * kStage * 4;
-        const uint32_t wps = warps_per_cta(warp_row_words(c->prm.warp_lg, kStage) * 4);
-        const size_t ss_w = (size_t)wps * warp_row_words(c->prm.warp_lg, kStage) * 4;
+        const uint32_t wps = warps_per_cta(warp_row_words(c->prm.warp_lg, kWarpStage) * 4);
+        const size_t ss_w = (size_t)wps * warp_row_words(c->prm.warp_lg, kWarpStage) * 4;
         const size_t ss_t = 8 * kPackWords * 4;
         if (dp.on) {
             k_dense_reserve<<<1, 1, 0, st>>>(dp.coff + (uint64_t)dp.nd * dp.cpr, &sc->cursor, cap, &sc->dense_base);
@@ -999,7 +999,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         rc.flat_avg = kFlatAvgWarp;
         if (has_w) {
             k_single_warp<<<resident_grid(c, k_single_warp, 32 * wps, ss_w), 32 * wps, ss_w, st>>>(
-                rc, rs, L.w, L.nw, c->prm.warp_lg, kStage);
+                rc, rs, L.w, L.nw, c->prm.warp_lg, kWarpStage);
             CHECK_LAUNCH();
         }
         if (has_t) {

@@ -20,6 +20,11 @@ namespace dim3g {
 #define DIM3G_STAGE 512
 #endif
 constexpr uint32_t kStage = DIM3G_STAGE;  // staged z values per warp (2 KB)
+// Staged pairs of a warp-class warp: the least a step of candidates needs, so
+// that three 8-warp CTAs fit an SM (512 pairs and two CTAs: 338 us against
+// 297 for the 20M-edge 2-hop slice's warp rows).
+constexpr uint32_t kWarpStage = 128;
+static_assert(kWarpStage >= 32 * kUnroll, "a step of candidates fits the stage");
 
 struct Reserve {
     unsigned long long* cursor;
