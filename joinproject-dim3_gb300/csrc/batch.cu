@@ -115,12 +115,23 @@ struct QueryScratch {
     size_t qmem_bytes = 0;
     QueryRes* h_res = nullptr;  // pinned
     uint32_t h_res_n = 0;
+    // The row kernels of a pass are independent (each has its own list and
+    // counter; results meet in the queries' cursors), so they fork from the
+    // pass's stream onto these and join again: a kernel whose last rows are
+    // huge leaves the rest of the GPU to the next.
+    cudaStream_t side[2] = {};
+    cudaEvent_t fork = nullptr, join[2] = {};
     QueryScratch() = default;
     QueryScratch(const QueryScratch&) = delete;
     QueryScratch& operator=(const QueryScratch&) = delete;
     ~QueryScratch() {
         if (qmem) cudaFree(qmem);
         if (h_res) cudaFreeHost(h_res);
+        for (int k = 0; k < 2; k++) {
+            if (side[k]) cudaStreamDestroy(side[k]);
+            if (join[k]) cudaEventDestroy(join[k]);
+        }
+        if (fork) cudaEventDestroy(fork);
     }
 };
 
@@ -467,6 +478,14 @@ int query_plan(dim3g_relset* s, QueryScratch& qs, const dim3g_query* q, uint32_t
         }
         qs.qmem_bytes = o.total;
     }
+    if (!qs.fork) {
+        cudaError_t e = cudaEventCreateWithFlags(&qs.fork, cudaEventDisableTiming);
+        for (int i = 0; i < 2; i++) {
+            if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&qs.side[i], cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&qs.join[i], cudaEventDisableTiming);
+        }
+        if (e != cudaSuccess) return I::fail(ctx, DIM3G_ERR_CUDA, "query pass streams: %s", cudaGetErrorString(e));
+    }
     if (qs.h_res_n < nq) {
         if (qs.h_res) cudaFreeHost(qs.h_res);
         qs.h_res = nullptr;
@@ -563,6 +582,8 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
         k_row_lists<<<(unsigned)((qp.nrows + kListTile - 1) / kListTile), 256, 0, st>>>(
             Q.bucket, (uint32_t)qp.nrows, op ? kCountBuckets : 0, n + 16, n + 24, qp.lists, n, nb);
         BLAUNCH();
+        BCU(cudaEventRecord(qs.fork, st));
+        for (int i = 0; i < 2; i++) BCU(cudaStreamWaitEvent(qs.side[i], qs.fork, 0));
         if (op == 0) {
             const size_t ss_m = (size_t)bm_words * 4 + 16 * kStage * 4;
             k_b_single_bitmap<<<resident(k_b_single_bitmap, 512, ss_m, sm), 512, ss_m, st>>>(
@@ -587,11 +608,11 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
             }
             const uint32_t wps = warps_for(warp_row_words(tu.warp_lg, kWarpStage) * 4);
             const size_t ss_w = (size_t)wps * warp_row_words(tu.warp_lg, kWarpStage) * 4;
-            k_b_single_warp<<<resident(k_b_single_warp, 32 * wps, ss_w, sm), 32 * wps, ss_w, st>>>(
+            k_b_single_warp<<<resident(k_b_single_warp, 32 * wps, ss_w, sm), 32 * wps, ss_w, qs.side[0]>>>(
                 Q, BatchRows{lw, &n[1], nullptr, nullptr}, tu.warp_lg, kWarpStage);
             BLAUNCH();
             const size_t ss_t = 8 * kPackWords * 4;
-            k_b_single_pack<<<resident(k_b_single_pack, 256, ss_t, sm), 256, ss_t, st>>>(
+            k_b_single_pack<<<resident(k_b_single_pack, 256, ss_t, sm), 256, ss_t, qs.side[1]>>>(
                 Q, BatchRows{lt, &n[5], nullptr, nullptr});
             BLAUNCH();
         } else {
@@ -602,7 +623,7 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
             auto map_rows = [&](const BatchRows& rows, uint32_t lg) -> int {
                 const int thr = lg >= 14 ? 1024 : (lg == 13 ? 512 : (lg == 12 ? 256 : 128));
                 const size_t ss = (size_t)8 << lg;
-                k_b_agg_map<<<resident(k_b_agg_map, thr, ss, sm), thr, ss, st>>>(Q, rows, lg);
+                k_b_agg_map<<<resident(k_b_agg_map, thr, ss, sm), thr, ss, qs.side[0]>>>(Q, rows, lg);
                 BLAUNCH();
                 return DIM3G_OK;
             };
@@ -618,9 +639,13 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
             if (!r) r = map_rows(BatchRows{lw, &n[1], nullptr, &next[0]}, tu.warp_lg);
             if (r) return r;
             const size_t ss_t = 8 * kAggPackWords * 4;
-            k_b_agg_pack<<<resident(k_b_agg_pack, 256, ss_t, sm), 256, ss_t, st>>>(
+            k_b_agg_pack<<<resident(k_b_agg_pack, 256, ss_t, sm), 256, ss_t, qs.side[1]>>>(
                 Q, BatchRows{lt, &n[5], nullptr, nullptr});
             BLAUNCH();
+        }
+        for (int i = 0; i < 2; i++) {
+            BCU(cudaEventRecord(qs.join[i], qs.side[i]));
+            BCU(cudaStreamWaitEvent(st, qs.join[i], 0));
         }
     }
     BCU(cudaMemcpyAsync(qs.h_res, Q.res, (size_t)nq * sizeof(QueryRes), cudaMemcpyDeviceToHost, st));
