@@ -118,7 +118,7 @@ struct Scalars {
     unsigned long long cursor;     // single-pass output cursor
     unsigned long long nrows[6];   // rows per class (index = class)
     unsigned long long outj_cls[6];  // candidates per class (index = class)
-    unsigned long long cursor_at[3]; // single-pass cursor after the bitmap / block / warp kernel
+    unsigned long long n_cls[2];     // single-pass pairs of the block and the warp kernels
     unsigned long long dense_base;   // single-pass start of the dense block's pairs (~0: past the capacity)
     unsigned int err;
     unsigned long long nrows_b[3];  // block-class rows by hash-set size (single pass, block_split)
@@ -147,6 +147,9 @@ struct dim3g_ctx {
     void* d_sum = nullptr;  // per-A-tile summary accumulators
     size_t d_sum_bytes = 0;
     Scalars* h_sc = nullptr;  // pinned
+    // Streams of the row kernels beside the context's (RowStreams).
+    cudaStream_t side[2] = {};
+    cudaEvent_t ev_fork = nullptr, ev_join[2] = {};
     cudaEvent_t ev[6] = {};
     cudaEvent_t evc[8] = {};  // per row-class kernel timing
     cudaEvent_t evd[4] = {};  // dense block: selection, operands, product, light pass
@@ -247,7 +250,9 @@ struct RowLists {
     const uint32_t *w, *b, *m;                          // class 1, class 2, classes 4 then 3
     const unsigned long long *nw, *nb, *n3, *n4;        // their sizes (device)
 };
-int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc, const uint32_t* list_t);
+struct RowStreams;
+int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc, const uint32_t* list_t,
+                  RowStreams& rst);
 
 // Warps per CTA of a warp-per-row kernel whose warps each own per_warp
 // bytes of shared memory: up to 8, within about a third of an SM's shared
@@ -268,6 +273,40 @@ unsigned resident_grid(dim3g_ctx* c, K kernel, int block, size_t smem) {
     }
     return (unsigned)(per * c->sm_count);
 }
+
+// The row kernels of a pass are independent: each has its own list and row
+// counter, and they meet only in the output cursor (or at exact offsets).  So
+// where several have rows they fork from the context's stream -- the bitmap
+// rows stay on it, the block rows and the warp rows take one side stream each
+// -- and join it again, and a kernel that is down to a few huge rows leaves
+// the rest of the GPU to the next.  Whole calls, in turn and forked: 1.2M-edge
+// 2-hop 1.48 and 1.44 ms, its COUNT 3.63 and 3.40, 200k rows ordered 0.79 and
+// 0.76, an eighth of the 20M-edge 2-hop 10.37 and 10.23.
+struct RowStreams {
+    dim3g_ctx* c;
+    bool on, open = false;
+    cudaStream_t m, b, w;
+    RowStreams(dim3g_ctx* c, bool on)
+        : c(c), on(on), m(c->stream), b(on ? c->side[0] : c->stream), w(on ? c->side[1] : c->stream) {}
+    cudaError_t fork() {
+        if (!on) return cudaSuccess;
+        open = true;
+        cudaError_t e = cudaEventRecord(c->ev_fork, c->stream);
+        for (int k = 0; k < 2 && e == cudaSuccess; k++) e = cudaStreamWaitEvent(c->side[k], c->ev_fork, 0);
+        return e;
+    }
+    cudaError_t join() {
+        cudaError_t e = cudaSuccess;
+        for (int k = 0; open && k < 2; k++) {
+            if (e == cudaSuccess) e = cudaEventRecord(c->ev_join[k], c->side[k]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_join[k], 0);
+        }
+        open = false;
+        return e;
+    }
+    RowStreams(const RowStreams&) = delete;
+    ~RowStreams() { join(); }  // an error return between the two
+};
 
 // The block class's launches: its rows in three lists by distinct bound u (<=
 // 2^(b-3), <= 2^(b-2), the rest; b = block_slots_log2), 2^lg table words each:
@@ -868,13 +907,14 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
                            dp.counted ? h.nrows_b[2] != 0 : m > rb.cap_m};
     const bool has_any_b = !dp.counted || h.nrows[2], has_w = !dp.counted || h.nrows[1],
                has_t = !dp.counted || h.nrows[5];
+    RowStreams rst(c, dp.counted ? has_m + has_any_b + (has_w || has_t) > 1 : !small && jp.aggregate);
 
     if (jp.sum.tiles) {
         // summaries: the expansion kernels hash instead of writing; COUNT
         // needs no count pass (nothing is placed)
         CU(cudaEventRecord(c->evc[4], st));
         if (jp.aggregate) {
-            int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, nullptr);
+            int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, nullptr, rst);
             if (r) return r;
         } else {
             k_sum_bitmap<<<resident_grid(c, k_sum_bitmap, blk_m, smem_m), blk_m, smem_m, st>>>(rc, jp.sum, L.m,
@@ -916,7 +956,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         rc.out = sp_out;
     }
     if (single && jp.aggregate) {
-        int r = run_aggregate(c, rc, AggOut{sp_cnt, SumAcc{}, Reserve{&sc->cursor, cap}}, L, sc, list_t);
+        int r = run_aggregate(c, rc, AggOut{sp_cnt, SumAcc{}, Reserve{&sc->cursor, cap}}, L, sc, list_t, rst);
         if (r) return r;
         CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
         CU(cudaEventRecord(c->ev[3], st));
@@ -960,6 +1000,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
                 list_m, dp.nd, dp.D, dp.Wd, dp.Wm, dp.cpr, dp.coff, id2x, id2z, out, nullptr, &sc->dense_base);
             CHECK_LAUNCH();
         }
+        CU(rst.fork());
         // the cross-segment gather's threshold per row class, measured on
         // the 2-hop (bitmap rows 45.5 -> 44.7 ms at 160, block rows 26.3 ->
         // 25.7 at 560, warp rows 2.62 -> 2.58 at 160; every setting exact)
@@ -967,46 +1008,46 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         if (!has_m) {
         } else if (c->prm.stream_rows && stream_smem_bytes(bm_words) <= kMaxSmemOptin) {
             const size_t ss_s = stream_smem_bytes(bm_words);
-            k_stream_bitmap<<<resident_grid(c, k_stream_bitmap, kStreamThreads, ss_s), kStreamThreads, ss_s, st>>>(
+            k_stream_bitmap<<<resident_grid(c, k_stream_bitmap, kStreamThreads, ss_s), kStreamThreads, ss_s, rst.m>>>(
                 rc, rs, L.m, L.n3, L.n4, bm_words);
             CHECK_LAUNCH();
         } else {
-            k_single_bitmap<<<resident_grid(c, k_single_bitmap, blk_m, ss_m), blk_m, ss_m, st>>>(rc, rs, L.m, L.n3,
+            k_single_bitmap<<<resident_grid(c, k_single_bitmap, blk_m, ss_m), blk_m, ss_m, rst.m>>>(rc, rs, L.m, L.n3,
                                                                                              L.n4, bm_words);
             CHECK_LAUNCH();
         }
-        CU(cudaEventRecord(c->evc[5], st));
-        CU(cudaMemcpyAsync(&sc->cursor_at[0], &sc->cursor, 8, cudaMemcpyDeviceToDevice, st));
+        CU(cudaEventRecord(c->evc[5], rst.m));
         rc.flat_avg = kFlatAvgBlock;
         if (!has_any_b) {
         } else if (c->prm.prefetch_rows && c->prm.cta_rr == 3) {
             const size_t ss_p = (((size_t)1 << c->prm.block_lg) + (size_t)kPfWorkers * kStage) * 4;
-            k_single_block_pf<<<resident_grid(c, k_single_block_pf, kPfThreads, ss_p), kPfThreads, ss_p, st>>>(
-                rc, rs, L.b, L.nb, c->prm.block_lg);
+            k_single_block_pf<<<resident_grid(c, k_single_block_pf, kPfThreads, ss_p), kPfThreads, ss_p, rst.b>>>(
+                rc, rs, &sc->n_cls[0], L.b, L.nb, c->prm.block_lg);
             CHECK_LAUNCH();
         } else {
             for (uint32_t k = 0; k < parts.n; k++) {
                 if (parts.n > 1 && !has_b[k]) continue;
                 const BlockPart& p = parts.p[k];
                 const size_t ss = ((size_t)1 << p.lg << 2) + (size_t)(p.threads / 32) * kStage * 4;
-                k_single_block<<<resident_grid(c, k_single_block, p.threads, ss), p.threads, ss, st>>>(
-                    rc, rs, L.b, parts.rows(sc, k), p.lg, parts.skip0(sc, k), parts.skip1(sc, k), 4 + k);
+                k_single_block<<<resident_grid(c, k_single_block, p.threads, ss), p.threads, ss, rst.b>>>(
+                    rc, rs, &sc->n_cls[0], L.b, parts.rows(sc, k), p.lg, parts.skip0(sc, k), parts.skip1(sc, k), 4 + k);
                 CHECK_LAUNCH();
             }
         }
-        CU(cudaEventRecord(c->evc[6], st));
-        CU(cudaMemcpyAsync(&sc->cursor_at[1], &sc->cursor, 8, cudaMemcpyDeviceToDevice, st));
+        CU(cudaEventRecord(c->evc[6], rst.b));
         rc.flat_avg = kFlatAvgWarp;
         if (has_w) {
-            k_single_warp<<<resident_grid(c, k_single_warp, 32 * wps, ss_w), 32 * wps, ss_w, st>>>(
-                rc, rs, L.w, L.nw, c->prm.warp_lg, kWarpStage);
+            k_single_warp<<<resident_grid(c, k_single_warp, 32 * wps, ss_w), 32 * wps, ss_w, rst.w>>>(
+                rc, rs, &sc->n_cls[1], L.w, L.nw, c->prm.warp_lg, kWarpStage);
             CHECK_LAUNCH();
         }
         if (has_t) {
-            k_single_pack<<<resident_grid(c, k_single_pack, 256, ss_t), 256, ss_t, st>>>(rc, rs, list_t, &sc->nrows[5]);
+            k_single_pack<<<resident_grid(c, k_single_pack, 256, ss_t), 256, ss_t, rst.w>>>(
+                rc, rs, &sc->n_cls[1], list_t, &sc->nrows[5]);
             CHECK_LAUNCH();
         }
-        CU(cudaEventRecord(c->evc[7], st));
+        CU(cudaEventRecord(c->evc[7], rst.w));
+        CU(rst.join());
         CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
         CU(cudaEventRecord(c->ev[3], st));
         CU(cudaStreamSynchronize(st));
@@ -1015,9 +1056,9 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         const uint64_t total = c->h_sc->cursor;
         if (small) id_counts();
         S.out_j = c->h_sc->outj;
-        S.n_out_cls[0] = c->h_sc->cursor_at[0];
-        S.n_out_cls[1] = c->h_sc->cursor_at[1] - c->h_sc->cursor_at[0];
-        S.n_out_cls[2] = total - c->h_sc->cursor_at[1];
+        S.n_out_cls[1] = c->h_sc->n_cls[0];
+        S.n_out_cls[2] = c->h_sc->n_cls[1];
+        S.n_out_cls[0] = total - S.n_out_cls[1] - S.n_out_cls[2];
         S.n_out = total;
         S.rows_warp = (uint32_t)(c->h_sc->nrows[1] + c->h_sc->nrows[5]);
         S.rows_block = (uint32_t)c->h_sc->nrows[2];
@@ -1030,7 +1071,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         cudaEventElapsedTime(&a, c->ev[0], c->ev[1]);
         cudaEventElapsedTime(&b, c->ev[1], c->ev[2]);
         cudaEventElapsedTime(&e, c->ev[2], c->ev[3]);
-        for (int i = 0; i < 3; i++) cudaEventElapsedTime(&S.ms_write_cls[i], c->evc[4 + i], c->evc[5 + i]);
+        for (int i = 0; i < 3; i++) cudaEventElapsedTime(&S.ms_write_cls[i], c->evc[rst.on ? 4 : 4 + i], c->evc[5 + i]);
         S.ms_map = a;
         S.ms_csr = b;
         S.ms_write = e;
@@ -1050,37 +1091,39 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     // the row kernels of one pass over the classes, with an event after each
     auto pass = [&](auto write, cudaEvent_t* ev) -> int {
         constexpr bool W = decltype(write)::value;
+        CU(rst.fork());
         if (has_m) {
-            k_rows_bitmap<W><<<resident_grid(c, k_rows_bitmap<W>, blk_m, smem_m), blk_m, smem_m, st>>>(rc, L.m, L.n3, L.n4);
+            k_rows_bitmap<W><<<resident_grid(c, k_rows_bitmap<W>, blk_m, smem_m), blk_m, smem_m, rst.m>>>(rc, L.m, L.n3, L.n4);
             CHECK_LAUNCH();
         }
-        CU(cudaEventRecord(ev[1], st));
+        CU(cudaEventRecord(ev[1], rst.m));
         for (uint32_t k = 0; k < parts.n; k++) {
             if (!has_any_b || (parts.n > 1 && !has_b[k])) continue;
             const BlockPart& p = parts.p[k];
             const size_t ss = (size_t)1 << p.lg << 2;
-            k_rows_block<W><<<resident_grid(c, k_rows_block<W>, p.threads, ss), p.threads, ss, st>>>(
+            k_rows_block<W><<<resident_grid(c, k_rows_block<W>, p.threads, ss), p.threads, ss, rst.b>>>(
                 rc, L.b, parts.rows(sc, k), p.lg, parts.skip0(sc, k), parts.skip1(sc, k), 4 + k);
             CHECK_LAUNCH();
         }
-        CU(cudaEventRecord(ev[2], st));
+        CU(cudaEventRecord(ev[2], rst.b));
         if (has_w) {
-            k_rows_warp<W><<<resident_grid(c, k_rows_warp<W>, 32 * wpc, smem_w), 32 * wpc, smem_w, st>>>(
+            k_rows_warp<W><<<resident_grid(c, k_rows_warp<W>, 32 * wpc, smem_w), 32 * wpc, smem_w, rst.w>>>(
                 rc, L.w, L.nw, c->prm.warp_lg);
             CHECK_LAUNCH();
         }
         if (tiny && has_t) {
             const size_t ss = 8 * kRowsPackWords * 4;
-            k_rows_pack<W><<<resident_grid(c, k_rows_pack<W>, 256, ss), 256, ss, st>>>(rc, list_t, &sc->nrows[5]);
+            k_rows_pack<W><<<resident_grid(c, k_rows_pack<W>, 256, ss), 256, ss, rst.w>>>(rc, list_t, &sc->nrows[5]);
             CHECK_LAUNCH();
         }
+        CU(cudaEventRecord(ev[3], rst.w));
+        CU(rst.join());
         return DIM3G_OK;
     };
     {
         int r = pass(std::false_type{}, &c->evc[0]);
         if (r) return r;
     }
-    CU(cudaEventRecord(c->evc[3], st));
     SCAN(U32Src{cnt}, OffDst{off}, (uint64_t)n + 1, bsum2, &sc->total, &sc->err);
     CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
     CU(cudaEventRecord(c->ev[3], st));
@@ -1088,7 +1131,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     if (c->h_sc->err) return fail(c, DIM3G_ERR_DEVICE, "device bound violated in count pass (flags %u)", c->h_sc->err);
     dense_times(c, dp);
     const uint64_t total = c->h_sc->total;
-    for (int i = 0; i < 3; i++) cudaEventElapsedTime(&S.ms_count_cls[i], c->evc[i], c->evc[i + 1]);
+    for (int i = 0; i < 3; i++) cudaEventElapsedTime(&S.ms_count_cls[i], c->evc[rst.on ? 0 : i], c->evc[i + 1]);
     S.out_j = c->h_sc->outj;
     S.n_out = total;
     S.rows_warp = (uint32_t)(c->h_sc->nrows[1] + c->h_sc->nrows[5]);
@@ -1117,7 +1160,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     CU(cudaMemsetAsync(sc->next_row, 0, sizeof(sc->next_row), st));
     if (total > 0) {
         if (jp.aggregate) {
-            int r = run_aggregate(c, rc, AggOut{out_cnt, SumAcc{}, Reserve{nullptr, 0}}, L, sc, nullptr);
+            int r = run_aggregate(c, rc, AggOut{out_cnt, SumAcc{}, Reserve{nullptr, 0}}, L, sc, nullptr, rst);
             if (r) return r;
         } else {
             CU(cudaEventRecord(c->evc[4], st));
@@ -1128,7 +1171,6 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
             }
             int r = pass(std::true_type{}, &c->evc[4]);
             if (r) return r;
-            CU(cudaEventRecord(c->evc[7], st));
         }
     }
     CU(cudaMemcpyAsync(&c->h_sc->err, &sc->err, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
@@ -1146,7 +1188,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     S.ms_write = e;
     S.ms_total = a + b + d + e;
     if (total > 0 && !jp.aggregate)
-        for (int i = 0; i < 3; i++) cudaEventElapsedTime(&S.ms_write_cls[i], c->evc[4 + i], c->evc[5 + i]);
+        for (int i = 0; i < 3; i++) cudaEventElapsedTime(&S.ms_write_cls[i], c->evc[rst.on ? 4 : 4 + i], c->evc[5 + i]);
     return DIM3G_OK;
 }
 
@@ -1154,22 +1196,21 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
 // rows from the largest maps down, then the tiny rows (list_t; null: none).
 // CTAs by map size, so that small maps run many rows an SM.
 int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc,
-                  const uint32_t* list_t) {
-    cudaStream_t st = c->stream;
-    const int sm = c->sm_count;
+                  const uint32_t* list_t, RowStreams& rst) {
+    CU(rst.fork());
     // one ranked CTA an SM with all of its shared memory, or two where a
     // half leaves 60 KB for the counters
     const bool half = rank_layout(rc.tile_width, 16, 0).words * 6 + (60u << 10) <= (102u << 10);
     const int thr_m = half ? 512 : 1024;
     const size_t smem_m = half ? 102 << 10 : 200 << 10;
-    k_agg_ranked<<<resident_grid(c, k_agg_ranked, thr_m, smem_m), thr_m, smem_m, st>>>(
+    k_agg_ranked<<<resident_grid(c, k_agg_ranked, thr_m, smem_m), thr_m, smem_m, rst.m>>>(
         rc, ao, L.m, L.n3, L.n4, rank_layout(rc.tile_width, thr_m / 32, smem_m));
     CHECK_LAUNCH();
     auto map_rows = [&](const uint32_t* rows, const unsigned long long* n, uint32_t lg, const unsigned long long* s0,
                         const unsigned long long* s1, uint32_t ctr) -> int {
         const int thr = lg >= 14 ? 1024 : (lg == 13 ? 512 : (lg == 12 ? 256 : 128));
         const size_t smem = (size_t)8 << lg;
-        k_agg_map<<<resident_grid(c, k_agg_map, thr, smem), thr, smem, st>>>(rc, ao, rows, n, lg, s0, s1, ctr);
+        k_agg_map<<<resident_grid(c, k_agg_map, thr, smem), thr, smem, rst.b>>>(rc, ao, rows, n, lg, s0, s1, ctr);
         CHECK_LAUNCH();
         return DIM3G_OK;
     };
@@ -1186,9 +1227,10 @@ int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, 
     if (r) return r;
     if (list_t) {
         const size_t smem = 8 * kAggPackWords * 4;
-        k_agg_pack<<<resident_grid(c, k_agg_pack, 256, smem), 256, smem, st>>>(rc, ao, list_t, &sc->nrows[5]);
+        k_agg_pack<<<resident_grid(c, k_agg_pack, 256, smem), 256, smem, rst.w>>>(rc, ao, list_t, &sc->nrows[5]);
         CHECK_LAUNCH();
     }
+    CU(rst.join());
     return DIM3G_OK;
 }
 
@@ -1382,6 +1424,11 @@ int dim3g_create(int device, dim3g_ctx** out) {
     dim3g_ctx* c = new dim3g_ctx();
     c->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&c->side[0], cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&c->side[1], cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_join[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_join[1], cudaEventDisableTiming) != cudaSuccess ||
         cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaMallocHost((void**)&c->h_sc, sizeof(Scalars)) != cudaSuccess) {
         cudaGetLastError();
@@ -1448,6 +1495,11 @@ void dim3g_destroy(dim3g_ctx* c) {
         if (e) cudaEventDestroy(e);
     for (auto& e : c->evd)
         if (e) cudaEventDestroy(e);
+    if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+    for (int k = 0; k < 2; k++) {
+        if (c->ev_join[k]) cudaEventDestroy(c->ev_join[k]);
+        if (c->side[k]) cudaStreamDestroy(c->side[k]);
+    }
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
 }

@@ -143,10 +143,12 @@ struct PackSink {
     uint2* out;
     Reserve rs;
     uint32_t n = 0;
+    unsigned long long done = 0;  // pairs flushed
 
     __device__ __forceinline__ uint32_t tag(const RowCtx& c, uint32_t x) const { return c.id2x[x]; }
     __device__ __forceinline__ void flush() {
         if (n == 0) return;
+        done += n;
         unsigned long long base = 0;
         if (lane_id() == 0) base = atomicAdd(rs.cursor, (unsigned long long)n);
         base = __shfl_sync(0xffffffffu, base, 0);
@@ -175,7 +177,8 @@ struct PackSink {
 };
 
 // One join's small rows.
-static __global__ void __launch_bounds__(256, 4) k_single_pack(RowCtx c, Reserve rs, const uint32_t* __restrict__ rows,
+static __global__ void __launch_bounds__(256, 4) k_single_pack(RowCtx c, Reserve rs, unsigned long long* cls,
+                                                               const uint32_t* __restrict__ rows,
                                                                const unsigned long long* __restrict__ nrows_p) {
     extern __shared__ uint32_t smem[];
     const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
@@ -192,6 +195,7 @@ static __global__ void __launch_bounds__(256, 4) k_single_pack(RowCtx c, Reserve
         pack_rows(c, x, 0, n, tab, sink);
     }
     sink.flush();
+    if (lane == 0 && sink.done) atomicAdd(cls, sink.done);
 }
 
 }  // namespace dim3g

@@ -233,6 +233,7 @@ __device__ __forceinline__ void pf_work(const RowCtx& c, PfSmem& sm, uint32_t* t
 // Class 2 of the single pass with prefetched rows: 2^block_lg table words,
 // then one kStage staging buffer per expanding warp.
 static __global__ void __launch_bounds__(kPfThreads) k_single_block_pf(RowCtx c, Reserve rs,
+                                                                       unsigned long long* cls,
                                                                        const uint32_t* __restrict__ rows,
                                                                        const unsigned long long* __restrict__ nrows_p,
                                                                        uint32_t block_lg) {
@@ -258,6 +259,7 @@ static __global__ void __launch_bounds__(kPfThreads) k_single_block_pf(RowCtx c,
         uint32_t* stage = pf_raw + (1u << block_lg) + ((threadIdx.x >> 5) - 1) * kStage;
         StageSink sink{stage, c.out, rs, 0};
         pf_work(c, sm, pf_raw, block_lg, sink, &s_cc);
+        if (lane_id() == 0 && sink.done) atomicAdd(cls, sink.done);
     }
 }
 

@@ -39,9 +39,11 @@ struct StageSink {
     uint32_t xv;
     uint32_t n = 0;        // staged entries (warp-uniform)
     uint32_t cap = kStage;  // at least 32 * kUnroll
+    unsigned long long done = 0;  // pairs flushed
 
     __device__ __forceinline__ void flush() {
         if (n == 0) return;
+        done += n;
         unsigned long long base = 0;
         if (lane_id() == 0) base = atomicAdd(rs.cursor, (unsigned long long)n);
         base = __shfl_sync(0xffffffffu, base, 0);
@@ -83,9 +85,11 @@ struct PairStageSink {
     uint32_t xv;
     uint32_t cap;  // staged pairs the buffer holds (at least 32 * kUnroll)
     uint32_t n = 0;
+    unsigned long long done = 0;  // pairs flushed
 
     __device__ __forceinline__ void flush() {
         if (n == 0) return;
+        done += n;
         unsigned long long base = 0;
         if (lane_id() == 0) base = atomicAdd(rs.cursor, (unsigned long long)n);
         base = __shfl_sync(0xffffffffu, base, 0);
@@ -405,7 +409,8 @@ __host__ __device__ constexpr size_t warp_row_words(uint32_t warp_lg, uint32_t s
 }
 
 // Classes 1 and 5 (tiny): one warp per row.
-static __global__ void __launch_bounds__(256) k_single_warp(RowCtx c, Reserve rs, const uint32_t* __restrict__ rows,
+static __global__ void __launch_bounds__(256) k_single_warp(RowCtx c, Reserve rs, unsigned long long* cls,
+                                                            const uint32_t* __restrict__ rows,
                                                             const unsigned long long* __restrict__ nrows_p,
                                                             uint32_t warp_lg, uint32_t stage) {
     extern __shared__ uint32_t smem[];
@@ -416,20 +421,23 @@ static __global__ void __launch_bounds__(256) k_single_warp(RowCtx c, Reserve rs
     for (uint32_t ri = blockIdx.x * nw + wib; ri < nrows; ri += gridDim.x * nw)
         single_warp_row(c, rows[ri], tab, sink, warp_lg);
     sink.flush();
+    if (lane_id() == 0 && sink.done) atomicAdd(cls, sink.done);
 }
 
 // Class 2: one CTA per row; 2^block_lg table words, then one staging buffer
 // per warp.
 // Rows rows[skip0 + skip1 + i], i < *nrows_p (skips: device counts, either
 // may be null), taken through row counter c.next_row[ctr].
-static __global__ void __launch_bounds__(1024) k_single_block(RowCtx c, Reserve rs, const uint32_t* __restrict__ rows,
+static __global__ void __launch_bounds__(1024) k_single_block(RowCtx c, Reserve rs, unsigned long long* cls,
+                                                              const uint32_t* __restrict__ rows,
                                                               const unsigned long long* __restrict__ nrows_p,
                                                               uint32_t block_lg, const unsigned long long* skip0,
                                                               const unsigned long long* skip1, uint32_t ctr) {
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t s_row;
+    __shared__ unsigned long long s_done;
     __shared__ CtaChunks s_cc;
-    if (threadIdx.x == 0) s_cc.n = 0;
+    if (threadIdx.x == 0) s_cc.n = 0, s_done = 0;
     uint32_t* stage = smem + (1u << block_lg) + (threadIdx.x >> 5) * kStage;
     const uint32_t nrows = (uint32_t)*nrows_p;
     rows += (skip0 ? *skip0 : 0ull) + (skip1 ? *skip1 : 0ull);
@@ -438,7 +446,10 @@ static __global__ void __launch_bounds__(1024) k_single_block(RowCtx c, Reserve 
         StageSink sink{stage, c.out, rs, c.id2x[x]};
         single_block_row(c, x, smem, sink, block_lg, &s_cc);
         sink.flush();
+        if (lane_id() == 0) atomicAdd(&s_done, sink.done);
     }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_done) atomicAdd(cls, s_done);
 }
 
 // Classes 3/4: one CTA per row; a bitmap of bitmap_words, then one staging
