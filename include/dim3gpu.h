@@ -56,7 +56,9 @@ typedef struct {
     float ms_total;            /* device ms: whole call (inputs resident) */
     uint64_t launches;         /* kernels launched on this context since creation */
     float ms_count_cls[3];     /* count pass device ms per row kernel: bitmap, block, warp */
-    float ms_write_cls[3];     /* write pass device ms per row kernel: bitmap, block, warp */
+    float ms_write_cls[3];     /* write pass device ms per row kernel: bitmap, block, warp (of a join whose larger
+                                  relation has at most 2^22 tuples the kernels run beside each other: each from
+                                  the pass's start to its own end; ms_count_cls likewise) */
     uint64_t out_j_cls[3];     /* candidates (join tuples) per row kernel: bitmap, block, warp */
     uint64_t n_out_cls[3];     /* distinct pairs per row kernel (single pass): bitmap, block, warp */
     float ms_dense[3];         /* dense block device ms: selection + operands, tensor-core product, light pass */
@@ -81,7 +83,8 @@ const char* dim3g_last_error(const dim3g_ctx* ctx);
 int dim3g_get_stats(const dim3g_ctx* ctx, dim3g_stats* out);
 /* Tuning knobs, validated on set: "warp_slots_log2" (5..14, warp-class hash
  * set size), "block_slots_log2" (8..14, block-class hash set size),
- * "tile_bits_log2" (10..20, bitmap-class z tile width), "ordered_output" (0: one expansion per row, rows in unspecified order;
+ * "tile_bits_log2" (10..20, bitmap-class z tile width; at most 19 for
+ * materialised COUNT), "ordered_output" (0: one expansion per row, rows in unspecified order;
  * 1: count pass + write pass, pairs grouped by first value),
  * "block_threads" (256, 512 or 1024: CTA width of the block class),
  * "host_direct_output" (1: pinned host outputs written directly),
@@ -96,7 +99,9 @@ int dim3g_get_stats(const dim3g_ctx* ctx, dim3g_stats* out);
  * "dense_mem_mb" (bitmap budget of that product, default 16384: it takes as
  * many heavy rows as their x z bitmap fits, the largest first),
  * "sized_tables" (1: the mapping's hash tables are sized by a distinct-key
- * sketch to fit the L2 where keys repeat; 0: by the tuple counts),
+ * sketch to fit the L2 where keys repeat; 0: by the tuple counts, as always
+ * where both relations have at most 2^16 tuples and table_slack_pct is at
+ * least 100),
  * "table_slack_pct" (5..1000, default 150: slots of a sketch-sized table per
  * estimated distinct key, in percent; a table that overfills is rebuilt at
  * full size),

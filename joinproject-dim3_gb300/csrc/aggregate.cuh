@@ -114,6 +114,15 @@ struct CountRanked {
         return false;
     }
 };
+struct CountGlobal {  // ranked rows of many ranks, second pass
+    RankedTile t;
+    uint32_t lo;
+    uint32_t* g;
+    __device__ __forceinline__ bool insert(uint32_t z, bool act) {
+        if (act) atomicAdd(&g[t.rank(z - lo)], 1u);
+        return false;
+    }
+};
 struct NullSink {
     static constexpr bool kValues = false;
     template <uint32_t N>
@@ -263,10 +272,14 @@ __device__ __forceinline__ RankHead rank_head(const RowCtx& c, uint32_t item, ui
 // to the row's next places.  Called after a barrier that follows the previous
 // row; *s_pos as the caller keeps it for the row.  ahead() runs on thread 0
 // during the first pass (the other warps take its share of the pieces).
+// g: the CTA's tile_width counters in global memory, all zero between calls,
+// or null.  A tile of more than two windows of ranks counts there in one walk
+// instead of one walk a window.
 template <class Ahead>
 __device__ __forceinline__ void agg_ranked_tile(const RowCtx& c, const AggOut& ao, const RankHead& h, uint32_t t,
                                                 uint32_t* smem, const RankLayout& l, CtaChunks* cc, uint32_t* s_pos,
-                                                uint32_t* s_wbase, unsigned long long* s_base, Ahead ahead) {
+                                                uint32_t* s_wbase, unsigned long long* s_base, uint32_t* g,
+                                                Ahead ahead) {
     const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
     const uint32_t x = h.x, e0 = h.e0, e1 = h.e1, ne = e1 - e0, lo = t * c.tile_width, xv = h.xv;
     uint32_t* bm = smem;
@@ -317,6 +330,41 @@ __device__ __forceinline__ void agg_ranked_tile(const RowCtx& c, const AggOut& a
     }
     GroupSums gs;
     const RankedTile rt{bm, pre, s_wbase, l.wsh};
+    if (g && d > 2 * l.cap) {
+        __syncthreads();  // *s_base; cc->n
+        CountGlobal cg{rt, lo, g};
+        if (staged) balanced_expand(c, ne, cg, sink, cc->st.seg.s0, cc->st.seg.incl, cc->ctot, pol, wib, nw, &cc->n, kDynPiece);
+        else cta_expand_balanced(c, e0, e1, t, t + 1, cg, sink, cc);
+        __syncthreads();
+        const unsigned long long base = ao.sum.tiles ? 0ull : *s_base;
+        for (uint32_t wb = w0; wb < w1; wb += 4) {  // a warp's own words, a lane a bit
+            uint32_t r[4], v[4], z[4];
+            bool on[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                const uint32_t b = bm[wb + k];
+                on[k] = b >> lane & 1u;
+                r[k] = s_wbase[wib] + pre[wb + k] + __popc(b & lanemask_lt());
+                v[k] = on[k] ? __ldcg(&g[r[k]]) : 0u;
+                z[k] = on[k] ? __ldg(&c.id2z[lo + (wb + k) * 32 + lane]) : 0u;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                if (!on[k]) continue;
+                __stcg(&g[r[k]], 0u);
+                if (ao.sum.tiles) {
+                    gs.add(xv, z[k], v[k]);
+                } else if (base != ~0ull) {
+                    st_stream(&c.out[base + r[k]], make_uint2(xv, z[k]));
+                    __stcs(&ao.cnt[base + r[k]], (unsigned long long)v[k]);
+                }
+            }
+        }
+        if (threadIdx.x == 0) cc->n = 0;
+        __syncthreads();  // the next row's bitmap
+        if (ao.sum.tiles) ao.sum.commit(xv, gs.g, gs.cs, gs.h);
+        return;
+    }
     for (uint32_t r0 = 0; r0 < d; r0 += l.cap) {
         const uint32_t n = min(l.cap, d - r0);
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) ctr[i] = 0;
@@ -351,6 +399,81 @@ __device__ __forceinline__ void agg_ranked_tile(const RowCtx& c, const AggOut& a
         __syncthreads();  // the next window's counters; the next row's bitmap
     }
     if (ao.sum.tiles) ao.sum.commit(xv, gs.g, gs.cs, gs.h);
+}
+
+// ---------------------------------------------------------- direct rows
+// Rows of many candidates: a counter per z of a tile of at most
+// 2^kAggDirectLg ids, so the candidates are walked once -- ranked rows walk
+// them twice and once more for every window of ranks past the first, which is
+// what a dense row pays for most (a 1/16 slice of the 16M-tuple COUNT on the
+// sparse kernels, 830K candidates a row over 1M z: ranked 47 s, direct 0.65).
+constexpr uint32_t kAggDirectLg = 15;
+// The whole CTA, as agg_ranked_tile; ctr holds a word a z of the tile.  The
+// caller commits a summary's sums, once a row.
+template <class Ahead>
+__device__ __forceinline__ void agg_direct_tile(const RowCtx& c, const AggOut& ao, const RankHead& h, uint32_t t,
+                                                uint32_t* ctr, CtaChunks* cc, uint32_t* s_pos, uint32_t* s_wbase,
+                                                unsigned long long* s_base, GroupSums& gs, Ahead ahead) {
+    const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
+    const uint32_t ne = h.e1 - h.e0, lo = t * c.tile_width, width = min(c.tile_width, c.m - lo), xv = h.xv;
+    const uint64_t pol = l2_keep_policy();
+    const bool staged = ne <= kRowBlk;
+    NullSink sink;
+    for (uint32_t i = threadIdx.x; i < width; i += blockDim.x) ctr[i] = 0;
+    if (staged) balanced_stage(c, h.e0, ne, t, t + 1, cc, pol, wib, nw);
+    if (threadIdx.x == 0) cc->n = 0;
+    __syncthreads();
+    if (threadIdx.x == 0) ahead();
+    __syncwarp();
+    CountTile set{ctr, lo};
+    if (staged) balanced_expand(c, ne, set, sink, cc->st.seg.s0, cc->st.seg.incl, cc->ctot, pol, wib, nw, &cc->n, 0);
+    else cta_expand_balanced(c, h.e0, h.e1, t, t + 1, set, sink, cc);
+    __syncthreads();
+    const uint32_t per = (((width + nw - 1) / nw) + 31) & ~31u, s0 = min(width, wib * per), s1 = min(width, s0 + per);
+    if (ao.sum.tiles) {
+        for (uint32_t i = s0 + lane; i < s1; i += 32)
+            if (ctr[i]) gs.add(xv, __ldg(&c.id2z[lo + i]), ctr[i]);
+        __syncthreads();  // the next tile's counters
+        return;
+    }
+    // the warps' places in one reservation a tile
+    uint32_t n = 0;
+    for (uint32_t i = s0 + lane; i < s1; i += 32) n += ctr[i] != 0;
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) s_wbase[wib] = n;
+    __syncthreads();
+    if (wib == 0) {
+        const uint32_t v = lane < nw ? s_wbase[lane] : 0u, inc = warp_incl_scan(v);
+        const uint32_t d = __shfl_sync(0xffffffffu, inc, 31);
+        __syncwarp();
+        s_wbase[lane] = inc - v;
+        const unsigned long long base = d ? group_place(c, ao, h.x, d, s_pos) : ~0ull;
+        if (lane == 0) *s_base = base;
+    }
+    __syncthreads();
+    if (*s_base != ~0ull) {
+        unsigned long long base = *s_base + s_wbase[wib];
+        for (uint32_t sb = s0; sb < s1; sb += 128) {  // four id gathers in flight
+            uint32_t v[4], z[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                const uint32_t i = sb + k * 32 + lane;
+                v[k] = i < s1 ? ctr[i] : 0u;
+                z[k] = v[k] ? __ldg(&c.id2z[lo + i]) : 0u;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                const uint32_t b = __ballot_sync(0xffffffffu, v[k] != 0);
+                if (v[k]) {
+                    const unsigned long long pos = base + __popc(b & lanemask_lt());
+                    st_stream(&c.out[pos], make_uint2(xv, z[k]));
+                    __stcs(&ao.cnt[pos], (unsigned long long)v[k]);
+                }
+                base += __popc(b);
+            }
+        }
+    }
+    __syncthreads();  // the next tile's counters
 }
 
 // ------------------------------------------------------------ tiny rows
@@ -471,8 +594,11 @@ static __global__ void __launch_bounds__(1024, 1) k_agg_map(RowCtx c, AggOut ao,
 }
 
 // Ranked rows (classes 4, then 3).  Cursor and summaries: one CTA a row and
-// tile, so a huge row's tiles run side by side; offsets: one CTA a row.  The
+// tile, so a huge row's tiles run side by side; offsets, and the summaries of
+// direct rows (their sums meet in a few addresses, once a row): one CTA a row.  The
 // next item is claimed and its header loaded during the current one.
+// DIRECT: direct rows, `l` unused.
+template <bool DIRECT>
 static __global__ void __launch_bounds__(1024, 1) k_agg_ranked(RowCtx c, AggOut ao, const uint32_t* __restrict__ rows,
                                                             const unsigned long long* __restrict__ n3,
                                                             const unsigned long long* __restrict__ n4, RankLayout l) {
@@ -481,7 +607,7 @@ static __global__ void __launch_bounds__(1024, 1) k_agg_ranked(RowCtx c, AggOut 
     __shared__ unsigned long long s_base;
     __shared__ RankHead s_head[2];
     __shared__ CtaChunks s_cc;
-    const uint32_t per = ao.rs.cursor || ao.sum.tiles ? c.T : 1u;
+    const uint32_t per = ao.rs.cursor || (ao.sum.tiles && !DIRECT) ? c.T : 1u;
     const uint32_t items = (uint32_t)(*n3 + *n4) * per;
     auto claim = [&](RankHead* dst) {
         const uint32_t i = atomicAdd(&c.next_row[3], 1u);
@@ -493,17 +619,17 @@ static __global__ void __launch_bounds__(1024, 1) k_agg_ranked(RowCtx c, AggOut 
         const RankHead h = s_head[k];
         if (h.item >= items) break;
         if (threadIdx.x == 0) s_pos = 0;
-        if (per == c.T) {
-            agg_ranked_tile(c, ao, h, h.item % per, smem, l, &s_cc, &s_pos, s_wbase, &s_base,
-                            [&] { claim(&s_head[k ^ 1]); });
-        } else {
-            for (uint32_t t = 0; t < c.T; t++) {
-                agg_ranked_tile(c, ao, h, t, smem, l, &s_cc, &s_pos, s_wbase, &s_base, [&] {
-                    if (t == 0) claim(&s_head[k ^ 1]);
-                });
-                __syncthreads();
-            }
+        const uint32_t t0 = per == c.T ? h.item % per : 0u, t1 = per == c.T ? t0 + 1 : c.T;
+        GroupSums gs;
+        for (uint32_t t = t0; t < t1; t++) {
+            auto ahead = [&] {
+                if (t == t0) claim(&s_head[k ^ 1]);
+            };
+            if (DIRECT) agg_direct_tile(c, ao, h, t, smem, &s_cc, &s_pos, s_wbase, &s_base, gs, ahead);
+            else agg_ranked_tile(c, ao, h, t, smem, l, &s_cc, &s_pos, s_wbase, &s_base, nullptr, ahead);
+            __syncthreads();
         }
+        if (DIRECT && ao.sum.tiles) ao.sum.commit(h.xv, gs.g, gs.cs, gs.h);
         __syncthreads();
     }
 }

@@ -9,9 +9,9 @@
 //   -> CSR scans (by f, by (y, f tile); bounded by the layout's counts)
 //   -> k_ix_scatter (a batch builds only the CSR each relation's query reads)
 // Query pass over queries (P, Q) of a set:
-//   k_q_setup -> k_q_ymap -> k_q_entries -> k_q_rows -> k_q_row_work
-//   -> class lists (one partition) -> project row kernels -> COUNT row
-//   kernels -> per-query results to pinned host memory
+//   k_q_setup -> k_q_ymap -> k_q_work -> class lists (one partition)
+//   -> project and COUNT row kernels on forked streams -> per-query results
+//   to pinned host memory
 // Every size the launches depend on is known on the host from the tuple
 // counts; counts that depend on the data (distinct values, rows per class,
 // output sizes) stay on the device.  The data-dependent bounds -- the
@@ -115,6 +115,8 @@ struct QueryScratch {
     size_t qmem_bytes = 0;
     QueryRes* h_res = nullptr;  // pinned
     uint32_t h_res_n = 0;
+    uint32_t* agg = nullptr;  // COUNT rows of many ranks: a CTA's counters a tile id
+    size_t agg_bytes = 0;
     // The row kernels of a pass are independent (each has its own list and
     // counter; results meet in the queries' cursors), so they fork from the
     // pass's stream onto these and join again: a kernel whose last rows are
@@ -126,6 +128,7 @@ struct QueryScratch {
     QueryScratch& operator=(const QueryScratch&) = delete;
     ~QueryScratch() {
         if (qmem) cudaFree(qmem);
+        if (agg) cudaFree(agg);
         if (h_res) cudaFreeHost(h_res);
         for (int k = 0; k < 2; k++) {
             if (side[k]) cudaStreamDestroy(side[k]);
@@ -618,7 +621,7 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
         } else {
             const size_t ss_m = 200 << 10;
             k_b_agg_ranked<<<resident(k_b_agg_ranked, 1024, ss_m, sm), 1024, ss_m, st>>>(
-                Q, BatchRows{lm, &n[4], &n[3], &next[2]}, ss_m);
+                Q, BatchRows{lm, &n[4], &n[3], &next[2]}, ss_m, qs.agg, s->tile_lg);
             BLAUNCH();
             auto map_rows = [&](const BatchRows& rows, uint32_t lg) -> int {
                 const int thr = lg >= 14 ? 1024 : (lg == 13 ? 512 : (lg == 12 ? 256 : 128));
@@ -665,6 +668,24 @@ int set_batch_attributes(dim3g_ctx* ctx) {
     BCU(cudaFuncSetAttribute(k_b_agg_map, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 << 14));
     BCU(cudaFuncSetAttribute(k_b_agg_ranked, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10));
     BCU(cudaFuncSetAttribute(k_b_agg_pack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * kAggPackWords * 4)));
+    return DIM3G_OK;
+}
+
+// One CTA of k_b_agg_ranked an SM (200 KB of shared memory each).
+int ensure_agg_scratch(dim3g_relset* s, QueryScratch& qs) {
+    dim3g_ctx* ctx = s->ctx;
+    const size_t need = (size_t)I::sm_count(ctx) * ((size_t)1 << s->tile_lg) * 4;
+    if (qs.agg_bytes >= need) return DIM3G_OK;
+    if (qs.agg) cudaFree(qs.agg);
+    qs.agg = nullptr;
+    qs.agg_bytes = 0;
+    if (cudaMalloc(&qs.agg, need) != cudaSuccess) {
+        cudaGetLastError();
+        return I::fail(ctx, DIM3G_ERR_NOMEM, "COUNT scratch: device allocation of %zu bytes failed", need);
+    }
+    // counters start at zero; every row resets the counters it touched
+    BCU(cudaMemset(qs.agg, 0, need));
+    qs.agg_bytes = need;
     return DIM3G_OK;
 }
 
@@ -810,6 +831,7 @@ int dim3g_relset_join(dim3g_relset* s, dim3g_query* q, uint32_t n) {
     cudaStream_t st = I::stream(ctx);
     QueryPlan qp;
     int r = query_plan(s, s->qs, q, n, qp);
+    if (!r && qp.has_count) r = ensure_agg_scratch(s, s->qs);
     if (!r) r = query_upload(s, qp);
     if (r) return r;
     uint64_t launches = 0;
@@ -854,6 +876,7 @@ int dim3g_batch_create(dim3g_ctx* ctx, const dim3g_relation* rels, const dim3g_q
     if (!r) r = relset_sketch(&b->set, b->rels.data(), 2 * n);
     if (!r) r = relset_plan(&b->set, b->rels.data(), 2 * n, 0);
     if (!r) r = query_plan(&b->set, b->set.qs, b->queries.data(), n, b->qp);
+    if (!r && b->qp.has_count) r = ensure_agg_scratch(&b->set, b->set.qs);
     if (!r) r = batch_capture(b);
     if (r) {
         delete b;
@@ -1224,6 +1247,8 @@ int dim3g_server_create(dim3g_relset* set, uint32_t lanes, uint32_t max_batch, u
             return I::fail(ctx, DIM3G_ERR_NOMEM, "server lane pinned staging");
         }
         L->qs.h_res_n = max_batch;
+        int r = ensure_agg_scratch(set, L->qs);
+        if (r) return r;
         fixed += L->qs.qmem_bytes;
         S->lanes.push_back(std::move(L));
     }

@@ -773,7 +773,8 @@ static __global__ void __launch_bounds__(1024, 1) k_b_agg_map(QueryPools Q, Batc
 
 // Ranked rows: a row's z tiles are taken in turn; the next row is claimed, and
 // its query and header looked up, during the current one.
-static __global__ void __launch_bounds__(1024, 1) k_b_agg_ranked(QueryPools Q, BatchRows L, size_t smem_bytes) {
+static __global__ void __launch_bounds__(1024, 1) k_b_agg_ranked(QueryPools Q, BatchRows L, size_t smem_bytes,
+                                                                uint32_t* ctr, uint32_t tile_lg) {
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t s_q[2], s_pos, s_wbase[33];
     __shared__ unsigned long long s_base;
@@ -798,7 +799,7 @@ static __global__ void __launch_bounds__(1024, 1) k_b_agg_ranked(QueryPools Q, B
         const RankHead h = s_head[k];
         const RankLayout l = rank_layout(c.tile_width, blockDim.x >> 5, smem_bytes);
         for (uint32_t t = 0; t < c.T; t++) {
-            agg_ranked_tile(c, ao, h, t, smem, l, &s_cc, &s_pos, s_wbase, &s_base, [&] {
+            agg_ranked_tile(c, ao, h, t, smem, l, &s_cc, &s_pos, s_wbase, &s_base, ctr + ((size_t)blockIdx.x << tile_lg), [&] {
                 if (t == 0) claim(k ^ 1);
             });
             __syncthreads();

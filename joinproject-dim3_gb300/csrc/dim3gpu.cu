@@ -5,11 +5,13 @@
 //             insertion, dense ids by prefix sums over occupied slots
 //             (replaces mapping_step + LS_mapper, dim3.hpp:394-883)
 //   CSR       R by x id, S by (y id, z tile) (divide_R / divide_S,
-//             dim3.hpp:1058-1259), per-row work and row binning
-//   count     per-row distinct counts, prefix sum to output offsets
-//   write     the same expansion emitting (x value, z value) pairs
-// (Hybrid_solution, dim3.hpp:889-974).  Two host synchronisations: one for
-// the id domain sizes, one for the output size.
+//             dim3.hpp:1058-1259), per-row work and row lists
+//   rows      one expansion of every row by class, emitting through a cursor
+//             (ordered output: a count pass, offsets, a write pass), the
+//             classes' kernels on forked streams
+// (Hybrid_solution, dim3.hpp:889-974).  The host waits for the sketch, the
+// id domain sizes, the rows per class and the output size; a small join only
+// for the last.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdarg.h>
@@ -111,6 +113,16 @@ struct Params {
 constexpr uint64_t kSmallSlots = (uint64_t)1 << 17;  // tuple-sized tables this small are not sized by a sketch
 constexpr size_t kMaxSmemOptin = 227 * 1024;  // dynamic shared memory a CTA may opt into
 constexpr uint32_t kFlatAvgBitmap = 160, kFlatAvgBlock = 560, kFlatAvgWarp = 160;  // single pass, per row class
+// COUNT joins of more possible candidates than this are not small: their row
+// classes are read back (kAggDirectCand).  2^24 candidates are about as long as
+// the round trip that saves.
+constexpr uint64_t kSmallAggCand = 1ull << 24;
+// Candidates a z tile of 2^kAggDirectLg ids (aggregate.cuh), on average over
+// the bitmap rows, from which COUNT rows count directly: below, the tiles' fixed cost
+// is the larger.  Direct and ranked: 2000 rows of 40K candidates over 200K z
+// (5.7K a tile) 1.25 and 1.49 ms, of 8K (1.1K a tile) 1.18 and 0.46; 3000 rows
+// of 10K over 30K z 0.46 and 0.45.
+constexpr uint64_t kAggDirectCand = 4096;
 constexpr uint32_t kAggTileLgMax = 19;  // join-aggregate z tile (its bitmap and ranks are 96 KB)
 
 struct Scalars {
@@ -150,6 +162,7 @@ struct dim3g_ctx {
     // Streams of the row kernels beside the context's (RowStreams).
     cudaStream_t side[2] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {};
+    bool rows_in_turn = false;  // no forks: each class's kernels timed alone
     cudaEvent_t ev[6] = {};
     cudaEvent_t evc[8] = {};  // per row-class kernel timing
     cudaEvent_t evd[4] = {};  // dense block: selection, operands, product, light pass
@@ -252,7 +265,7 @@ struct RowLists {
 };
 struct RowStreams;
 int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc, const uint32_t* list_t,
-                  RowStreams& rst);
+                  RowStreams& rst, bool direct);
 
 // Warps per CTA of a warp-per-row kernel whose warps each own per_warp
 // bytes of shared memory: up to 8, within about a third of an SM's shared
@@ -282,6 +295,12 @@ unsigned resident_grid(dim3g_ctx* c, K kernel, int block, size_t smem) {
 // the rest of the GPU to the next.  Whole calls, in turn and forked: 1.2M-edge
 // 2-hop 1.48 and 1.44 ms, its COUNT 3.63 and 3.40, 200k rows ordered 0.79 and
 // 0.76, an eighth of the 20M-edge 2-hop 10.37 and 10.23.
+//
+// Calls of more than kForkTuples driving tuples keep the kernels in turn: their
+// tails are a small part there (20M-edge 2-hop 74.97 ms in
+// turn, 74.70 forked), and the per-class times of the
+// statistics stay each kernel's own.
+constexpr uint64_t kForkTuples = 1ull << 22;
 struct RowStreams {
     dim3g_ctx* c;
     bool on, open = false;
@@ -702,6 +721,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     const bool small_tables = fullP <= kSmallSlots && fullQ <= kSmallSlots && c->prm.table_slack_pct >= 100;
     const uint32_t dense_mode = jp.aggregate ? 0 : c->prm.dense;
     const bool small = small_tables && jp.single_pass && !jp.count_only && jp.nQ <= (1ull << c->prm.tile_lg) &&
+                       (!jp.aggregate || jp.nP * jp.nQ <= kSmallAggCand) &&
                        (dense_mode == 0 || (dense_mode == 1 && (jp.nP * jp.nQ < kDenseMinCand ||
                                                                 jp.nQ <= (1ull << (c->prm.block_lg - 1)))));
     // table capacities from the distinct-key sketch (see mapping.cuh)
@@ -783,9 +803,16 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     if (m >= 0x80000000u || n >= 0x80000000u)
         return fail(c, DIM3G_ERR_UNSUPPORTED, "key domains of 2^31 or more distinct values are not supported");
 
+    // COUNT rows of many candidates count directly (agg_direct_tile), in z
+    // tiles of at most 2^kAggDirectLg ids: known once the rows are binned, S's
+    // CSR is then built again in those tiles
+    bool direct = false, retiled = false;
+    DensePlan dp;
+retile:
     // z tiles for the bitmap class
     uint32_t tile_lg = c->prm.tile_lg;
     if (jp.aggregate && tile_lg > kAggTileLgMax) tile_lg = kAggTileLgMax;
+    if (direct && tile_lg > kAggDirectLg) tile_lg = kAggDirectLg;
     uint32_t T = 1, tile_shift = 31, tile_width = m;
     if (m > (1u << tile_lg)) {
         tile_shift = tile_lg;
@@ -880,11 +907,27 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
                                                                              sc->nrows, sc->nrows_b);
     CHECK_LAUNCH();
     CU(cudaEventRecord(c->ev[2], st));
-    DensePlan dp;
-    {
+    if (!retiled) {
         S.dense_skip = dense_mode == 0 ? 1 : 2;  // off, or too little heavy work
         int r = small ? DIM3G_OK : run_dense(c, jp, rc, sc, list_m, k, m, &dp);
         if (r) return r;
+    }
+    if (jp.aggregate && !small && !dp.on && !retiled) {
+        if (!dp.counted) {
+            CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
+            CU(cudaStreamSynchronize(st));
+            if (c->h_sc->err) return fail(c, DIM3G_ERR_DEVICE, "device bound violated in row binning (flags %u)", c->h_sc->err);
+            dp.counted = true;
+        }
+        const uint64_t rows = c->h_sc->nrows[3] + c->h_sc->nrows[4], cand = c->h_sc->outj_cls[3] + c->h_sc->outj_cls[4];
+        const uint64_t Td = ((uint64_t)m + (1u << kAggDirectLg) - 1) >> kAggDirectLg;
+        direct = rows && cand >= rows * Td * kAggDirectCand && (uint64_t)k * Td < (1ull << 31);
+        if (direct && tile_width > (1u << kAggDirectLg)) {
+            // everything k_row_work and k_row_lists counted, once more
+            CU(cudaMemsetAsync((char*)sc + offsetof(Scalars, outj), 0, sizeof(Scalars) - offsetof(Scalars, outj), st));
+            retiled = true;
+            goto retile;
+        }
     }
 
     // Row counts are read on the device; grids are resident CTAs x SMs.
@@ -907,14 +950,15 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
                            dp.counted ? h.nrows_b[2] != 0 : m > rb.cap_m};
     const bool has_any_b = !dp.counted || h.nrows[2], has_w = !dp.counted || h.nrows[1],
                has_t = !dp.counted || h.nrows[5];
-    RowStreams rst(c, dp.counted ? has_m + has_any_b + (has_w || has_t) > 1 : !small && jp.aggregate);
+    RowStreams rst(c, jp.nP <= kForkTuples && !c->rows_in_turn &&
+                          (dp.counted ? has_m + has_any_b + (has_w || has_t) > 1 : !small && jp.aggregate));
 
     if (jp.sum.tiles) {
         // summaries: the expansion kernels hash instead of writing; COUNT
         // needs no count pass (nothing is placed)
         CU(cudaEventRecord(c->evc[4], st));
         if (jp.aggregate) {
-            int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, nullptr, rst);
+            int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, nullptr, rst, direct);
             if (r) return r;
         } else {
             k_sum_bitmap<<<resident_grid(c, k_sum_bitmap, blk_m, smem_m), blk_m, smem_m, st>>>(rc, jp.sum, L.m,
@@ -956,7 +1000,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
         rc.out = sp_out;
     }
     if (single && jp.aggregate) {
-        int r = run_aggregate(c, rc, AggOut{sp_cnt, SumAcc{}, Reserve{&sc->cursor, cap}}, L, sc, list_t, rst);
+        int r = run_aggregate(c, rc, AggOut{sp_cnt, SumAcc{}, Reserve{&sc->cursor, cap}}, L, sc, list_t, rst, direct);
         if (r) return r;
         CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
         CU(cudaEventRecord(c->ev[3], st));
@@ -1160,7 +1204,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     CU(cudaMemsetAsync(sc->next_row, 0, sizeof(sc->next_row), st));
     if (total > 0) {
         if (jp.aggregate) {
-            int r = run_aggregate(c, rc, AggOut{out_cnt, SumAcc{}, Reserve{nullptr, 0}}, L, sc, nullptr, rst);
+            int r = run_aggregate(c, rc, AggOut{out_cnt, SumAcc{}, Reserve{nullptr, 0}}, L, sc, nullptr, rst, direct);
             if (r) return r;
         } else {
             CU(cudaEventRecord(c->evc[4], st));
@@ -1196,15 +1240,21 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
 // rows from the largest maps down, then the tiny rows (list_t; null: none).
 // CTAs by map size, so that small maps run many rows an SM.
 int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc,
-                  const uint32_t* list_t, RowStreams& rst) {
+                  const uint32_t* list_t, RowStreams& rst, bool direct) {
     CU(rst.fork());
     // one ranked CTA an SM with all of its shared memory, or two where a
     // half leaves 60 KB for the counters
     const bool half = rank_layout(rc.tile_width, 16, 0).words * 6 + (60u << 10) <= (102u << 10);
     const int thr_m = half ? 512 : 1024;
     const size_t smem_m = half ? 102 << 10 : 200 << 10;
-    k_agg_ranked<<<resident_grid(c, k_agg_ranked, thr_m, smem_m), thr_m, smem_m, rst.m>>>(
-        rc, ao, L.m, L.n3, L.n4, rank_layout(rc.tile_width, thr_m / 32, smem_m));
+    if (direct) {
+        const size_t sd = (size_t)rc.tile_width * 4;
+        k_agg_ranked<true><<<resident_grid(c, k_agg_ranked<true>, 1024, sd), 1024, sd, rst.m>>>(rc, ao, L.m, L.n3, L.n4,
+                                                                                            RankLayout{});
+    } else {
+        k_agg_ranked<false><<<resident_grid(c, k_agg_ranked<false>, thr_m, smem_m), thr_m, smem_m, rst.m>>>(
+            rc, ao, L.m, L.n3, L.n4, rank_layout(rc.tile_width, thr_m / 32, smem_m));
+    }
     CHECK_LAUNCH();
     auto map_rows = [&](const uint32_t* rows, const unsigned long long* n, uint32_t lg, const unsigned long long* s0,
                         const unsigned long long* s1, uint32_t ctr) -> int {
@@ -1241,7 +1291,8 @@ bool set_aggregate_attributes() {
            cudaFuncSetAttribute(k_sum_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 1 << 14 << 2) == cudaSuccess &&
            cudaFuncSetAttribute(k_sum_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, (1 << 20) / 8) == cudaSuccess &&
            cudaFuncSetAttribute(k_agg_map, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 << 14) == cudaSuccess &&
-           cudaFuncSetAttribute(k_agg_ranked, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10) == cudaSuccess;
+           cudaFuncSetAttribute(k_agg_ranked<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10) == cudaSuccess &&
+           cudaFuncSetAttribute(k_agg_ranked<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kAggDirectLg) == cudaSuccess;
 }
 
 int ensure_dev(dim3g_ctx* c, void** p, size_t* have, size_t need) {
@@ -1395,6 +1446,7 @@ namespace dim3g_internal {
 cudaStream_t stream(const dim3g_ctx* c) { return c->stream; }
 int device(const dim3g_ctx* c) { return c->device; }
 int sm_count(const dim3g_ctx* c) { return c->sm_count; }
+void rows_in_turn(dim3g_ctx* c, bool on) { c->rows_in_turn = on; }
 void add_launches(dim3g_ctx* c, uint64_t n) { c->launches += n; }
 void set_sparse_rate(dim3g_ctx* c, double bytes_per_s) {
     if (bytes_per_s > 0) c->cm.sparse_bw = bytes_per_s;

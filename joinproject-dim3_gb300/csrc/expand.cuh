@@ -440,6 +440,11 @@ __device__ __forceinline__ void balanced_stage(const RowCtx& c, uint32_t eb, uin
 // dyn (optional, zeroed before the barrier that precedes this): a shared
 // counter from which the warps take pieces of dyn_piece candidates instead
 // of equal static shares.
+// dyn_piece 0: a warp's share of the candidates, at least 256 and at most
+// this many (direct COUNT rows, whose tiles hold 4K candidates and up: a slice
+// of the 16M-tuple COUNT takes 1024 ms in pieces of 256, 698 up to 1024, 646
+// up to 4096).
+constexpr uint32_t kDynPieceMax = 4096;
 template <class Set, class Sink>
 __device__ __forceinline__ void balanced_expand(const RowCtx& c, uint32_t ne, Set& set, Sink& sink,
                                                 const uint32_t* s0a, const uint32_t* lena, const uint32_t* ctota,
@@ -452,7 +457,8 @@ __device__ __forceinline__ void balanced_expand(const RowCtx& c, uint32_t ne, Se
     const uint32_t inc = warp_incl_scan(v);
     if (__any_sync(0xffffffffu, inc < v)) raise_error(c.err, kErrCountRange);
     const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-    const uint32_t piece = dyn ? dyn_piece : total / nw + (total % nw ? 1u : 0u);
+    const uint32_t share = total / nw + (total % nw ? 1u : 0u);
+    const uint32_t piece = !dyn ? share : (dyn_piece ? dyn_piece : min(max((share + 127) & ~127u, 256u), kDynPieceMax));
     for (uint32_t round = 0;; round++) {
     uint32_t p0;
     if (dyn) {

@@ -92,6 +92,31 @@ def test_row_widths(built, name, prm):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("prm", [{}, {"tile_bits_log2": 12}, {"dense_block": 0, "warp_slots_log2": 6, "block_slots_log2": 10}],
+                         ids=lambda p: ",".join(f"{k}={v}" for k, v in p.items()) or "default")
+@pytest.mark.parametrize("m", [9000, 32_768, 32_769, 98_305])
+def test_count_rows_of_many_candidates(built, m, prm):
+    """COUNT rows of 4096 and more candidates a tile, in the output and in the
+    summaries, beside rows of a few and of one tile's."""
+    import dim3gpu
+    rng = np.random.default_rng(m)
+    S = [np.stack([rng.choice(m, 8000, replace=False), np.full(8000, y)], 1) for y in range(40)]
+    S = np.concatenate(S + [np.stack([np.arange(m), np.full(m, 40)], 1)]).astype(np.uint32)
+    R = np.array([(x, y) for x in range(30) for y in range(40)] + [(77, 40), (78, 0), (79, 99)] +
+                 [(100 + i, i % 40) for i in range(20)] + [(5, 7)] * 40, dtype=np.uint32)
+    c = dim3gpu.Context(0)
+    for k, v in {"keep_roles": 1, **prm}.items():
+        c.set_param(k, v)
+    check(c, R, S, (m, prm))
+    import torch
+    dR, dS = (torch.from_numpy(a.view(np.int32)).cuda() for a in (R, S))
+    wg, wc, _, _, _ = O.join_count(R, S)
+    want = O.tile_summary(np.ascontiguousarray(wg[:, ::-1]), wc, 4)  # the oracle's pairs are (z, x)
+    assert np.array_equal(c.join_count_summary(dR, R.shape[0], dS, S.shape[0], 4), want)
+    c.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("nx", [1, 2, 4095, 4096, 4097, 3 * 4096 + 1, 70_001])
 def test_scan_tiles(built, nx):
     """Ids, row offsets and lists over prefix sums of one tile, its edges and
