@@ -594,6 +594,7 @@ int run_dense(dim3g_ctx* c, const JoinPlan& jp, const RowCtx& rc, Scalars* sc, c
         CHECK_LAUNCH();
         k_dense_maxcnt<<<grid_for(ntile, sm), 256, 0, st>>>(tcnt, ntile, flag + 1);
         CHECK_LAUNCH();
+        // (32-bit sums: a bucket above kDenseBucketMax is refused below)
         SCAN(U32Src{tcnt}, RowPtrDst{toff, tcur}, ntile + 1, bsum, ltotal, &sc->err);
         unsigned int hflag[2] = {0, 0};
         unsigned long long hl = 0;
@@ -1168,7 +1169,7 @@ retile:
         int r = pass(std::false_type{}, &c->evc[0]);
         if (r) return r;
     }
-    SCAN(U32Src{cnt}, OffDst{off}, (uint64_t)n + 1, bsum2, &sc->total, &sc->err);
+    SCAN(RowCountSrc{cnt}, OffDst{off}, (uint64_t)n + 1, bsum2, &sc->total, &sc->err);
     CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
     CU(cudaEventRecord(c->ev[3], st));
     CU(cudaStreamSynchronize(st));

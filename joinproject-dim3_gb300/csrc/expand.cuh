@@ -788,6 +788,13 @@ static __global__ void __launch_bounds__(256) k_row_lists(const uint8_t* __restr
         if (b[k] < kRowBuckets) s_at[b[k]][rank[k]] = (uint32_t)(t0 + k * 256 + threadIdx.x);
 }
 
+// Output offsets from the rows' distinct counts.  A row has up to m pairs, so
+// 4096 rows pass 2^32 from 2^20 pairs a row on.
+struct RowCountSrc {
+    using Sum = uint64_t;
+    const uint32_t* a;
+    __device__ uint64_t operator()(uint64_t i) const { return a[i]; }
+};
 struct OffDst {
     unsigned long long* off;
     __device__ void operator()(uint64_t i, uint64_t e, uint64_t) const { off[i] = e; }

@@ -57,6 +57,7 @@ __device__ __forceinline__ unsigned long long* mapper_slot(DevTable t, uint32_t 
 
 // first[i] = 1 when occurrence i is its key's first occurrence in the batch.
 struct FirstOccSrc {
+    using Sum = uint32_t;
     DevTable t;
     const uint32_t* keys;
     __device__ uint64_t operator()(uint64_t i) const {

@@ -216,6 +216,7 @@ static __global__ void __launch_bounds__(256) k_probe_q(const uint2* __restrict_
 
 // Table compaction: ids by prefix sum over occupied slots.
 struct OccupiedSrc {
+    using Sum = uint32_t;
     const unsigned long long* slots;
     __device__ uint64_t operator()(uint64_t i) const { return slots[i] != kEmpty64 ? 1u : 0u; }
 };
@@ -272,6 +273,7 @@ static __global__ void __launch_bounds__(256) k_map(MapArgs a) {
 
 // Row pointers from a histogram: JR[i] = cursor[i] = exclusive prefix.
 struct U32Src {
+    using Sum = uint32_t;
     const uint32_t* a;
     __device__ uint64_t operator()(uint64_t i) const { return a[i]; }
 };

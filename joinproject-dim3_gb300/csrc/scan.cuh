@@ -22,8 +22,10 @@ constexpr unsigned long long kScanSum = 1, kScanPrefix = 2;
 // Polls of one look-back window before a tile gives up (about a second).
 constexpr uint32_t kScanPolls = 1u << 21;
 
-// One scan.  Src: uint32_t operator()(i), the value of item i, i < n (a
-// tile's values add up to less than 2^32).
+// One scan.  Src: uint32_t operator()(i), the value of item i, i < n, and
+// Src::Sum, the type that a tile's values are added up in: uint32_t where 4096
+// consecutive ones stay below 2^32 (0/1 flags, and counts of the tuples of a
+// relation, which holds fewer), else uint64_t.
 // Dst: void operator()(i, prefix, value).  state: scan_storage(n) zeroed
 // words.  *total (may be null) receives the sum.  lim (may be null): the
 // length where only the device knows it (the launch covers the host's bound
@@ -75,8 +77,9 @@ __device__ __forceinline__ uint64_t scan_look_back(unsigned long long* state, ui
 // Up to two scans of one kind (blockIdx.y) in one launch.
 template <class Src, class Dst>
 __global__ void __launch_bounds__(kScanBlock) k_scan(ScanJob<Src, Dst> a, ScanJob<Src, Dst> b, uint32_t* err) {
+    using Sum = typename Src::Sum;
     constexpr int kWarps = kScanBlock / 32;
-    __shared__ uint32_t s_warp[kWarps];
+    __shared__ Sum s_warp[kWarps];
     __shared__ uint64_t s_tile, s_before;
     const ScanJob<Src, Dst> j = blockIdx.y ? b : a;
     const uint64_t n = j.lim && *j.lim < j.n ? *j.lim : j.n;
@@ -91,7 +94,8 @@ __global__ void __launch_bounds__(kScanBlock) k_scan(ScanJob<Src, Dst> a, ScanJo
     // step come from a warp scan.  (kScanItems consecutive items a thread
     // made every store of a warp touch 32 sectors.)
     const uint64_t first = tile * kScanTile + wib * (32 * kScanItems) + lane;
-    uint32_t v[kScanItems], e[kScanItems], run = 0;
+    uint32_t v[kScanItems];
+    Sum e[kScanItems], run = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
         const uint64_t i = first + 32 * k;
@@ -99,15 +103,15 @@ __global__ void __launch_bounds__(kScanBlock) k_scan(ScanJob<Src, Dst> a, ScanJo
     }
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        const uint32_t inc = warp_incl_scan(v[k]);
+        const Sum inc = warp_incl_scan<Sum>(v[k]);
         e[k] = run + inc - v[k];
         run += __shfl_sync(0xffffffffu, inc, 31);
     }
     if (lane == 0) s_warp[wib] = run;
     __syncthreads();
     if (wib == 0) {
-        const uint32_t t = lane < kWarps ? s_warp[lane] : 0u;
-        const uint32_t inc = warp_incl_scan(t);
+        const Sum t = lane < kWarps ? s_warp[lane] : Sum(0);
+        const Sum inc = warp_incl_scan(t);
         const uint64_t sum = __shfl_sync(0xffffffffu, inc, kWarps - 1);
         if (lane < kWarps) s_warp[lane] = inc - t;
         const uint64_t before = scan_look_back(j.state, tile, sum, err);
