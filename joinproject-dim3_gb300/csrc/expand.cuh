@@ -14,6 +14,7 @@
 // expands it twice, counting and then writing at exact offsets.
 #pragma once
 #include "common.cuh"
+#include "items.h"
 
 namespace dim3g {
 
@@ -438,8 +439,8 @@ __device__ __forceinline__ void balanced_stage(const RowCtx& c, uint32_t eb, uin
 // s0 / len / ctot: the staged segment starts and lengths and the chunk
 // totals (a CtaChunks' arrays, or a prefetched row's).
 // dyn (optional, zeroed before the barrier that precedes this): a shared
-// counter from which the warps take pieces of dyn_piece candidates instead
-// of equal static shares.
+// counter of pieces of dyn_piece candidates, which the warps take instead of
+// equal static shares.
 // dyn_piece 0: a warp's share of the candidates, at least 256 and at most
 // this many (direct COUNT rows, whose tiles hold 4K candidates and up: a slice
 // of the 16M-tuple COUNT takes 1024 ms in pieces of 256, 698 up to 1024, 646
@@ -458,21 +459,19 @@ __device__ __forceinline__ void balanced_expand(const RowCtx& c, uint32_t ne, Se
     if (__any_sync(0xffffffffu, inc < v)) raise_error(c.err, kErrCountRange);
     const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
     const uint32_t share = total / nw + (total % nw ? 1u : 0u);
-    const uint32_t piece = !dyn ? share : (dyn_piece ? dyn_piece : min(max((share + 127) & ~127u, 256u), kDynPieceMax));
+    const Pieces pieces(dyn_piece ? dyn_piece : min(max((share + 127) & ~127u, 256u), kDynPieceMax), total);
     for (uint32_t round = 0;; round++) {
-    uint32_t p0;
+    uint32_t p0, p1;
     if (dyn) {
-        p0 = 0;
-        if (lane == 0) p0 = atomicAdd(dyn, piece);
-        p0 = __shfl_sync(0xffffffffu, p0, 0);
-        if (p0 >= total) break;
-    } else {
-        if (round) break;
-        p0 = min(wib * piece, total);
+        uint32_t k0 = 0;
+        if (lane == 0) k0 = atomicAdd(dyn, 1u);
+        k0 = __shfl_sync(0xffffffffu, k0, 0);
+        if (!pieces.at(k0, &p0, &p1)) break;
+    } else if (round || !share_of(wib, nw, total, &p0, &p1)) {
+        break;
     }
-    const uint32_t p1 = min(p0 + piece, total);
     // first chunk holding candidate p0: chunks with incl <= p0 form a prefix
-    for (uint32_t k = __popc(__ballot_sync(0xffffffffu, lane < nch && inc <= p0)); p0 < p1 && k < nch; k++) {
+    for (uint32_t k = __popc(__ballot_sync(0xffffffffu, lane < nch && inc <= p0)); k < nch; k++) {
         const uint32_t cin = __shfl_sync(0xffffffffu, inc, k), ctot = __shfl_sync(0xffffffffu, v, k);
         const uint32_t cex = cin - ctot;
         if (cex >= p1) break;

@@ -337,12 +337,12 @@ __device__ __forceinline__ void bitmap_row_staged(const RowCtx& c, uint32_t e0, 
         // pieces of kDynPiece candidates taken from a shared counter: a warp
         // slowed by short segments takes fewer, so the tile's barrier waits
         // on at most one piece
+        const Pieces pieces(kDynPiece, total);
         for (;;) {
-            uint32_t p0 = 0;
-            if (lane == 0) p0 = atomicAdd(&cc->n, kDynPiece);
-            p0 = __shfl_sync(0xffffffffu, p0, 0);
-            if (p0 >= total) break;
-            const uint32_t p1 = min(p0 + kDynPiece, total);
+            uint32_t k0 = 0, p0, p1;
+            if (lane == 0) k0 = atomicAdd(&cc->n, 1u);
+            k0 = __shfl_sync(0xffffffffu, k0, 0);
+            if (!pieces.at(k0, &p0, &p1)) break;
             for (uint32_t k = __popc(__ballot_sync(0xffffffffu, lane < nch && inc <= p0)); k < nch; k++) {
                 const uint32_t cin = __shfl_sync(0xffffffffu, inc, k), ctot = __shfl_sync(0xffffffffu, v, k);
                 const uint32_t cex = cin - ctot;

@@ -84,3 +84,62 @@ def test_ordered_rows_past_2_32(built):
 
 def test_sizes_used_here():
     assert 4096 * NZ >= 1 << 32 and np.iinfo(np.uint32).max < NX * NZ
+
+
+WIDE_Z = 9000  # a bitmap row of one tile
+
+
+def wide_row(pad):
+    """R: 1024 times (3, 0), and pad tuples without a partner; S: 2^22 - 1
+    tuples of WIDE_Z values.  Row 3 has 2^32 - 1024 candidates, in one tile."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(2)
+    z = torch.randint(0, WIDE_Z, ((1 << 22) - 1,), generator=g, device="cuda", dtype=torch.int32)
+    x = torch.full((1024 + pad,), 3, dtype=torch.int32, device="cuda")
+    y = torch.zeros_like(x)
+    x[1024:], y[1024:] = 4, 1
+    mult = torch.bincount(z.to(torch.int64), minlength=WIDE_Z)
+    assert 1024 * int(mult.sum()) == (1 << 32) - 1024 and int(mult.min()) > 0
+    return torch.stack([x, y], 1).contiguous(), torch.stack([z, torch.zeros_like(z)], 1).contiguous(), 1024 * mult
+
+
+def check_wide(out, cnt, n, mult):
+    assert n == WIDE_Z and bool((out[:n, 0] == 3).all())
+    z = out[:n, 1].to("cpu").numpy()
+    assert np.array_equal(np.sort(z), np.arange(WIDE_Z))
+    assert cnt is None or np.array_equal(cnt[:n].cpu().numpy(), mult.cpu().numpy()[z])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [0, 1])
+def test_row_of_almost_2_32_candidates(built, count):
+    """One join: the whole-tile bitmap row, and COUNT's counter a z."""
+    import torch
+    R, S, mult = wide_row(0)
+    out = torch.empty((WIDE_Z, 2), dtype=torch.int32, device="cuda")
+    cnt = torch.empty(WIDE_Z, dtype=torch.int64, device="cuda") if count else None
+    c = context(dense_block=0)
+    a = (R, R.shape[0], S, S.shape[0], out)
+    n = c.join_count_device(*a, cnt, WIDE_Z) if count else c.join_project_device(*a, WIDE_Z)
+    check_wide(out, cnt, n, mult)
+    c.close()
+
+
+@pytest.mark.gpu
+def test_query_row_of_almost_2_32_candidates(built):
+    """A query pass: the bitmap row and the ranked row."""
+    import torch
+
+    import dim3gpu
+    R, S, mult = wide_row(1 << 22)
+    c = dim3gpu.Context(0)
+    rs = dim3gpu.RelSet(c, [(R, R.shape[0]), (S, S.shape[0])])
+    outs = [torch.empty((WIDE_Z, 2), dtype=torch.int32, device="cuda") for _ in range(2)]
+    cnt = torch.empty(WIDE_Z, dtype=torch.int64, device="cuda")
+    got = rs.join([{"r": 0, "s": 1, "op": op, "out": outs[op], "cnt": cnt, "capacity": WIDE_Z}
+                   for op in (dim3gpu.OP_PROJECT, dim3gpu.OP_COUNT)])
+    for op, r in enumerate(got):
+        assert r["out_j"] == (1 << 32) - 1024
+        check_wide(outs[op], cnt if op else None, r["n_out"], mult)
+    rs.close()
+    c.close()
