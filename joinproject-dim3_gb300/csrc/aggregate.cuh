@@ -260,12 +260,13 @@ __host__ __device__ inline RankLayout rank_layout(uint32_t tile_width, uint32_t 
 }
 
 // A row (or row and tile) of the ranked class: item number, row, its entries
-// and first value.
+// and first value, tile.
 struct RankHead {
-    uint32_t item, x, e0, e1, xv;
+    uint64_t item;
+    uint32_t x, e0, e1, xv, t;
 };
-__device__ __forceinline__ RankHead rank_head(const RowCtx& c, uint32_t item, uint32_t x) {
-    return RankHead{item, x, c.JR_R[x], c.JR_R[x + 1], c.id2x[x]};
+__device__ __forceinline__ RankHead rank_head(const RowCtx& c, uint64_t item, uint32_t x, uint32_t t) {
+    return RankHead{item, x, c.JR_R[x], c.JR_R[x + 1], c.id2x[x], t};
 }
 
 // The whole CTA: row h.x over tile t.  Groups go to the cursor, or (offsets)
@@ -601,25 +602,26 @@ static __global__ void __launch_bounds__(1024, 1) k_agg_map(RowCtx c, AggOut ao,
 template <bool DIRECT>
 static __global__ void __launch_bounds__(1024, 1) k_agg_ranked(RowCtx c, AggOut ao, const uint32_t* __restrict__ rows,
                                                             const unsigned long long* __restrict__ n3,
-                                                            const unsigned long long* __restrict__ n4, RankLayout l) {
+                                                            const unsigned long long* __restrict__ n4, RankLayout l,
+                                                            unsigned long long* next_item) {
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t s_pos, s_wbase[33];
     __shared__ unsigned long long s_base;
     __shared__ RankHead s_head[2];
     __shared__ CtaChunks s_cc;
     const uint32_t per = ao.rs.cursor || (ao.sum.tiles && !DIRECT) ? c.T : 1u;
-    const uint32_t items = (uint32_t)(*n3 + *n4) * per;
+    const TileItems it{*n3 + *n4, per};
     auto claim = [&](RankHead* dst) {
-        const uint32_t i = atomicAdd(&c.next_row[3], 1u);
-        *dst = i < items ? rank_head(c, i, rows[i / per]) : RankHead{i, 0, 0, 0, 0};
+        const uint64_t i = atomicAdd(next_item, 1ull);
+        *dst = i < it.count() ? rank_head(c, i, rows[it.row(i)], it.tile(i)) : RankHead{i, 0, 0, 0, 0, 0};
     };
     if (threadIdx.x == 0) claim(&s_head[0]);
     __syncthreads();
     for (uint32_t k = 0;; k ^= 1) {
         const RankHead h = s_head[k];
-        if (h.item >= items) break;
+        if (h.item >= it.count()) break;
         if (threadIdx.x == 0) s_pos = 0;
-        const uint32_t t0 = per == c.T ? h.item % per : 0u, t1 = per == c.T ? t0 + 1 : c.T;
+        const uint32_t t0 = h.t, t1 = per == c.T ? t0 + 1 : c.T;
         GroupSums gs;
         for (uint32_t t = t0; t < t1; t++) {
             auto ahead = [&] {

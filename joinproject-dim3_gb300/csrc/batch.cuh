@@ -789,7 +789,7 @@ static __global__ void __launch_bounds__(1024, 1) k_b_agg_ranked(QueryPools Q, B
         uint32_t x;
         s_q[k] = query_of_row(Q, L.list[i], &x);
         s_c[k] = Q.rc[s_q[k]];
-        s_head[k] = rank_head(s_c[k], i, x);
+        s_head[k] = rank_head(s_c[k], i, x, 0);
     };
     if (threadIdx.x == 0) claim(0);
     __syncthreads();

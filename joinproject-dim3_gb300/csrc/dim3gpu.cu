@@ -136,7 +136,7 @@ struct Scalars {
     unsigned long long nrows_b[3];  // block-class rows by hash-set size (single pass, block_split)
     unsigned long long nbucket[kRowBuckets], list_cur[kRowBuckets];  // rows per bucket, list cursors (k_row_lists)
     unsigned int next_row[8];      // dynamic row counters of the CTA classes (4..6: block_split launches)
-    unsigned int pad;
+    unsigned long long next_item;  // COUNT's ranked rows: items (row and z tile) taken
 };
 
 }  // namespace
@@ -264,7 +264,7 @@ struct RowLists {
     const unsigned long long *nw, *nb, *n3, *n4;        // their sizes (device)
 };
 struct RowStreams;
-int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc, const uint32_t* list_t,
+int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, Scalars* sc, const uint32_t* list_t,
                   RowStreams& rst, bool direct);
 
 // Warps per CTA of a warp-per-row kernel whose warps each own per_warp
@@ -1240,7 +1240,7 @@ retile:
 // COUNT's row kernels (aggregate.cuh): the ranked rows first, then the map
 // rows from the largest maps down, then the tiny rows (list_t; null: none).
 // CTAs by map size, so that small maps run many rows an SM.
-int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, const Scalars* sc,
+int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, Scalars* sc,
                   const uint32_t* list_t, RowStreams& rst, bool direct) {
     CU(rst.fork());
     // one ranked CTA an SM with all of its shared memory, or two where a
@@ -1251,10 +1251,10 @@ int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, 
     if (direct) {
         const size_t sd = (size_t)rc.tile_width * 4;
         k_agg_ranked<true><<<resident_grid(c, k_agg_ranked<true>, 1024, sd), 1024, sd, rst.m>>>(rc, ao, L.m, L.n3, L.n4,
-                                                                                            RankLayout{});
+                                                                                            RankLayout{}, &sc->next_item);
     } else {
         k_agg_ranked<false><<<resident_grid(c, k_agg_ranked<false>, thr_m, smem_m), thr_m, smem_m, rst.m>>>(
-            rc, ao, L.m, L.n3, L.n4, rank_layout(rc.tile_width, thr_m / 32, smem_m));
+            rc, ao, L.m, L.n3, L.n4, rank_layout(rc.tile_width, thr_m / 32, smem_m), &sc->next_item);
     }
     CHECK_LAUNCH();
     auto map_rows = [&](const uint32_t* rows, const unsigned long long* n, uint32_t lg, const unsigned long long* s0,

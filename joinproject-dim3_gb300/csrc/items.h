@@ -37,4 +37,14 @@ DIM3G_HD bool share_of(uint32_t k, uint32_t parts, uint32_t total, uint32_t* p0,
     return true;
 }
 
+// Work items of rows taken `per` z tiles apart: item i is tile i % per of row
+// i / per.  33M heavy rows over 128 tiles are 2^32 of them.
+struct TileItems {
+    uint64_t rows;
+    uint32_t per;
+    DIM3G_HD uint64_t count() const { return rows * per; }
+    DIM3G_HD uint32_t row(uint64_t i) const { return (uint32_t)(i / per); }
+    DIM3G_HD uint32_t tile(uint64_t i) const { return (uint32_t)(i % per); }
+};
+
 }  // namespace dim3g

@@ -44,6 +44,9 @@ uint64_t shares(uint32_t parts, uint32_t total) {
     }
     return covered;
 }
+uint64_t items(uint64_t rows, uint32_t per) { return TileItems{rows, per}.count(); }
+uint32_t item_row(uint64_t rows, uint32_t per, uint64_t i) { return TileItems{rows, per}.row(i); }
+uint32_t item_tile(uint64_t rows, uint32_t per, uint64_t i) { return TileItems{rows, per}.tile(i); }
 }
 """
 
@@ -60,6 +63,11 @@ def lib(tmp_path_factory):
     L.walk.argtypes = [ctypes.c_uint32] * 3 + [ctypes.POINTER(ctypes.c_uint64)]
     L.shares.restype = ctypes.c_uint64
     L.shares.argtypes = [ctypes.c_uint32] * 2
+    L.items.restype = ctypes.c_uint64
+    L.items.argtypes = [ctypes.c_uint64, ctypes.c_uint32]
+    for f in (L.item_row, L.item_tile):
+        f.restype = ctypes.c_uint32
+        f.argtypes = [ctypes.c_uint64, ctypes.c_uint32, ctypes.c_uint64]
     return L
 
 
@@ -76,3 +84,13 @@ def test_pieces_cover_all_candidates_once(lib, piece, total):
 def test_shares_cover_all_candidates_once(lib, parts):
     for total in [*range(0, 1100), *range((1 << 32) - 1100, 1 << 32)]:
         assert lib.shares(parts, total) == total
+
+
+@pytest.mark.parametrize("rows,per", [(1, 1), (7, 3), (2_100_000, 2048), (33 << 20, 128), ((1 << 31) - 1, 8192)])
+def test_items_of_rows_and_tiles(lib, rows, per):
+    """2.1M ranked rows over 2048 tiles, 33M over 128: every row and tile once."""
+    n = lib.items(rows, per)
+    assert n == rows * per
+    for i in {0, per - 1, per, n // 2, (1 << 32) - 1, 1 << 32, n - per, n - 1}:
+        if 0 <= i < n:
+            assert (lib.item_row(rows, per, i), lib.item_tile(rows, per, i)) == (i // per, i % per)
