@@ -820,7 +820,7 @@ void dim3g_relset_destroy(dim3g_relset* s) {
 }
 
 uint64_t dim3g_relset_bytes(const dim3g_relset* s) {
-    return s ? (uint64_t)(s->mem_bytes + s->qs.qmem_bytes) : 0;
+    return s ? (uint64_t)(s->mem_bytes + s->qs.qmem_bytes + s->qs.agg_bytes) : 0;
 }
 
 int dim3g_relset_join(dim3g_relset* s, dim3g_query* q, uint32_t n) {
@@ -1011,7 +1011,7 @@ int dim3g_batch_info(const dim3g_batch* b, float* ms_last, uint64_t* launches_pe
     if (!b) return DIM3G_ERR_INVALID;
     if (ms_last) *ms_last = b->ms_last;
     if (launches_per_run) *launches_per_run = b->launches_per_run;
-    if (device_bytes) *device_bytes = (uint64_t)(b->set.mem_bytes + b->set.qs.qmem_bytes);
+    if (device_bytes) *device_bytes = (uint64_t)(b->set.mem_bytes + b->set.qs.qmem_bytes + b->set.qs.agg_bytes);
     return DIM3G_OK;
 }
 
@@ -1249,7 +1249,7 @@ int dim3g_server_create(dim3g_relset* set, uint32_t lanes, uint32_t max_batch, u
         L->qs.h_res_n = max_batch;
         int r = ensure_agg_scratch(set, L->qs);
         if (r) return r;
-        fixed += L->qs.qmem_bytes;
+        fixed += L->qs.qmem_bytes + L->qs.agg_bytes;
         S->lanes.push_back(std::move(L));
     }
     if (fixed >= budget_bytes)
