@@ -671,8 +671,10 @@ int set_batch_attributes(dim3g_ctx* ctx) {
     return DIM3G_OK;
 }
 
-// One CTA of k_b_agg_ranked an SM (200 KB of shared memory each).
-int ensure_agg_scratch(dim3g_relset* s, QueryScratch& qs) {
+// One CTA of k_b_agg_ranked an SM (200 KB of shared memory each).  st: the
+// stream of the passes that will use the counters (a server's lanes run on
+// streams of their own, which nothing else orders behind the clear).
+int ensure_agg_scratch(dim3g_relset* s, QueryScratch& qs, cudaStream_t st) {
     dim3g_ctx* ctx = s->ctx;
     const size_t need = (size_t)I::sm_count(ctx) * ((size_t)1 << s->tile_lg) * 4;
     if (qs.agg_bytes >= need) return DIM3G_OK;
@@ -684,7 +686,7 @@ int ensure_agg_scratch(dim3g_relset* s, QueryScratch& qs) {
         return I::fail(ctx, DIM3G_ERR_NOMEM, "COUNT scratch: device allocation of %zu bytes failed", need);
     }
     // counters start at zero; every row resets the counters it touched
-    BCU(cudaMemset(qs.agg, 0, need));
+    BCU(cudaMemsetAsync(qs.agg, 0, need, st));
     qs.agg_bytes = need;
     return DIM3G_OK;
 }
@@ -831,7 +833,7 @@ int dim3g_relset_join(dim3g_relset* s, dim3g_query* q, uint32_t n) {
     cudaStream_t st = I::stream(ctx);
     QueryPlan qp;
     int r = query_plan(s, s->qs, q, n, qp);
-    if (!r && qp.has_count) r = ensure_agg_scratch(s, s->qs);
+    if (!r && qp.has_count) r = ensure_agg_scratch(s, s->qs, st);
     if (!r) r = query_upload(s, qp);
     if (r) return r;
     uint64_t launches = 0;
@@ -876,7 +878,7 @@ int dim3g_batch_create(dim3g_ctx* ctx, const dim3g_relation* rels, const dim3g_q
     if (!r) r = relset_sketch(&b->set, b->rels.data(), 2 * n);
     if (!r) r = relset_plan(&b->set, b->rels.data(), 2 * n, 0);
     if (!r) r = query_plan(&b->set, b->set.qs, b->queries.data(), n, b->qp);
-    if (!r && b->qp.has_count) r = ensure_agg_scratch(&b->set, b->set.qs);
+    if (!r && b->qp.has_count) r = ensure_agg_scratch(&b->set, b->set.qs, I::stream(ctx));
     if (!r) r = batch_capture(b);
     if (r) {
         delete b;
@@ -1247,7 +1249,7 @@ int dim3g_server_create(dim3g_relset* set, uint32_t lanes, uint32_t max_batch, u
             return I::fail(ctx, DIM3G_ERR_NOMEM, "server lane pinned staging");
         }
         L->qs.h_res_n = max_batch;
-        int r = ensure_agg_scratch(set, L->qs);
+        int r = ensure_agg_scratch(set, L->qs, L->st);
         if (r) return r;
         fixed += L->qs.qmem_bytes + L->qs.agg_bytes;
         S->lanes.push_back(std::move(L));

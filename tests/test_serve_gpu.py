@@ -186,3 +186,55 @@ def test_server_admission_limits_and_shutdown(ctx, golden):
     srv.submit(0, 1)
     srv.close()
     rs.close()
+
+
+def test_count_counters_are_cleared_before_a_lanes_first_pass(ctx):
+    """A lane's counters are cleared on its own stream.  Here the legacy stream
+    is half a second behind: a clear queued there would come while rows count.
+    The rows have more distinct values than two windows of ranks, so they count
+    in that memory."""
+    import time
+
+    import torch
+    import dim3gpu
+    m, wide, n_y, n_x = 100_000, 60_000, 4, 500
+    rng = np.random.default_rng(3)
+    zs = [rng.choice(m, wide, replace=False) for _ in range(n_y)]
+    S = np.concatenate([np.stack([z, np.full(wide, y)], 1) for y, z in enumerate(zs)])
+    R = np.array([(x, y) for x in range(n_x) for y in range(n_y)] + [(10_000 + i, 99) for i in range(n_y * wide)])
+    dev = [torch.from_numpy(a.astype(np.int32)).cuda() for a in (R, S)]
+    rs = dim3gpu.RelSet(ctx, [(d, d.shape[0]) for d in dev])
+    want = torch.from_numpy(np.bincount(np.concatenate(zs), minlength=m)).cuda()
+    n_out = n_x * int((want > 0).sum())
+    torch.cuda.synchronize()
+    stop = threading.Event()
+
+    def fall_behind():
+        while not stop.is_set():
+            torch.cuda._sleep(100_000_000)  # about 50 ms of the legacy stream
+            time.sleep(0.02)
+
+    t = threading.Thread(target=fall_behind)
+    t.start()
+    try:
+        time.sleep(0.2)
+        srv = dim3gpu.Server(rs, lanes=2, max_batch=1, budget_bytes=1 << 45)
+    finally:
+        stop.set()
+        t.join()
+    behind = torch.cuda.Event()
+    behind.record()
+    queued, after, served = [], 6, 0  # after: requests past the last queued work
+    with torch.cuda.stream(torch.cuda.Stream()):
+        while after or queued:
+            while after and len(queued) < 6:
+                queued.append(srv.submit(0, 1, dim3gpu.OP_COUNT))
+                after -= behind.query()
+            r = srv.wait(queued[0])
+            assert r["status"] == 0 and r["n_out"] == n_out
+            z = dim3gpu.device_tensor(r["d_out"], (n_out, 2), "<i4")[:, 1].long()
+            assert bool((dim3gpu.device_tensor(r["d_cnt"], (n_out,), "<i8") == want[z]).all()), served
+            srv.release(queued.pop(0))
+            served += 1
+    srv.close()
+    rs.close()
