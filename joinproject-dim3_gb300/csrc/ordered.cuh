@@ -98,13 +98,15 @@ static __global__ void __launch_bounds__(256) k_rows_warp(RowCtx c, const uint32
 }
 
 // Tiny rows, many to a warp: the pack's candidates carry the lane of their
-// row, whose count (or next place) is a shared counter.
-constexpr size_t kRowsPackWords = ((size_t)1 << kPackLg) + 128;  // table, then a row's counter, value and offset
+// row, whose count (or next place) is a shared counter.  A place past the row's
+// count is not written.
+constexpr size_t kRowsPackWords = ((size_t)1 << kPackLg) + 160;  // table, then a row's counter, value, offset and count
 template <bool WRITE>
 struct PackRowSink {
     static constexpr bool kValues = WRITE;
-    uint32_t* pos;  // 32 counters, 32 first values, 32 offsets (two words each)
+    uint32_t* pos;  // 32 counters, 32 first values, 32 offsets (two words each), 32 counts
     uint2* out;
+    uint32_t* err;
     __device__ __forceinline__ uint32_t tag(const RowCtx&, uint32_t) const { return lane_id(); }
     template <uint32_t N>
     __device__ __forceinline__ void take(const uint32_t (&b)[N], const uint32_t (&r)[N], const uint32_t (&v)[N]) {
@@ -114,7 +116,8 @@ struct PackRowSink {
                 const uint32_t p = atomicAdd(&pos[r[u]], 1u);
                 if (WRITE) {
                     const unsigned long long off = reinterpret_cast<const unsigned long long*>(pos + 64)[r[u]];
-                    st_stream(&out[off + p], make_uint2(pos[32 + r[u]], v[u]));
+                    if (p < pos[128 + r[u]]) st_stream(&out[off + p], make_uint2(pos[32 + r[u]], v[u]));
+                    else raise_error(err, kErrOutputBound);
                 }
             }
     }
@@ -126,7 +129,7 @@ static __global__ void __launch_bounds__(256, 4) k_rows_pack(RowCtx c, const uin
     extern __shared__ uint32_t smem[];
     const uint32_t nw = blockDim.x >> 5, wib = threadIdx.x >> 5, lane = lane_id();
     uint32_t* tab = smem + (size_t)wib * kRowsPackWords;
-    PackRowSink<WRITE> sink{tab + (1u << kPackLg), c.out};
+    PackRowSink<WRITE> sink{tab + (1u << kPackLg), c.out, c.err};
     const uint32_t nrows = (uint32_t)*nrows_p, warps = gridDim.x * nw;
     uint32_t take = (nrows + warps - 1) / warps;
     take = take > 32 ? 32 : take;
@@ -137,11 +140,12 @@ static __global__ void __launch_bounds__(256, 4) k_rows_pack(RowCtx c, const uin
         if (WRITE && lane < n) {
             sink.pos[32 + lane] = c.id2x[x];
             reinterpret_cast<unsigned long long*>(sink.pos + 64)[lane] = c.off[x];
+            sink.pos[128 + lane] = c.cnt[x];
         }
         __syncwarp();
         pack_rows(c, x, 0, n, tab, sink);
         if (!WRITE && lane < n) c.cnt[x] = sink.pos[lane];
-        if (WRITE && lane < n && sink.pos[lane] != c.cnt[x]) raise_error(c.err, kErrOutputBound);
+        if (WRITE && lane < n && sink.pos[lane] != sink.pos[128 + lane]) raise_error(c.err, kErrOutputBound);
         __syncwarp();
     }
 }
