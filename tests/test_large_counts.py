@@ -143,3 +143,19 @@ def test_query_row_of_almost_2_32_candidates(built):
         check_wide(outs[op], cnt if op else None, r["n_out"], mult)
     rs.close()
     c.close()
+
+
+@pytest.mark.gpu
+def test_sizes_around_the_wide_sums(built):
+    """Rows of 2^20 - 1 and 2^20 pairs: on either side of where a tile's sum
+    can pass 2^32, alone and in one result."""
+    import torch
+    nz = 1 << 20
+    z = torch.arange(nz, dtype=torch.int32, device="cuda")
+    S = torch.cat([torch.stack([z, torch.zeros_like(z)], 1), torch.stack([z[1:], torch.ones_like(z[1:])], 1)]).contiguous()
+    c = context(dense_block=0)
+    for ys in ([0] * 4096, [1] * 4096, [1] * 4096 + [0] + [1] * 4095, [1] * 5000 + [2] * 5000 + [0] * 3000):
+        R = torch.tensor([[x, y] for x, y in enumerate(ys)], dtype=torch.int32, device="cuda")
+        n = sum({0: nz, 1: nz - 1, 2: 0}[y] for y in ys)
+        assert c.join_project_count_device(R, len(ys), S, S.shape[0]) == n
+    c.close()
