@@ -661,17 +661,43 @@ struct RowBuckets {
 // so the rows in flight bound the time: 2^lg lanes take a row, about as many
 // as a row has entries on average (row_work_lanes), and a row of more than
 // 4 x 2^lg entries is finished by its whole warp.  A warp for every row took
-// 281 us for 1M rows of 10 entries.  The sums and the rows per bucket are
+// 281 us for 1M rows of 10 entries.  Rows of more than kLongRow entries are
+// left to the whole CTA at its end, kLongRows of them (where there are more,
+// their warps do them side by side): a hub of 2M entries among 4M tuples held
+// one warp, and the GPU with it -- the whole join 29.5 ms, 19.7 with the CTA;
+// 20M-edge and 10M uniform joins the same either way.  The sums and the rows per bucket are
 // added up per CTA in shared memory, then one atomic a CTA and counter.
+constexpr uint32_t kLongRow = 2048, kLongRows = 4;
 static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, uint32_t lg, RowBuckets rb,
                                                          bool check_range, SumAcc sel, uint32_t* __restrict__ ucap,
                                                          uint8_t* __restrict__ bucket, unsigned long long* outj,
                                                          unsigned long long* outj_cls, unsigned long long* nbucket) {
     __shared__ unsigned long long s_acc[6];
     __shared__ uint32_t s_n[kRowBuckets + 1];
+    __shared__ uint32_t s_nlong;
+    __shared__ uint3 s_long[kLongRows];  // row, its entries
+    __shared__ unsigned long long s_w[kLongRows];
     if (threadIdx.x < 6) s_acc[threadIdx.x] = 0;
     if (threadIdx.x <= kRowBuckets) s_n[threadIdx.x] = 0;
+    if (threadIdx.x < kLongRows) s_w[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s_nlong = 0;
     __syncthreads();
+    auto candidates = [&](uint32_t e) {
+        const uint64_t r = (uint64_t)__ldg(&c.IC_R[e]) * c.T;
+        return __ldg(&c.JR_S[r + c.T]) - __ldg(&c.JR_S[r]);
+    };
+    auto finish = [&](uint64_t x, unsigned long long w) {
+        const uint32_t u = (uint32_t)(w < c.m ? w : c.m);
+        const uint32_t k = row_class(w, u, rb.cap_w, rb.cap_b, rb.tiny), q = rb.of(k, u);
+        ucap[x] = u;
+        bucket[x] = (uint8_t)q;
+        atomicAdd(&s_n[q], 1u);
+        if (check_range && w >= 0xFFFFFFFFull) raise_error(c.err, kErrCountRange);
+        if (w) {
+            atomicAdd(&s_acc[0], w);
+            atomicAdd(&s_acc[k], w);
+        }
+    };
     const uint32_t lane = lane_id(), G = 1u << lg, gl = lane & (G - 1), per = 32 >> lg;
     const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -683,8 +709,17 @@ static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, u
             e0 = c.JR_R[x];
             e1 = c.JR_R[x + 1];
         }
+        bool later = e1 - e0 > kLongRow;
+        if (__any_sync(0xffffffffu, later)) {
+            uint32_t slot = 0;
+            if (later && gl == 0) slot = atomicAdd(&s_nlong, 1u);
+            slot = __shfl_sync(0xffffffffu, slot, lane & ~(G - 1));
+            later = later && slot < kLongRows;
+            if (later && gl == 0) s_long[slot] = make_uint3((uint32_t)x, e0, e1);
+            if (later) e1 = e0;
+        }
         unsigned long long w = 0;
-        const uint32_t head = min(e1, e0 + 4 * G);
+        const uint32_t head = e0 + min(e1 - e0, 4 * G);
         uint32_t y[4];
 #pragma unroll
         for (uint32_t k = 0; k < 4; k++) y[k] = e0 + gl + k * G < head ? __ldg(&c.IC_R[e0 + gl + k * G]) : kEmpty32;
@@ -700,28 +735,28 @@ static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, u
             const uint32_t b = __shfl_sync(0xffffffffu, head, src), e = __shfl_sync(0xffffffffu, e1, src);
             unsigned long long v = 0;
 #pragma unroll 4
-            for (uint32_t k = b + lane; k < e; k += 32) {
-                const uint64_t r = (uint64_t)__ldg(&c.IC_R[k]) * c.T;
-                v += __ldg(&c.JR_S[r + c.T]) - __ldg(&c.JR_S[r]);
-            }
+            for (uint32_t k = b + lane; k < e; k += 32) v += candidates(k);
             v = warp_sum(v);
             if ((int)lane == src) w += v;
         }
         for (uint32_t o = G >> 1; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-        if (gl == 0 && x < n) {
-            const uint32_t u = (uint32_t)(w < c.m ? w : c.m);
-            const uint32_t k = row_class(w, u, rb.cap_w, rb.cap_b, rb.tiny), q = rb.of(k, u);
-            ucap[x] = u;
-            bucket[x] = (uint8_t)q;
-            atomicAdd(&s_n[q], 1u);
-            if (check_range && w >= 0xFFFFFFFFull) raise_error(c.err, kErrCountRange);
-            if (w) {
-                atomicAdd(&s_acc[0], w);
-                atomicAdd(&s_acc[k], w);
-            }
-        }
+        if (gl == 0 && x < n && !later) finish(x, w);
     }
     __syncthreads();
+    const uint32_t nlong = min(s_nlong, kLongRows);
+    if (nlong) {
+        for (uint32_t i = 0; i < nlong; i++) {
+            const uint3 l = s_long[i];
+            unsigned long long v = 0;
+#pragma unroll 4
+            for (uint32_t k = threadIdx.x; k < l.z - l.y; k += blockDim.x) v += candidates(l.y + k);
+            v = warp_sum(v);
+            if (lane == 0) atomicAdd(&s_w[i], v);
+        }
+        __syncthreads();
+        if (threadIdx.x < nlong) finish(s_long[threadIdx.x].x, s_w[threadIdx.x]);
+        __syncthreads();
+    }
     if (threadIdx.x < 6 && s_acc[threadIdx.x]) atomicAdd(threadIdx.x ? &outj_cls[threadIdx.x] : outj, s_acc[threadIdx.x]);
     if (threadIdx.x < kRowBuckets && s_n[threadIdx.x])
         atomicAdd(&nbucket[threadIdx.x], (unsigned long long)s_n[threadIdx.x]);
