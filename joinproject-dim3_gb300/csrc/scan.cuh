@@ -84,11 +84,10 @@ __device__ __forceinline__ uint64_t scan_look_back(unsigned long long* state, ui
 // touch 32 sectors.)
 template <class Sum, class Src, class Dst>
 __device__ __forceinline__ void scan_tile(const ScanJob<Src, Dst>& j, const uint32_t (&v)[kScanItems], uint64_t first,
-                                          uint64_t n, uint64_t tile, uint64_t nb, uint32_t* err) {
+                                          uint64_t n, uint64_t tile, uint64_t nb, uint32_t* err, uint32_t lane, uint32_t wib) {
     constexpr int kWarps = kScanBlock / 32;
     __shared__ Sum s_warp[kWarps];
     __shared__ uint64_t s_before;
-    const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
     Sum e[kScanItems], run = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
@@ -131,7 +130,8 @@ __global__ void __launch_bounds__(kScanBlock) k_scan(ScanJob<Src, Dst> a, ScanJo
     if (threadIdx.x == 0) s_tile = atomicAdd(j.state, 1ull);
     __syncthreads();
     const uint64_t tile = s_tile;
-    const uint64_t first = tile * kScanTile + (threadIdx.x >> 5) * (32 * kScanItems) + lane_id();
+    const uint32_t lane = lane_id(), wib = threadIdx.x >> 5;
+    const uint64_t first = tile * kScanTile + wib * (32 * kScanItems) + lane;
     uint32_t v[kScanItems];
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
@@ -143,11 +143,11 @@ __global__ void __launch_bounds__(kScanBlock) k_scan(ScanJob<Src, Dst> a, ScanJo
 #pragma unroll
         for (int k = 0; k < kScanItems; k++) bits |= v[k];
         if (__syncthreads_or(bits >= kScanNarrow)) {
-            scan_tile<uint64_t>(j, v, first, n, tile, nb, err);
+            scan_tile<uint64_t>(j, v, first, n, tile, nb, err, lane, wib);
             return;
         }
     }
-    scan_tile<uint32_t>(j, v, first, n, tile, nb, err);
+    scan_tile<uint32_t>(j, v, first, n, tile, nb, err, lane, wib);
 }
 
 // Host launches; the states are zeroed by the caller.  An empty scan launches
