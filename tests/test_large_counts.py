@@ -9,11 +9,18 @@ import pytest
 NX, NZ = 4200, 1_100_000  # more than 2^32 pairs in one 4096-row tile of the prefix sum
 
 
+def ready(*t):
+    """The library runs on streams of its own."""
+    import torch
+    torch.cuda.synchronize()
+    return t
+
+
 def all_pairs():
     import torch
     x = torch.arange(NX, dtype=torch.int32, device="cuda")
     z = torch.randperm(NZ, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda").to(torch.int32)
-    return (torch.stack([x, torch.zeros_like(x)], 1).contiguous(), torch.stack([z, torch.zeros_like(z)], 1).contiguous())
+    return ready(torch.stack([x, torch.zeros_like(x)], 1).contiguous(), torch.stack([z, torch.zeros_like(z)], 1).contiguous())
 
 
 def context(**prm):
@@ -46,8 +53,8 @@ def test_ordered_result_past_2_32_is_refused(built, count, dense):
     R, S = all_pairs()
     c = context(ordered_output=1, dense_block=dense)
     cap = 1024
-    out = torch.full((cap, 2), -5, dtype=torch.int32, device="cuda")
-    cnt = torch.full((cap,), -5, dtype=torch.int64, device="cuda")
+    out, cnt = ready(torch.full((cap, 2), -5, dtype=torch.int32, device="cuda"),
+                     torch.full((cap,), -5, dtype=torch.int64, device="cuda"))
     n = ctypes.c_uint64()
     L, p = dim3gpu.load(), ctypes.c_void_p
     if count:
@@ -100,7 +107,7 @@ def wide_row(pad):
     x[1024:], y[1024:] = 4, 1
     mult = torch.bincount(z.to(torch.int64), minlength=WIDE_Z)
     assert 1024 * int(mult.sum()) == (1 << 32) - 1024 and int(mult.min()) > 0
-    return torch.stack([x, y], 1).contiguous(), torch.stack([z, torch.zeros_like(z)], 1).contiguous(), 1024 * mult
+    return ready(torch.stack([x, y], 1).contiguous(), torch.stack([z, torch.zeros_like(z)], 1).contiguous(), 1024 * mult)
 
 
 def check_wide(out, cnt, n, mult):
@@ -155,7 +162,7 @@ def test_sizes_around_the_wide_sums(built):
     S = torch.cat([torch.stack([z, torch.zeros_like(z)], 1), torch.stack([z[1:], torch.ones_like(z[1:])], 1)]).contiguous()
     c = context(dense_block=0)
     for ys in ([0] * 4096, [1] * 4096, [1] * 4096 + [0] + [1] * 4095, [1] * 5000 + [2] * 5000 + [0] * 3000):
-        R = torch.tensor([[x, y] for x, y in enumerate(ys)], dtype=torch.int32, device="cuda")
+        R, = ready(torch.tensor([[x, y] for x, y in enumerate(ys)], dtype=torch.int32, device="cuda"))
         n = sum({0: nz, 1: nz - 1, 2: 0}[y] for y in ys)
         assert c.join_project_count_device(R, len(ys), S, S.shape[0]) == n
     c.close()
