@@ -9,7 +9,7 @@
 //   -> CSR scans (by f, by (y, f tile); bounded by the layout's counts)
 //   -> k_ix_scatter (a batch builds only the CSR each relation's query reads)
 // Query pass over queries (P, Q) of a set:
-//   k_q_setup -> k_q_ymap -> k_q_work -> class lists (one partition)
+//   k_q_setup -> k_q_ymap -> k_q_work, k_q_long -> class lists (one partition)
 //   -> project and COUNT row kernels on forked streams -> per-query results
 //   to pinned host memory
 // Every size the launches depend on is known on the host from the tuple
@@ -394,16 +394,19 @@ struct QueryPlan {
     std::vector<uint32_t> swapped;
     uint64_t ntot = 0, nrows = 0;
     bool has_project = false, has_count = false;
+    bool has_long = false;  // some driving relation can have a row for k_q_long
     QueryPools Q{};
     uint32_t* lists = nullptr;             // 3 x nrows
-    unsigned long long* ncls = nullptr;    // per op 32 words: class counts, split counts, bucket counts, list cursors
+    // per op 32 words: class counts, split counts, bucket counts, list cursors;
+    // words 12 and 13: long rows and their pieces
+    unsigned long long* ncls = nullptr;
     uint32_t* next_row = nullptr;          // 8 dynamic counters (4..6: split block launches)
 };
 
 // Device layout of a query pass's scratch (every size monotone in the
 // arguments, so scratch laid out for maxima fits every smaller pass).
 struct QLayout {
-    size_t qin, qt, qr, ymap, step, ICq, JRq, ucap, bucket, rc, rs, res, lists, ncls, next, total;
+    size_t qin, qt, qr, ymap, step, ICq, JRq, ucap, bucket, longs, pieces, rc, rs, res, lists, ncls, next, total;
 };
 QLayout query_layout(uint32_t nq, uint64_t ntot, uint64_t nrows) {
     Layout L;
@@ -417,6 +420,8 @@ QLayout query_layout(uint32_t nq, uint64_t ntot, uint64_t nrows) {
     o.JRq = L.add<uint32_t>(nrows);
     o.ucap = L.add<uint32_t>(nrows);
     o.bucket = L.add<uint8_t>(nrows);
+    o.longs = L.add<QLongRow>(q_long_rows(ntot));
+    o.pieces = L.add<uint2>(q_pieces(ntot));
     o.rc = L.add<RowCtx>(nq);
     o.rs = L.add<Reserve>(nq);
     o.res = L.add<QueryRes>(nq);
@@ -456,6 +461,7 @@ int query_plan(dim3g_relset* s, QueryScratch& qs, const dim3g_query* q, uint32_t
         const uint64_t np = (nr == 0 || ns == 0) ? 0 : s->h_in[qi.p].n;
         qp.h_qin[i] = qi;
         qp.swapped[i] = sw;
+        if (np > kQLongRow) qp.has_long = true;
         qp.h_qt_off[i + 1] = qp.h_qt_off[i] + np;
         // rows: the driving relation's distinct first values, at most its tuples
         const uint64_t rows = np && !s->h_nf.empty() && s->h_nf[qi.p] < np ? s->h_nf[qi.p] : np;
@@ -525,6 +531,8 @@ int query_plan(dim3g_relset* s, QueryScratch& qs, const dim3g_query* q, uint32_t
     Q.JRq = (uint32_t*)(m + o.JRq);
     Q.ucap = (uint32_t*)(m + o.ucap);
     Q.bucket = (uint8_t*)(m + o.bucket);
+    Q.longs = (QLongRow*)(m + o.longs);
+    Q.pieces = (uint2*)(m + o.pieces);
     Q.rc = (RowCtx*)(m + o.rc);
     Q.rs = (Reserve*)(m + o.rs);
     Q.res = (QueryRes*)(m + o.res);
@@ -532,6 +540,7 @@ int query_plan(dim3g_relset* s, QueryScratch& qs, const dim3g_query* q, uint32_t
     qp.ncls = (unsigned long long*)(m + o.ncls);
     qp.next_row = (uint32_t*)(m + o.next);
     for (int op = 0; op < 2; op++) Q.nbucket[op] = qp.ncls + 32 * op + 16;
+    Q.n_long = qp.ncls + 12;
     return DIM3G_OK;
 }
 
@@ -570,6 +579,10 @@ int query_enqueue(dim3g_relset* s, QueryScratch& qs, QueryPlan& qp, cudaStream_t
                         1u << (tu.block_lg - 3), 1u << (tu.block_lg - 2)};
     k_q_work<<<elem_grid(qp.ntot + 32 * (uint64_t)nq, sm), 256, 0, st>>>(Q, rb);
     BLAUNCH();
+    if (qp.has_long) {
+        k_q_long<<<elem_grid(32 * q_pieces(qp.ntot), sm), 256, 0, st>>>(Q, rb);
+        BLAUNCH();
+    }
     uint32_t* lw = qp.lists;
     uint32_t* lb = qp.lists + qp.nrows;
     uint32_t* lm = qp.lists + 2 * qp.nrows;

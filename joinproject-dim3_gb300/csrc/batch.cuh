@@ -339,6 +339,20 @@ struct QueryRes {
     uint32_t nx, ny, nz;        // rows (distinct P.f; 0 when a side is empty), P.y, Q.f
 };
 
+constexpr uint32_t kCountBuckets = 8, kNoBucket = 0xFF;
+// A row of more than kQLongRow entries, past the first that its lanes take, is
+// worked out in pieces of kQPiece by the whole grid (k_q_long).
+constexpr uint32_t kQLongRow = 4096, kQPiece = 2048;
+struct QLongRow {
+    unsigned long long w;  // candidates so far
+    uint64_t g;            // row of the row space
+    uint32_t qi, e1;
+    uint32_t left;         // pieces not done
+};
+// Rows and pieces that n entries may have.
+inline uint64_t q_long_rows(uint64_t n) { return n / kQLongRow + 1; }
+inline uint64_t q_pieces(uint64_t n) { return n / kQPiece + n / kQLongRow + 1; }
+
 struct QueryPools {
     const RelDev* rel;
     const QueryIn* qin;
@@ -361,6 +375,9 @@ struct QueryPools {
     uint32_t* ucap;   // nrows
     uint8_t* bucket;  // nrows: RowBuckets, COUNT rows from kCountBuckets on
     unsigned long long* nbucket[2];  // rows per bucket: join-project, COUNT
+    QLongRow* longs;
+    uint2* pieces;    // of the long rows: slot in longs, first entry
+    unsigned long long* n_long;  // long rows, and their pieces
     RowCtx* rc;       // nq
     Reserve* rs;      // nq
     QueryRes* res;    // nq
@@ -453,15 +470,28 @@ static __global__ void __launch_bounds__(1024) k_q_setup(QueryPools Q) {
     if (threadIdx.x == 0) Q.step_off[Q.nq] = carry;
 }
 
+// A row with its candidates counted: its distinct bound and bucket (kRowBuckets:
+// none).
+__device__ __forceinline__ uint32_t query_row(const QueryPools& Q, const RowBuckets& rb, uint32_t qi, uint64_t g,
+                                              unsigned long long w, uint32_t m, uint32_t fam) {
+    const uint32_t u = (uint32_t)(w < m ? w : m);
+    const uint32_t k = rb.of(row_class(w, u, rb.cap_w, fam ? agg_cap_b(m, rb.cap_b) : rb.cap_b, rb.tiny), u);
+    Q.ucap[g] = u;
+    if (fam && w >= 0xFFFFFFFFull) raise_error(&Q.res[qi].err, kErrCountRange);
+    if (k < kRowBuckets) Q.bucket[g] = (uint8_t)(fam * kCountBuckets + k);
+    return k;
+}
+
 // The rows of all queries: P's entries as Q's y ids, P's row pointers, the
 // row's candidates and its bucket.  A warp step is 32 >> lg rows of one query,
 // 2^lg lanes a row, about as many as its rows have entries on average (a row
 // of more than 4 x 2^lg is finished by the whole warp; see k_row_work).  Row
 // space planned from tuple counts, past a query's distinct first values, is
 // not visited.  An entry costs one random sector (its y id's ymap pair).
+// Rows of more than kQLongRow entries are left to k_q_long: a hub of 2M entries
+// among 4M held one warp for 28.7 ms.
 // In place of three passes with a per-entry atomic on the row's candidates
 // (16 resident queries of 35M entries: 1020 us; 48-join batch: 345 us).
-constexpr uint32_t kCountBuckets = 8, kNoBucket = 0xFF;
 static __global__ void __launch_bounds__(256) k_q_work(QueryPools Q, RowBuckets rb) {
     __shared__ uint32_t s_n[2][kRowBuckets + 1];
     if (threadIdx.x < 2 * (kRowBuckets + 1)) s_n[threadIdx.x / (kRowBuckets + 1)][threadIdx.x % (kRowBuckets + 1)] = 0;
@@ -506,7 +536,7 @@ static __global__ void __launch_bounds__(256) k_q_work(QueryPools Q, RowBuckets 
             e1 = live ? jp[x + 1] - tup_off : e0;
         }
         unsigned long long w = 0;
-        const uint32_t head = min(e1, e0 + 4 * G);
+        const uint32_t head = e0 + min(e1 - e0, 4 * G);
         uint32_t y[4];
 #pragma unroll
         for (uint32_t k = 0; k < 4; k++) y[k] = e0 + gl + k * G < head ? __ldg(&icf[e0 + gl + k * G]) : kEmpty32;
@@ -517,10 +547,29 @@ static __global__ void __launch_bounds__(256) k_q_work(QueryPools Q, RowBuckets 
                 icq[e0 + gl + k * G] = t.x;
                 w += t.y;
             }
-        // the rest of the warp's long rows, all lanes on one row at a time
+        // the rest of the warp's long rows, all lanes on one row at a time, or
+        // its pieces for k_q_long
+        uint32_t slot = kEmpty32;
         for (uint32_t longs = __ballot_sync(0xffffffffu, gl == 0 && head < e1); longs; longs &= longs - 1) {
             const int src = __ffs(longs) - 1;
             const uint32_t b0 = __shfl_sync(0xffffffffu, head, src), b1 = __shfl_sync(0xffffffffu, e1, src);
+            if (b1 - b0 > kQLongRow) {
+                const uint32_t np = (b1 - b0 - 1) / kQPiece + 1;
+                uint32_t sl = 0;
+                unsigned long long at = 0;
+                if (lane == 0) {
+                    sl = (uint32_t)atomicAdd(&Q.n_long[0], 1ull);
+                    at = atomicAdd(&Q.n_long[1], (unsigned long long)np);
+                }
+                sl = __shfl_sync(0xffffffffu, sl, 0);
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if ((int)lane == src) {
+                    slot = sl;
+                    Q.longs[sl] = QLongRow{0, g, qi, b1, np};
+                }
+                for (uint32_t k = lane; k < np; k += 32) Q.pieces[at + k] = make_uint2(sl, b0 + k * kQPiece);
+                continue;
+            }
             unsigned long long v = 0;
 #pragma unroll 4
             for (uint32_t e = b0 + lane; e < b1; e += 32) {
@@ -533,14 +582,12 @@ static __global__ void __launch_bounds__(256) k_q_work(QueryPools Q, RowBuckets 
         }
         for (uint32_t o = G >> 1; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
         if (gl == 0 && live) {
-            const uint32_t u = (uint32_t)(w < m ? w : m);
-            const uint32_t k = rb.of(row_class(w, u, rb.cap_w, fam ? agg_cap_b(m, rb.cap_b) : rb.cap_b, rb.tiny), u);
-            Q.ucap[g] = u;
-            if (fam && w >= 0xFFFFFFFFull) raise_error(&Q.res[qi].err, kErrCountRange);
-            acc += w;
-            if (k < kRowBuckets) {
-                Q.bucket[g] = (uint8_t)(fam * kCountBuckets + k);
-                atomicAdd(&s_n[fam][k], 1u);
+            if (slot == kEmpty32) {
+                const uint32_t k = query_row(Q, rb, qi, g, w, m, fam);
+                acc += w;
+                if (k < kRowBuckets) atomicAdd(&s_n[fam][k], 1u);
+            } else {
+                Q.longs[slot].w = w;
             }
         }
     }
@@ -550,6 +597,43 @@ static __global__ void __launch_bounds__(256) k_q_work(QueryPools Q, RowBuckets 
     if (threadIdx.x < 2 * (kRowBuckets + 1)) {
         const uint32_t fam = threadIdx.x / (kRowBuckets + 1), k = threadIdx.x % (kRowBuckets + 1);
         if (k < kRowBuckets && s_n[fam][k]) atomicAdd(&Q.nbucket[fam][k], (unsigned long long)s_n[fam][k]);
+    }
+}
+
+// The long rows that k_q_work left, a warp a piece; whoever does a row's last
+// piece bins it.
+static __global__ void __launch_bounds__(256) k_q_long(QueryPools Q, RowBuckets rb) {
+    const uint32_t lane = lane_id();
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5, n = Q.n_long[1];
+    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < n; t += nwarps) {
+        const uint2 piece = Q.pieces[t];
+        QLongRow& l = Q.longs[piece.x];
+        const uint32_t qi = l.qi, b0 = piece.y, ne = min(l.e1 - b0, kQPiece);
+        const QueryIn qn = Q.qin[qi];
+        const RelDev& p = Q.rel[qn.p];
+        const uint32_t* icf = Q.ICf + p.tup_off + b0;
+        const uint2* ymap = Q.ymap + Q.qt_off[qi] - p.ybase;
+        uint32_t* icq = Q.ICq + Q.qt_off[qi] + b0;
+        unsigned long long v = 0;
+#pragma unroll 4
+        for (uint32_t e = lane; e < ne; e += 32) {
+            const uint2 y = __ldg(&ymap[__ldg(&icf[e])]);
+            icq[e] = y.x;
+            v += y.y;
+        }
+        v = warp_sum(v);
+        if (lane == 0) {
+            if (v) atomicAdd(&l.w, v);
+            __threadfence();
+            if (atomicSub(&l.left, 1u) == 1u) {
+                __threadfence();
+                const unsigned long long w = atomicAdd(&l.w, 0ull);
+                const uint32_t fam = qn.op == kOpCount, k = query_row(Q, rb, qi, l.g, w, Q.res[qi].nz, fam);
+                if (w) atomicAdd(&Q.res[qi].out_j, w);
+                if (k < kRowBuckets) atomicAdd(&Q.nbucket[fam][k], 1ull);
+            }
+        }
+        __syncwarp();
     }
 }
 

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 # entries of the long rows: about the lengths at which a row goes to the CTA,
 # or to the whole grid in pieces
-LENGTHS = [2047, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 10_241, 20_000]
+LENGTHS = [2047, 2048, 2049, 4096, 4097, 4112, 4113, 6160, 6161, 8192, 10_241, 20_000]
 
 
 def hubs(lengths, short, seed):
@@ -59,6 +59,7 @@ def star(n, hub):
     p = torch.randperm(n, generator=g, device="cuda")
     R = torch.stack([x[p], y[p]], 1).to(torch.int32).contiguous()
     S = torch.stack([ints(n // 8, n - 1000), ints(n_y, n - 1000)], 1).to(torch.int32).contiguous()
+    torch.cuda.synchronize()  # the library runs on streams of its own
     return R, S
 
 
@@ -75,3 +76,70 @@ def test_hub_row_is_binned_in_less_than_its_expansion(ctx):
         for k in ("ms_csr", "ms_write"):
             best[k] = min(best.get(k, 1e9), st[k])
     assert best["ms_csr"] < best["ms_write"], best
+
+
+def check_query(spec, res, R, S):
+    import dim3gpu
+    assert res["status"] == 0
+    k = O.pair_keys(spec["out"][:res["n_out"]].cpu().numpy().view(np.uint32))
+    order = np.argsort(k)
+    if spec["op"] == dim3gpu.OP_PROJECT:
+        assert np.array_equal(k[order], np.sort(O.pair_keys(O.join_project(R, S)[0])))
+        return
+    wg, wc = O.join_count(R, S)[:2]
+    b = np.argsort(O.pair_keys(wg))
+    assert np.array_equal(k[order], O.pair_keys(wg)[b])
+    assert np.array_equal(spec["cnt"][:res["n_out"]].cpu().numpy().view(np.uint64)[order], np.asarray(wc)[b])
+    assert res["out_j"] == int(wc.sum())
+
+
+@pytest.mark.parametrize("form", ["set", "batch"])
+def test_query_passes_with_hubs(ctx, form):
+    """Driving relations with rows on either side of the lengths at which a
+    row is cut, one relation a single row, one below any long row."""
+    import torch
+
+    import dim3gpu
+    host = [hubs(LENGTHS, 30_000, 1), hubs([4096, 4097, 4112, 4113, 4224, 4225], 12_000, 2), hubs([4160, 4161, 4128, 4129], 300, 5), hubs([30_000], 8000, 3), hubs([3000], 400, 4)]
+    host.append((np.stack([np.full(40_000, 5), np.arange(40_000)], 1).astype(np.uint32), host[0][1]))
+    dev = [tuple((torch.from_numpy(a.view(np.int32)).cuda(), a.shape[0]) for a in h) for h in host]
+    specs = []
+    for k in range(len(host)):
+        for op in (dim3gpu.OP_PROJECT, dim3gpu.OP_COUNT):
+            specs.append({"r": 2 * k, "s": 2 * k + 1, "op": op, "capacity": 400_000,
+                          "out": torch.empty((400_000, 2), dtype=torch.int32, device="cuda"),
+                          "cnt": torch.empty(400_000, dtype=torch.int64, device="cuda")})
+    if form == "set":
+        h = dim3gpu.RelSet(ctx, [r for d in dev for r in d])
+        run = lambda: h.join(specs)  # noqa: E731
+    else:
+        h = dim3gpu.Batch(ctx, [d for d in dev for _ in range(2)], specs)
+        run = h.run
+    for _ in range(2):
+        for i, (spec, res) in enumerate(zip(specs, run())):
+            check_query(spec, res, *host[i // 2])
+    h.close()
+
+
+def test_query_pass_of_a_hub_takes_little_more_than_its_expansion(ctx):
+    """The pass against the row kernels of the same join: one warp working out
+    the hub's row took twice as long as they."""
+    import time
+
+    import torch
+
+    import dim3gpu
+    R, S = star(4_000_000, 2_000_000)
+    out = torch.empty((16_000_000, 2), dtype=torch.int32, device="cuda")
+    n = ctx.join_project_device(R, R.shape[0], S, S.shape[0], out, out.shape[0])
+    ctx.join_project_device(R, R.shape[0], S, S.shape[0], out, out.shape[0])
+    rows = ctx.stats()["ms_write"]
+    rs = dim3gpu.RelSet(ctx, [(R, R.shape[0]), (S, S.shape[0])])
+    best = 1e9
+    for _ in range(4):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        assert rs.join([{"r": 0, "s": 1, "out": out, "capacity": out.shape[0]}])[0]["n_out"] == n
+        best = min(best, 1e3 * (time.perf_counter() - t))
+    assert best < 2 * rows, (best, rows)
+    rs.close()
