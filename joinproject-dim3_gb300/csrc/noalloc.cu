@@ -40,7 +40,6 @@ constexpr unsigned long long kEmptyPair = ~0ull;
 // join values with long buckets do not leave their candidates to one warp.
 constexpr uint32_t kPiece = 1024, kMaxTasks = kMaxTuples / 32 * 16;
 constexpr int kThreads = 512, kCtasPerSm = 3;
-constexpr uint32_t kBarrierPolls = 1u << 22;  // a grid barrier gives up after this many (seconds)
 
 // Layout of the scratch array (byte offsets, 256-aligned).  The counters and
 // bucket counts are zeroed together.
@@ -56,17 +55,16 @@ static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
 struct Counters {
     unsigned long long n_out;    // distinct pairs found
-    unsigned long long flags;    // bit 1: a probe walked the whole pair table; bit 2: a grid barrier gave up
+    unsigned long long flags;    // bit 1: a probe walked the whole pair table
     unsigned long long all_ones; // the all-ones pair seen
     uint32_t placed;             // sorted tuples given to buckets
     uint32_t n_tasks, next_task;
-    uint32_t barrier[4];         // CTAs arrived
 };
 static_assert(sizeof(Counters) <= 256, "counters' room");
 
 struct Scratch {
     Counters* c;
-    uint32_t* count;  // tuples per bucket (counted down again as they are placed)
+    uint32_t* count;  // tuples per bucket
     uint32_t* base;   // first sorted tuple of each bucket; its end once placed
     uint2* sorted;    // the larger relation, bucket by bucket
     uint32_t* tasks;  // run of 32 probe tuples * pieces a run + piece
@@ -96,25 +94,6 @@ __device__ __forceinline__ uint32_t warp_scan(uint32_t v) {  // inclusive
         if ((int)lane() >= o) v += t;
     }
     return v;
-}
-
-// All CTAs of the grid (co-resident: a cooperative launch).  False once a
-// wait has given up; the caller returns.
-__device__ bool grid_barrier(const Scratch& s, uint32_t k) {
-    __shared__ bool ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(&s.c->barrier[k], 1u);
-        uint32_t polls = 0;
-        while (*(volatile uint32_t*)&s.c->barrier[k] < gridDim.x && ++polls < kBarrierPolls) {
-        }
-        ok = polls < kBarrierPolls;
-        if (!ok) atomicOr(&s.c->flags, 4ull);
-        __threadfence();
-    }
-    __syncthreads();
-    return ok;
 }
 
 // Distinct-pair set: 64-bit keys (P.first << 32 | Q.first) with linear
@@ -154,28 +133,38 @@ __device__ __forceinline__ Run load_run(const uint2* __restrict__ Q, uint32_t nQ
     return r;
 }
 
-// The whole join in one cooperative launch.  The larger relation P is placed
-// bucket by bucket of its join key (count, give every bucket a range, place;
-// the ranges are in no order, so no prefix sum), then the smaller one, Q,
-// probes: the candidates of 32 probe tuples are flattened over a warp, each
-// lane comparing one sorted tuple's key, and new pairs take one reservation
-// per group of 128 candidates.
+// The join.  The larger relation P is placed bucket by bucket of its join key
+// (count, give every bucket a range, place; the ranges are in no order, so no
+// prefix sum), then the smaller one, Q, probes: the candidates of 32 probe
+// tuples are flattened over a warp, each lane comparing one sorted tuple's key,
+// and new pairs take one reservation per group of 128 candidates.
 //
 // Bound by the latency of dependent accesses.  A linked list per bucket,
 // walked by one thread a probe tuple, with a reservation a pair, took 205 us
-// in the probe alone for 150K x 90K tuples.
-__global__ void __launch_bounds__(kThreads, kCtasPerSm)
-    k_na_join(const uint2* __restrict__ P, uint32_t nP, const uint2* __restrict__ Q, uint32_t nQ, Scratch s, uint2* out,
-              unsigned long long cap) {
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-    const uint32_t warp = tid >> 5, warps = stride >> 5, ln = lane();
-    const uint32_t lt = (1u << ln) - 1u;
-    // count
-    for (uint32_t i = tid; i < nP; i += stride) atomicAdd(&s.count[bucket_of(__ldg(&P[i]).y)], 1u);
-    if (!grid_barrier(s, 0)) return;
-    // ranges: a warp's 128 buckets take one range, four buckets a lane
+// in the probe alone for 150K x 90K tuples.  The steps are plain launches, each
+// with what does not depend on the one before (150K x 90K tuples: 77 us).  One
+// cooperative launch with grid barriers between them took 83, and could only
+// start once its whole grid fitted beside whatever else ran on the GPU.
+__device__ __forceinline__ uint32_t thread_id() { return blockIdx.x * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ uint32_t thread_count() { return gridDim.x * blockDim.x; }
+
+// Counts P's buckets; empties the pair set (the previous call's pairs).
+__global__ void __launch_bounds__(kThreads) k_na_count(const uint2* __restrict__ P, uint32_t nP, Scratch s) {
+    for (uint32_t i = thread_id(); i < nP; i += thread_count()) atomicAdd(&s.count[bucket_of(__ldg(&P[i]).y)], 1u);
+    const uint32_t ones = 0xFFFFFFFFu;
+    for (uint32_t i = thread_id(); i < kPairSlots / 2; i += thread_count())
+        reinterpret_cast<uint4*>(s.pairs)[i] = make_uint4(ones, ones, ones, ones);
+}
+
+// Pieces a run of 32 probe tuples may have.
+__device__ __forceinline__ uint32_t most_pieces(uint32_t nQ) { return kMaxTasks / ((nQ + 31) / 32); }
+
+// Ranges: a warp's 128 buckets take one range, four buckets a lane.  Tasks:
+// the pieces of every run of 32 probe tuples.
+__global__ void __launch_bounds__(kThreads) k_na_ranges(const uint2* __restrict__ Q, uint32_t nQ, Scratch s) {
+    const uint32_t warp = thread_id() >> 5, warps = thread_count() >> 5, ln = lane();
     for (uint32_t b0 = warp * 128; b0 < kBuckets; b0 += warps * 128) {
-        const uint4 n = __ldcg(reinterpret_cast<const uint4*>(s.count + b0) + ln);
+        const uint4 n = reinterpret_cast<const uint4*>(s.count + b0)[ln];
         const uint32_t sum = n.x + n.y + n.z + n.w, inc = warp_scan(sum);
         const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
         if (tot == 0) continue;
@@ -184,18 +173,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         at = __shfl_sync(0xffffffffu, at, 0) + inc - sum;
         reinterpret_cast<uint4*>(s.base + b0)[ln] = make_uint4(at, at + n.x, at + n.x + n.y, at + n.x + n.y + n.z);
     }
-    if (!grid_barrier(s, 1)) return;
-    // place (base becomes the bucket's end)
-    for (uint32_t i = tid; i < nP; i += stride) {
-        const uint2 p = __ldg(&P[i]);
-        s.sorted[atomicAdd(&s.base[bucket_of(p.y)], 1u)] = p;
-    }
-    if (!grid_barrier(s, 2)) return;
-    // tasks: the pieces of every run of 32 probe tuples
-    const uint32_t runs = (nQ + 31) / 32, most = kMaxTasks / runs;
+    const uint32_t runs = (nQ + 31) / 32, most = most_pieces(nQ);
     for (uint32_t r = warp; r < runs; r += warps) {
-        const Run run = load_run(Q, nQ, r * 32, s);
-        unsigned long long w = run.len;
+        const uint32_t i = r * 32 + ln;
+        unsigned long long w = i < nQ ? s.count[bucket_of(__ldg(&Q[i]).y)] : 0u;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
         if (w == 0) continue;
@@ -205,7 +186,19 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         at = __shfl_sync(0xffffffffu, at, 0);
         for (uint32_t k = ln; k < n; k += 32) s.tasks[at + k] = r * most + k;
     }
-    if (!grid_barrier(s, 3)) return;
+}
+
+// Places P's tuples (base becomes the bucket's end).
+__global__ void __launch_bounds__(kThreads) k_na_place(const uint2* __restrict__ P, uint32_t nP, Scratch s) {
+    for (uint32_t i = thread_id(); i < nP; i += thread_count()) {
+        const uint2 p = __ldg(&P[i]);
+        s.sorted[atomicAdd(&s.base[bucket_of(p.y)], 1u)] = p;
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+    k_na_join(const uint2* __restrict__ Q, uint32_t nQ, Scratch s, uint2* out, unsigned long long cap) {
+    const uint32_t most = most_pieces(nQ), ln = lane(), lt = (1u << ln) - 1u;
     const uint32_t tasks = __ldcg(&s.c->n_tasks);
     for (;;) {
         uint32_t t = 0;
@@ -293,13 +286,7 @@ int scratch_for_device(int dev, unsigned char** base, int* grid) {
                 cudaGetLastError();
                 return DIM3G_ERR_CUDA;
             }
-            int per_sm = 0;  // the CTAs wait on one another, so all must be resident
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_na_join, kThreads, 0) != cudaSuccess ||
-                per_sm < 1) {
-                cudaGetLastError();
-                return DIM3G_ERR_CUDA;
-            }
-            g_grid[dev] = sms * (per_sm < kCtasPerSm ? per_sm : kCtasPerSm);
+            g_grid[dev] = sms * kCtasPerSm;
             p = (unsigned char*)addr;
             g_base[dev].store(p, std::memory_order_release);
         }
@@ -341,26 +328,25 @@ extern "C" int dim3g_join_project_noalloc(const uint32_t* d_R, uint64_t nR, cons
     Scratch s{(Counters*)(base + kOffCounters), (uint32_t*)(base + kOffCount), (uint32_t*)(base + kOffBase),
               (uint2*)(base + kOffSorted), (uint32_t*)(base + kOffTasks), (unsigned long long*)(base + kOffPairs)};
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    // the previous call's contents stay in the array: reset what must start
-    // empty (counters, bucket counts, pair set)
-    if (cudaMemsetAsync(s.c, 0, kOffBase - kOffCounters, st) != cudaSuccess ||
-        cudaMemsetAsync(s.pairs, 0xff, (size_t)kPairSlots * 8, st) != cudaSuccess) {
+    // the previous call's contents stay in the array: the counters and bucket
+    // counts start at zero, k_na_count empties the pair set
+    if (cudaMemsetAsync(s.c, 0, kOffBase - kOffCounters, st) != cudaSuccess) {
         cudaGetLastError();
         return DIM3G_ERR_CUDA;
     }
-    // a CTA per 512 tuples (the barriers cost by the CTAs), at least one an SM
-    // (the candidates are not known), at most what is resident
-    const uint2* out = (const uint2*)d_out;
-    uint32_t n_p = (uint32_t)nP, n_q = (uint32_t)nQ;
-    unsigned long long cap = capacity;
-    int ctas = (int)((nP + nQ + kThreads - 1) / kThreads);
-    if (ctas < grid / kCtasPerSm) ctas = grid / kCtasPerSm;
-    if (ctas > grid) ctas = grid;
-    void* args[] = {&P, &n_p, &Q, &n_q, &s, &out, &cap};
+    auto ctas = [&](uint64_t threads) {
+        const uint64_t n = (threads + kThreads - 1) / kThreads;
+        return (unsigned)(n < (uint64_t)grid ? n : (uint64_t)grid);
+    };
+    const uint32_t n_p = (uint32_t)nP, n_q = (uint32_t)nQ;
+    k_na_count<<<(unsigned)grid, kThreads, 0, st>>>(P, n_p, s);
+    k_na_ranges<<<ctas(nQ > kBuckets / 4 ? nQ : kBuckets / 4), kThreads, 0, st>>>(Q, n_q, s);
+    k_na_place<<<ctas(nP), kThreads, 0, st>>>(P, n_p, s);
+    // the candidates are not known: at least a CTA an SM
+    const unsigned c_join = ctas(nP + nQ), c_sm = (unsigned)(grid / kCtasPerSm);
+    k_na_join<<<c_join > c_sm ? c_join : c_sm, kThreads, 0, st>>>(Q, n_q, s, (uint2*)d_out, capacity);
     unsigned long long h[2] = {0, 0};  // n_out, flags
-    if (cudaLaunchCooperativeKernel((const void*)k_na_join, dim3((unsigned)ctas), dim3(kThreads), args, 0, st) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(h, s.c, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(h, s.c, sizeof h, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {
         cudaGetLastError();
         return DIM3G_ERR_CUDA;
