@@ -83,8 +83,8 @@ const char* dim3g_last_error(const dim3g_ctx* ctx);
 int dim3g_get_stats(const dim3g_ctx* ctx, dim3g_stats* out);
 /* Tuning knobs, validated on set: "warp_slots_log2" (5..14, warp-class hash
  * set size), "block_slots_log2" (8..14, block-class hash set size),
- * "tile_bits_log2" (10..20, bitmap-class z tile width; at most 19 for
- * materialised COUNT), "ordered_output" (0: one expansion per row, rows in unspecified order;
+ * "tile_bits_log2" (10..20, bitmap-class z tile width; COUNT uses 15..19 of
+ * it), "ordered_output" (0: one expansion per row, rows in unspecified order;
  * 1: count pass + write pass, pairs grouped by first value),
  * "block_threads" (256, 512 or 1024: CTA width of the block class),
  * "host_direct_output" (1: pinned host outputs written directly),

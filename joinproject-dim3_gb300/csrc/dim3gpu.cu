@@ -811,9 +811,11 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     DensePlan dp;
 retile:
     // z tiles for the bitmap class
+    // (COUNT has row pointers of S by tile and a work item a row and tile for
+    // no gain from narrow tiles: it takes no narrower ones than direct rows do)
     uint32_t tile_lg = c->prm.tile_lg;
     if (jp.aggregate && tile_lg > kAggTileLgMax) tile_lg = kAggTileLgMax;
-    if (direct && tile_lg > kAggDirectLg) tile_lg = kAggDirectLg;
+    if (jp.aggregate && (direct || tile_lg < kAggDirectLg)) tile_lg = kAggDirectLg;
     uint32_t T = 1, tile_shift = 31, tile_width = m;
     if (m > (1u << tile_lg)) {
         tile_shift = tile_lg;

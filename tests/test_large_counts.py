@@ -166,3 +166,24 @@ def test_sizes_around_the_wide_sums(built):
         n = sum({0: nz, 1: nz - 1, 2: 0}[y] for y in ys)
         assert c.join_project_count_device(R, len(ys), S, S.shape[0]) == n
     c.close()
+
+
+@pytest.mark.gpu
+def test_count_over_wide_domains_takes_any_tile_width(built):
+    """1.2M join values and 4M z: 2^32 row pointers at 2^10 z a tile, which
+    COUNT does not need."""
+    import torch
+    ny, nz = 1_200_000, 4_000_000
+    y, z = torch.arange(ny, device="cuda"), torch.arange(nz, device="cuda")
+    R, S = ready(torch.stack([y % 1000, y], 1).to(torch.int32).contiguous(),
+                 torch.stack([z, z % ny], 1).to(torch.int32).contiguous())
+    out = torch.empty((nz, 2), dtype=torch.int32, device="cuda")
+    cnt = torch.empty(nz, dtype=torch.int64, device="cuda")
+    c = context(tile_bits_log2=10)
+    assert ny * (nz >> 10) >= 1 << 32
+    assert c.join_count_device(R, ny, S, nz, out, cnt, nz) == nz
+    assert bool((cnt == 1).all())
+    order = torch.argsort(out[:, 1])
+    assert torch.equal(out[order, 1].long(), z) and torch.equal(out[order, 0].long(), (z % ny) % 1000)
+    assert c.stats()["z_tiles"] <= 1 << 9
+    c.close()
