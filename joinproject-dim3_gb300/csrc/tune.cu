@@ -141,26 +141,26 @@ int dim3g_autotune(dim3g_ctx* ctx, const uint32_t* d_R, uint64_t nR, const uint3
             std::vector<int64_t> cand = best;
             cand[i] = v;
             if (set_all(ctx, knobs, cand)) continue;  // a combination the context rejects
-            float ms = 0;
-            r = trial(ctx, d_R, nR, d_S, nS, d_out, n_out, reps, &ms);
+            // heavy rows on the sparse kernels: their measured rate becomes
+            // the cost model's sparse rate (4 algorithmic bytes a candidate).
+            // It is the bitmap rows' alone, so the trial's last run takes the
+            // row classes in turn and not beside each other.
+            const bool sparse = i == kDenseKnob && v == 0;
+            float ms = 0, alone = 0;
+            r = trial(ctx, d_R, nR, d_S, nS, d_out, n_out, sparse ? reps - 1 : reps, &ms);
+            if (!r && sparse) {
+                I::rows_in_turn(ctx, true);
+                r = trial(ctx, d_R, nR, d_S, nS, d_out, n_out, 1, &alone);
+                I::rows_in_turn(ctx, false);
+                if (alone < ms) ms = alone;
+            }
             trials++;
             if (r) break;
             dim3g_stats ts;
             dim3g_get_stats(ctx, &ts);
             if (ts.rows_dense) dense_ran = true;
-            // heavy rows on the sparse kernels: their measured rate becomes
-            // the cost model's sparse rate (4 algorithmic bytes a candidate)
-            // (of a run with the row classes in turn, not beside each other)
-            if (i == kDenseKnob && v == 0 && ts.out_j_cls[0]) {
-                float alone = 0;
-                I::rows_in_turn(ctx, true);
-                r = trial(ctx, d_R, nR, d_S, nS, d_out, n_out, 1, &alone);
-                I::rows_in_turn(ctx, false);
-                if (r) break;
-                dim3g_get_stats(ctx, &ts);
-                if (ts.ms_write_cls[0] > 0)
-                    I::set_sparse_rate(ctx, 4.0 * (double)ts.out_j_cls[0] / (ts.ms_write_cls[0] * 1e-3));
-            }
+            if (sparse && ts.out_j_cls[0] && ts.ms_write_cls[0] > 0)
+                I::set_sparse_rate(ctx, 4.0 * (double)ts.out_j_cls[0] / (ts.ms_write_cls[0] * 1e-3));
             if (ms < best_ms) {
                 best_ms = ms;
                 best = cand;
