@@ -151,7 +151,9 @@ int dim3g_join_project_count_device(dim3g_ctx* ctx, const uint32_t* d_R, uint64_
 /* ---- join-aggregate COUNT(*) GROUP BY (x, z) -------------------------
  * Replaces DIM3JoinAggregate<...>::doJoinAggregate (dim3.hpp:1313-1373) with
  * a COUNT aggregate: for every distinct (P.first, Q.first) the number of
- * joining tuple pairs, exact in 64 bits. */
+ * joining tuple pairs, exact in 64 bits.  Groups come in unspecified order
+ * unless "ordered_output" is 1.  On DIM3G_ERR_CAPACITY *n_out holds the groups
+ * needed and the buffers' contents are unspecified. */
 int dim3g_join_count(dim3g_ctx* ctx, const uint32_t* R_xy, uint64_t nR, const uint32_t* S_zy, uint64_t nS,
                      uint32_t** out_xz, uint64_t** out_cnt, uint64_t* n_out);
 int dim3g_join_count_device(dim3g_ctx* ctx, const uint32_t* d_R, uint64_t nR, const uint32_t* d_S, uint64_t nS,
@@ -243,7 +245,8 @@ typedef struct {
  * in the whole set. */
 int dim3g_relset_create(dim3g_ctx* ctx, const dim3g_relation* rels, uint32_t n, dim3g_relset** set);
 void dim3g_relset_destroy(dim3g_relset* set);
-/* Device bytes the set holds (indexes and query scratch). */
+/* Device bytes the set holds (indexes and query scratch, from its first COUNT
+ * query on with that query's counters). */
 uint64_t dim3g_relset_bytes(const dim3g_relset* set);
 /* Runs n queries over the set in one pass on the context's stream;
  * synchronous.  Each query gets its own status; the call returns DIM3G_OK
@@ -327,8 +330,8 @@ void dim3g_batch_destroy(dim3g_batch* b);
  * and the fastest are applied to the context.  The trial that runs the
  * heavy rows on the sparse kernels also sets the context's measured sparse
  * rate, which the dense block's cost model uses from then on (see
- * dim3g_calibrate for the product's rates).  max_trials bounds the joins run
- * (0: no bound). */
+ * dim3g_calibrate for the product's rates).  max_trials bounds the settings
+ * timed (0: no bound): two joins each, after one pass for the output's size. */
 typedef struct {
     int32_t tile_bits_log2, block_threads, block_slots_log2, warp_slots_log2, cta_walk;
     int32_t dense_block, dense_k_max;

@@ -293,8 +293,8 @@ unsigned resident_grid(dim3g_ctx* c, K kernel, int block, size_t smem) {
 // rows stay on it, the block rows and the warp rows take one side stream each
 // -- and join it again, and a kernel that is down to a few huge rows leaves
 // the rest of the GPU to the next.  Whole calls, in turn and forked: 1.2M-edge
-// 2-hop 1.48 and 1.44 ms, its COUNT 3.63 and 3.40, 200k rows ordered 0.79 and
-// 0.76, an eighth of the 20M-edge 2-hop 10.37 and 10.23.
+// 2-hop 1.48 and 1.44 ms, COUNT of 1M x 800K Zipf tuples 3.63 and 3.40, 200K
+// tuples ordered 0.79 and 0.76, an eighth of the 20M-edge 2-hop 10.37 and 10.23.
 //
 // Calls of more than kForkTuples driving tuples keep the kernels in turn: their
 // tails are a small part there (20M-edge 2-hop 74.97 ms in
@@ -716,7 +716,7 @@ int run_join(dim3g_ctx* c, const JoinPlan& jp, uint64_t* n_out) {
     // one z tile covers Q and the dense block cannot pay -- too few candidates
     // (at most |P| |Q|), or no row can pass the block class -- the single pass
     // runs on the tuple counts as bounds of the id counts, with nothing to wait
-    // for before its end: 1.2K x 0.9K tuples 175 us with four round trips, 98
+    // for before its end: 1.2K x 0.9K tuples 177 us with four round trips, 118
     // with one.  (A slack below 100 % asks for tables smaller than the keys,
     // which only the sketch gives.)
     const bool small_tables = fullP <= kSmallSlots && fullQ <= kSmallSlots && c->prm.table_slack_pct >= 100;
@@ -841,7 +841,6 @@ retile:
     const bool single = jp.single_pass && !jp.count_only;
     const bool want_ids = !single || jp.aggregate, want_pairs = !jp.aggregate && !jp.count_only;
     uint32_t* IC_S = want_ids ? ws_get<uint32_t>(c, nq) : nullptr;
-    uint32_t* VS = nullptr;  // the value paths read the pairs in ISV
     // +2: the streamed bitmap rows copy 16-byte-aligned supersets of S
     // segments, up to one pair past the last one
     uint2* ISV = want_pairs ? ws_get<uint2>(c, nq + 2) : nullptr;
@@ -877,7 +876,7 @@ retile:
     rc.IC_R = IC_R;
     rc.JR_S = JR_S;
     rc.IC_S = IC_S;
-    rc.VS = VS;
+    rc.VS = nullptr;  // the value paths read the pairs in ISV
     rc.ISV = ISV;
     rc.T = T;
     rc.tile_width = tile_width;

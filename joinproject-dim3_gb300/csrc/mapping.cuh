@@ -74,10 +74,6 @@ __device__ __forceinline__ uint2 sketch_slot(uint32_t key) {
     const unsigned long long w = h << kSketchLg;
     return make_uint2((uint32_t)(h >> (64 - kSketchLg)), (w ? (uint32_t)__clzll(w) : 64u - kSketchLg) + 1);
 }
-__device__ __forceinline__ void sketch_add(uint32_t* r, uint32_t key) {
-    const uint2 s = sketch_slot(key);
-    atomicMax(&r[s.x], s.y);
-}
 
 inline uint64_t next_pow2(uint64_t v) {
     uint64_t p = 1;
@@ -85,8 +81,8 @@ inline uint64_t next_pow2(uint64_t v) {
     return p;
 }
 
-// sketch_add without the atomic when the register already holds the rank
-// (most updates once the registers have filled).
+// Adds a key: no atomic when the register already holds the rank (most
+// updates once the registers have filled).
 __device__ __forceinline__ void sketch_add_if_larger(uint32_t* r, uint32_t key) {
     const uint2 s = sketch_slot(key);
     if (*(volatile uint32_t*)&r[s.x] < s.y) atomicMax(&r[s.x], s.y);

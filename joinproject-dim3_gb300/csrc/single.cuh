@@ -408,7 +408,7 @@ __host__ __device__ constexpr size_t warp_row_words(uint32_t warp_lg, uint32_t s
     return ((size_t)1 << warp_lg) + 2 * (size_t)stage;
 }
 
-// Classes 1 and 5 (tiny): one warp per row.
+// Class 1: one warp per row (tiny rows go many to a warp, packed.cuh).
 static __global__ void __launch_bounds__(256) k_single_warp(RowCtx c, Reserve rs, unsigned long long* cls,
                                                             const uint32_t* __restrict__ rows,
                                                             const unsigned long long* __restrict__ nrows_p,
@@ -469,7 +469,6 @@ static __global__ void __launch_bounds__(DIM3G_BM_BOUNDS, DIM3G_BM_MINB) k_singl
                                                                const unsigned long long* __restrict__ n4,
                                                                uint32_t bitmap_words) {
     extern __shared__ uint32_t bm[];
-    __shared__ uint32_t s_row;
     __shared__ CtaChunks s_cc;
     if (threadIdx.x == 0) s_cc.n = 0;
     uint32_t* stage = bm + bitmap_words + (threadIdx.x >> 5) * kStage;
