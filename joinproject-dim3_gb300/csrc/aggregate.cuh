@@ -275,7 +275,9 @@ __device__ __forceinline__ RankHead rank_head(const RowCtx& c, uint64_t item, ui
 // during the first pass (the other warps take its share of the pieces).
 // g: the CTA's tile_width counters in global memory, all zero between calls,
 // or null.  A tile of more than two windows of ranks counts there in one walk
-// instead of one walk a window.
+// instead of one walk a window.  (A query pass of 600 rows, windows of 23K
+// ranks, there and in windows: 28K distinct z a row 0.62 and 0.48 ms, 40K 0.77
+// and 0.64, 52K 0.95 and 1.01, 90K 1.54 and 2.04.)
 template <class Ahead>
 __device__ __forceinline__ void agg_ranked_tile(const RowCtx& c, const AggOut& ao, const RankHead& h, uint32_t t,
                                                 uint32_t* smem, const RankLayout& l, CtaChunks* cc, uint32_t* s_pos,
@@ -598,18 +600,22 @@ static __global__ void __launch_bounds__(1024, 1) k_agg_map(RowCtx c, AggOut ao,
 // tile, so a huge row's tiles run side by side; offsets, and the summaries of
 // direct rows (their sums meet in a few addresses, once a row): one CTA a row.  The
 // next item is claimed and its header loaded during the current one.
-// DIRECT: direct rows, `l` unused.
-template <bool DIRECT>
+// FORM: direct rows (`l` and `ctr` unused), ranked rows in windows (ctr
+// unused), or ranked rows with every CTA's counters for agg_ranked_tile at
+// ctr.  (Without a use for them they cost registers: count_1m 3.41 and 3.48
+// ms.)
+enum RankForm { kRankDirect, kRankWindows, kRankCounters };
+template <RankForm FORM>
 static __global__ void __launch_bounds__(1024, 1) k_agg_ranked(RowCtx c, AggOut ao, const uint32_t* __restrict__ rows,
                                                             const unsigned long long* __restrict__ n3,
                                                             const unsigned long long* __restrict__ n4, RankLayout l,
-                                                            unsigned long long* next_item) {
+                                                            unsigned long long* next_item, uint32_t* ctr) {
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t s_pos, s_wbase[33];
     __shared__ unsigned long long s_base;
     __shared__ RankHead s_head[2];
     __shared__ CtaChunks s_cc;
-    const uint32_t per = ao.rs.cursor || (ao.sum.tiles && !DIRECT) ? c.T : 1u;
+    const uint32_t per = ao.rs.cursor || (ao.sum.tiles && FORM != kRankDirect) ? c.T : 1u;
     const TileItems it{*n3 + *n4, per};
     auto claim = [&](RankHead* dst) {
         const uint64_t i = atomicAdd(next_item, 1ull);
@@ -627,11 +633,12 @@ static __global__ void __launch_bounds__(1024, 1) k_agg_ranked(RowCtx c, AggOut 
             auto ahead = [&] {
                 if (t == t0) claim(&s_head[k ^ 1]);
             };
-            if (DIRECT) agg_direct_tile(c, ao, h, t, smem, &s_cc, &s_pos, s_wbase, &s_base, gs, ahead);
-            else agg_ranked_tile(c, ao, h, t, smem, l, &s_cc, &s_pos, s_wbase, &s_base, nullptr, ahead);
+            if (FORM == kRankDirect) agg_direct_tile(c, ao, h, t, smem, &s_cc, &s_pos, s_wbase, &s_base, gs, ahead);
+            else agg_ranked_tile(c, ao, h, t, smem, l, &s_cc, &s_pos, s_wbase, &s_base,
+                                 FORM == kRankCounters ? ctr + (size_t)blockIdx.x * c.tile_width : nullptr, ahead);
             __syncthreads();
         }
-        if (DIRECT && ao.sum.tiles) ao.sum.commit(h.xv, gs.g, gs.cs, gs.h);
+        if (FORM == kRankDirect && ao.sum.tiles) ao.sum.commit(h.xv, gs.g, gs.cs, gs.h);
         __syncthreads();
     }
 }

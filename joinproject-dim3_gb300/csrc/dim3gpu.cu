@@ -265,7 +265,7 @@ struct RowLists {
 };
 struct RowStreams;
 int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, Scalars* sc, const uint32_t* list_t,
-                  RowStreams& rst, bool direct);
+                  RowStreams& rst, bool direct, bool huge_rows);
 
 // Warps per CTA of a warp-per-row kernel whose warps each own per_warp
 // bytes of shared memory: up to 8, within about a third of an SM's shared
@@ -952,6 +952,9 @@ retile:
                            dp.counted ? h.nrows_b[2] != 0 : m > rb.cap_m};
     const bool has_any_b = !dp.counted || h.nrows[2], has_w = !dp.counted || h.nrows[1],
                has_t = !dp.counted || h.nrows[5];
+    // COUNT rows that ranks may have to take in many windows: huge ones beside
+    // so many others that the rows are not counted directly
+    const bool huge_rows = dp.counted && h.nrows[4] != 0;
     RowStreams rst(c, jp.nP <= kForkTuples && !c->rows_in_turn &&
                           (dp.counted ? has_m + has_any_b + (has_w || has_t) > 1 : !small && jp.aggregate));
 
@@ -960,7 +963,7 @@ retile:
         // needs no count pass (nothing is placed)
         CU(cudaEventRecord(c->evc[4], st));
         if (jp.aggregate) {
-            int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, nullptr, rst, direct);
+            int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, nullptr, rst, direct, huge_rows);
             if (r) return r;
         } else {
             k_sum_bitmap<<<resident_grid(c, k_sum_bitmap, blk_m, smem_m), blk_m, smem_m, st>>>(rc, jp.sum, L.m,
@@ -1002,7 +1005,7 @@ retile:
         rc.out = sp_out;
     }
     if (single && jp.aggregate) {
-        int r = run_aggregate(c, rc, AggOut{sp_cnt, SumAcc{}, Reserve{&sc->cursor, cap}}, L, sc, list_t, rst, direct);
+        int r = run_aggregate(c, rc, AggOut{sp_cnt, SumAcc{}, Reserve{&sc->cursor, cap}}, L, sc, list_t, rst, direct, huge_rows);
         if (r) return r;
         CU(cudaMemcpyAsync(c->h_sc, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
         CU(cudaEventRecord(c->ev[3], st));
@@ -1206,7 +1209,7 @@ retile:
     CU(cudaMemsetAsync(sc->next_row, 0, sizeof(sc->next_row), st));
     if (total > 0) {
         if (jp.aggregate) {
-            int r = run_aggregate(c, rc, AggOut{out_cnt, SumAcc{}, Reserve{nullptr, 0}}, L, sc, nullptr, rst, direct);
+            int r = run_aggregate(c, rc, AggOut{out_cnt, SumAcc{}, Reserve{nullptr, 0}}, L, sc, nullptr, rst, direct, huge_rows);
             if (r) return r;
         } else {
             CU(cudaEventRecord(c->evc[4], st));
@@ -1242,7 +1245,7 @@ retile:
 // rows from the largest maps down, then the tiny rows (list_t; null: none).
 // CTAs by map size, so that small maps run many rows an SM.
 int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, Scalars* sc,
-                  const uint32_t* list_t, RowStreams& rst, bool direct) {
+                  const uint32_t* list_t, RowStreams& rst, bool direct, bool huge_rows) {
     CU(rst.fork());
     // one ranked CTA an SM with all of its shared memory, or two where a
     // half leaves 60 KB for the counters
@@ -1251,11 +1254,20 @@ int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, 
     const size_t smem_m = half ? 102 << 10 : 200 << 10;
     if (direct) {
         const size_t sd = (size_t)rc.tile_width * 4;
-        k_agg_ranked<true><<<resident_grid(c, k_agg_ranked<true>, 1024, sd), 1024, sd, rst.m>>>(rc, ao, L.m, L.n3, L.n4,
-                                                                                            RankLayout{}, &sc->next_item);
+        k_agg_ranked<kRankDirect><<<resident_grid(c, k_agg_ranked<kRankDirect>, 1024, sd), 1024, sd, rst.m>>>(
+            rc, ao, L.m, L.n3, L.n4, RankLayout{}, &sc->next_item, nullptr);
     } else {
-        k_agg_ranked<false><<<resident_grid(c, k_agg_ranked<false>, thr_m, smem_m), thr_m, smem_m, rst.m>>>(
-            rc, ao, L.m, L.n3, L.n4, rank_layout(rc.tile_width, thr_m / 32, smem_m), &sc->next_item);
+        const RankLayout l = rank_layout(rc.tile_width, thr_m / 32, smem_m);
+        const unsigned grid = resident_grid(c, k_agg_ranked<kRankCounters>, thr_m, smem_m);
+        const uint64_t words = (uint64_t)grid * rc.tile_width;
+        uint32_t* ctr = huge_rows && rc.tile_width > 2 * l.cap ? ws_get<uint32_t>(c, words) : nullptr;
+        if (ctr) {  // (no room for them: windows)
+            CU(cudaMemsetAsync(ctr, 0, words * 4, rst.m));
+            k_agg_ranked<kRankCounters><<<grid, thr_m, smem_m, rst.m>>>(rc, ao, L.m, L.n3, L.n4, l, &sc->next_item, ctr);
+        } else {
+            k_agg_ranked<kRankWindows><<<resident_grid(c, k_agg_ranked<kRankWindows>, thr_m, smem_m), thr_m, smem_m, rst.m>>>(
+                rc, ao, L.m, L.n3, L.n4, l, &sc->next_item, nullptr);
+        }
     }
     CHECK_LAUNCH();
     auto map_rows = [&](const uint32_t* rows, const unsigned long long* n, uint32_t lg, const unsigned long long* s0,
@@ -1293,8 +1305,9 @@ bool set_aggregate_attributes() {
            cudaFuncSetAttribute(k_sum_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 1 << 14 << 2) == cudaSuccess &&
            cudaFuncSetAttribute(k_sum_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, (1 << 20) / 8) == cudaSuccess &&
            cudaFuncSetAttribute(k_agg_map, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 << 14) == cudaSuccess &&
-           cudaFuncSetAttribute(k_agg_ranked<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10) == cudaSuccess &&
-           cudaFuncSetAttribute(k_agg_ranked<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kAggDirectLg) == cudaSuccess;
+           cudaFuncSetAttribute(k_agg_ranked<kRankWindows>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10) == cudaSuccess &&
+           cudaFuncSetAttribute(k_agg_ranked<kRankCounters>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10) == cudaSuccess &&
+           cudaFuncSetAttribute(k_agg_ranked<kRankDirect>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kAggDirectLg) == cudaSuccess;
 }
 
 int ensure_dev(dim3g_ctx* c, void** p, size_t* have, size_t need) {
