@@ -408,7 +408,7 @@ static __global__ void k_q_ymap(QueryPools Q) {
     }
 }
 
-// Lanes a row (log2) of a query's k_q_work steps.
+// Lanes a row (log2) of a query's k_q_work steps (as row_work_lanes).
 __device__ __forceinline__ uint32_t query_lanes(const RelDev& p) {
     const uint64_t per_row = p.nf ? p.nt / p.nf : 0;
     return per_row > 64 ? 5u : (per_row > 24 ? 4u : (per_row > 8 ? 3u : 2u));

@@ -51,8 +51,10 @@ __device__ __forceinline__ uint32_t row_class(unsigned long long w, uint32_t u, 
 // The block class's distinct bound for COUNT rows: larger rows are ranked over
 // a bitmap (aggregate.cuh), which costs by the z domain where a map costs by
 // its slots; below 128 z a distinct z the ranks are cheaper than the larger
-// maps (1M-tuple COUNT, m = 196K: rows of 2K to 8K distinct z 2.6 ms in maps
-// of 2^13 and 2^14).
+// maps.  4000 rows, ranked and in maps: of 2500 distinct z, m = 173K 0.226 and
+// 0.231 ms, m = 346K 0.325 and 0.222; of 5000, m = 173K 0.32 and 0.45, m = 346K
+// 0.41 and 0.45, m = 691K 0.66 and 0.43.  (The 1M-tuple COUNT, m = 196K: 3.41
+// ms, 3.57 with the bound at cap_b / 2, 4.49 with none.)
 __host__ __device__ __forceinline__ uint32_t agg_cap_b(uint64_t m, uint32_t cap_b) {
     return m <= 128ull * (cap_b / 4) ? cap_b / 4 : (m <= 128ull * (cap_b / 2) ? cap_b / 2 : cap_b);
 }
@@ -761,7 +763,10 @@ static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, u
     if (threadIdx.x < kRowBuckets && s_n[threadIdx.x])
         atomicAdd(&nbucket[threadIdx.x], (unsigned long long)s_n[threadIdx.x]);
 }
-// Lanes a row (log2) for rows of `per_row` entries on average.
+// Lanes a row (log2) for rows of `per_row` entries on average.  Both CSRs and
+// the row work of 4M x 500K tuples, us with 4, 8, 16 and 32 lanes: 2 a row 296
+// 309 397 606, 5 a row 246 242 272 363, 12 a row 214 211 215 258, 40 a row 192
+// 189 187 194, 64 a row 197 190 188 188.
 inline uint32_t row_work_lanes(double per_row) { return per_row > 64 ? 5 : (per_row > 24 ? 4 : (per_row > 8 ? 3 : 2)); }
 
 // Every row into its bucket's list: list_w, list_b (buckets 1, 2, 3 in
