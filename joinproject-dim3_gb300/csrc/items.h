@@ -21,8 +21,7 @@ struct Pieces {
     DIM3G_HD bool at(uint32_t k, uint32_t* p0, uint32_t* p1) const {
         if (k >= n) return false;
         *p0 = k * piece;
-        const uint32_t left = total - *p0;
-        *p1 = *p0 + (piece < left ? piece : left);
+        *p1 = k + 1 < n ? *p0 + piece : total;
         return true;
     }
 };
