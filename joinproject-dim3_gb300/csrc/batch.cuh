@@ -473,9 +473,9 @@ static __global__ void __launch_bounds__(1024) k_q_setup(QueryPools Q) {
 // A row with its candidates counted: its distinct bound and bucket (kRowBuckets:
 // none).
 __device__ __forceinline__ uint32_t query_row(const QueryPools& Q, const RowBuckets& rb, uint32_t qi, uint64_t g,
-                                              unsigned long long w, uint32_t m, uint32_t fam) {
+                                              uint32_t ne, unsigned long long w, uint32_t m, uint32_t fam) {
     const uint32_t u = (uint32_t)(w < m ? w : m);
-    const uint32_t k = rb.of(row_class(w, u, rb.cap_w, fam ? agg_cap_b(m, rb.cap_b) : rb.cap_b, rb.tiny), u);
+    const uint32_t k = rb.of(row_class(w, u, ne, rb.cap_w, fam ? agg_cap_b(m, rb.cap_b) : rb.cap_b, rb.tiny), u);
     Q.ucap[g] = u;
     if (fam && w >= 0xFFFFFFFFull) raise_error(&Q.res[qi].err, kErrCountRange);
     if (k < kRowBuckets) Q.bucket[g] = (uint8_t)(fam * kCountBuckets + k);
@@ -583,7 +583,7 @@ static __global__ void __launch_bounds__(256) k_q_work(QueryPools Q, RowBuckets 
         for (uint32_t o = G >> 1; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
         if (gl == 0 && live) {
             if (slot == kEmpty32) {
-                const uint32_t k = query_row(Q, rb, qi, g, w, m, fam);
+                const uint32_t k = query_row(Q, rb, qi, g, e1 - e0, w, m, fam);
                 acc += w;
                 if (k < kRowBuckets) atomicAdd(&s_n[fam][k], 1u);
             } else {
@@ -628,7 +628,7 @@ static __global__ void __launch_bounds__(256) k_q_long(QueryPools Q, RowBuckets 
             if (atomicSub(&l.left, 1u) == 1u) {
                 __threadfence();
                 const unsigned long long w = atomicAdd(&l.w, 0ull);
-                const uint32_t fam = qn.op == kOpCount, k = query_row(Q, rb, qi, l.g, w, Q.res[qi].nz, fam);
+                const uint32_t fam = qn.op == kOpCount, k = query_row(Q, rb, qi, l.g, kQLongRow, w, Q.res[qi].nz, fam);
                 if (w) atomicAdd(&Q.res[qi].out_j, w);
                 if (k < kRowBuckets) atomicAdd(&Q.nbucket[fam][k], 1ull);
             }

@@ -21,6 +21,10 @@ namespace dim3g {
 constexpr uint32_t kEmpty32 = 0xFFFFFFFFu;
 constexpr uint32_t kHugeRow = 1u << 16;
 constexpr uint32_t kWarpWorkMax = 1u << 14;  // candidates a single warp takes alone
+// Entries a single warp takes alone.  A hub's row may have next to no
+// candidates and hundreds of thousands of entries to look up: 320K entries took
+// a warp 3.9 ms, and a pack, which does more an entry, 5.3.
+constexpr uint32_t kWarpEntries = 1024;
 // Tiny rows (few distinct z, few candidates) are expanded many to a warp
 // (packed.cuh).
 constexpr uint32_t kTinyU = 256, kTinyW = 4096;
@@ -40,11 +44,11 @@ __device__ __forceinline__ bool use_row_bitmap(uint32_t m, uint32_t u, uint32_t 
 // for few distinct z and few candidates, 2 (one CTA, hash set or bitmap) up
 // to cap_b distinct, 3 / 4 (one CTA, z-tile bitmaps; 4 = huge, scheduled
 // first) beyond; 0 for an empty row.
-__device__ __forceinline__ uint32_t row_class(unsigned long long w, uint32_t u, uint32_t cap_w, uint32_t cap_b,
-                                              bool tiny) {
+__device__ __forceinline__ uint32_t row_class(unsigned long long w, uint32_t u, uint32_t ne, uint32_t cap_w,
+                                              uint32_t cap_b, bool tiny) {
     if (u == 0) return 0;
-    if (tiny && u <= kTinyU && w <= kTinyW) return 5;
-    if (u <= cap_w && w <= kWarpWorkMax) return 1;
+    if (tiny && u <= kTinyU && w <= kTinyW && ne <= kWarpEntries) return 5;
+    if (u <= cap_w && w <= kWarpWorkMax && ne <= kWarpEntries) return 1;
     if (u <= cap_b) return 2;
     return u <= kHugeRow ? 3 : 4;
 }
@@ -688,9 +692,9 @@ static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, u
         const uint64_t r = (uint64_t)__ldg(&c.IC_R[e]) * c.T;
         return __ldg(&c.JR_S[r + c.T]) - __ldg(&c.JR_S[r]);
     };
-    auto finish = [&](uint64_t x, unsigned long long w) {
+    auto finish = [&](uint64_t x, uint32_t ne, unsigned long long w) {
         const uint32_t u = (uint32_t)(w < c.m ? w : c.m);
-        const uint32_t k = row_class(w, u, rb.cap_w, rb.cap_b, rb.tiny), q = rb.of(k, u);
+        const uint32_t k = row_class(w, u, ne, rb.cap_w, rb.cap_b, rb.tiny), q = rb.of(k, u);
         ucap[x] = u;
         bucket[x] = (uint8_t)q;
         atomicAdd(&s_n[q], 1u);
@@ -711,7 +715,8 @@ static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, u
             e0 = c.JR_R[x];
             e1 = c.JR_R[x + 1];
         }
-        bool later = e1 - e0 > kLongRow;
+        const uint32_t ne = e1 - e0;
+        bool later = ne > kLongRow;
         if (__any_sync(0xffffffffu, later)) {
             uint32_t slot = 0;
             if (later && gl == 0) slot = atomicAdd(&s_nlong, 1u);
@@ -742,7 +747,7 @@ static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, u
             if ((int)lane == src) w += v;
         }
         for (uint32_t o = G >> 1; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-        if (gl == 0 && x < n && !later) finish(x, w);
+        if (gl == 0 && x < n && !later) finish(x, ne, w);
     }
     __syncthreads();
     const uint32_t nlong = min(s_nlong, kLongRows);
@@ -756,7 +761,7 @@ static __global__ void __launch_bounds__(256) k_row_work(RowCtx c, uint32_t n, u
             if (lane == 0) atomicAdd(&s_w[i], v);
         }
         __syncthreads();
-        if (threadIdx.x < nlong) finish(s_long[threadIdx.x].x, s_w[threadIdx.x]);
+        if (threadIdx.x < nlong) finish(s_long[threadIdx.x].x, s_long[threadIdx.x].z - s_long[threadIdx.x].y, s_w[threadIdx.x]);
         __syncthreads();
     }
     if (threadIdx.x < 6 && s_acc[threadIdx.x]) atomicAdd(threadIdx.x ? &outj_cls[threadIdx.x] : outj, s_acc[threadIdx.x]);

@@ -143,3 +143,35 @@ def test_query_pass_of_a_hub_takes_little_more_than_its_expansion(ctx):
         best = min(best, 1e3 * (time.perf_counter() - t))
     assert best < 2 * rows, (best, rows)
     rs.close()
+
+
+def test_hub_rows_without_partners_are_not_left_to_a_warp(ctx):
+    """Rows of many entries and next to no candidates: a warp looked all of them
+    up alone."""
+    import torch
+
+    import dim3gpu
+    rng = np.random.default_rng(8)
+    n_y, hub = 1_000_000, 400_000
+    # the same tuples, as two rows of 400K and in rows of about ten
+    y = np.concatenate([rng.choice(n_y, hub, replace=False) for _ in range(2)])
+    S = np.stack([rng.integers(0, 50, 3000), rng.integers(0, n_y, 3000)], 1).astype(np.uint32)
+    ms = []
+    for x in (np.repeat([7, 8], hub), rng.integers(0, 80_000, 2 * hub)):
+        R = np.stack([x, y], 1).astype(np.uint32)
+        dR, dS = (torch.from_numpy(a.view(np.int32)).cuda() for a in (R, S))
+        n = O.join_project(R, S)[1]
+        out = torch.empty((n, 2), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        best = 1e9
+        for _ in range(5):
+            assert ctx.join_project_device(dR, R.shape[0], dS, S.shape[0], out, n) == n
+            best = min(best, ctx.stats()["ms_write"])
+        ms.append(best)
+        rs = dim3gpu.RelSet(ctx, [(dR, R.shape[0]), (dS, S.shape[0])])
+        spec = {"r": 0, "s": 1, "op": dim3gpu.OP_COUNT, "capacity": n, "out": out,
+                "cnt": torch.empty(n, dtype=torch.int64, device="cuda")}
+        torch.cuda.synchronize()
+        check_query(spec, rs.join([spec])[0], R, S)
+        rs.close()
+    assert ms[0] < ms[1] + 1.5, ms
