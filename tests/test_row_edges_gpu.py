@@ -246,3 +246,32 @@ def test_query_pass_row_widths(built):
                 assert np.array_equal(got[a], np.asarray(w[1], np.uint64)[b])
     rs.close()
     c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ordered", [0, 1])
+def test_few_block_rows_get_the_full_cta_width(built, ordered):
+    """120 rows of a million candidates over 1000 z: split by set size, they take
+    no longer than in one launch of full-width CTAs (time against time)."""
+    import torch
+
+    import dim3gpu
+    rng = np.random.default_rng(9)
+    R = np.stack([np.repeat(np.arange(120), 1000), np.tile(np.arange(1000), 120)], 1).astype(np.uint32)
+    S = np.stack([rng.integers(0, 1000, 1_000_000), rng.integers(0, 1000, 1_000_000)], 1).astype(np.uint32)
+    dR, dS = (torch.from_numpy(a.view(np.int32)).cuda() for a in (R, S))
+    out = torch.empty((120 * 1000, 2), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ms = []
+    for split in (0, 1):
+        c = dim3gpu.Context(0)
+        for k, v in dict(keep_roles=1, ordered_output=ordered, block_split=split).items():
+            c.set_param(k, v)
+        best = 1e9
+        for _ in range(6):
+            assert c.join_project_device(dR, R.shape[0], dS, S.shape[0], out, out.shape[0]) == out.shape[0]
+            best = min(best, c.stats()["ms_write"])
+        assert c.stats()["rows_block"] == 120
+        ms.append(best)
+        c.close()
+    assert ms[1] < 1.2 * ms[0] + 0.02, ms
