@@ -895,11 +895,11 @@ retile:
     rc.id2z = id2z;
     rc.out = nullptr;
     rc.err = &sc->err;
-    // tiny rows go many to a warp but in summaries and COUNT at exact
-    // offsets; the block class is split by hash-set size (2^lg slots for 2u
+    // tiny rows go many to a warp, but in COUNT's summaries and at its exact
+    // offsets one, and in project summaries they are warp rows; the block class is split by hash-set size (2^lg slots for 2u
     // keys)
     const bool block_split = c->prm.block_split && !(single && !jp.aggregate && c->prm.prefetch_rows && c->prm.cta_rr == 3);
-    const bool tiny = single || (!jp.aggregate && !jp.sum.tiles);
+    const bool tiny = jp.aggregate || !jp.sum.tiles;
     const uint32_t cap_w = 1u << (c->prm.warp_lg - 1), cap_b = 1u << (c->prm.block_lg - 1);
     const RowBuckets rb{cap_w, jp.aggregate ? agg_cap_b(m, cap_b) : cap_b, tiny, block_split,
                         1u << (c->prm.block_lg - 3), 1u << (c->prm.block_lg - 2)};
@@ -969,7 +969,7 @@ retile:
         // needs no count pass (nothing is placed)
         CU(cudaEventRecord(c->evc[4], st));
         if (jp.aggregate) {
-            int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, nullptr, rst, direct, huge_rows);
+            int r = run_aggregate(c, rc, AggOut{nullptr, jp.sum, Reserve{nullptr, 0}}, L, sc, list_t, rst, direct, huge_rows);
             if (r) return r;
         } else {
             k_sum_bitmap<<<resident_grid(c, k_sum_bitmap, blk_m, smem_m), blk_m, smem_m, st>>>(rc, jp.sum, L.m,
@@ -989,7 +989,7 @@ retile:
         if (c->h_sc->err) return fail(c, DIM3G_ERR_DEVICE, "device bound violated in summary (flags %u)", c->h_sc->err);
         dense_times(c, dp);
         S.out_j = c->h_sc->outj;
-        S.rows_warp = (uint32_t)c->h_sc->nrows[1];
+        S.rows_warp = (uint32_t)(c->h_sc->nrows[1] + c->h_sc->nrows[5]);
         S.rows_block = (uint32_t)c->h_sc->nrows[2];
         S.rows_bitmap = (uint32_t)(c->h_sc->nrows[3] + c->h_sc->nrows[4]);
         float a, b, e;
@@ -1215,7 +1215,7 @@ retile:
     CU(cudaMemsetAsync(sc->next_row, 0, sizeof(sc->next_row), st));
     if (total > 0) {
         if (jp.aggregate) {
-            int r = run_aggregate(c, rc, AggOut{out_cnt, SumAcc{}, Reserve{nullptr, 0}}, L, sc, nullptr, rst, direct, huge_rows);
+            int r = run_aggregate(c, rc, AggOut{out_cnt, SumAcc{}, Reserve{nullptr, 0}}, L, sc, list_t, rst, direct, huge_rows);
             if (r) return r;
         } else {
             CU(cudaEventRecord(c->evc[4], st));
@@ -1248,7 +1248,7 @@ retile:
 }
 
 // COUNT's row kernels (aggregate.cuh): the ranked rows first, then the map
-// rows from the largest maps down, then the tiny rows (list_t; null: none).
+// rows from the largest maps down, then the tiny rows (list_t).
 // CTAs by map size, so that small maps run many rows an SM.
 int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, Scalars* sc,
                   const uint32_t* list_t, RowStreams& rst, bool direct, bool huge_rows) {
@@ -1295,11 +1295,14 @@ int run_aggregate(dim3g_ctx* c, const RowCtx& rc, AggOut ao, const RowLists& L, 
     }
     if (!r) r = map_rows(L.w, L.nw, c->prm.warp_lg, nullptr, nullptr, 2);
     if (r) return r;
-    if (list_t) {
+    if (ao.rs.cursor) {
         const size_t smem = 8 * kAggPackWords * 4;
         k_agg_pack<<<resident_grid(c, k_agg_pack, 256, smem), 256, smem, rst.w>>>(rc, ao, list_t, &sc->nrows[5]);
-        CHECK_LAUNCH();
+    } else {
+        const size_t smem = (size_t)8 * 4 << (kAggPackLg + 1);
+        k_agg_warp<<<resident_grid(c, k_agg_warp, 256, smem), 256, smem, rst.w>>>(rc, ao, list_t, &sc->nrows[5]);
     }
+    CHECK_LAUNCH();
     CU(rst.join());
     return DIM3G_OK;
 }
