@@ -542,22 +542,32 @@ __device__ __forceinline__ void agg_pack_rows(const RowCtx& c, uint32_t x, uint3
         const bool in = lane >= first && lane < end;
         uint32_t lg = ceil_log2(2 * sum);
         lg = lg < 5 ? 5 : lg;
-        uint32_t* vals = keys + (1u << lg);
-        for (uint32_t s = lane; s < (1u << lg); s += 32) {
-            keys[s] = kEmpty32;
-            vals[s] = 0;
+        // a counter a row and z where those are no more than the map's words
+        const uint64_t cells = (uint64_t)(end - first) * c.m;
+        const bool direct = cells <= (2u << lg);
+        const uint32_t span = direct ? (uint32_t)cells : 1u << lg;
+        uint32_t* vals = direct ? keys : keys + (1u << lg);
+        for (uint32_t s = lane; s < span; s += 32) {
+            keys[s] = direct ? 0u : kEmpty32;
+            if (!direct) vals[s] = 0;
         }
         __syncwarp();
-        CountMap set{keys, vals, lg, c.err};
         NullSink sink;
-        pack_expand<false>(c, e0, in ? ne : 0u, in ? (lane - first) * c.m : 0u, xv, set, sink);
+        const uint32_t n = in ? ne : 0u, key0 = in ? (lane - first) * c.m : 0u;
+        if (direct) {
+            CountTile set{keys, 0};
+            pack_expand<false>(c, e0, n, key0, xv, set, sink);
+        } else {
+            CountMap set{keys, vals, lg, c.err};
+            pack_expand<false>(c, e0, n, key0, xv, set, sink);
+        }
         __syncwarp();
-        for (uint32_t sb = 0; sb < (1u << lg); sb += 32) {
-            const uint32_t key = keys[sb + lane];
-            const bool have = key != kEmpty32;
-            const uint32_t r = have ? key / c.m : 0u;
+        for (uint32_t sb = 0; sb < span; sb += 32) {
+            const uint32_t s = sb + lane, v = s < span ? vals[s] : 0u;
+            const bool have = v != 0;
+            const uint32_t key = have ? (direct ? s : keys[s]) : 0u, r = have ? key / c.m : 0u;
             const uint32_t gx = __shfl_sync(0xffffffffu, xv, first + r);
-            gs.add(have, gx, have ? __ldg(&c.id2z[key - r * c.m]) : 0u, have ? vals[sb + lane] : 0u);
+            gs.add(have, gx, have ? __ldg(&c.id2z[key - r * c.m]) : 0u, v);
         }
         __syncwarp();
         first = end;

@@ -66,6 +66,29 @@ __device__ __forceinline__ void pack_expand(const RowCtx& c, uint32_t e0, uint32
         }
         const uint32_t inc = warp_incl_scan(len), exc = inc - len;
         const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+        // long segments: the lanes stride each, without a search a candidate
+        uint32_t segs = __ballot_sync(0xffffffffu, len != 0);
+        if (total >= kFlatAvgMax * __popc(segs)) {
+            for (; segs; segs &= segs - 1) {
+                const int k = __ffs(segs) - 1;
+                const uint32_t ks0 = __shfl_sync(0xffffffffu, s0, k), klen = __shfl_sync(0xffffffffu, len, k);
+                const uint32_t kk = __shfl_sync(0xffffffffu, ek, k), kx = __shfl_sync(0xffffffffu, ex, k);
+                for (uint32_t jb = 0; jb < klen; jb += 32 * kUnroll) {
+                    uint32_t z[kUnroll], v[kUnroll], x[kUnroll], b[kUnroll];
+#pragma unroll
+                    for (uint32_t u = 0; u < kUnroll; u++) {
+                        const uint32_t j = jb + u * 32 + lane;
+                        x[u] = kx;
+                        load_cand<kPair, Sink::kValues>(c, ks0 + j, j < klen, pol, z[u], v[u]);
+                    }
+#pragma unroll
+                    for (uint32_t u = 0; u < kUnroll; u++)
+                        b[u] = jb + u * 32 < klen ? __ballot_sync(0xffffffffu, set.insert(kk + z[u], z[u] != kEmpty32)) : 0u;
+                    sink.take(b, x, v);
+                }
+            }
+            continue;
+        }
         for (uint32_t cb = 0; cb < total; cb += 32 * kUnroll) {
             uint32_t z[kUnroll], v[kUnroll], key[kUnroll], x[kUnroll], b[kUnroll];
 #pragma unroll
